@@ -1,8 +1,10 @@
 // spectrum.cu -- the spectrum stage of eSPec on the GPU, FP64, batched over
 // packets: total correlation assembly (espec.f:1545-1576), lifetime
 // broadening HWHM (hwhm.f:59-77), window and half swap of SPECTRUMTD
-// (spectrumtd.f:58-81) fused into one pass, then the inverse DFT of FFTNT
-// (cfft.f:6-106) as radix-2 Stockham passes (natural order in and out).
+// (spectrumtd.f:58-81), applied as the inverse DFT of FFTNT (cfft.f:6-106)
+// reads its input; the DFT as radix-2 Stockham passes (natural order in and
+// out) taken four at a time in registers, whole transforms in shared memory up
+// to 2^13 points.
 // Also the Fortran drop-ins hwhm_ and spectrumtd_ (with the printed table).
 #include <cuda_runtime.h>
 
@@ -33,83 +35,224 @@ struct PrepArgs {
   double dem, ta;         // -DE*1.5192676, TAL*1.5192676
   int window;             // 1: .SG
   double taux;            // TMAX^2 / ln(1/WP)^2
-  double2* out;           // [npk][2^mf], halves swapped
+  const double2* factor;  // HWHM and window factor of each time, or null (neither)
+  double2* out;           // [npk][2^mf]
 };
 
-// one element j of packet p: assembled (or read) C value, HWHM, window;
-// written to the half-swapped position (spectrumtd.f:73-80)
-__global__ void spec_prep_kernel(PrepArgs a) {
-  const long N = 1L << a.mf;
-  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= N * a.npk) return;
-  const long p = gid / N, j = gid % N;
-  double u, v;
-  if (a.assemble) {
-    // espec.f:1549-1563: C(-t) = C(t)* mirrored onto 2 MC points, MC = N/2
-    const long mc = N / 2;
+// HWHM (hwhm.f:63-73) and window (spectrumtd.f:62-68) of time j as one complex
+// factor: every packet has the same times, so the sine, cosine and exponentials
+// are taken once per call and not once per packet (a third of the prep time)
+__device__ __forceinline__ double2 time_factor(const PrepArgs& a, long j) {
+  const double t = -a.tf + (double)j * a.dtf;
+  double sn = 0.0, cs = 1.0, f = 1.0;
+  if (a.hwhm) {
+    sincos(a.dem * t, &sn, &cs);
+    f = exp(-fabs(t) * a.ta);
+  }
+  if (a.window) f *= exp(-(t * t) / a.taux);
+  return make_double2(cs * f, sn * f);
+}
+
+// element i of the transform's input for packet p: the half swap of
+// spectrumtd.f:73-80 puts time j = i + N/2 (mod N) there; assembled
+// (espec.f:1549-1563: C(-t) = C(t)* mirrored onto 2 MC points, MC = N/2) or
+// read, times the factor of its time
+__device__ __forceinline__ double2 prep_value(const PrepArgs& a, long p, long i) {
+  const long N = 1L << a.mf, mc = N / 2;
+  const long j = i < mc ? i + mc : i - mc;  // N = 1: 0
+  double2 z;
+  if (a.assemble && N > 1) {
     const double2* c = a.in + p * a.ldc;
-    if (j == 0) {
-      u = c[mc - 1].x;
-      v = -c[mc - 1].y;
-    } else if (j <= mc) {
-      u = c[mc - j].x;
-      v = -c[mc - j].y;
+    if (j > mc) {
+      z = __ldg(c + (j - mc));
     } else {
-      u = c[j - mc].x;
-      v = c[j - mc].y;
+      z = __ldg(c + (j == 0 ? mc - 1 : mc - j));
+      z.y = -z.y;
     }
   } else {
-    const double2 z = a.in[p * a.ldc + j];
-    u = z.x;
-    v = z.y;
+    z = __ldg(a.in + p * a.ldc + j);
   }
-  const double t = -a.tf + (double)j * a.dtf;
-  if (a.hwhm) {  // hwhm.f:63-73
-    double sn, cs;
-    sincos(a.dem * t, &sn, &cs);
-    const double cstl = exp(-fabs(t) * a.ta);
-    const double ui = u;
-    u = cs * u - sn * v;
-    v = cs * v + sn * ui;
-    u = cstl * u;
-    v = cstl * v;
+  if (a.factor) {
+    const double2 f = __ldg(a.factor + j);
+    z = make_double2(f.x * z.x - f.y * z.y, f.x * z.y + f.y * z.x);
   }
-  if (a.window) {  // spectrumtd.f:62-68
-    const double cstl = exp(-(t * t) / a.taux);
-    u = cstl * u;
-    v = cstl * v;
-  }
-  const long js = (j + N / 2) % N;
-  a.out[p * N + js] = make_double2(u, v);
+  return z;
 }
 
-// twiddles w_k = exp(+i twopi k / N), k < N/2 (the backward sign of FFTNT)
-__global__ void spec_twiddle_kernel(double2* tw, long nh, double twopi_over_n) {
+// twiddles w_k = exp(+i twopi k / N), k < N/2 (the backward sign of FFTNT),
+// and, when asked for, the factor of every time
+__global__ void spec_table_kernel(PrepArgs a, double2* tw, double2* factor, double twopi_over_n) {
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nh) return;
-  double s, c;
-  sincos(twopi_over_n * (double)k, &s, &c);
-  tw[k] = make_double2(c, s);
+  const long N = 1L << a.mf;
+  if (k < N / 2) {
+    double s, c;
+    sincos(twopi_over_n * (double)k, &s, &c);
+    tw[k] = make_double2(c, s);
+  }
+  if (factor && k < N) factor[k] = time_factor(a, k);
 }
 
-// one radix-2 Stockham pass (natural order after the last pass) of all
-// packets; the last pass divides by N (cfft.f:102-105)
-__global__ void spec_pass_kernel(const double2* x, double2* y, const double2* tw, int npk, int mf,
-                                 int s, double scale) {
-  const long N = 1L << mf, NH = N / 2;
+// HWHM and window alone, natural order (hwhm_)
+__global__ void spec_hwhm_kernel(PrepArgs a) {
+  const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= (1L << a.mf)) return;
+  const double2 z = a.in[j], f = time_factor(a, j);
+  a.out[j] = make_double2(f.x * z.x - f.y * z.y, f.x * z.y + f.y * z.x);
+}
+
+// LOGR consecutive radix-2 Stockham passes s, s+1, ... on the 2^LOGR points
+// that meet in them, in registers.  Pass s takes elements j and j + N/2 to
+// ((j >> s) << (s + 1)) | k and that + 2^s (k = j mod 2^s), so the points
+// j0 + q N / 2^LOGR (j0 < N / 2^LOGR) stay together through LOGR passes: a
+// block of the array per output bit found so far, halved by every pass, the
+// block's bits reversed extending k.  On return element r belongs at
+// (j0 - k) 2^LOGR + k + 2^s brev(r).  The twiddles are the table's for each
+// pass, so that FFTNT's single-precision 2 pi enters as it does in the
+// reference's radix-2 form.
+__host__ __device__ constexpr int brev_c(int v, int bits) {
+  int r = 0;
+  for (int i = 0; i < bits; ++i) r |= ((v >> i) & 1) << (bits - 1 - i);
+  return r;
+}
+template <int LOGR>
+__device__ __forceinline__ void passes(double2* v, const double2* __restrict__ tw, long k, int s,
+                                       int mf) {
+  constexpr int R = 1 << LOGR;
+#pragma unroll
+  for (int p = 0; p < LOGR; ++p) {
+    const int half = R >> (p + 1);
+#pragma unroll
+    for (int blk = 0; blk < (1 << p); ++blk) {
+      const double2 w = __ldg(tw + ((k + ((long)brev_c(blk, p) << s)) << (mf - 1 - s - p)));
+#pragma unroll
+      for (int q = 0; q < half; ++q) {
+        double2& x = v[blk * 2 * half + q];
+        double2& y = v[blk * 2 * half + q + half];
+        const double2 b = make_double2(y.x * w.x - y.y * w.y, y.x * w.y + y.y * w.x);
+        y = make_double2(x.x - b.x, x.y - b.y);
+        x = make_double2(x.x + b.x, x.y + b.y);
+      }
+    }
+  }
+}
+
+// Transforms of 2^mf points, 4 <= mf <= kOneMax, whole in shared memory: 16
+// points per thread, the passes taken four at a time in registers (REM of them,
+// the remainder, first), one exchange through shared memory between the groups; the
+// input is prepared as it is read and the last group writes the result.
+// Small transforms share a CTA.  The exchange adds one element in 16, which
+// keeps the stride-16 writes of the first groups on distinct banks.
+// HBM then carries the samples once and the spectrum once; with one kernel per
+// radix-2 pass every pass moved the whole batch (1024 x 4096 points: 12 passes
+// of 134 MB and a prep pass, 295 us).
+constexpr int kOneMax = 13;
+constexpr int kOneThreads = 256;
+__device__ __forceinline__ int padded(int i) { return i + (i >> 4); }
+
+template <int REM, int T>
+__global__ void __launch_bounds__(T, 512 / T) spec_one_kernel(PrepArgs a, const double2* __restrict__ tw,
+                                                     double scale) {
+  extern __shared__ double2 spec_sm[];
+  const int mf = a.mf, n = 1 << mf, tp = n >> 4;  // threads of a packet
+  const int g = threadIdx.x / tp, t = threadIdx.x % tp;
+  const long p = (long)blockIdx.x * (T / tp) + g;
+  const bool on = p < a.npk;
+  double2* sm = spec_sm + (size_t)g * (n + (n >> 4));
+  double2 v[16];
+  constexpr int R = 1 << REM, B = 16 / R;  // B groups of 2^REM points, k = 0
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    const int j0 = t + i * tp;
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+      v[i * R + q] = on ? prep_value(a, p, j0 + q * (n / R)) : make_double2(0.0, 0.0);
+  }
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    passes<REM>(v + i * R, tw, 0, 0, mf);
+    const int j0 = t + i * tp;
+    if (mf > REM) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) sm[padded(j0 * R + brev_c(r, REM))] = v[i * R + r];
+    } else if (on) {  // 16 points: one group is the whole transform
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        a.out[p * n + brev_c(r, REM)] = make_double2(v[r].x * scale, v[r].y * scale);
+    }
+  }
+  __syncthreads();
+  for (int s = REM; s < mf; s += 4) {
+    const int k = t & ((1 << s) - 1);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = sm[padded(t + q * tp)];
+    passes<4>(v, tw, k, s, mf);
+    const int o = (t - k) * 16 + k;
+    if (s + 4 < mf) {
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 16; ++r) sm[padded(o + (brev_c(r, 4) << s))] = v[r];
+      __syncthreads();
+    } else if (on) {
+      double2* out = a.out + p * n;
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+        out[o + (brev_c(r, 4) << s)] = make_double2(v[r].x * scale, v[r].y * scale);
+    }
+  }
+}
+
+// LOGR radix-2 passes of every packet from one buffer to the other (x null:
+// from the prepared input), for transforms of 1-3 passes and those above
+// kOneMax; one thread per group of 2^LOGR points
+template <int LOGR>
+__global__ void __launch_bounds__(256) spec_pass_kernel(PrepArgs a, const double2* x, double2* y,
+                                                        const double2* __restrict__ tw, int s,
+                                                        double scale) {
+  constexpr int R = 1 << LOGR;
+  const int mf = a.mf;
+  const long N = 1L << mf, M = N >> LOGR;
   const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= NH * npk) return;
-  const long p = gid / NH, j = gid % NH;
-  const long Ns = 1L << s;
-  const long k = j & (Ns - 1);
-  const double2* xp = x + p * N;
-  double2* yp = y + p * N;
-  const double2 a = xp[j], b0 = xp[j + NH];
-  const double2 w = tw[k << (mf - 1 - s)];
-  const double2 b = make_double2(b0.x * w.x - b0.y * w.y, b0.x * w.y + b0.y * w.x);
-  const long d = ((j >> s) << (s + 1)) | k;
-  yp[d] = make_double2((a.x + b.x) * scale, (a.y + b.y) * scale);
-  yp[d + Ns] = make_double2((a.x - b.x) * scale, (a.y - b.y) * scale);
+  if (gid >= M * a.npk) return;
+  const long p = gid >> (mf - LOGR), j0 = gid & (M - 1), k = j0 & ((1L << s) - 1);
+  double2 v[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q)
+    v[q] = x ? x[p * N + j0 + q * M] : prep_value(a, p, j0 + q * M);
+  passes<LOGR>(v, tw, k, s, mf);
+  double2* yp = y + p * N + ((j0 - k) << LOGR) + k;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    yp[(long)brev_c(r, LOGR) << s] = make_double2(v[r].x * scale, v[r].y * scale);
+}
+
+template <int REM, int T>
+cudaError_t launch_one(const PrepArgs& a, const double2* tw, double scale, cudaStream_t st) {
+  static DeviceFlags attr;
+  const size_t smem = sizeof(double2) * 17 * T;
+  cudaError_t e = set_max_smem_once(attr, spec_one_kernel<REM, T>, smem);
+  if (e != cudaSuccess) return e;
+  const int per = T >> (a.mf - 4);  // packets per CTA
+  spec_one_kernel<REM, T><<<(a.npk + per - 1) / per, T, smem, st>>>(a, tw, scale);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pass(int logr, const PrepArgs& a, const double2* x, double2* y,
+                        const double2* tw, int s, double scale, cudaStream_t st) {
+  const long th = ((1L << a.mf) >> logr) * a.npk;
+  const unsigned nb = (unsigned)((th + 255) / 256);
+  switch (logr) {
+    case 1: spec_pass_kernel<1><<<nb, 256, 0, st>>>(a, x, y, tw, s, scale); break;
+    case 2: spec_pass_kernel<2><<<nb, 256, 0, st>>>(a, x, y, tw, s, scale); break;
+    case 3: spec_pass_kernel<3><<<nb, 256, 0, st>>>(a, x, y, tw, s, scale); break;
+    default: spec_pass_kernel<4><<<nb, 256, 0, st>>>(a, x, y, tw, s, scale); break;
+  }
+  return cudaGetLastError();
+}
+
+// mf = 0: the prepared sample is the spectrum (FFTNT returns at N = 1)
+__global__ void spec_copy_kernel(PrepArgs a) {
+  const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < a.npk) a.out[p] = prep_value(a, p, 0);
 }
 
 }  // namespace
@@ -151,26 +294,62 @@ extern "C" int espec_spectrum_dev(int npk, int mf, const void* in, long ld, int 
     const double l = std::log(1.0 / wp);
     a.taux = tmax * tmax / (l * l);
   }
-  double2* bufs[2] = {(double2*)spec, (double2*)work};
-  // the passes ping-pong; start in the buffer that makes the last pass land in spec
-  int cur = (mf % 2 == 0) ? 0 : 1;
-  a.out = bufs[cur];
-  const long tot = N * npk;
-  spec_prep_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(a);
-  SPEC_CK(cudaGetLastError());
-  if (mf == 0) return ESPEC_OK;  // FFTNT returns at N = 1 (cfft.f:39)
+  a.out = (double2*)spec;
+  const bool scaled = a.hwhm || a.window;
+  if (mf == 0) {  // FFTNT returns at N = 1 (cfft.f:39)
+    // work may be null here: the one time's factor goes through spec
+    if (scaled) {
+      PrepArgs b = a;
+      b.factor = nullptr;
+      for (int p = 0; p < npk; ++p) {
+        b.in = a.in + p * ld;
+        b.out = a.out + p;
+        spec_hwhm_kernel<<<1, 1, 0, st>>>(b);
+      }
+    } else {
+      spec_copy_kernel<<<(npk + 255) / 256, 256, 0, st>>>(a);
+    }
+    SPEC_CK(cudaGetLastError());
+    return ESPEC_OK;
+  }
   // cfft.f:35 declares TWOPI with a default-real literal: single precision
   const double twopi = (quirks & ESPEC_Q_FFTNT_SP) ? (double)(float)kTwoPi : kTwoPi;
-  double2* tw = (double2*)work + tot;
-  spec_twiddle_kernel<<<(unsigned)((N / 2 + 255) / 256), 256, 0, st>>>(tw, N / 2, twopi / N);
+  const long tot = N * npk;
+  double2* wk = (double2*)work;
+  double2* tw = wk + tot;
+  // groups of up to four passes, the short one first; the groups ping-pong
+  // between work and spec and end in spec.  The time factors sit in the
+  // buffer that the first group does not write.
+  const int ngroups = (mf + 3) / 4;
+  const bool one = mf >= 4 && mf <= kOneMax;
+  double2* dst = one || ngroups % 2 == 1 ? a.out : wk;
+  double2* factor = scaled ? (dst == a.out ? wk : a.out) : nullptr;
+  a.factor = factor;
+  spec_table_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(a, tw, factor, twopi / N);
   SPEC_CK(cudaGetLastError());
-  const long nb = N / 2 * npk;
-  for (int s = 0; s < mf; ++s) {
-    const double scale = s == mf - 1 ? 1.0 / N : 1.0;
-    spec_pass_kernel<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(bufs[cur], bufs[cur ^ 1], tw,
-                                                                   npk, mf, s, scale);
-    SPEC_CK(cudaGetLastError());
-    cur ^= 1;
+  const double rn = 1.0 / N;  // cfft.f:102-105
+  if (one) {
+    cudaError_t e;
+    if (mf == kOneMax) {
+      e = launch_one<1, 2 * kOneThreads>(a, tw, rn, st);
+    } else {
+      switch (mf % 4) {
+        case 0: e = launch_one<4, kOneThreads>(a, tw, rn, st); break;
+        case 1: e = launch_one<1, kOneThreads>(a, tw, rn, st); break;
+        case 2: e = launch_one<2, kOneThreads>(a, tw, rn, st); break;
+        default: e = launch_one<3, kOneThreads>(a, tw, rn, st); break;
+      }
+    }
+    SPEC_CK(e);
+    return ESPEC_OK;
+  }
+  const double2* src = nullptr;
+  for (int s = 0; s < mf;) {
+    const int lr = s == 0 && mf % 4 ? mf % 4 : 4;
+    SPEC_CK(launch_pass(lr, a, src, dst, tw, s, s + lr == mf ? rn : 1.0, st));
+    src = dst;
+    dst = dst == a.out ? wk : a.out;
+    s += lr;
   }
   return ESPEC_OK;
 }
@@ -256,19 +435,11 @@ extern "C" void hwhm_(const int* m, const double* dt, const double* tf, double* 
   a.out = d_out;
   cudaMemcpy2D(d_in, 16, u, 8, 8, N, cudaMemcpyHostToDevice);
   cudaMemcpy2D((char*)d_in + 8, 16, v, 8, 8, N, cudaMemcpyHostToDevice);
-  spec_prep_kernel<<<(unsigned)((N + 255) / 256), 256>>>(a);
-  // prep writes half-swapped: read back with the halves exchanged
-  const size_t h = N / 2;
+  spec_hwhm_kernel<<<(unsigned)((N + 255) / 256), 256>>>(a);
   cudaError_t e = cudaGetLastError();
-  if (N == 1) {
-    cudaMemcpy2D(u, 8, d_out, 16, 8, 1, cudaMemcpyDeviceToHost);
-    cudaMemcpy2D(v, 8, (char*)d_out + 8, 16, 8, 1, cudaMemcpyDeviceToHost);
-  } else {
-    cudaMemcpy2D(u, 8, d_out + h, 16, 8, h, cudaMemcpyDeviceToHost);
-    cudaMemcpy2D(u + h, 8, d_out, 16, 8, h, cudaMemcpyDeviceToHost);
-    cudaMemcpy2D(v, 8, (char*)(d_out + h) + 8, 16, 8, h, cudaMemcpyDeviceToHost);
-    e = cudaMemcpy2D(v + h, 8, (char*)d_out + 8, 16, 8, h, cudaMemcpyDeviceToHost);
-  }
+  cudaMemcpy2D(u, 8, d_out, 16, 8, N, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess)
+    e = cudaMemcpy2D(v, 8, (char*)d_out + 8, 16, 8, N, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) std::fprintf(stderr, "espec_gpu HWHM: %s\n", cudaGetErrorString(e));
   cudaFree(d_in);
   cudaFree(d_out);
