@@ -17,6 +17,8 @@ void digt_nd_table(int ndim, const int* np, const double* sh, const double* sm, 
 // the spectrum block SPECTRUMTD prints (spectrumtd.f:84-97) for FFTNT's
 // output u + i v of 2^mf points
 std::string spectrum_table(int mf, double dt, double de, const double* u, const double* v);
+// polls before a grid-barrier wait gives up (espec_set_wait_limit)
+long grid_wait_limit();
 inline int ck(cudaError_t e, const char* what) {
   return e == cudaSuccess ? 0 : set_cuda_error(what, e);
 }

@@ -1247,6 +1247,10 @@ static void grid_free(espec_grid_plan* p) {
 static std::atomic<long> g_wait_limit{kSpinLimit};
 static std::atomic<int> g_short_arrivals{0};
 
+namespace espec {
+long grid_wait_limit() { return g_wait_limit.load(); }
+}  // namespace espec
+
 // column strips of the PSOD pass on a 2D grid (0: contiguous point ranges):
 // used when the CTA count is a multiple of the strip count and every band
 // holds at least kBandMinRows rows

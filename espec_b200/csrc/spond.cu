@@ -19,9 +19,12 @@
 // Strided passes stage a tile of 8 adjacent x columns in shared memory.  The
 // fftshift swaps of spofft.f:120-133/178-191 cancel and are not done; the
 // 1/N of the reference's B factor is folded into the kinetic table.
+#include <cuda/atomic>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -34,7 +37,9 @@ namespace espec {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kMaxWarps = 8;  // lines per CTA (one warp each); fewer on small grids
+constexpr int kFusedMinPlanes = 64;
+// dynamic shared memory of a CTA: 227 KB less the kernels' static part
+constexpr size_t kNdMaxSmem = 227 * 1024 - 2048;
 
 template <typename R>
 __device__ __forceinline__ cpx<R> cmul(cpx<R> a, cpx<R> b) {
@@ -48,7 +53,7 @@ template <typename R>
 __device__ __forceinline__ cpx<R> shx(cpx<R> v, int m) {
   return mk(__shfl_xor_sync(kFull, v.x, m), __shfl_xor_sync(kFull, v.y, m));
 }
-__host__ __device__ __forceinline__ int brev_bits(int v, int bits) {
+__host__ __device__ __forceinline__ constexpr int brev_bits(int v, int bits) {
   int r = 0;
   for (int i = 0; i < bits; ++i) r |= ((v >> i) & 1) << (bits - 1 - i);
   return r;
@@ -119,109 +124,168 @@ __host__ __device__ inline PhF make_phf(double phi, double a) {
   return o;
 }
 
-template <typename R, int P>
-struct WarpFft {
-  static constexpr int LP = log2i<P>();
+// Line transform of N = 2^LN points (32 <= N <= 512), E points per thread, the
+// line's L = N/E threads exchanging through shared memory.  The arithmetic is
+// the four-step form N = 32 P: radix-2 decimation in frequency over the P-point
+// index (twiddles W_P), the twiddle W_N^(l k1), then radix-2 decimation in
+// frequency over the 32-point index l -- one level per bit of the position
+// 32 j + l, from the top, in place.  A thread takes LE levels at a time: group
+// k holds LE bits of the position (the low end of the group at bit lo(k)) and
+// the thread number the other bits, so both partners of a butterfly are in one
+// thread.  (One warp per line with the lower five levels by __shfl_xor, the
+// form before, evaluated both branches of every butterfly in both lanes and
+// moved each word five times: 80 instructions per point against about 45.)
+// The inverse is the exact mirror with conjugate twiddles (unnormalised).
+template <typename R, int LN>
+struct LineFft {
+  static constexpr int N = 1 << LN, LE = LN == 9 ? 4 : 3, E = 1 << LE, LT = LN - LE, L = 1 << LT;
+  static constexpr int NG = (LN + LE - 1) / LE;  // groups: 5 = 3+2, 6 = 3+3, 7 = 3+3+1, ...
   using T = typename Rot<R>::type;
-  T wl[5];                         // lane stages m = 16 .. 1: W_2m^(lane & (m-1))
-  T wb[P];                         // W_N^(lane k1(r))
-  T wr[P > 1 ? P / 2 : 1];         // W_P^q, q < P/2
-  int lane;
+  static __host__ __device__ constexpr int lo(int k) {
+    return LN - LE * (k + 1) > 0 ? LN - LE * (k + 1) : 0;
+  }
+  static __host__ __device__ constexpr int hi(int k) { return LN - LE * k; }
+  // position of element e of thread t in group k
+  static __device__ __forceinline__ int pos(int k, int t, int e) {
+    const int l = lo(k);
+    return ((t >> l) << (l + LE)) | (e << l) | (t & ((1 << l) - 1));
+  }
+  // twiddle index of the level at bit b at position p: W_2h^(q), q the bits
+  // below b of the P-point or the 32-point index
+  static __device__ __forceinline__ int tw_index(int b, int p) {
+    return b >= 5 ? ((p >> 5) & ((1 << (b - 5)) - 1)) * (N >> (b - 4))
+                  : (p & ((1 << b) - 1)) * (N >> (b + 1));
+  }
+  T wl[NG][E];  // group k, level b, lower element e: at 2^(b - lo) + (e mod 2^(b - lo))
+  T wb[E];      // W_N^(l k1) of the first group's elements
+  int t;
 
   // every twiddle is W_N^k, k < N: read from the line's table (built once
   // per plan in FP64, tw_table_kernel)
-  __device__ void init(const T* tab) {
-    constexpr int N = 32 * P;
-    lane = threadIdx.x & 31;
+  __device__ __forceinline__ void init(const T* tab, int thread) {
+    t = thread;
 #pragma unroll
-    for (int s = 0; s < 5; ++s) {
-      const int m = 16 >> s;
-      wl[s] = tab[(lane & (m - 1)) * (N / (2 * m))];
+    for (int k = 0; k < NG; ++k)
+#pragma unroll
+      for (int b = hi(k) - 1; b >= lo(k); --b)
+#pragma unroll
+        for (int q = 0; q < (1 << (b - lo(k))); ++q)
+          if (!trivial(k, b, q)) wl[k][(1 << (b - lo(k))) + q] = tab[tw_index(b, pos(k, t, q))];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int k1 = brev_bits((e << lo(0)) >> 5, LN - 5);
+      if (k1) wb[e] = tab[(pos(0, t, e) & 31) * k1];
     }
-#pragma unroll
-    for (int r = 0; r < P; ++r) wb[r] = tab[lane * brev_bits(r, LP)];
-#pragma unroll
-    for (int q = 0; q < (P > 1 ? P / 2 : 1); ++q) wr[q] = tab[q * 32];
   }
-  __device__ void forward(cpx<R>* v) const {
+  // W^0 known at compile time (the rotation by it is exact in both forms)
+  static __host__ __device__ constexpr bool trivial(int k, int b, int q) {
+    return b >= 5 ? ((((q << lo(k)) >> 5) & ((1 << (b - 5)) - 1)) == 0) : (lo(k) == 0 && q == 0);
+  }
+  template <bool INV>
+  __device__ __forceinline__ void level(cpx<R>* v, int k, int b) const {
+    const int h = 1 << (b - lo(k));
 #pragma unroll
-    for (int h = P / 2; h >= 1; h /= 2)
-#pragma unroll
-      for (int b = 0; b < P; b += 2 * h)
-#pragma unroll
-        for (int q = 0; q < h; ++q) {
-          const cpx<R> a = v[b + q], c = v[b + q + h];
-          v[b + q] = a + c;
-          v[b + q + h] = rot<false>(wr[q * (P / (2 * h))], a - c);
-        }
-#pragma unroll
-    for (int r = 0; r < P; ++r) v[r] = rot<false>(wb[r], v[r]);
-#pragma unroll
-    for (int s = 0; s < 5; ++s) {
-      const int m = 16 >> s;
-      const bool up = lane & m;
-#pragma unroll
-      for (int r = 0; r < P; ++r) {
-        const cpx<R> mine = v[r], other = shx(mine, m);
-        v[r] = up ? rot<false>(wl[s], other - mine) : mine + other;
+    for (int e = 0; e < E; ++e) {
+      if (e & h) continue;
+      const int q = e & (h - 1);
+      if (!INV) {
+        const cpx<R> x = v[e], y = v[e + h];
+        v[e] = x + y;
+        v[e + h] = trivial(k, b, q) ? x - y : rot<false>(wl[k][h + q], x - y);
+      } else {
+        const cpx<R> x = v[e];
+        const cpx<R> y = trivial(k, b, q) ? v[e + h] : rot<true>(wl[k][h + q], v[e + h]);
+        v[e] = x + y;
+        v[e + h] = x - y;
       }
     }
   }
-  __device__ void inverse(cpx<R>* v) const {
+  template <bool INV>
+  __device__ __forceinline__ void twiddle(cpx<R>* v) const {
 #pragma unroll
-    for (int s = 4; s >= 0; --s) {
-      const int m = 16 >> s;
-      const bool up = lane & m;
+    for (int e = 0; e < E; ++e)
+      if (brev_bits((e << lo(0)) >> 5, LN - 5)) v[e] = rot<INV>(wb[e], v[e]);
+  }
+  // from the first group's layout to the last's; at(p): the exchange slot of
+  // position p, sync(): a barrier of the line's threads.  A thread writes only
+  // the positions it read last, so each exchange needs one barrier, and so
+  // does a transform that follows another on the same exchange space.
+  template <class At, class Sync>
+  __device__ __forceinline__ void forward(cpx<R>* v, At at, Sync sync) const {
 #pragma unroll
-      for (int r = 0; r < P; ++r) {
-        const cpx<R> mine = up ? rot<true>(wl[s], v[r]) : v[r];
-        const cpx<R> other = shx(mine, m);
-        v[r] = up ? other - mine : mine + other;
+    for (int k = 0; k < NG; ++k) {
+      if (k > 0) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) *at(pos(k - 1, t, e)) = v[e];
+        sync();
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[e] = *at(pos(k, t, e));
+      }
+#pragma unroll
+      for (int b = hi(k) - 1; b >= lo(k); --b) {
+        if (k == 0 && b == 4) twiddle<false>(v);
+        level<false>(v, k, b);
+      }
+      if (k == 0 && lo(k) == 5) twiddle<false>(v);
+    }
+  }
+  template <class At, class Sync>
+  __device__ __forceinline__ void inverse(cpx<R>* v, At at, Sync sync) const {
+#pragma unroll
+    for (int k = NG - 1; k >= 0; --k) {
+      if (k < NG - 1) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) *at(pos(k + 1, t, e)) = v[e];
+        sync();
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[e] = *at(pos(k, t, e));
+      }
+      if (k == 0 && lo(k) == 5) twiddle<true>(v);
+#pragma unroll
+      for (int b = lo(k); b < hi(k); ++b) {
+        level<true>(v, k, b);
+        if (k == 0 && b == 4) twiddle<true>(v);
       }
     }
-#pragma unroll
-    for (int r = 0; r < P; ++r) v[r] = rot<true>(wb[r], v[r]);
-#pragma unroll
-    for (int h = 1; h <= P / 2; h *= 2)
-#pragma unroll
-      for (int b = 0; b < P; b += 2 * h)
-#pragma unroll
-        for (int q = 0; q < h; ++q) {
-          const cpx<R> a = v[b + q], t = rot<true>(wr[q * (P / (2 * h))], v[b + q + h]);
-          v[b + q] = a + t;
-          v[b + q + h] = a - t;
-        }
   }
 };
 
+// what the passes of a step read; copied to shared memory by every CTA
 template <typename R>
 struct NdArgs {
-  int nx, ny, nz, ndim;
-  cpx<R>* psi;            // state
-  const double2* psi0;    // psi(0), natural order (FIRST pass input)
-  const double2* psi_start;  // resume / diagnostics: natural-order state read instead
-  double2* psi_out;       // psi(TF), natural order (LAST pass output)
+  int ln[3], ndim;        // log2 of the axis lengths (0 for an absent z)
+  long n;
+  cpx<R>* psi;            // state between the passes, storage order (NdLayout)
+  const double2* psi0;    // psi(0), natural order
+  const double2* psi_start;  // the natural-order state a run starts from
+  double2* psi_out;       // psi(TF), natural order
   using PhT = typename Ph<R>::type;
   const PhT* g;           // x-space factors, natural order
   const PhT* h;
   const PhT* hm;
   const double2* w;       // conj(psi0) hm, for C(t) (FP64 in both forms)
-  const PhT* K;           // kinetic factors in the kinetic pass's layout
-  const double* kq_c;     // reference-defect form: cos / sin(CST1 TC) in that layout
+  const PhT* K;           // kinetic factors in storage order
+  const double* kq_c;     // reference-defect form: cos / sin(CST1 TC), storage order
   const double* kq_s;
   double kq_scale;
-  double2* cpart;         // C(t) partial sums [step][x-pass CTA]
+  double2* cpart;         // C(t) partial sums [step][CTA]
   const typename Rot<R>::type* tw[3];  // W_n^k tables of the x, y, z line lengths
-  int step;
-  // second-order differences (psodfft.f / sodfft.f:64-126): dst <- dst - i f
+  // second-order differences (psodfft.f / sodfft.f:64-126): dst <- old - i f
   // (vc src + T src) [+ f ab src, or times the mask], natural order
-  const double2* sod_src;
-  double2* sod_dst;
+  double2 *cur, *prev;
   const double* vc;   // CST V
   const double* ab;   // CST VABC (.VOPTIC) or the .SMOOTHW mask
-  double f;
   int kabs;           // 0 none, 1 complex potential, 2 mask
+  // the run
+  int op;             // kOpSpo, kOpSod, kOpForward
+  int nsteps, from_start;
+  int fused;          // 3D: xy planes whole in shared memory
+  int lc;             // log2 of the adjacent columns of a tile
+  unsigned long long* bar;  // grid barrier arrivals of the launch (zeroed before it)
+  int* err;                 // set when a barrier wait gave up
+  long spin_limit;
 };
+enum { kOpSpo = 0, kOpSod = 1, kOpForward = 2 };
 
 // W_n^k = exp(-2 pi i k / n), k < n, in the form the line transforms apply
 template <typename R>
@@ -230,118 +294,459 @@ __global__ void tw_table_kernel(typename Rot<R>::type* tab, int n) {
   if (k < n) tab[k] = twid<R>(k, n);
 }
 
-enum { kFirst = 0, kMid = 1, kLast = 2, kFwd0 = 3, kSodUpd = 4 };
+// one row update of the second-order-differences form
+struct SodRow {
+  const double2 *src, *old;
+  double2* dst;
+  double f;
+};
 
-// x pass: one warp per row, 8 rows per CTA
-template <typename R, int P, int MODE>
-__global__ void __launch_bounds__(256) x_pass(NdArgs<R> a) {
-  constexpr int N = 32 * P;
-  __shared__ double2 s_c[kMaxWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
-  const long row = (long)blockIdx.x * nw + warp;
-  const long nrows = (long)a.ny * a.nz;
-  WarpFft<R, P> fft;
-  fft.init(a.tw[0]);
-  cpx<R> v[P];
-  double cr = 0.0, ci = 0.0;
-  if (row < nrows) {
-    const long base = row * N;
+// x-space work of a row between its inverse and its forward transform.  kFirst:
+// h psi of a natural-order state, |psi|^2; kMid / kLast: C(t) and the phase g
+// or hm; kFwd0: a natural-order state; kUpd / kUpdFwd: the leapfrog update
+enum { kFirst = 0, kMid = 1, kLast = 2, kFwd0 = 3, kUpd = 4, kUpdFwd = 5 };
+__host__ __device__ constexpr bool row_inverse(int mode) { return mode != kFirst && mode != kFwd0; }
+__host__ __device__ constexpr bool row_forward(int mode) { return mode != kLast && mode != kUpd; }
+
+// what row_points reads of a row's points; loaded before the inverse transform
+// where the registers allow (8 points per thread), so that the two overlap
+template <typename R, int E, int MODE>
+struct RowIn {
+  static constexpr bool kEarly = E == 8 && row_inverse(MODE);
+  double2 p[E], q[E];
+  typename Ph<R>::type ph[E];
+  __device__ __forceinline__ void load(const NdArgs<R>& a, const SodRow& o, int e, long x) {
     if (MODE == kFirst) {
-      const double2* src = a.psi_start ? a.psi_start : a.psi0;
+      p[e] = a.psi_start[x];
+      ph[e] = a.h[x];
+    } else if (MODE == kFwd0) {
+      p[e] = a.psi_start[x];
+    } else if (MODE == kMid || MODE == kLast) {
+      p[e] = __ldg(a.w + x);
+      ph[e] = MODE == kLast ? a.hm[x] : a.g[x];
+    } else {
+      p[e] = o.src[x];
+      q[e] = o.old[x];
+    }
+  }
+};
+
+template <typename R, int LN, int MODE>
+__device__ __forceinline__ void row_points(const NdArgs<R>& a, const SodRow& o, cpx<R>* v,
+                                           RowIn<R, LineFft<R, LN>::E, MODE>& in,
+                                           const LineFft<R, LN>& fft, long base, double& cr,
+                                           double& ci) {
+  constexpr int E = LineFft<R, LN>::E, L = LineFft<R, LN>::L;
 #pragma unroll
-      for (int j = 0; j < P; ++j) {
-        const long x = base + 32 * j + lane;
-        const double2 p = src[x];
-        cr += p.x * p.x + p.y * p.y;  // C(0) = <psi0|psi0> (not used when resuming)
-        v[j] = apply_ph(a.h[x], mk((R)p.x, (R)p.y));
-      }
-    } else if (MODE == kSodUpd) {
+  for (int e = 0; e < E; ++e) {
+    const long x = base + e * L + fft.t;
+    if (!in.kEarly) in.load(a, o, e, x);
+    const double2 p = in.p[e];
+    if (MODE == kFirst) {
+      cr += p.x * p.x + p.y * p.y;  // C(0) = <psi0|psi0> (not used when resuming)
+      v[e] = apply_ph(in.ph[e], mk((R)p.x, (R)p.y));
+    } else if (MODE == kFwd0) {
+      if (a.op == kOpSod) cr += p.x * p.x + p.y * p.y;
+      v[e] = mk((R)p.x, (R)p.y);
+    } else if (MODE == kMid || MODE == kLast) {
+      cr += p.x * (double)v[e].x - p.y * (double)v[e].y;
+      ci += p.x * (double)v[e].y + p.y * (double)v[e].x;
+      v[e] = apply_ph(in.ph[e], v[e]);
+      if (MODE == kLast) a.psi_out[x] = make_double2((double)v[e].x, (double)v[e].y);
+    } else {
       // T src by the inverse of the transformed copy, then the leapfrog update
-#pragma unroll
-      for (int j = 0; j < P; ++j) v[j] = a.psi[base + 32 * j + lane];
-      fft.inverse(v);
-#pragma unroll
-      for (int j = 0; j < P; ++j) {
-        const long x = base + 32 * j + lane;
-        const double2 sj = a.sod_src[x], dj = a.sod_dst[x];
-        const double vc = a.vc[x];
-        const double hx = fma(vc, sj.x, (double)v[j].x), hy = fma(vc, sj.y, (double)v[j].y);
-        double ox = fma(a.f, hy, dj.x), oy = fma(-a.f, hx, dj.y);
-        if (a.kabs == 1) {
-          const double abf = a.f * a.ab[x];
-          ox = fma(abf, sj.x, ox);
-          oy = fma(abf, sj.y, oy);
-        } else if (a.kabs == 2) {
-          ox *= a.ab[x];
-          oy *= a.ab[x];
-        }
-        a.sod_dst[x] = make_double2(ox, oy);
-        const double2 wj = a.w[x];  // conj(psi0)
-        cr += wj.x * ox - wj.y * oy;
-        ci += wj.x * oy + wj.y * ox;
+      const double2 sj = p, dj = in.q[e];
+      const double vc = a.vc[x];
+      const double hx = fma(vc, sj.x, (double)v[e].x), hy = fma(vc, sj.y, (double)v[e].y);
+      double ox = fma(o.f, hy, dj.x), oy = fma(-o.f, hx, dj.y);
+      if (a.kabs == 1) {
+        const double abf = o.f * a.ab[x];
+        ox = fma(abf, sj.x, ox);
+        oy = fma(abf, sj.y, oy);
+      } else if (a.kabs == 2) {
+        ox *= a.ab[x];
+        oy *= a.ab[x];
       }
-    } else if (MODE == kFwd0) {  // plain forward transform of a natural-order state
-#pragma unroll
-      for (int j = 0; j < P; ++j) {
-        const double2 p = a.psi_start[base + 32 * j + lane];
-        v[j] = mk((R)p.x, (R)p.y);
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < P; ++j) v[j] = a.psi[base + 32 * j + lane];
-      fft.inverse(v);
-#pragma unroll
-      for (int j = 0; j < P; ++j) {
-        const long x = base + 32 * j + lane;
-        const double2 wj = a.w[x];
-        cr += wj.x * (double)v[j].x - wj.y * (double)v[j].y;
-        ci += wj.x * (double)v[j].y + wj.y * (double)v[j].x;
-        v[j] = apply_ph(MODE == kLast ? a.hm[x] : a.g[x], v[j]);
-      }
+      o.dst[x] = make_double2(ox, oy);
+      const double2 wj = a.w[x];  // conj(psi0)
+      cr += wj.x * ox - wj.y * oy;
+      ci += wj.x * oy + wj.y * ox;
+      v[e] = mk((R)ox, (R)oy);
     }
-    if (MODE == kSodUpd) {
-      // written above
-    } else if (MODE == kLast) {
-#pragma unroll
-      for (int j = 0; j < P; ++j)
-        a.psi_out[base + 32 * j + lane] = make_double2((double)v[j].x, (double)v[j].y);
-    } else {
-      fft.forward(v);
-#pragma unroll
-      for (int j = 0; j < P; ++j) a.psi[base + 32 * j + lane] = v[j];
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    cr += __shfl_xor_sync(kFull, cr, o);
-    ci += __shfl_xor_sync(kFull, ci, o);
-  }
-  if (lane == 0) s_c[warp] = make_double2(cr, ci);
-  __syncthreads();
-  if (threadIdx.x == 0 && a.cpart) {
-    double sr = 0.0, si = 0.0;
-    for (int i = 0; i < nw; ++i) {
-      sr += s_c[i].x;
-      si += s_c[i].y;
-    }
-    a.cpart[(long)a.step * gridDim.x + blockIdx.x] = make_double2(sr, si);
   }
 }
 
-// C(0) = sum |psi0|^2 as x-pass-shaped partials (nb blocks)
-__global__ void c0_kernel(const double2* psi0, long n, double2* part) {
-  __shared__ double red[256];
-  const long lo = n * blockIdx.x / gridDim.x, hi = n * (blockIdx.x + 1) / gridDim.x;
-  double s = 0.0;
-  for (long i = lo + threadIdx.x; i < hi; i += blockDim.x) s += psi0[i].x * psi0[i].x + psi0[i].y * psi0[i].y;
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+__device__ __forceinline__ void bar_group(int id, int threads) {
+  if (threads <= 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ int skew(int p) { return p + (p >> 3); }
+
+// x pass: the rows of the grid, 32/L of them per warp; psi holds a row's
+// transform in storage order (coalesced for the last group's registers)
+template <typename R, int LN, int MODE>
+__device__ __noinline__ double2 rows_phase(const NdArgs<R>& a, const SodRow& o,
+                                           const typename Rot<R>::type* tab, cpx<R>* sm) {
+  using F = LineFft<R, LN>;
+  constexpr int N = F::N, E = F::E, L = F::L, LW = 32 / L;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nw = blockDim.x >> 5, sub = lane / L;
+  cpx<R>* ex = sm + (warp * LW + sub) * (N + N / 8);
+  F fft;
+  fft.init(tab, lane % L);
+  auto at = [&](int p) { return ex + skew(p); };
+  auto sync = [&]() { __syncwarp(); };
+  double cr = 0.0, ci = 0.0;
+  const int items = (int)(a.n >> LN) / LW, step = gridDim.x * nw;
+  for (int it = blockIdx.x + gridDim.x * warp; it < items; it += step) {
+    const long base = ((long)it * LW + sub) << LN;
+    cpx<R> v[E];
+    RowIn<R, E, MODE> in;
+    if (row_inverse(MODE)) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) v[e] = a.psi[base + e * L + fft.t];
+      if (in.kEarly) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) in.load(a, o, e, base + e * L + fft.t);
+      }
+      fft.inverse(v, at, sync);
+    }
+    row_points<R, LN, MODE>(a, o, v, in, fft, base, cr, ci);
+    if (row_forward(MODE)) {
+      fft.forward(v, at, sync);
+#pragma unroll
+      for (int e = 0; e < E; ++e) a.psi[base + e * L + fft.t] = v[e];
+    }
+    __syncwarp();
+  }
+  return make_double2(cr, ci);
+}
+
+enum { kFwd = 0, kInv = 1, kKin = 2 };
+
+// y or z pass: tiles of 2^lc adjacent x columns of one line set, a group of
+// 2^lc L threads per tile (consecutive threads: consecutive columns, so the
+// line's points go straight between global memory and registers)
+template <typename R, int LN, int MODE>
+__device__ __noinline__ void cols_phase(const NdArgs<R>& a, int axis,
+                                        const typename Rot<R>::type* tab, cpx<R>* sm) {
+  using F = LineFft<R, LN>;
+  constexpr int N = F::N, E = F::E, L = F::L;
+  const int lc = a.lc, gt = L << lc;  // threads of a group
+  const int group = threadIdx.x / gt, ng = blockDim.x / gt;
+  const int c = threadIdx.x & ((1 << lc) - 1);
+  cpx<R>* ex = sm + ((group * (N + N / 8)) << lc) + c;
+  F fft;
+  fft.init(tab, (threadIdx.x >> lc) & (L - 1));
+  auto at = [&](int p) { return ex + (skew(p) << lc); };
+  auto sync = [&]() { bar_group(1 + group, gt); };
+  const int ltx = a.ln[0] - lc;  // log2 of the tiles along x
+  const long stride = axis == 1 ? 1L << a.ln[0] : 1L << (a.ln[0] + a.ln[1]);
+  const int lset = axis == 1 ? a.ln[0] + a.ln[1] : a.ln[0];  // log2 of a line set's pitch
+  const int items = (int)(a.n >> (LN + lc));
+  for (int it = blockIdx.x + gridDim.x * group; it < items; it += gridDim.x * ng) {
+    const long base = ((long)(it >> ltx) << lset) + ((long)(it & ((1 << ltx) - 1)) << lc) + c;
+    cpx<R> v[E];
+    typename Ph<R>::type kf[E];
+    constexpr bool kEarly = MODE == kKin && E == 8;  // as RowIn
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = a.psi[base + (e * L + fft.t) * stride];
+    if (kEarly && !a.kq_c) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) kf[e] = a.K[base + (e * L + fft.t) * stride];
+    }
+    if (MODE != kInv) fft.forward(v, at, sync);
+    if (MODE == kKin) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const long f = base + (e * L + fft.t) * stride;
+        if (a.kq_c) {
+          // spofft.f:148-154 as written: V(I) uses the already updated U(I)
+          const double kc = a.kq_c[f], ks = a.kq_s[f];
+          const double un = kc * (double)v[e].x + ks * (double)v[e].y;
+          const double vn = kc * (double)v[e].y - ks * un;
+          v[e] = mk((R)(un * a.kq_scale), (R)(vn * a.kq_scale));
+        } else {
+          v[e] = apply_ph(kEarly ? kf[e] : a.K[f], v[e]);
+        }
+      }
+    }
+    if (MODE != kFwd) {
+      fft.inverse(v, at, sync);
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) a.psi[base + (e * L + fft.t) * stride] = v[e];
+    sync();
+  }
+}
+
+// the columns of a plane in shared memory, in place (positions along y), the
+// exchange through the lines' own places
+template <typename R, int LN, bool INV, int THREADS>
+__device__ __noinline__ void plane_cols(const NdArgs<R>& a, const typename Rot<R>::type* tab,
+                                        cpx<R>* sm) {
+  using F = LineFft<R, LN>;
+  constexpr int E = F::E, L = F::L;
+  // columns of a group: 128 bytes of them, within the CTA's threads
+  constexpr int C = sizeof(R) == 4 && 16 * L <= THREADS ? 16 : 8, GT = C * L;
+  const int nx = 1 << a.ln[0], pitch = nx + nx / 8;
+  const int group = threadIdx.x / GT, ng = blockDim.x / GT;
+  F fft;
+  fft.init(tab, (threadIdx.x / C) % L);
+  auto sync = [&]() { bar_group(1 + group, GT); };
+  for (int xt = group; xt < nx / C; xt += ng) {
+    cpx<R>* col = sm + skew(xt * C + threadIdx.x % C);
+    auto at = [&](int p) { return col + p * pitch; };
+    cpx<R> v[E];
+    constexpr int k0 = INV ? F::NG - 1 : 0, k1 = INV ? 0 : F::NG - 1;
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = *at(F::pos(k0, fft.t, e));
+    if (INV) fft.inverse(v, at, sync);
+    else fft.forward(v, at, sync);
+#pragma unroll
+    for (int e = 0; e < E; ++e) *at(F::pos(k1, fft.t, e)) = v[e];
+  }
+}
+
+// the rows of a plane in shared memory, in place
+template <typename R, int LN, int MODE>
+__device__ __noinline__ double2 plane_rows(const NdArgs<R>& a, const SodRow& o,
+                                           const typename Rot<R>::type* tab, cpx<R>* sm,
+                                           long plane) {
+  using F = LineFft<R, LN>;
+  constexpr int N = F::N, E = F::E, L = F::L, LW = 32 / L;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int ny = 1 << a.ln[1];
+  F fft;
+  fft.init(tab, lane % L);
+  auto sync = [&]() { __syncwarp(); };
+  double cr = 0.0, ci = 0.0;
+  for (int y = warp * LW + lane / L; y < ny; y += nw * LW) {
+    cpx<R>* row = sm + y * (N + N / 8);
+    auto at = [&](int p) { return row + skew(p); };
+    const long base = ((plane << a.ln[1]) + y) << LN;
+    cpx<R> v[E];
+    RowIn<R, E, MODE> in;
+    if (row_inverse(MODE)) {
+      if (in.kEarly) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) in.load(a, o, e, base + e * F::L + fft.t);
+      }
+#pragma unroll
+      for (int e = 0; e < E; ++e) v[e] = *at(F::pos(F::NG - 1, fft.t, e));
+      fft.inverse(v, at, sync);
+    }
+    row_points<R, LN, MODE>(a, o, v, in, fft, base, cr, ci);
+    if (row_forward(MODE)) {
+      fft.forward(v, at, sync);
+#pragma unroll
+      for (int e = 0; e < E; ++e) *at(F::pos(F::NG - 1, fft.t, e)) = v[e];
+    }
+  }
+  return make_double2(cr, ci);
+}
+
+// runs f<LN>() for the line length 2^ln; MAXLN bounds the instantiations
+template <int MAXLN, class F>
+__device__ __forceinline__ void for_len(int ln, F f) {
+  switch (ln) {
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 7: f(std::integral_constant<int, 7>{}); break;
+    case 8: if constexpr (MAXLN >= 8) f(std::integral_constant<int, 8>{}); break;
+    default: if constexpr (MAXLN >= 9) f(std::integral_constant<int, 9>{}); break;
+  }
+}
+
+// x pass of the whole grid, or with `fused` the x and y transforms of whole xy
+// planes (y inverse, the x pass, y forward) in shared memory
+template <typename R, int T, int MAXLN, int MODE>
+__device__ __forceinline__ double2 x_phase(const NdArgs<R>& a, const SodRow& o,
+                                           const typename Rot<R>::type* const* tab, cpx<R>* sm) {
+  double2 c = make_double2(0.0, 0.0);
+  if (!a.fused) {
+    for_len<MAXLN>(a.ln[0], [&](auto ln) {
+      c = rows_phase<R, decltype(ln)::value, MODE>(a, o, tab[0], sm);
+    });
+    return c;
+  }
+  const int lx = a.ln[0], lp = lx + a.ln[1], pitch = (1 << lx) + (1 << (lx - 3));
+  for (long z = blockIdx.x; z < (1L << a.ln[2]); z += gridDim.x) {
+    cpx<R>* g = a.psi + (z << lp);
+    auto slot = [&](int i) { return sm + (i >> lx) * pitch + skew(i & ((1 << lx) - 1)); };
+    if (row_inverse(MODE)) {
+#pragma unroll 8
+      for (int i = threadIdx.x; i < (1 << lp); i += blockDim.x) *slot(i) = g[i];
+      __syncthreads();
+      for_len<MAXLN>(a.ln[1], [&](auto ln) {
+        plane_cols<R, decltype(ln)::value, true, T>(a, tab[1], sm);
+      });
+      __syncthreads();
+    }
+    for_len<MAXLN>(lx, [&](auto ln) {
+      const double2 d = plane_rows<R, decltype(ln)::value, MODE>(a, o, tab[0], sm, z);
+      c.x += d.x;
+      c.y += d.y;
+    });
+    if (row_forward(MODE)) {
+      __syncthreads();
+      for_len<MAXLN>(a.ln[1], [&](auto ln) {
+        plane_cols<R, decltype(ln)::value, false, T>(a, tab[1], sm);
+      });
+      __syncthreads();
+#pragma unroll 8
+      for (int i = threadIdx.x; i < (1 << lp); i += blockDim.x) g[i] = *slot(i);
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = make_double2(red[0], 0.0);
+  return c;
+}
+
+template <typename R, int MAXLN, int MODE>
+__device__ __forceinline__ void axis_phase(const NdArgs<R>& a, int axis,
+                                           const typename Rot<R>::type* const* tab, cpx<R>* sm) {
+  for_len<MAXLN>(a.ln[axis], [&](auto ln) {
+    cols_phase<R, decltype(ln)::value, MODE>(a, axis, tab[axis], sm);
+  });
+}
+
+// End of a pass: with step >= 0 the CTA's C(t) partial sum of that step, then
+// (unless it is the last pass) a grid barrier.  Thread 0's arrival is a
+// release ordered after the CTA's writes by bar.sync; every arrival continues
+// the release sequence of the earlier ones, so the acquire load that sees the
+// last one synchronises with all.  false: a wait gave up.
+template <typename R>
+__device__ __forceinline__ bool end_pass(const NdArgs<R>& a, double2 c, int step, bool last,
+                                         unsigned& passed, double2* s_c, int* s_ok) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (step >= 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      c.x += __shfl_xor_sync(kFull, c.x, o);
+      c.y += __shfl_xor_sync(kFull, c.y, o);
+    }
+    if (lane == 0) s_c[warp] = c;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (step >= 0) {
+      double2 t = make_double2(0.0, 0.0);
+      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
+        t.x += s_c[i].x;
+        t.y += s_c[i].y;
+      }
+      a.cpart[(long)step * gridDim.x + blockIdx.x] = t;
+    }
+    *s_ok = 1;
+    if (!last && gridDim.x > 1) {
+      const unsigned long long target = (unsigned long long)(passed + 1u) * gridDim.x;
+      cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> cnt(*a.bar);
+      cuda::atomic_ref<int, cuda::thread_scope_device> err(*a.err);
+      if (cnt.fetch_add(1ull, cuda::memory_order_acq_rel) + 1ull < target) {
+        long spins = 0;
+        while (cnt.load(cuda::memory_order_acquire) < target) {
+          if (++spins > a.spin_limit || err.load(cuda::memory_order_relaxed) != 0) {
+            err.store(1, cuda::memory_order_relaxed);
+            *s_ok = 0;
+            break;
+          }
+          if (spins > 4096) __nanosleep(32);
+        }
+      }
+    }
+  }
+  ++passed;
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+// A whole run in one cooperative launch: the passes of every step separated by
+// grid barriers.  The state (1 MB for 256 x 256 FP64) stays in L2, and a pass
+// of a small grid is a chain of latencies: one launch per pass cost 9 us each
+// (launch, table loads and one warp per SM), a pass here about a third.
+template <typename R, int T, int MAXLN>
+__global__ void __launch_bounds__(T, 1) nd_kernel(const NdArgs<R> ga) {
+  extern __shared__ __align__(16) unsigned char nd_raw[];
+  __shared__ NdArgs<R> a;
+  __shared__ double2 s_c[T / 32];
+  __shared__ int s_ok;
+  using Tw = typename Rot<R>::type;
+  if (threadIdx.x == 0) a = ga;
+  // twiddle tables of the axes, then the exchange space
+  Tw* tab[3];
+  Tw* next = reinterpret_cast<Tw*>(nd_raw);
+  for (int ax = 0; ax < ga.ndim; ++ax) {
+    tab[ax] = next;
+    for (int i = threadIdx.x; i < (1 << ga.ln[ax]); i += T) next[i] = ga.tw[ax][i];
+    next += 1 << ga.ln[ax];
+  }
+  if (ga.ndim < 3) tab[2] = tab[1];
+  cpx<R>* sm = reinterpret_cast<cpx<R>*>(next);
+  __syncthreads();
+  unsigned passed = 0;
+  const double2 zero = make_double2(0.0, 0.0);
+  auto fence = [&](double2 c, int step, bool last) {
+    return end_pass<R>(a, c, step, last, passed, s_c, &s_ok);
+  };
+  // the passes between two x passes
+  auto kin = [&]() -> bool {
+    if (a.ndim == 2) {
+      axis_phase<R, MAXLN, kKin>(a, 1, tab, sm);
+      return fence(zero, -1, false);
+    }
+    if (!a.fused) {
+      axis_phase<R, MAXLN, kFwd>(a, 1, tab, sm);
+      if (!fence(zero, -1, false)) return false;
+    }
+    axis_phase<R, MAXLN, kKin>(a, 2, tab, sm);
+    if (!fence(zero, -1, false)) return false;
+    if (!a.fused) {
+      axis_phase<R, MAXLN, kInv>(a, 1, tab, sm);
+      return fence(zero, -1, false);
+    }
+    return true;
+  };
+  SodRow o{};
+  if (a.op == kOpSpo) {
+    double2 c = x_phase<R, T, MAXLN, kFirst>(a, o, tab, sm);
+    if (!fence(c, 0, a.nsteps == 0)) return;
+    for (int s = 1; s <= a.nsteps; ++s) {
+      if (!kin()) return;
+      const bool end = s == a.nsteps;
+      c = end ? x_phase<R, T, MAXLN, kLast>(a, o, tab, sm) : x_phase<R, T, MAXLN, kMid>(a, o, tab, sm);
+      if (!fence(c, s, end)) return;
+    }
+  } else if (a.op == kOpForward) {
+    x_phase<R, T, MAXLN, kFwd0>(a, o, tab, sm);
+    if (!a.fused) {
+      if (!fence(zero, -1, false)) return;
+      axis_phase<R, MAXLN, kFwd>(a, 1, tab, sm);
+    }
+    if (a.ndim == 3) {
+      if (!fence(zero, -1, false)) return;
+      axis_phase<R, MAXLN, kFwd>(a, 2, tab, sm);
+    }
+  } else if constexpr (sizeof(R) == 8) {  // SOD plans are FP64
+    // every update's new state is the next one's source: its row is
+    // transformed in the same pass.  The start-up (psodfft.f:120-152) is two
+    // half steps from psi0 and then psi(t - dt) = psi0.
+    const int updates = a.nsteps + (a.from_start && a.nsteps > 0 ? 1 : 0);
+    double2* buf[2] = {a.prev, a.cur};
+    double2 c = x_phase<R, T, MAXLN, kFwd0>(a, o, tab, sm);
+    if (!fence(c, a.from_start ? 0 : -1, updates == 0)) return;
+    for (int u = 0; u < updates; ++u) {
+      if (!kin()) return;
+      o.src = u == 0 ? a.psi_start : buf[(u & 1) ^ 1];
+      o.dst = buf[u & 1];
+      o.old = a.from_start && u < 3 ? a.psi0 : o.dst;
+      o.f = a.from_start && u < 2 ? 0.5 : 1.0;
+      const bool end = u + 1 == updates;
+      c = end ? x_phase<R, T, MAXLN, kUpd>(a, o, tab, sm) : x_phase<R, T, MAXLN, kUpdFwd>(a, o, tab, sm);
+      // updates 0 and 1 both lead to step 1; the sample is the second's
+      const int step = a.from_start ? (u == 0 ? -1 : u) : u + 1;
+      if (!fence(c, step, end)) return;
+    }
+  }
 }
 
 // SOD tables: vc = CST V, ab = CST VABC or the mask, w = conj(psi0)
@@ -382,78 +787,94 @@ __global__ void nd_energy_kernel(const double2* psi, const double* vpot, const c
   if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-enum { kFwd = 0, kInv = 1, kKin = 2 };
-
-// strided pass along axis 1 (y) or 2 (z): CTA = blockDim/32 adjacent x columns
-// of one line set, staged through shared memory; warp w transforms column w
-template <typename R, int P, int MODE, bool QUIRK>
-__global__ void __launch_bounds__(256) axis_pass(NdArgs<R> a, int axis) {
-  constexpr int N = 32 * P;
-  extern __shared__ __align__(16) unsigned char sm_raw[];
-  const int kTile = blockDim.x >> 5;  // adjacent x columns per CTA, one warp each
-  cpx<R>* tile = reinterpret_cast<cpx<R>*>(sm_raw);  // [N][kTile + 1]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ntx = a.nx / kTile;
-  const long xt = blockIdx.x % ntx, other = blockIdx.x / ntx;
-  long stride, base;
-  if (axis == 1) {  // lines along y: x = 8 xt + c, z = other
-    stride = a.nx;
-    base = other * (long)a.nx * a.ny + xt * kTile;
-  } else {          // lines along z: x = 8 xt + c, y = other
-    stride = (long)a.nx * a.ny;
-    base = other * (long)a.nx + xt * kTile;
-  }
-  for (int e = threadIdx.x; e < N * kTile; e += blockDim.x) {
-    const int t = e / kTile, c = e % kTile;
-    tile[t * (kTile + 1) + c] = a.psi[base + t * stride + c];
-  }
-  __syncthreads();
-  WarpFft<R, P> fft;
-  fft.init(a.tw[axis]);
-  cpx<R> v[P];
-#pragma unroll
-  for (int j = 0; j < P; ++j) v[j] = tile[(32 * j + lane) * (kTile + 1) + warp];
-  if (MODE == kFwd || MODE == kKin) fft.forward(v);
-  if (MODE == kKin) {
-    // kinetic table line: x position and the other coordinate
-    const long line = (xt * kTile + warp) + (long)a.nx * other;
-    const long kb = line * N;
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const long f = kb + 32 * j + lane;
-      if constexpr (QUIRK) {
-        // spofft.f:148-154 as written: V(I) uses the already updated U(I)
-        const double c = a.kq_c[f], s = a.kq_s[f];
-        const double un = c * (double)v[j].x + s * (double)v[j].y;
-        const double vn = c * (double)v[j].y - s * un;
-        v[j] = mk((R)(un * a.kq_scale), (R)(vn * a.kq_scale));
-      } else {
-        v[j] = apply_ph(a.K[f], v[j]);
-      }
-    }
-  }
-  if (MODE == kInv || MODE == kKin) fft.inverse(v);
-#pragma unroll
-  for (int j = 0; j < P; ++j) tile[(32 * j + lane) * (kTile + 1) + warp] = v[j];
-  __syncthreads();
-  for (int e = threadIdx.x; e < N * kTile; e += blockDim.x) {
-    const int t = e / kTile, c = e % kTile;
-    a.psi[base + t * stride + c] = tile[t * (kTile + 1) + c];
-  }
-}
-
-// C(t) of each step: the x-pass partial sums in CTA order
+// C(t) of each step: the partial sums of the CTAs, a warp per step; NaN where
+// a grid barrier of the run gave up
 __global__ void csum_kernel(const double2* cpart, int nparts, int nsteps, int first,
-                            double2* c_out) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x + first;
+                            double2* c_out, const int* err) {
+  const int lane = threadIdx.x & 31;
+  const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) + first;
   if (s > nsteps) return;
   double sr = 0.0, si = 0.0;
-  for (int i = 0; i < nparts; ++i) {
+  for (int i = lane; i < nparts; i += 32) {
     const double2 p = cpart[(long)s * nparts + i];
     sr += p.x;
     si += p.y;
   }
-  c_out[s] = make_double2(sr, si);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sr += __shfl_xor_sync(kFull, sr, o);
+    si += __shfl_xor_sync(kFull, si, o);
+  }
+  if (err && *err) sr = si = nan("");
+  if (lane == 0) c_out[s] = make_double2(sr, si);
+}
+
+// Frequency (FFT order) at place s of an axis's transform.  Positions p of the
+// line transform hold frequency brev_P(p / 32) + P brev_32(p % 32), N = 32 P; a
+// pass that stores its registers writes position (t << LE) | e at place e L + t
+// (coalesced), a fused plane is stored by position.
+__host__ __device__ inline int freq_at(int s, int ln, bool by_pos) {
+  const int le = ln == 9 ? 4 : 3, lt = ln - le;
+  const int p = by_pos ? s : ((s & ((1 << lt) - 1)) << le) | (s >> lt);
+  return brev_bits(p >> 5, ln - 5) + (brev_bits(p & 31, 5) << (ln - 5));
+}
+struct NdLayout {
+  int ln[3];
+  bool by_pos[3];
+};
+// index into the reference's FFT-order table of the frequency stored at i,
+// mirrored to its FFT sign (fft3d.f: ISN = +1 is exp(+2 pi i jk/n))
+__device__ __forceinline__ long tc_index(const NdLayout& l, long i) {
+  long idx = 0;
+  int shift = 0;
+  for (int ax = 0; ax < 3 && l.ln[ax] > 0; ++ax) {
+    const int n = 1 << l.ln[ax];
+    const int s = (int)(i >> shift) & (n - 1);
+    idx += (long)((n - freq_at(s, l.ln[ax], l.by_pos[ax])) & (n - 1)) << shift;
+    shift += l.ln[ax];
+  }
+  return idx;
+}
+// TC of FFT-order index idx: the sum of the axis tables t (x, y, z one after the
+// other), or with `defect` the only TC(1..NP1) that dkeft.f:80-137 fills
+__device__ __forceinline__ double tc_value(const NdLayout& l, const double* t, bool defect,
+                                           long idx) {
+  const long nx = 1L << l.ln[0], ny = 1L << l.ln[1];
+  if (defect) return idx < nx ? t[idx] : 0.0;
+  double s = t[idx & (nx - 1)] + t[nx + ((idx >> l.ln[0]) & (ny - 1))];
+  if (l.ln[2] > 0) s += t[nx + ny + (idx >> (l.ln[0] + l.ln[1]))];
+  return s;
+}
+__device__ __forceinline__ void put_k(cpx<double>* o, double th, double n) {
+  double s, c;
+  sincos(th, &s, &c);
+  *o = mk(c / n, -s / n);
+}
+__device__ __forceinline__ void put_k(PhF* o, double th, double n) { *o = make_phf(-th, 1.0 / n); }
+
+// kinetic factors in storage order: e^{-i CST1 TC}/N (and cos, sin for the
+// reference-defect form), or CST TC/N for second-order differences
+template <typename R>
+__global__ void nd_kinetic_kernel(NdLayout l, long n, const double* t, bool defect, bool sod,
+                                  double cst, typename Ph<R>::type* K, double* kq) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double th = cst * tc_value(l, t, defect, tc_index(l, i));
+  if (sod) {  // CST TC B (sodfft.f:100-104,119)
+    if constexpr (sizeof(R) == 8) K[i] = mk(th / n, 0.0);
+    return;
+  }
+  put_k(K + i, th, (double)n);
+  if (kq) {
+    double s, c;
+    sincos(th, &s, &c);
+    kq[i] = c;
+    kq[n + i] = s;
+  }
+}
+__global__ void nd_tc_kernel(NdLayout l, long n, const double* t, bool defect, double* tcp) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) tcp[i] = tc_value(l, t, defect, tc_index(l, i));
 }
 
 // x-space tables (spofft.f:120-133, 162-191): h = e^{-i cst2 V} (x e^{cst2
@@ -515,7 +936,11 @@ struct espec_spond_plan {
   double2* d_cpart = nullptr;
   double2* d_c = nullptr;
   void* d_tw[3] = {nullptr, nullptr, nullptr};
-  int c_cap = -1, xblocks = 0;
+  int c_cap = -1;
+  int nsm = 0;
+  double* d_tax = nullptr;         // DIGT axis tables (or the defect's TC(1..NP1))
+  bool k_ready = false;            // the kinetic table is built (it depends on the plan alone)
+  unsigned long long* d_bar = nullptr;  // grid barrier arrivals, then the error flag
   bool has_state = false;          // d_out holds the state of the last run
   // energy diagnostics (FP64 in both forms)
   cpx<double>* d_khat = nullptr;
@@ -528,12 +953,6 @@ struct espec_spond_plan {
 namespace {
 
 bool line_ok(int n) { return n == 32 || n == 64 || n == 128 || n == 256 || n == 512; }
-
-// frequency held at stored position pos of a line of n = 32 P points
-int freq_of(int pos, int n) {
-  const int P = n / 32, lp = P == 1 ? 0 : (P == 2 ? 1 : (P == 4 ? 2 : (P == 8 ? 3 : 4)));
-  return brev_bits(pos / 32, lp) + P * brev_bits(pos % 32, 5);
-}
 
 const double kDigtTwoPi = 6.283185307;  // dkeft.f:38
 
@@ -614,6 +1033,85 @@ void digt_nd(const espec_spond_plan* p, std::vector<double>& tc) {
     if (e_ != cudaSuccess) return set_cuda_error(#call, e_); \
   } while (0)
 
+// how a grid's passes are cut
+struct NdConfig {
+  int threads = 256, grid = 1, lc = 3, fused = 0;
+  size_t smem = 0;
+  NdLayout layout{};
+};
+
+// longest line (log2) of the 512-thread form
+template <typename R>
+constexpr int kMaxLn512 = sizeof(R) == 8 ? 7 : 8;
+
+// Threads: 512 where a thread's points, twiddles and preloaded factors fit 128
+// registers, else 256 (FP64 lines of 256 and 512 points, FP32 of 512).
+// Fused xy planes: where a plane fits in shared memory and there are planes
+// for most SMs -- the y passes then cost no memory traffic and no grid
+// barrier, but a plane runs on one SM.
+// Tiles of the column passes: 8 adjacent columns (128 bytes in FP64), fewer
+// where that would leave SMs without a tile.  CTAs: the fewest that keep the
+// largest share, at most one per SM.
+template <typename R>
+NdConfig nd_config(const espec_spond_plan* p) {
+  NdConfig c;
+  int mx = 0;
+  for (int ax = 0; ax < p->ndim; ++ax) {
+    int l = 5;
+    while ((1 << l) < p->np[ax]) ++l;
+    c.layout.ln[ax] = l;
+    mx = l > mx ? l : mx;
+  }
+  const int* ln = c.layout.ln;
+  c.threads = mx <= kMaxLn512<R> ? 512 : 256;
+  const size_t plane = sizeof(cpx<R>) * (size_t)(p->np[0] + p->np[0] / 8) * p->np[1];
+  size_t tw = 0;
+  for (int ax = 0; ax < p->ndim; ++ax) tw += sizeof(typename Rot<R>::type) * p->np[ax];
+  c.fused = p->ndim == 3 && tw + plane <= kNdMaxSmem && p->np[2] >= kFusedMinPlanes;
+  for (int ax = 0; ax < 2; ++ax) c.layout.by_pos[ax] = c.fused;
+  auto threads_of = [&](int ax) { return ln[ax] == 9 ? 5 : ln[ax] - 3; };  // log2, per line
+  auto tiles = [&](int lc) {
+    long t = p->n >> (ln[p->ndim - 1] + lc);
+    if (p->ndim == 3 && !c.fused) t = std::min(t, p->n >> (ln[1] + lc));
+    return t;
+  };
+  int lmin = 5 - threads_of(p->ndim - 1);  // a tile's group is whole warps
+  if (p->ndim == 3 && !c.fused) lmin = std::max(lmin, 5 - threads_of(1));
+  lmin = std::max(lmin, 1);
+  while (c.lc > lmin && tiles(c.lc) < 96) --c.lc;
+  const long rows = c.fused ? p->np[2] : (p->n >> ln[0]) >> (5 - threads_of(0));
+  long want = std::max(rows, tiles(c.lc));
+  if (want > p->nsm) {
+    const long per = (want + p->nsm - 1) / p->nsm;
+    want = (want + per - 1) / per;
+  }
+  c.grid = (int)want;
+  const int e = mx == 9 ? 16 : 8;
+  size_t ex = sizeof(cpx<R>) * (size_t)c.threads * e * 9 / 8;
+  if (c.fused) ex = std::max(ex, plane);
+  c.smem = tw + ex;
+  return c;
+}
+
+// DIGT's axis tables x, y, z, or with ESPEC_Q_DIGT_ND the TC(1..NP1) it fills
+int upload_axis_tables(espec_spond_plan* p, cudaStream_t st) {
+  std::vector<double> t;
+  if (p->quirks & ESPEC_Q_DIGT_ND) {
+    digt_nd(p, t);
+    t.resize(p->np[0]);
+  } else {
+    size_t o = 0;
+    for (int ax = 0; ax < p->ndim; ++ax) {
+      t.resize(o + p->np[ax]);
+      digt_axis_host(p->np[ax], p->sh[ax], p->sm[ax], t.data() + o);
+      o += p->np[ax];
+    }
+  }
+  ND_CK(cudaMemcpyAsync(p->d_tax, t.data(), 8 * t.size(), cudaMemcpyHostToDevice, st));
+  ND_CK(cudaStreamSynchronize(st));  // the host vector goes out of scope
+  return ESPEC_OK;
+}
+
 // table block: g, h, hm (PhT) | w (double2) | K (PhT), n entries each
 template <typename R>
 struct NdTabs {
@@ -630,13 +1128,6 @@ struct NdTabs {
     K = hm + n;
   }
 };
-
-inline cpx<double> k_factor(double th, long n, double) {
-  return mk(std::cos(th) / n, -std::sin(th) / n);
-}
-inline PhF k_factor(double th, long n, float) { return make_phf(-th, 1.0 / n); }
-inline cpx<double> k_real(double v, double) { return mk(v, 0.0); }
-inline PhF k_real(double v, float) { return make_phf(0.0, v); }
 
 inline int sod_kabs(const espec_spond_plan* p) {
   if (p->absorb == ESPEC_ABS_VOPTIC) return 1;
@@ -659,146 +1150,73 @@ int build_tables(espec_spond_plan* p, cudaStream_t st) {
         n, p->d_vpot, p->d_vabc, p->absorb, cst2, p->d_psi0, tb.g, tb.h, tb.hm, tb.w);
   }
   ND_CK(cudaGetLastError());
-  // kinetic factors in the kinetic pass's layout: line (x position, other
-  // position), position along the kinetic axis; frequencies mirrored to the
-  // reference's FFT sign (fft3d.f: ISN = +1 is exp(+2 pi i jk/n))
-  std::vector<double> tc;
-  digt_nd(p, tc);
-  const int nx = p->np[0], ny = p->np[1], nz = p->ndim > 2 ? p->np[2] : 1;
-  const int ka = p->ndim - 1;  // kinetic axis: y (2D) or z (3D)
-  const int nk = p->np[ka];
-  std::vector<typename Ph<R>::type> K((size_t)n);
-  std::vector<double> qc, qs;
-  const bool quirk = (p->quirks & ESPEC_Q_SPO_INPLACE) != 0;
-  if (quirk) {
-    qc.resize((size_t)n);
-    qs.resize((size_t)n);
-  }
-  const long nlines = n / nk;
-  for (long line = 0; line < nlines; ++line) {
-    const int px = (int)(line % nx);
-    const int po = (int)(line / nx);  // y position (3D) or unused (2D)
-    const int fx = (nx - freq_of(px, nx)) % nx;
-    const int fy2 = p->ndim > 2 ? (ny - freq_of(po, ny)) % ny : 0;
-    for (int pos = 0; pos < nk; ++pos) {
-      const int fk = (nk - freq_of(pos, nk)) % nk;
-      size_t idx;
-      if (p->ndim == 2) idx = fx + (size_t)nx * fk;
-      else idx = fx + (size_t)nx * (fy2 + (size_t)ny * fk);
-      const double th = cst1 * tc[idx];
-      const size_t o = (size_t)line * nk + pos;
-      if (sod) {
-        K[o] = k_real(cst_sod * tc[idx] / n, R(0));  // CST TC B (sodfft.f:100-104,119)
-      } else {
-        K[o] = k_factor(th, n, R(0));
-      }
-      if (quirk) {
-        qc[o] = std::cos(th);
-        qs[o] = std::sin(th);
-      }
+  if (!p->k_ready) {
+    const NdConfig cf = nd_config<R>(p);
+    const bool defect = (p->quirks & ESPEC_Q_DIGT_ND) != 0;
+    const int rc = upload_axis_tables(p, st);
+    if (rc) return rc;
+    nd_kinetic_kernel<R><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+        cf.layout, n, p->d_tax, defect, sod, sod ? cst_sod : cst1, tb.K, p->d_kq);
+    ND_CK(cudaGetLastError());
+    for (int ax = 0; ax < p->ndim; ++ax) {
+      const int nl = p->np[ax];
+      tw_table_kernel<R><<<(nl + 255) / 256, 256, 0, st>>>((typename Rot<R>::type*)p->d_tw[ax], nl);
+      ND_CK(cudaGetLastError());
     }
+    p->k_ready = true;
   }
-  (void)nz;
-  ND_CK(cudaMemcpyAsync(tb.K, K.data(), sizeof(K[0]) * n, cudaMemcpyHostToDevice, st));
-  if (quirk) {
-    ND_CK(cudaMemcpyAsync(p->d_kq, qc.data(), 8 * n, cudaMemcpyHostToDevice, st));
-    ND_CK(cudaMemcpyAsync(p->d_kq + n, qs.data(), 8 * n, cudaMemcpyHostToDevice, st));
-  }
-  ND_CK(cudaStreamSynchronize(st));  // the host vectors go out of scope
+  // a caller may reuse its arrays, and load on another stream next
+  ND_CK(cudaStreamSynchronize(st));
   return ESPEC_OK;
 }
 
-// warps per CTA: 8, or fewer when that leaves SMs idle (2 CTAs per SM wanted)
-int warps_for(long lines) {
-  int w = kMaxWarps;
-  while (w > 1 && lines / w < 2 * 148) w /= 2;
-  return w;
-}
-
-template <typename R, int P>
-cudaError_t launch_x(int mode, const NdArgs<R>& a, int blocks, cudaStream_t st) {
-  const long rows = (long)a.ny * a.nz;
-  const int w = warps_for(rows);
-  blocks = (int)((rows + w - 1) / w);
-  switch (mode) {
-    case kFirst: x_pass<R, P, kFirst><<<blocks, 32 * w, 0, st>>>(a); break;
-    case kMid: x_pass<R, P, kMid><<<blocks, 32 * w, 0, st>>>(a); break;
-    case kFwd0: x_pass<R, P, kFwd0><<<blocks, 32 * w, 0, st>>>(a); break;
-    case kSodUpd:
-      if constexpr (sizeof(R) == 8) {
-        x_pass<R, P, kSodUpd><<<blocks, 32 * w, 0, st>>>(a);
-        break;
-      }
-      return cudaErrorInvalidValue;  // SOD plans are FP64
-    case kLast: x_pass<R, P, kLast><<<blocks, 32 * w, 0, st>>>(a); break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-template <typename R>
-cudaError_t launch_x_n(int nx, int mode, const NdArgs<R>& a, int blocks, cudaStream_t st) {
-  switch (nx) {
-    case 32: return launch_x<R, 1>(mode, a, blocks, st);
-    case 64: return launch_x<R, 2>(mode, a, blocks, st);
-    case 128: return launch_x<R, 4>(mode, a, blocks, st);
-    case 256: return launch_x<R, 8>(mode, a, blocks, st);
-    default: return launch_x<R, 16>(mode, a, blocks, st);
-  }
-}
-
-template <typename R, int P, int MODE, bool Q>
-cudaError_t launch_axis1(const NdArgs<R>& a, int axis, long, cudaStream_t st) {
+template <typename R, int T, int MAXLN>
+int nd_launch_as(const NdConfig& c, NdArgs<R>& a, cudaStream_t st) {
   static DeviceFlags attr;
-  {
-    const size_t smax = sizeof(cpx<R>) * 32 * P * (kMaxWarps + 1);
-    cudaError_t e = set_max_smem_once(attr, axis_pass<R, P, MODE, Q>, smax);
-    if (e != cudaSuccess) return e;
-  }
-  const long other = axis == 1 ? a.nz : a.ny;  // line sets beside the x tiles
-  const int w = warps_for((long)a.nx * other);
-  const long blocks = (long)(a.nx / w) * other;
-  const size_t smem = sizeof(cpx<R>) * 32 * P * (w + 1);
-  axis_pass<R, P, MODE, Q><<<(unsigned)blocks, 32 * w, smem, st>>>(a, axis);
-  return cudaGetLastError();
-}
-
-template <typename R, int P>
-cudaError_t launch_axis_p(int mode, bool quirk, const NdArgs<R>& a, int axis, long blocks,
-                          cudaStream_t st) {
-  if (mode == kFwd) return launch_axis1<R, P, kFwd, false>(a, axis, blocks, st);
-  if (mode == kInv) return launch_axis1<R, P, kInv, false>(a, axis, blocks, st);
-  if constexpr (sizeof(R) == 8) {
-    if (quirk) return launch_axis1<R, P, kKin, true>(a, axis, blocks, st);
-  }
-  return launch_axis1<R, P, kKin, false>(a, axis, blocks, st);
+  ND_CK(set_max_smem_once(attr, nd_kernel<R, T, MAXLN>, kNdMaxSmem));
+  void* args[] = {&a};
+  ND_CK(cudaLaunchCooperativeKernel((const void*)nd_kernel<R, T, MAXLN>, dim3(c.grid), dim3(T),
+                                    args, c.smem, st));
+  return ESPEC_OK;
 }
 
 template <typename R>
-cudaError_t launch_axis(int n, int mode, bool quirk, const NdArgs<R>& a, int axis, long blocks,
-                        cudaStream_t st) {
-  switch (n) {
-    case 32: return launch_axis_p<R, 1>(mode, quirk, a, axis, blocks, st);
-    case 64: return launch_axis_p<R, 2>(mode, quirk, a, axis, blocks, st);
-    case 128: return launch_axis_p<R, 4>(mode, quirk, a, axis, blocks, st);
-    case 256: return launch_axis_p<R, 8>(mode, quirk, a, axis, blocks, st);
-    default: return launch_axis_p<R, 16>(mode, quirk, a, axis, blocks, st);
-  }
+NdArgs<R> nd_args(const espec_spond_plan* p, const NdConfig& c) {
+  NdArgs<R> a{};
+  for (int ax = 0; ax < 3; ++ax) a.ln[ax] = c.layout.ln[ax];
+  a.ndim = p->ndim;
+  a.n = p->n;
+  a.fused = c.fused;
+  a.lc = c.lc;
+  a.psi0 = p->d_psi0;
+  a.bar = p->d_bar;
+  a.err = (int*)(p->d_bar + 1);
+  a.spin_limit = grid_wait_limit();
+  return a;
+}
+
+template <typename R>
+int nd_launch(espec_spond_plan* p, const NdConfig& c, NdArgs<R>& a, cudaStream_t st) {
+  // the arrival count; a diagnostic transform keeps the last run's error flag,
+  // so that it fails too
+  ND_CK(cudaMemsetAsync(p->d_bar, 0, (a.op == kOpForward ? 1 : 2) * sizeof(unsigned long long),
+                        st));
+  if (c.threads == 256) return nd_launch_as<R, 256, 9>(c, a, st);
+  return nd_launch_as<R, 512, kMaxLn512<R>>(c, a, st);
 }
 
 template <typename R>
 int run_steps(espec_spond_plan* p, int nsteps, bool from_start, cudaStream_t st) {
-  NdArgs<R> a{};
-  a.nx = p->np[0];
-  a.ny = p->np[1];
-  a.nz = p->ndim > 2 ? p->np[2] : 1;
-  a.ndim = p->ndim;
-  a.psi = (cpx<R>*)p->d_psi;
-  a.psi0 = p->d_psi0;
-  a.psi_out = p->d_out;
-  a.psi_start = from_start ? nullptr : p->d_out;
+  const NdConfig c = nd_config<R>(p);
+  NdArgs<R> a = nd_args<R>(p, c);
   const long n = p->n;
   NdTabs<R> tb(p->d_tab, n);
+  a.op = kOpSpo;
+  a.nsteps = nsteps;
+  a.from_start = from_start;
+  a.psi = (cpx<R>*)p->d_psi;
+  a.psi_out = p->d_out;
+  a.psi_start = from_start ? p->d_psi0 : p->d_out;
   a.g = tb.g;
   a.h = tb.h;
   a.hm = tb.hm;
@@ -808,107 +1226,45 @@ int run_steps(espec_spond_plan* p, int nsteps, bool from_start, cudaStream_t st)
   a.kq_s = p->d_kq ? p->d_kq + n : nullptr;
   a.kq_scale = 1.0 / (double)n;
   a.cpart = p->d_cpart;
-  for (int ax = 0; ax < 3; ++ax)
-    a.tw[ax] = (const typename Rot<R>::type*)(ax < p->ndim ? p->d_tw[ax] : nullptr);
-  const bool quirk = (p->quirks & ESPEC_Q_SPO_INPLACE) != 0;
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const int xb = p->xblocks;
-  const long yb = 0, zb = 0;  // grid sizes are chosen by the launchers
-  cudaError_t e = cudaSuccess;
-  auto kin_step = [&]() {
-    if (p->ndim == 2) {
-      e = launch_axis<R>(ny, kKin, quirk, a, 1, yb, st);
-    } else {
-      e = launch_axis<R>(ny, kFwd, false, a, 1, yb, st);
-      if (e == cudaSuccess) e = launch_axis<R>(nz, kKin, quirk, a, 2, zb, st);
-      if (e == cudaSuccess) e = launch_axis<R>(ny, kInv, false, a, 1, yb, st);
-    }
-  };
-  if (nsteps == 0) {
-    if (from_start) {
-      a.step = 0;
-      e = launch_x_n<R>(nx, kFirst, a, xb, st);  // C(0); the state is left in k layout
-      if (e != cudaSuccess) return set_cuda_error("x pass", e);
-      // psi(TF) = psi(0)
-      ND_CK(cudaMemcpyAsync(p->d_out, p->d_psi0, 16 * n, cudaMemcpyDeviceToDevice, st));
-    }
-    return ESPEC_OK;
-  }
-  for (int s = 0; s <= nsteps; ++s) {
-    a.step = s;
-    const int mode = s == 0 ? kFirst : (s == nsteps ? kLast : kMid);
-    e = launch_x_n<R>(nx, mode, a, xb, st);
-    if (e != cudaSuccess) return set_cuda_error("x pass", e);
-    if (s < nsteps) {
-      kin_step();
-      if (e != cudaSuccess) return set_cuda_error("axis pass", e);
-    }
-  }
-  return ESPEC_OK;
+  for (int ax = 0; ax < p->ndim; ++ax) a.tw[ax] = (const typename Rot<R>::type*)p->d_tw[ax];
+  if (nsteps == 0)  // psi(TF) = psi(0)
+    ND_CK(cudaMemcpyAsync(p->d_out, p->d_psi0, 16 * n, cudaMemcpyDeviceToDevice, st));
+  return nd_launch<R>(p, c, a, st);
 }
 
 // second-order differences on the grid (psodfft.f:77-206): start-up of two
 // half steps from psi0 (psodfft.f:120-152), then leapfrog steps; the newest
 // state ends in d_out, the one before in d_prev
 int run_sod(espec_spond_plan* p, int nsteps, bool from_start, cudaStream_t st) {
-  NdArgs<double> a{};
-  a.nx = p->np[0];
-  a.ny = p->np[1];
-  a.nz = p->ndim > 2 ? p->np[2] : 1;
-  a.ndim = p->ndim;
-  a.psi = (cpx<double>*)p->d_psi;  // transform scratch
+  const NdConfig c = nd_config<double>(p);
+  NdArgs<double> a = nd_args<double>(p, c);
   const long n = p->n;
   NdTabs<double> tb(p->d_tab, n);
+  a.op = kOpSod;
+  a.nsteps = nsteps;
+  a.from_start = from_start;
+  a.psi = (cpx<double>*)p->d_psi;  // transform scratch
+  a.psi_start = from_start ? p->d_psi0 : p->d_out;
+  a.cur = p->d_out;
+  a.prev = p->d_prev;
   a.w = tb.w;
   a.K = tb.K;
   a.vc = p->d_sod;
   a.ab = p->d_sod + n;
   a.kabs = sod_kabs(p);
   a.cpart = p->d_cpart;
-  for (int ax = 0; ax < 3; ++ax) a.tw[ax] = ax < p->ndim ? (const RotD*)p->d_tw[ax] : nullptr;
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  cudaError_t e = cudaSuccess;
-  auto op = [&](const double2* src, double2* dst, double f, int step) {
-    a.step = step;
-    a.psi_start = src;
-    e = launch_x_n<double>(nx, kFwd0, a, 0, st);
-    if (e != cudaSuccess) return;
-    if (p->ndim == 2) {
-      e = launch_axis<double>(ny, kKin, false, a, 1, 0, st);
-    } else {
-      e = launch_axis<double>(ny, kFwd, false, a, 1, 0, st);
-      if (e == cudaSuccess) e = launch_axis<double>(nz, kKin, false, a, 2, 0, st);
-      if (e == cudaSuccess) e = launch_axis<double>(ny, kInv, false, a, 1, 0, st);
-    }
-    if (e != cudaSuccess) return;
-    a.sod_src = src;
-    a.sod_dst = dst;
-    a.f = f;
-    e = launch_x_n<double>(nx, kSodUpd, a, 0, st);
-  };
-  double2* cur = p->d_out;
-  double2* prev = p->d_prev;
-  int s0 = 1;
-  if (from_start) {
-    ND_CK(cudaMemcpyAsync(cur, p->d_psi0, 16 * n, cudaMemcpyDeviceToDevice, st));
-    ND_CK(cudaMemcpyAsync(prev, p->d_psi0, 16 * n, cudaMemcpyDeviceToDevice, st));
-    c0_kernel<<<p->xblocks, 256, 0, st>>>(p->d_psi0, n, p->d_cpart);
-    ND_CK(cudaGetLastError());
-    if (nsteps >= 1) {
-      op(cur, prev, 0.5, 1);  // prev = psi0 - i/2 H psi0
-      if (e == cudaSuccess) op(prev, cur, 0.5, 1);  // cur = psi0 - i/2 H prev = psi(dt)
-      if (e != cudaSuccess) return set_cuda_error("SOD start-up", e);
-      ND_CK(cudaMemcpyAsync(prev, p->d_psi0, 16 * n, cudaMemcpyDeviceToDevice, st));
-    }
-    s0 = 2;
+  for (int ax = 0; ax < p->ndim; ++ax) a.tw[ax] = (const RotD*)p->d_tw[ax];
+  if (from_start && nsteps == 0) {
+    ND_CK(cudaMemcpyAsync(p->d_out, p->d_psi0, 16 * n, cudaMemcpyDeviceToDevice, st));
+    ND_CK(cudaMemcpyAsync(p->d_prev, p->d_psi0, 16 * n, cudaMemcpyDeviceToDevice, st));
   }
-  for (int s = s0; s <= nsteps; ++s) {
-    op(cur, prev, 1.0, s);
-    if (e != cudaSuccess) return set_cuda_error("SOD step", e);
-    std::swap(cur, prev);
-  }
-  p->d_out = cur;
-  p->d_prev = prev;
+  const int rc = nd_launch<double>(p, c, a, st);
+  if (rc) return rc;
+  if (from_start && nsteps == 1)  // the start-up's half-step state is no psi(t - dt)
+    ND_CK(cudaMemcpyAsync(p->d_prev, p->d_psi0, 16 * n, cudaMemcpyDeviceToDevice, st));
+  // update u writes d_prev for even u, d_out for odd u
+  const int updates = nsteps + (from_start && nsteps > 0 ? 1 : 0);
+  if (updates % 2 == 1) std::swap(p->d_out, p->d_prev);
   return ESPEC_OK;
 }
 
@@ -969,10 +1325,12 @@ extern "C" int espec_spond_create_method(espec_spond_plan** out, int method, int
   p->precision = precision;
   p->absorb = absorb;
   p->quirks = quirks;
-  {
-    const long rows = p->n / np[0];
-    const int w = warps_for(rows);
-    p->xblocks = (int)((rows + w - 1) / w);  // the x pass's grid (C(t) partials per step)
+  int dev = 0;
+  cudaError_t de = cudaGetDevice(&dev);
+  if (de == cudaSuccess) de = cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (de != cudaSuccess) {
+    delete p;
+    return set_cuda_error("device query", de);
   }
   const size_t n = (size_t)p->n;
   const size_t cb = precision == ESPEC_FP64 ? 16 : 8;
@@ -980,7 +1338,7 @@ extern "C" int espec_spond_create_method(espec_spond_plan** out, int method, int
   auto fail = [&](int code) {
     void* b[] = {p->d_psi,   p->d_psi0,  p->d_out,   p->d_vpot,  p->d_vabc, p->d_tab,
                  p->d_kq,    p->d_cpart, p->d_c,     p->d_tw[0], p->d_tw[1], p->d_tw[2],
-                 p->d_prev,  p->d_sod};
+                 p->d_prev,  p->d_sod,   p->d_tax,   p->d_bar};
     for (void* x : b)
       if (x) cudaFree(x);
     delete p;
@@ -1000,6 +1358,12 @@ extern "C" int espec_spond_create_method(espec_spond_plan** out, int method, int
     if ((rc = ck(cudaMalloc(&p->d_prev, 16 * n), "cudaMalloc"))) return fail(rc);
     if ((rc = ck(cudaMalloc(&p->d_sod, 16 * n), "cudaMalloc"))) return fail(rc);
   }
+  size_t tax = 0;
+  for (int ax = 0; ax < ndim; ++ax) tax += np[ax];
+  if ((rc = ck(cudaMalloc(&p->d_tax, 8 * tax), "cudaMalloc"))) return fail(rc);
+  if ((rc = ck(cudaMalloc(&p->d_bar, 2 * sizeof(unsigned long long)), "cudaMalloc"))) return fail(rc);
+  if ((rc = ck(cudaMemset(p->d_bar, 0, 2 * sizeof(unsigned long long)), "cudaMemset")))
+    return fail(rc);
   for (int ax = 0; ax < ndim; ++ax)
     if ((rc = ck(cudaMalloc(&p->d_tw[ax], sizeof(RotD) * np[ax]), "cudaMalloc"))) return fail(rc);
   *out = p;
@@ -1041,16 +1405,12 @@ extern "C" int espec_spond_load(espec_spond_plan* p, const double* vpot, const d
                                             : build_tables<float>(p, st);
   if (rc) return rc;
   p->has_state = false;
-  for (int ax = 0; ax < p->ndim; ++ax) {
-    const int nl = p->np[ax];
-    if (p->precision == ESPEC_FP64)
-      tw_table_kernel<double><<<(nl + 255) / 256, 256, 0, st>>>((RotD*)p->d_tw[ax], nl);
-    else
-      tw_table_kernel<float><<<(nl + 255) / 256, 256, 0, st>>>((RotF*)p->d_tw[ax], nl);
-    ND_CK(cudaGetLastError());
-  }
   p->loaded = true;
   return ESPEC_OK;
+}
+
+static int nd_grid(const espec_spond_plan* p) {
+  return p->precision == ESPEC_FP64 ? nd_config<double>(p).grid : nd_config<float>(p).grid;
 }
 
 extern "C" int espec_spond_run(espec_spond_plan* p, int nsteps, void* stream) {
@@ -1063,7 +1423,7 @@ extern "C" int espec_spond_run(espec_spond_plan* p, int nsteps, void* stream) {
     p->d_c = nullptr;
     p->d_cpart = nullptr;
     ND_CK(cudaMalloc(&p->d_c, sizeof(double2) * ((size_t)nsteps + 1)));
-    ND_CK(cudaMalloc(&p->d_cpart, sizeof(double2) * ((size_t)nsteps + 1) * p->xblocks));
+    ND_CK(cudaMalloc(&p->d_cpart, sizeof(double2) * ((size_t)nsteps + 1) * nd_grid(p)));
     p->c_cap = nsteps;
   }
   const int rc = p->method == ESPEC_SOD
@@ -1071,8 +1431,8 @@ extern "C" int espec_spond_run(espec_spond_plan* p, int nsteps, void* stream) {
                      : (p->precision == ESPEC_FP64 ? run_steps<double>(p, nsteps, true, st)
                                                    : run_steps<float>(p, nsteps, true, st));
   if (rc) return rc;
-  csum_kernel<<<(nsteps + 1 + 255) / 256, 256, 0, st>>>(p->d_cpart, p->xblocks, nsteps, 0,
-                                                         p->d_c);
+  csum_kernel<<<(nsteps + 1 + 7) / 8, 256, 0, st>>>(p->d_cpart, nd_grid(p), nsteps, 0, p->d_c,
+                                                     (const int*)(p->d_bar + 1));
   ND_CK(cudaGetLastError());
   p->has_state = true;
   return ESPEC_OK;
@@ -1088,7 +1448,7 @@ extern "C" int espec_spond_continue(espec_spond_plan* p, int nsteps, void* strea
     p->d_c = nullptr;
     p->d_cpart = nullptr;
     ND_CK(cudaMalloc(&p->d_c, sizeof(double2) * ((size_t)nsteps + 1)));
-    ND_CK(cudaMalloc(&p->d_cpart, sizeof(double2) * ((size_t)nsteps + 1) * p->xblocks));
+    ND_CK(cudaMalloc(&p->d_cpart, sizeof(double2) * ((size_t)nsteps + 1) * nd_grid(p)));
     p->c_cap = nsteps;
   }
   if (nsteps == 0) return ESPEC_OK;
@@ -1097,28 +1457,9 @@ extern "C" int espec_spond_continue(espec_spond_plan* p, int nsteps, void* strea
                      : (p->precision == ESPEC_FP64 ? run_steps<double>(p, nsteps, false, st)
                                                    : run_steps<float>(p, nsteps, false, st));
   if (rc) return rc;
-  csum_kernel<<<(nsteps + 255) / 256, 256, 0, st>>>(p->d_cpart, p->xblocks, nsteps, 1, p->d_c);
+  csum_kernel<<<(nsteps + 7) / 8, 256, 0, st>>>(p->d_cpart, nd_grid(p), nsteps, 1, p->d_c,
+                                                 (const int*)(p->d_bar + 1));
   ND_CK(cudaGetLastError());
-  return ESPEC_OK;
-}
-
-// TC of the diagnostic transform's storage order (all axes permuted)
-static int nd_energy_tables(espec_spond_plan* p) {
-  std::vector<double> tc;
-  digt_nd(p, tc);
-  const int nx = p->np[0], ny = p->np[1], nz = p->ndim > 2 ? p->np[2] : 1;
-  std::vector<double> tcp((size_t)p->n);
-  for (int k = 0; k < nz; ++k) {
-    const int fz = p->ndim > 2 ? (nz - freq_of(k, nz)) % nz : 0;
-    for (int j = 0; j < ny; ++j) {
-      const int fy = (ny - freq_of(j, ny)) % ny;
-      for (int i = 0; i < nx; ++i) {
-        const int fx = (nx - freq_of(i, nx)) % nx;
-        tcp[i + (size_t)nx * (j + (size_t)ny * k)] = tc[fx + (size_t)nx * (fy + (size_t)ny * fz)];
-      }
-    }
-  }
-  ND_CK(cudaMemcpy(p->d_tcp, tcp.data(), 8 * tcp.size(), cudaMemcpyHostToDevice));
   return ESPEC_OK;
 }
 
@@ -1137,26 +1478,25 @@ extern "C" int espec_spond_energies(espec_spond_plan* p, double* e, double* norm
       tw_table_kernel<double><<<(p->np[ax] + 255) / 256, 256, 0, st>>>(p->d_tw64[ax], p->np[ax]);
       ND_CK(cudaGetLastError());
     }
-    const int rc = nd_energy_tables(p);
+    const int rc = upload_axis_tables(p, st);
     if (rc) return rc;
+    // TC in the storage order of the FP64 transform
+    nd_tc_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+        nd_config<double>(p).layout, n, p->d_tax, (p->quirks & ESPEC_Q_DIGT_ND) != 0, p->d_tcp);
+    ND_CK(cudaGetLastError());
+    ND_CK(cudaStreamSynchronize(st));  // later calls may come on other streams
   }
-  NdArgs<double> a{};
-  a.nx = p->np[0];
-  a.ny = p->np[1];
-  a.nz = p->ndim > 2 ? p->np[2] : 1;
-  a.ndim = p->ndim;
+  const NdConfig c = nd_config<double>(p);
+  NdArgs<double> a = nd_args<double>(p, c);
+  a.op = kOpForward;
   a.psi = p->d_khat;
   a.psi_start = p->has_state ? p->d_out : p->d_psi0;
-  for (int ax = 0; ax < 3; ++ax) a.tw[ax] = ax < p->ndim ? p->d_tw64[ax] : nullptr;
-  cudaError_t err = launch_x_n<double>(a.nx, kFwd0, a, p->xblocks, st);
-  if (err == cudaSuccess)
-    err = launch_axis<double>(a.ny, kFwd, false, a, 1, 0, st);
-  if (err == cudaSuccess && p->ndim > 2)
-    err = launch_axis<double>(a.nz, kFwd, false, a, 2, 0, st);
-  if (err != cudaSuccess) return set_cuda_error("energy transform", err);
+  for (int ax = 0; ax < p->ndim; ++ax) a.tw[ax] = p->d_tw64[ax];
+  const int rl = nd_launch<double>(p, c, a, st);
+  if (rl) return rl;
   nd_energy_kernel<<<nb, 256, 0, st>>>(a.psi_start, p->d_vpot, p->d_khat, p->d_tcp, n,
                                        1.0 / (double)n, p->d_epart);
-  csum_kernel<<<1, 1, 0, st>>>(p->d_epart, nb, 0, 0, p->d_epart + nb);
+  csum_kernel<<<1, 32, 0, st>>>(p->d_epart, nb, 0, 0, p->d_epart + nb, a.err);
   ND_CK(cudaGetLastError());
   double2 h;
   ND_CK(cudaMemcpyAsync(&h, p->d_epart + nb, sizeof h, cudaMemcpyDeviceToHost, st));
@@ -1174,7 +1514,12 @@ extern "C" int espec_spond_results(espec_spond_plan* p, double* c_re, double* c_
   int rc = get_complex(p->stage, p->d_c, c_re, c_im, nc, where, st);
   if (rc == ESPEC_OK) rc = get_complex(p->stage, p->d_out, psi_re, psi_im, n, where, st);
   if (rc) return rc;
-  if (where == ESPEC_MEM_HOST) ND_CK(cudaStreamSynchronize(st));
+  if (where == ESPEC_MEM_HOST) {
+    int err = 0;
+    ND_CK(cudaMemcpyAsync(&err, p->d_bar + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ND_CK(cudaStreamSynchronize(st));
+    if (err) return set_error(ESPEC_ECUDA, "a grid barrier of the split-operator kernel timed out");
+  }
   return ESPEC_OK;
 }
 
@@ -1183,7 +1528,7 @@ extern "C" void espec_spond_destroy(espec_spond_plan* p) {
   void* b[] = {p->d_psi,    p->d_psi0,  p->d_out,   p->d_vpot,  p->d_vabc,   p->d_tab,
                p->d_kq,     p->d_cpart, p->d_c,     p->d_tw[0], p->d_tw[1],  p->d_tw[2],
                p->d_khat,   p->d_tcp,   p->d_epart, p->d_tw64[0], p->d_tw64[1], p->d_tw64[2],
-               p->d_prev,   p->d_sod};
+               p->d_prev,   p->d_sod,   p->d_tax,    p->d_bar};
   for (void* x : b)
     if (x) cudaFree(x);
   p->stage.release();
