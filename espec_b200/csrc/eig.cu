@@ -26,7 +26,13 @@
 namespace espec {
 namespace {
 
-constexpr int kEigThreads = 1024;  // 32 warps: enough loads in flight per SM
+// 16 warps of up to 128 registers: a thread keeps 16 to 32 loads in flight
+constexpr int kEigThreads = 512;
+// CTA sums run over kEigChains accumulation chains (chain u: points u, u +
+// kEigChains, ...), each thread two of them, chains added in warps of 32
+constexpr int kEigChains = 1024;
+// points of a current vector kept in shared memory (beside 31 KB of static arrays)
+constexpr int kEigMaxSmemN = 24 * 1024;
 constexpr int kEigMaxM = 40;      // NREORT = 40 in lanczsc.f:55
 constexpr int kEigMaxStates = 16;  // locked states held in the reorthogonalisation
 
@@ -36,7 +42,7 @@ struct EigArgs {
   const double* vpot;   // [nprob][n]
   const double* start;  // [nprob][nstates][n]
   double* L;            // [nprob][m][n]
-  double* work;         // [nprob][n]
+  double* work;         // [nprob][n]: H vi - bt v_prev of an iteration
   double* vec;          // [nprob][nstates][n]
   double* eval;         // [nprob][nstates]
   double* resid;        // [nprob][nstates]
@@ -63,72 +69,102 @@ __device__ __forceinline__ double hx(const EigArgs& a, const double* V, const do
   return s;
 }
 
-// CTA sum of cnt per-thread values (acc[0..cnt)) into out[0..cnt)
-template <int MAXV>
-__device__ __forceinline__ void cta_sums(const double (&acc)[MAXV], int cnt, double* ws,
-                                         double* out) {
+// CTA sum of the two chains of every thread (chains t and t + kEigThreads)
+__device__ __forceinline__ double cta_sum(double x0, double x1, double* ws) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    if (i >= cnt) break;
-    double s = acc[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) ws[warp * MAXV + i] = s;
+  for (int o = 16; o > 0; o >>= 1) {
+    x0 += __shfl_xor_sync(0xffffffffu, x0, o);
+    x1 += __shfl_xor_sync(0xffffffffu, x1, o);
+  }
+  if (lane == 0) {
+    ws[warp] = x0;
+    ws[warp + kEigThreads / 32] = x1;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-    double s = 0.0;
-    for (int w = 0; w < kEigThreads / 32; ++w) s += ws[w * MAXV + i];
-    out[i] = s;
-  }
+  double s = 0.0;
+  for (int w = 0; w < kEigChains / 32; ++w) s += ws[w];
   __syncthreads();
+  return s;
 }
 
-// as cta_sums for the slots [0, e1) and [b2, e2) of acc only
-template <int MAXV>
-__device__ __forceinline__ void cta_sums2(const double (&acc)[MAXV], int e1, int b2, int e2,
-                                          double* ws, double* out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    if (!(i < e1 || (i >= b2 && i < e2))) continue;  // uniform over the CTA
-    double s = acc[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) ws[warp * MAXV + i] = s;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < MAXV; i += blockDim.x) {
-    if (!(i < e1 || (i >= b2 && i < e2))) continue;
-    double s = 0.0;
-    for (int w = 0; w < kEigThreads / 32; ++w) s += ws[w * MAXV + i];
-    out[i] = s;
-  }
-  __syncthreads();
-}
-
-// red[q] = <x, Y_q>, q < nl + nlock, with Y_q = L_q (q < nl) or lock_(q-nl):
-// one warp per vector, lanes striding the points (coalesced streams, one per
-// warp); x is read from L1/L2 by every warp
+// red[q] = <x, Y_q>, q < nl + nlock, with Y_q = L_q (q < nl) or lock_(q-nl).
+// Each product is two accumulation chains per lane (points lane + 64 i and
+// lane + 32 + 64 i); a warp takes one chain set of one vector at a time, so
+// that even the first iterations of a restart keep every warp loading, with
+// kDotLoads loads of the vector in flight per lane (with two, one CTA drew
+// about 20 GB/s).  part: [2 (kEigMaxM + kEigMaxStates)][32] in shared memory.
+constexpr int kDotLoads = 32;
 __device__ __forceinline__ void warp_dots(const double* x, const double* L, int nl,
-                                          const double* lock, int nlock, int n, double* red) {
+                                          const double* lock, int nlock, int n, double* part,
+                                          double* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int q = warp; q < nl + nlock; q += kEigThreads / 32) {
+  const int nv = nl + nlock;
+  for (int task = warp; task < 2 * nv; task += kEigThreads / 32) {
+    const int q = task >> 1;
     const double* y = q < nl ? L + (long)q * n : lock + (long)(q - nl) * n;
-    double s0 = 0.0, s1 = 0.0;
-    int k = lane;
-    for (; k + 32 < n; k += 64) {
-      s0 += x[k] * y[k];
-      s1 += x[k + 32] * y[k + 32];
+    double s = 0.0;
+    int k = lane + 32 * (task & 1);
+    for (; k + 64 * (kDotLoads - 1) < n; k += 64 * kDotLoads) {
+      double v[kDotLoads];
+#pragma unroll
+      for (int j = 0; j < kDotLoads; ++j) v[j] = __ldcg(y + k + 64 * j);
+#pragma unroll
+      for (int j = 0; j < kDotLoads; ++j) s += x[k + 64 * j] * v[j];
     }
-    for (; k < n; k += 32) s0 += x[k] * y[k];
-    double s = s0 + s1;
+    for (; k < n; k += 64) s += x[k] * __ldcg(y + k);
+    part[task * 32 + lane] = s;
+  }
+  __syncthreads();
+  for (int q = warp; q < nv; q += kEigThreads / 32) {
+    double s = part[2 * q * 32 + lane] + part[(2 * q + 1) * 32 + lane];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) red[q] = s;
   }
   __syncthreads();
+}
+
+// w[i] = init(k_i) - sum_j lock_j(k_i) a_j - sum_q L_q(k_i) b_q (sgn = -1), or
+// + (sgn = 1), for the thread's points k_i = t + i kEigThreads, four at a time so
+// that their loads overlap; put(k, w) takes each, in order
+template <class Init, class Put>
+__device__ __forceinline__ void combine(const double* lock, const double* ca, int nlock,
+                                        const double* L, const double* cb, int nl, int n,
+                                        bool plus, Init init, Put put) {
+  constexpr int P = 4;
+  for (int k0 = threadIdx.x; k0 < n; k0 += P * kEigThreads) {
+    double w[P];
+    int kk[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      kk[i] = min(k0 + i * kEigThreads, n - 1);
+      w[i] = init(kk[i]);
+    }
+    for (int j = 0; j < nlock; ++j) {
+      const double c = ca[j];
+#pragma unroll
+      for (int i = 0; i < P; ++i) w[i] -= c * __ldcg(lock + (long)j * n + kk[i]);
+    }
+    if (plus) {
+#pragma unroll 4
+      for (int q = 0; q < nl; ++q) {
+        const double c = cb[q];
+#pragma unroll
+        for (int i = 0; i < P; ++i) w[i] += c * __ldcg(L + (long)q * n + kk[i]);
+      }
+    } else {
+#pragma unroll 4
+      for (int q = 0; q < nl; ++q) {
+        const double c = cb[q];
+#pragma unroll
+        for (int i = 0; i < P; ++i) w[i] -= c * __ldcg(L + (long)q * n + kk[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+      if (k0 + i * kEigThreads < n) put(k0 + i * kEigThreads, i & 1, w[i]);
+  }
 }
 
 // number of eigenvalues of the tridiagonal (d, e) below x (Sturm count)
@@ -187,94 +223,93 @@ __host__ __device__ inline void tri_solve_pivoted(int m, const double* al, const
 
 }  // namespace
 
+// SM: the current vector in shared memory (grids up to kEigMaxSmemN points);
+// otherwise it is the work array in global memory
+template <bool SM>
 __global__ void __launch_bounds__(kEigThreads) eig_kernel(EigArgs a) {
   constexpr int NV = kEigMaxM + kEigMaxStates;
-  __shared__ double ws[(kEigThreads / 32) * NV];
+  extern __shared__ double eig_dyn[];
+  __shared__ double part[2 * NV * 32];
+  __shared__ double ws[kEigChains / 32];
   __shared__ double red[NV];
-  __shared__ double s_lk[kEigMaxStates];
   __shared__ double s_al[kEigMaxM], s_bt[kEigMaxM], s_e2[kEigMaxM], s_y[kEigMaxM];
-  __shared__ double s_r[kEigMaxM];
-  __shared__ double s_theta, s_bt0;
+  __shared__ double s_theta;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int p = blockIdx.x, n = a.n, m = a.m;
   const double* V = a.vpot + (long)p * n;
   double* L = a.L + (long)p * m * n;
   double* work = a.work + (long)p * n;
+  double* F = SM ? eig_dyn : work;  // the current vector
 
   for (int K = 0; K < a.nstates; ++K) {
     const double* st = a.start + ((long)p * a.nstates + K) * n;
-    double* v = a.vec + ((long)p * a.nstates + K) * n;  // the current vector
-    for (int k = t; k < n; k += kEigThreads) v[k] = st[k];
+    double* v = a.vec + ((long)p * a.nstates + K) * n;
+    for (int k = t; k < n; k += kEigThreads) F[k] = st[k];
     __syncthreads();
     int count = 0;
     double res = 0.0;
     const double* lock = a.vec + (long)p * a.nstates * n;  // states 0..K-1
     for (int rs = 0; rs < a.maxrest; ++rs) {
-      // ---- project the locked states out of v
+      // ---- project the locked states out of the current vector
       if (K > 0) {
-        warp_dots(v, nullptr, 0, lock, K, n, red);
-        for (int k = t; k < n; k += kEigThreads) {
-          double vk = v[k];
-          for (int j = 0; j < K; ++j) vk -= red[j] * lock[(long)j * n + k];
-          v[k] = vk;
-        }
+        warp_dots(F, nullptr, 0, lock, K, n, part, red);
+        combine(lock, red, K, nullptr, nullptr, 0, n, false, [&](int k) { return F[k]; },
+                [&](int k, int, double w) { F[k] = w; });
         __syncthreads();
       }
-      // ---- m Lanczos steps from v (lnz.f:76-119)
-      {
-        double acc[1] = {0.0};
-        for (int k = t; k < n; k += kEigThreads) acc[0] += v[k] * v[k];
-        cta_sums<1>(acc, 1, ws, red);
-        if (t == 0) s_bt0 = sqrt(red[0]);
-        __syncthreads();
+      // ---- m Lanczos steps (lnz.f:76-119)
+      double nn[2] = {0.0, 0.0};
+      for (int k = t, c = 0; k < n; k += kEigThreads, c ^= 1) {
+        if (c) nn[1] += F[k] * F[k];
+        else nn[0] += F[k] * F[k];
       }
+      double bt0 = sqrt(cta_sum(nn[0], nn[1], ws));
       for (int it = 0; it < m; ++it) {
-        const double bt0 = s_bt0;
-        const double* src = it == 0 ? v : work;
         double* Li = L + (long)it * n;
-        for (int k = t; k < n; k += kEigThreads) Li[k] = src[k] / bt0;
+        const double* Lp = it ? L + (long)(it - 1) * n : nullptr;
+#pragma unroll 4
+        for (int k = t; k < n; k += kEigThreads) {
+          const double vi = F[k] / bt0;
+          Li[k] = vi;
+          if (SM) F[k] = vi;
+        }
         __syncthreads();
         // w = H vi - bt0 v_prev into work, al = <vi, w> (lnz.f:96-107)
-        {
-          double acc[1] = {0.0};
-          for (int k = t; k < n; k += kEigThreads) {
-            const double vp = it ? L[(long)(it - 1) * n + k] : 0.0;
-            const double w = hx(a, V, Li, k, 1.0) - bt0 * vp;
-            work[k] = w;
-            acc[0] += Li[k] * w;
+        const double* x = SM ? F : Li;
+        nn[0] = nn[1] = 0.0;
+#pragma unroll 2
+        for (int k0 = t; k0 < n; k0 += kEigChains) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int k = k0 + c * kEigThreads;
+            if (k < n) {
+              const double vp = it ? Lp[k] : 0.0;
+              const double w = hx(a, V, x, k, 1.0) - bt0 * vp;
+              work[k] = w;
+              nn[c] += x[k] * w;
+            }
           }
-          cta_sums<1>(acc, 1, ws, red);
-          if (t == 0) s_al[it] = red[0];
-          __syncthreads();
         }
+        const double al = cta_sum(nn[0], nn[1], ws);
+        if (t == 0) s_al[it] = al;
         ++count;
         // work = w - al vi, then classical Gram-Schmidt against the locked
         // states and L_0..L_it (reort.f:65-80: all dot products, then all
         // updates): one pass for the dots, one for the updates and the norm
-        const double al = s_al[it];
-        for (int k = t; k < n; k += kEigThreads) work[k] = work[k] - al * Li[k];
+#pragma unroll 4
+        for (int k = t; k < n; k += kEigThreads) F[k] = work[k] - al * x[k];
         __syncthreads();
-        warp_dots(work, L, it + 1, lock, K, n, red);
-        if (t == 0) {
-          for (int q = 0; q <= it; ++q) s_r[q] = red[q];
-          for (int j = 0; j < K; ++j) s_lk[j] = red[it + 1 + j];
-        }
-        __syncthreads();
-        double nn[1] = {0.0};
-        for (int k = t; k < n; k += kEigThreads) {
-          double w = work[k];
-          for (int j = 0; j < K; ++j) w -= s_lk[j] * lock[(long)j * n + k];
-          for (int q = 0; q <= it; ++q) w -= s_r[q] * L[(long)q * n + k];
-          work[k] = w;
-          nn[0] += w * w;
-        }
-        cta_sums<1>(nn, 1, ws, red);
-        if (t == 0) {
-          s_bt[it] = sqrt(red[0]);
-          s_bt0 = s_bt[it];
-        }
-        __syncthreads();
+        warp_dots(F, L, it + 1, lock, K, n, part, red);
+        nn[0] = nn[1] = 0.0;
+        combine(lock, red + it + 1, K, L, red, it + 1, n, false, [&](int k) { return F[k]; },
+                [&](int k, int c, double w) {
+                  F[k] = w;
+                  nn[c] += w * w;
+                });
+        bt0 = sqrt(cta_sum(nn[0], nn[1], ws));
+        if (t == 0) s_bt[it] = bt0;
       }
+      __syncthreads();
       // ---- lowest Ritz pair of T (DSTEVX('V','I',...,IL,IU))
       if (warp == 0) {
         if (lane == 0) {
@@ -320,34 +355,29 @@ __global__ void __launch_bounds__(kEigThreads) eig_kernel(EigArgs a) {
         }
       }
       __syncthreads();
-      // ---- v = L y, normalised (lanczsc.f:99-113, FATN = ECNORM)
-      {
-        double acc[1] = {0.0};
-        for (int k = t; k < n; k += kEigThreads) {
-          double s = 0.0;
-          for (int j = 0; j < m; ++j) s += s_y[j] * L[(long)j * n + k];
-          v[k] = s;
-          acc[0] += s * s;
-        }
-        cta_sums<1>(acc, 1, ws, red);
-        const double inv = 1.0 / sqrt(red[0]);
-        for (int k = t; k < n; k += kEigThreads) v[k] *= inv;
-        __syncthreads();
-      }
+      // ---- the new vector L y, normalised (lanczsc.f:99-113, FATN = ECNORM)
+      nn[0] = nn[1] = 0.0;
+      combine(nullptr, nullptr, 0, L, s_y, m, n, true, [](int) { return 0.0; },
+              [&](int k, int c, double w) {
+                F[k] = w;
+                nn[c] += w * w;
+              });
+      const double inv = 1.0 / sqrt(cta_sum(nn[0], nn[1], ws));
+      for (int k = t; k < n; k += kEigThreads) F[k] *= inv;
+      __syncthreads();
       // ---- true residual |H v - theta v|
-      {
-        double acc[1] = {0.0};
-        const double th = s_theta;
-        for (int k = t; k < n; k += kEigThreads) {
-          const double r = hx(a, V, v, k, 1.0) - th * v[k];
-          acc[0] += r * r;
-        }
-        ++count;
-        cta_sums<1>(acc, 1, ws, red);
-        res = sqrt(red[0]);
+      const double th = s_theta;
+      nn[0] = nn[1] = 0.0;
+      for (int k = t, c = 0; k < n; k += kEigThreads, c ^= 1) {
+        const double r = hx(a, V, F, k, 1.0) - th * F[k];
+        if (c) nn[1] += r * r;
+        else nn[0] += r * r;
       }
+      ++count;
+      res = sqrt(cta_sum(nn[0], nn[1], ws));
       if (res <= a.tol) break;
     }
+    for (int k = t; k < n; k += kEigThreads) v[k] = F[k];
     if (t == 0) {
       const long o = (long)p * a.nstates + K;
       a.eval[o] = s_theta;
@@ -460,7 +490,13 @@ extern "C" int espec_eig_solve_dev(int nprob, const int* np, const double* shm,
   a.m = m;
   a.maxrest = maxrest;
   a.tol = tol;
-  eig_kernel<<<nprob, kEigThreads, 0, (cudaStream_t)stream>>>(a);
+  if (a.n > kEigMaxSmemN) {
+    eig_kernel<false><<<nprob, kEigThreads, 0, (cudaStream_t)stream>>>(a);
+  } else {
+    static DeviceFlags attr;
+    EIG_CK(set_max_smem_once(attr, eig_kernel<true>, sizeof(double) * kEigMaxSmemN));
+    eig_kernel<true><<<nprob, kEigThreads, sizeof(double) * a.n, (cudaStream_t)stream>>>(a);
+  }
   EIG_CK(cudaGetLastError());
   return ESPEC_OK;
 }
