@@ -16,7 +16,8 @@ SOURCES = ["spo1d.cu", "capi.cu", "spo1d_inst_f32_pow2.cu", "spo1d_inst_f32_r3.c
            "spo1d_inst_f64_pow2.cu", "spo1d_inst_f64_r3.cu", "spo1d_persist.cu", "spo1d_any.cu", "spo_tc.cu", "spo1d_static.cu", "sod1d_inst.cu",
            "diag1d.cu", "dropin.cu", "sil.cu",
            "spectrum.cu", "potential.cu", "eig.cu", "mlp.cu", "mlp_tc.cu",
-           "spond.cu", "deck.cpp", "pulse.cpp"]
+           "spond.cu", "spond_inst_f64_256.cu", "spond_inst_f64_512.cu", "spond_inst_f32_256.cu",
+           "spond_inst_f32_512.cu", "deck.cpp", "pulse.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # per-file flags: the analytic potentials follow the reference's arithmetic
 # (no fused multiply-add), so that they match it to the last bit of exp/cos
