@@ -19,6 +19,7 @@
 #include "spo1d_any.cuh"
 #include "spo1d_launch.cuh"
 #include "spo1d_persist.cuh"
+#include "spo1d_smooth.cuh"
 
 namespace espec {
 
@@ -218,7 +219,15 @@ void spo_tc256_final_freq(int* kap);
 cudaError_t spo_tc256_launch(const SpoArgs<float>& a, int npk, cudaStream_t st);
 int spo_tc_status(int* timed_out);
 
-static void plan_info(int n, int v, std::vector<int>& kap, int& n3) {
+// smooth: the packets run spo1d_smooth.cu (split operator, any size)
+static void plan_info(int n, int v, bool smooth, std::vector<int>& kap, int& n3) {
+  SmoothPlan sp;
+  if (smooth && smooth_plan(n, sp)) {
+    kap.assign(n, 0);
+    smooth_final_freq(sp, kap.data());
+    n3 = 0;
+    return;
+  }
   if (v == ESPEC_VARIANT_TC) {  // n == 256, mixed: no radix-3 stage
     kap.assign(256, 0);
     spo_tc256_final_freq(kap.data());
@@ -234,7 +243,7 @@ static void plan_info(int n, int v, std::vector<int>& kap, int& n3) {
     case 1536: plan_info_n<1536>(v, kap, n3); break;
     case 2048: plan_info_n<2048>(v, kap, n3); break;
     case 4096: plan_info_n<4096>(v, kap, n3); break;
-    default:  // the any-size kernels: natural order
+    default:  // the Stockham kernels of any size: natural order
       kap.resize(n);
       for (int j = 0; j < n; ++j) kap[j] = j;
       n3 = 0;
@@ -308,7 +317,9 @@ struct espec_spo_plan {
     int* d_kfreq;      // FFT index at each final position of the diagnostic FFT
     bool any;          // a size outside the register plans (spo1d_any.cu)
     AnyPlan ap;
-    double2* d_tw;     // its twiddle table
+    double2* d_tw;     // its twiddles e^{2 pi i e/n}, then the smooth stages'
+    bool smooth;       // split operator through spo1d_smooth.cu (prime factors <= 13)
+    SmoothPlan sp;
   };
   bool index_dirty = true;
   std::vector<Class> classes;
@@ -387,6 +398,8 @@ static int spo_index_tables(espec_spo_plan* p) {
   std::vector<double> tc(np), kscale(npk);
   std::vector<int> kperm(np), pk_of(np);
   std::map<int, int> var_of;
+  std::map<int, bool> smooth_of;
+  for (auto& c : p->classes) smooth_of[c.n] = c.smooth;
   const bool persist = p->launch == ESPEC_LAUNCH_PERSISTENT;
   // the reference-defect form always runs DefaultPlan<N> (launch_variant),
   // so its tables take that plan's final layout whatever the class's variant
@@ -402,7 +415,7 @@ static int spo_index_tables(espec_spo_plan* p) {
     if (it == kap_cache.end()) {
       std::vector<int> kap;
       int n3 = 0;
-      plan_info(n, var_of[n], kap, n3);
+      plan_info(n, var_of[n], smooth_of[n], kap, n3);
       it = kap_cache.emplace(n, std::make_pair(kap, n3)).first;
     }
     for (int j = 0; j < n; ++j) {
@@ -490,7 +503,8 @@ extern "C" int espec_prop_create(espec_spo_plan** out, int npk, const int* npts,
   for (auto& kv : cls) {
     espec_spo_plan::Class c{kv.first, (int)kv.second.size(), nullptr,
                             method == ESPEC_SOD ? 0 : default_variant(kv.first, precision),
-                            nullptr, nullptr, !native(kv.first), AnyPlan{}, nullptr};
+                            nullptr, nullptr, !native(kv.first), AnyPlan{}, nullptr, false,
+                            SmoothPlan{}};
     p->classes.push_back(c);  // owned by the plan from here on (freed by plan_free)
     auto& cc = p->classes.back();
     if ((rc = ck(cudaMalloc(&cc.d_pk, sizeof(SpoPacket) * cc.count), "cudaMalloc"))) return fail(rc);
@@ -499,11 +513,13 @@ extern "C" int espec_prop_create(espec_spo_plan** out, int npk, const int* npts,
     if ((rc = ck(cudaMalloc(&cc.d_kfreq, sizeof(int) * cc.n), "cudaMalloc"))) return fail(rc);
     if (cc.any) {
       any_plan(cc.n, cc.ap);
-      std::vector<double2> tw(cc.n);
+      cc.smooth = method == ESPEC_SPO && smooth_plan(cc.n, cc.sp);
+      std::vector<double2> tw(cc.n + (cc.smooth ? cc.sp.ntw : 0));
       any_twiddles(cc.n, tw.data());
-      if ((rc = ck(cudaMalloc(&cc.d_tw, sizeof(double2) * cc.n), "cudaMalloc"))) return fail(rc);
-      if ((rc = ck(cudaMemcpy(cc.d_tw, tw.data(), sizeof(double2) * cc.n, cudaMemcpyHostToDevice),
-                   "H2D")))
+      if (cc.smooth) smooth_twiddles(cc.sp, tw.data(), tw.data() + cc.n);
+      const size_t tb = sizeof(double2) * tw.size();
+      if ((rc = ck(cudaMalloc(&cc.d_tw, tb), "cudaMalloc"))) return fail(rc);
+      if ((rc = ck(cudaMemcpy(cc.d_tw, tw.data(), tb, cudaMemcpyHostToDevice), "H2D")))
         return fail(rc);
     }
     {
@@ -512,7 +528,7 @@ extern "C" int espec_prop_create(espec_spo_plan** out, int npk, const int* npts,
         if (p->n[i] == cc.n) pkd.push_back(SpoPacket{p->off[i], i});
       std::vector<int> kap;
       int n3 = 0;
-      plan_info(cc.n, 0, kap, n3);
+      plan_info(cc.n, 0, false, kap, n3);
       if ((rc = ck(cudaMemcpy(cc.d_pkd, pkd.data(), sizeof(SpoPacket) * pkd.size(),
                               cudaMemcpyHostToDevice), "H2D")))
         return fail(rc);
@@ -867,8 +883,9 @@ static int prop_launch(espec_spo_plan* p, int nsteps, bool resume, cudaStream_t 
       a.kq_scale = 1.0 / c.n;
       a.nsteps = nsteps;
       a.nonfinite = p->d_nonfinite;
-      e = c.any ? spo_any_launch(a, c.ap, c.d_tw, quirk, c.count, cs)
-                : launch_n<double>(c.n, c.variant, a, c.count, quirk, cs);
+      e = c.smooth ? spo_smooth_launch(a, c.sp, c.d_tw + c.n, quirk, c.count, cs)
+          : c.any  ? spo_any_launch(a, c.ap, c.d_tw, quirk, c.count, cs)
+                   : launch_n<double>(c.n, c.variant, a, c.count, quirk, cs);
     } else {
       SpoArgs<float> a{};
       a.tab = p->t32;

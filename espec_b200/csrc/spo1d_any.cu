@@ -1,5 +1,7 @@
 // spo1d_any.cu -- the 1D split-operator, SOD-with-FFT and energy kernels for
 // packet sizes outside the register plans of spo1d.cuh: any even size, FP64.
+// (The split operator of sizes without a prime factor above 13 runs in
+// spo1d_smooth.cu.)
 //
 // eSPec's FFT (fft3d.f, Singleton's mixed-radix transform) takes any N, so
 // its .PFSPO / .PFSOD runs do too.  Here one CTA owns one packet and keeps it
