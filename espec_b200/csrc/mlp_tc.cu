@@ -9,15 +9,21 @@
 // GEMM: C[M,N] (f32) = alpha op(A) op(B) + beta C, A and B bfloat16.  One CTA
 // of 128 threads owns a 128 x BN output tile whose FP32 accumulator lives in
 // tensor memory (TMEM lane = tile row, column = tile column).  K advances in
-// stages of 64: all threads stage the A and B tiles in shared memory as
-// "core matrices" (8 x 16 bytes, no swizzle; K-major or MN-major, whichever
-// keeps the source's 16-byte runs whole) with vector loads, one thread
-// issues four tcgen05.mma (M = 128, N = BN, K = 16, kind::f16 with BF16
-// inputs) and commits them to an mbarrier; the next stage is staged into the
-// other buffer while they run.  The epilogue reads the accumulator with
-// tcgen05.ld (one warp per 32 TMEM lanes).  Every mbarrier wait is bounded:
-// on timeout the kernel records it in a device status word, skips the
-// epilogue and still releases its TMEM.
+// stages of 64 through a ring of four shared-memory buffers: all threads copy the
+// A and B tiles two stages ahead with cp.async (16-byte pieces, zero-filled at the
+// edges) as "core matrices" (8 x 16 bytes, no swizzle; K-major or MN-major,
+// whichever keeps the source's 16-byte runs whole), one thread issues four
+// tcgen05.mma (M = 128, N = BN, K = 16, kind::f16 with BF16 inputs) per stage and
+// commits them to the buffer's mbarrier.  BN is the largest of 256, 128, 64 that
+// gives every SM a tile, else 32: the network's products have few tiles, and what
+// bounds them is the chain of stages.  The epilogue reads the accumulator with
+// tcgen05.ld (one warp per 32 TMEM lanes) and turns it in shared memory so that
+// rows are written 128 bytes at a time, adding the bias and the activation (or
+// its derivative) on the way.  Every mbarrier wait is bounded: on timeout the
+// kernel records it in a device status word, skips the epilogue and still releases
+// its TMEM.
+// 256 x 256 x 4096 (4 tiles of 128 x 128, staged through registers one stage
+// ahead with 8-way bank conflicts, rows written 4 bytes per lane): 248 us before.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -45,7 +51,14 @@ struct TcGemm {
   float* C;
   int ldc;
   int a_vec, b_vec;  // 16-byte loads allowed: ld % 8 == 0 and a 16-byte aligned base
+  // epilogue kBias: C = acc + bias (row), h = bf16(act ? gelu(C) : C);
+  // kGeluBack: C = acc gelu'(z), h = bf16(C)
+  const float* bias;
+  const float* z;
+  uint16_t* h;
+  int act;
 };
+enum { kPlain = 0, kBias = 1, kGeluBack = 2 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -79,52 +92,43 @@ __device__ __forceinline__ uint32_t pack2(uint16_t lo, uint16_t hi) {
 //    matrices, 16-byte row = 8 consecutive k of one row;
 //  * otherwise (element at X[k ld + row]): MN-major core matrices, 16-byte
 //    row = 8 consecutive rows at one k.
-// Either way a 16-byte row is 16 contiguous source bytes, loaded as one
-// vector when vec (aligned, in bounds) and element by element at the edges
-// (rows >= nrows, k >= K read as zero).  Consecutive threads take
-// consecutive 16-byte pieces of the source.
+// Either way a 16-byte row is 16 contiguous source bytes, copied asynchronously
+// when vec (aligned; the part beyond nrows or K is zero-filled), else element by
+// element.  Eight consecutive threads fill one core matrix (128 contiguous bytes
+// of shared memory), a warp four neighbouring ones (64 contiguous source bytes).
 template <int R>
 __device__ __forceinline__ void stage_tile(uint8_t* dst, const uint16_t* X, int ld, bool kcontig,
                                            bool vec, int row0, int nrows, int k0, int K) {
   constexpr int kIter = R * (kBK / 8) / kTcThreads;  // 16-byte pieces per thread
-  uint4 v[kIter];
-  int off[kIter];
-  // all loads first (independent, in flight together), then the stores
 #pragma unroll
   for (int i = 0; i < kIter; ++i) {
-    const int it = threadIdx.x + i * kTcThreads;
+    const int it = threadIdx.x + i * kTcThreads, lo = it & 7, hi = it >> 3;
+    int off, cnt;      // place; elements that exist
+    const uint16_t* src;
     if (kcontig) {
-      const int r = it / (kBK / 8), q = it % (kBK / 8);
-      const int row = row0 + r, kb = k0 + 8 * q;
-      off[i] = q * (R * 16) + (r >> 3) * 128 + (r & 7) * 16;
-      if (vec && row < nrows && kb + 8 <= K) {
-        v[i] = __ldg(reinterpret_cast<const uint4*>(X + (long)row * ld + kb));
-      } else {
-        uint16_t e[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          e[j] = (row < nrows && kb + j < K) ? X[(long)row * ld + kb + j] : (uint16_t)0;
-        v[i] = make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]), pack2(e[4], e[5]),
-                          pack2(e[6], e[7]));
-      }
+      const int q = hi & 7, g = hi >> 3, row = row0 + g * 8 + lo, kb = k0 + 8 * q;
+      off = q * (R * 16) + g * 128 + lo * 16;
+      cnt = row < nrows ? min(max(K - kb, 0), 8) : 0;
+      src = X + (long)row * ld + kb;
     } else {
-      const int g = it % (R / 8), k = it / (R / 8);
-      const int kk = k0 + k, m = row0 + 8 * g;
-      off[i] = (k >> 3) * (R * 16) + g * 128 + (k & 7) * 16;
-      if (vec && kk < K && m + 8 <= nrows) {
-        v[i] = __ldg(reinterpret_cast<const uint4*>(X + (long)kk * ld + m));
-      } else {
-        uint16_t e[8];
+      const int g = hi % (R / 8), kq = hi / (R / 8), kk = k0 + 8 * kq + lo, m = row0 + 8 * g;
+      off = kq * (R * 16) + g * 128 + lo * 16;
+      cnt = kk < K ? min(max(nrows - m, 0), 8) : 0;
+      src = X + (long)kk * ld + m;
+    }
+    if (cnt == 0) src = X;
+    if (vec) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst + off)),
+                   "l"(src), "r"(2 * cnt)
+                   : "memory");
+    } else {
+      uint16_t e[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          e[j] = (kk < K && m + j < nrows) ? X[(long)kk * ld + m + j] : (uint16_t)0;
-        v[i] = make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]), pack2(e[4], e[5]),
-                          pack2(e[6], e[7]));
-      }
+      for (int j = 0; j < 8; ++j) e[j] = j < cnt ? src[j] : (uint16_t)0;
+      *reinterpret_cast<uint4*>(dst + off) =
+          make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]), pack2(e[4], e[5]), pack2(e[6], e[7]));
     }
   }
-#pragma unroll
-  for (int i = 0; i < kIter; ++i) *reinterpret_cast<uint4*>(dst + off[i]) = v[i];
 }
 
 // bounded wait for the completion of the mbarrier phase with this parity
@@ -161,28 +165,56 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-template <int BN>
-constexpr size_t tc_smem_bytes() {
-  return 1024 + 2 * (size_t)(kBM + BN) * kBK * 2 + 64;
+__device__ __forceinline__ uint16_t bf16_bits(float v) {
+  return __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
 
+// GELU(z) = z Phi(z), Phi the standard normal distribution function
+__device__ __forceinline__ float gelu(float z) {
+  return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
+}
+__device__ __forceinline__ float gelu_grad(float z) {
+  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) +
+         z * 0.39894228040143268f * expf(-0.5f * z * z);
+}
+
+constexpr int kRing = 4;   // stage buffers
+constexpr int kAhead = 2;  // stages copied ahead of the one multiplied
+
 template <int BN>
+constexpr size_t tc_smem_bytes() {
+  return 1024 + kRing * (size_t)(kBM + BN) * kBK * 2 + 64;
+}
+
+template <int BN, int EPI>
 __global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
-  static_assert(BN == 128 || BN == 256, "TMEM columns: a power of two, N tile of one MMA");
+  static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256,
+                "TMEM columns: a power of two from 32, N tile of one MMA");
   constexpr int kA = kBM * kBK * 2, kB = BN * kBK * 2;
+  static_assert(kRing * kA >= kTcThreads * 33 * 4, "the epilogue turns tiles in the stage buffers");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA[2] = {base, base + kA};
-  uint8_t* sB[2] = {base + 2 * kA, base + 2 * kA + kB};
-  uint64_t* bar = (uint64_t*)(base + 2 * (kA + kB));
-  uint32_t* tmem_slot = (uint32_t*)(bar + 2);
+  uint8_t* sA = base;
+  uint8_t* sB = base + kRing * kA;
+  uint64_t* bar = (uint64_t*)(base + kRing * (kA + kB));
+  uint32_t* tmem_slot = (uint32_t*)(bar + kRing);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
   const bool a_kc = !g.ta, b_kc = g.tb != 0;
+  const int nk = (g.K + kBK - 1) / kBK;
+  auto stage = [&](int kt) {
+    if (kt < nk) {
+      const int b = kt % kRing;
+      stage_tile<kBM>(sA + b * kA, g.A, g.lda, a_kc, g.a_vec, m0, g.M, kt * kBK, g.K);
+      stage_tile<BN>(sB + b * kB, g.B, g.ldb, b_kc, g.b_vec, n0, g.N, kt * kBK, g.K);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
 
+  for (int kt = 0; kt < kAhead; ++kt) stage(kt);
   if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(bar)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(bar + 1)));
+    for (int b = 0; b < kRing; ++b)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(bar + b)));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 0) {
@@ -191,20 +223,23 @@ __global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
                  "r"(BN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
   }
-  stage_tile<kBM>(sA[0], g.A, g.lda, a_kc, g.a_vec, m0, g.M, 0, g.K);
-  stage_tile<BN>(sB[0], g.B, g.ldb, b_kc, g.b_vec, n0, g.N, 0, g.K);
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const int nk = (g.K + kBK - 1) / kBK;
   const uint32_t idesc = idesc_bf16<BN>(a_kc ? 0u : 1u, b_kc ? 0u : 1u);
   bool ok = true;
   for (int kt = 0; kt < nk; ++kt) {
-    const int b = kt & 1;
+    // buffer (kt + kAhead) % kRing was read by the MMAs of stage kt + kAhead - kRing
+    const int old = kt + kAhead - kRing;
+    if (old >= 0) ok = wait_phase(bar + old % kRing, (old / kRing) & 1) && ok;
+    stage(kt + kAhead);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kAhead) : "memory");
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
     if (threadIdx.x == 0) {
-      const uint32_t a0 = smem_u32(sA[b]), b0 = smem_u32(sB[b]);
+      const int b = kt % kRing;
+      const uint32_t a0 = smem_u32(sA + b * kA), b0 = smem_u32(sB + b * kB);
 #pragma unroll
       for (int j = 0; j < kBK / 16; ++j) {
         const uint64_t da = smem_desc(a0 + j * 2 * (kBM * 16), kBM * 16, 128);
@@ -221,67 +256,58 @@ __global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
               smem_u32(bar + b))
           : "memory");
     }
-    if (kt + 1 < nk) {
-      // the other buffer was read by the MMAs of stage kt - 1
-      if (kt >= 1) ok = wait_phase(bar + (b ^ 1), ((kt - 1) >> 1) & 1) && ok;
-      stage_tile<kBM>(sA[b ^ 1], g.A, g.lda, a_kc, g.a_vec, m0, g.M, (kt + 1) * kBK, g.K);
-      stage_tile<BN>(sB[b ^ 1], g.B, g.ldb, b_kc, g.b_vec, n0, g.N, (kt + 1) * kBK, g.K);
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-      __syncthreads();
-      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    }
   }
-  // the last two commits (every earlier one was waited for above)
-  if (nk >= 2) ok = wait_phase(bar + ((nk - 2) & 1), ((nk - 2) >> 1) & 1) && ok;
-  if (nk >= 1) ok = wait_phase(bar + ((nk - 1) & 1), ((nk - 1) >> 1) & 1) && ok;
+  // the commits not waited for above: the last kRing - kAhead stages
+  for (int kt = max(0, nk - (kRing - kAhead)); kt < nk; ++kt)
+    ok = wait_phase(bar + kt % kRing, (kt / kRing) & 1) && ok;
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   ok = __syncthreads_and(ok) != 0;
-  if (ok && nk >= 1) {
-    const int row = m0 + warp * 32 + lane;
-    float* crow = g.C + (long)row * g.ldc;
+  if (ok) {
+    // 32 columns at a time: each warp's 32 x 32 piece through shared memory
+    float* turn = reinterpret_cast<float*>(base) + warp * (32 * 33);
+    const int row0 = m0 + warp * 32;
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 32) {
       uint32_t r[32];
-      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
-      if (row < g.M) {
+      if (nk > 0) {
+        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
+      } else {  // empty sum
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int n = n0 + c0 + j;
-          if (n < g.N) {
-            float v = g.alpha * __uint_as_float(r[j]);
-            if (g.beta != 0.0f) v = fmaf(g.beta, crow[n], v);
-            crow[n] = v;
+        for (int j = 0; j < 32; ++j) r[j] = 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = __uint_as_float(r[j]);
+      __syncwarp();
+      const int n = n0 + c0 + lane;
+      const float bias = EPI == kBias && n < g.N ? g.bias[n] : 0.0f;
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i) {
+        const int row = row0 + i;
+        if (row < g.M && n < g.N) {
+          const long o = (long)row * g.ldc + n;
+          float v = turn[i * 33 + lane];
+          if (EPI == kPlain) {
+            v = g.alpha * v;
+            if (g.beta != 0.0f) v = nk > 0 ? fmaf(g.beta, g.C[o], v) : g.beta * g.C[o];
+            else if (nk == 0) v = 0.0f;
+          } else if (EPI == kBias) {
+            v = v + bias;
+            if (g.h) g.h[o] = bf16_bits(g.act ? gelu(v) : v);
+          } else {
+            v = v * gelu_grad(g.z[o]);
+            g.h[o] = bf16_bits(v);
           }
+          g.C[o] = v;
         }
       }
-    }
-  } else if (nk == 0) {  // empty sum: C = beta C
-    for (int e = threadIdx.x; e < kBM * BN; e += kTcThreads) {
-      const int row = m0 + e / BN, n = n0 + e % BN;
-      if (row < g.M && n < g.N) {
-        float* c = g.C + (long)row * g.ldc + n;
-        *c = g.beta == 0.0f ? 0.0f : g.beta * *c;
-      }
+      __syncwarp();
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN));
-}
-
-__device__ __forceinline__ uint16_t bf16_bits(float v) {
-  return __bfloat16_as_ushort(__float2bfloat16_rn(v));
-}
-
-// GELU(z) = z Phi(z), Phi the standard normal distribution function
-__device__ __forceinline__ float gelu(float z) {
-  return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
-}
-__device__ __forceinline__ float gelu_grad(float z) {
-  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) +
-         z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
 // z += b (row broadcast); h = bf16(gelu(z)) when act, else bf16(z) (h optional)
@@ -327,19 +353,33 @@ __global__ void adam_bf16_kernel(float* w, const float* g, float* m1, float* m2,
 
 inline unsigned nblk(long count) { return (unsigned)((count + 255) / 256); }
 
-template <int BN>
+template <int BN, int EPI>
 int launch_tc(const TcGemm& g, cudaStream_t st) {
   static DeviceFlags attr;
   {
-    const cudaError_t e = set_max_smem_once(attr, gemm_bf16_tc<BN>, tc_smem_bytes<BN>());
+    const cudaError_t e = set_max_smem_once(attr, gemm_bf16_tc<BN, EPI>, tc_smem_bytes<BN>());
     if (e != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute", e);
   }
   dim3 grid((g.N + BN - 1) / BN, (g.M + kBM - 1) / kBM);
-  gemm_bf16_tc<BN><<<grid, kTcThreads, tc_smem_bytes<BN>(), st>>>(g);
+  gemm_bf16_tc<BN, EPI><<<grid, kTcThreads, tc_smem_bytes<BN>(), st>>>(g);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_cuda_error("tensor-core GEMM launch", e);
   return ESPEC_OK;
 }
+
+// the widest tiles that still give every SM one
+template <int EPI>
+int launch_any(const TcGemm& g, cudaStream_t st) {
+  auto tiles = [&](int bn) {
+    return (long)((g.N + bn - 1) / bn) * ((g.M + kBM - 1) / kBM);
+  };
+  if (tiles(256) >= 148) return launch_tc<256, EPI>(g, st);
+  if (tiles(128) >= 148) return launch_tc<128, EPI>(g, st);
+  if (tiles(64) >= 148) return launch_tc<64, EPI>(g, st);
+  return launch_tc<32, EPI>(g, st);
+}
+
+inline int vec_ok(const void* p, int ld) { return ld % 8 == 0 && ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
 }  // namespace espec
@@ -359,13 +399,33 @@ extern "C" int espec_gemm_bf16(int M, int N, int K, float alpha, const void* A, 
     return set_error(ESPEC_EINVAL, "bad GEMM");
   if (lda < (ta ? M : K) || ldb < (tb ? K : N) || ldc < N)
     return set_error(ESPEC_EINVAL, "leading dimension smaller than the row length");
-  auto vec_ok = [](const void* p, int ld) { return ld % 8 == 0 && ((uintptr_t)p & 15) == 0; };
   TcGemm g{M, N, K, alpha, beta, (const uint16_t*)A, lda, ta ? 1 : 0, (const uint16_t*)B, ldb,
-           tb ? 1 : 0, C, ldc, vec_ok(A, lda) ? 1 : 0, vec_ok(B, ldb) ? 1 : 0};
-  // N tiles of 256 only when that still gives a CTA per SM
-  const long tiles256 = (long)((N + 255) / 256) * ((M + kBM - 1) / kBM);
-  return (N > 128 && tiles256 >= 148) ? launch_tc<256>(g, (cudaStream_t)stream)
-                                      : launch_tc<128>(g, (cudaStream_t)stream);
+           tb ? 1 : 0, C, ldc, vec_ok(A, lda), vec_ok(B, ldb)};
+  return launch_any<kPlain>(g, (cudaStream_t)stream);
+}
+
+extern "C" int espec_mlp_layer(int rows, int fin, int fout, const void* x, const void* w,
+                               const float* b, int act, float* z, void* h, void* stream) {
+  if (rows <= 0 || fin <= 0 || fout <= 0 || !x || !w || !b || !z)
+    return set_error(ESPEC_EINVAL, "bad network layer");
+  TcGemm g{rows, fout, fin, 1.0f, 0.0f, (const uint16_t*)x, fin, 0, (const uint16_t*)w, fout, 0,
+           z, fout, vec_ok(x, fin), vec_ok(w, fout)};
+  g.bias = b;
+  g.h = (uint16_t*)h;
+  g.act = act;
+  return launch_any<kBias>(g, (cudaStream_t)stream);
+}
+
+extern "C" int espec_mlp_layer_back(int rows, int fin, int fout, const void* dz, const void* w,
+                                    const float* z_in, float* dz_in, void* dz_in_bf16,
+                                    void* stream) {
+  if (rows <= 0 || fin <= 0 || fout <= 0 || !dz || !w || !z_in || !dz_in || !dz_in_bf16)
+    return set_error(ESPEC_EINVAL, "bad network layer");
+  TcGemm g{rows, fin, fout, 1.0f, 0.0f, (const uint16_t*)dz, fout, 0, (const uint16_t*)w, fout, 1,
+           dz_in, fin, vec_ok(dz, fout), vec_ok(w, fout)};
+  g.z = z_in;
+  g.h = (uint16_t*)dz_in_bf16;
+  return launch_any<kGeluBack>(g, (cudaStream_t)stream);
 }
 
 namespace espec {

@@ -165,13 +165,14 @@ class MLP:
         torch = _torch()
         lib = N.load()
         hs, zs = [Xb.contiguous()], []
-        L = len(self.W)
+        rows, L, st = hs[0].shape[0], len(self.W), _st(Xb)
         for i, (Wb, b) in enumerate(zip(self.Wb, self.b)):
-            Z = gemm_bf16(hs[-1], Wb)
+            Z = torch.empty((rows, b.numel()), dtype=torch.float32, device=b.device)
             h = torch.empty(Z.shape, dtype=torch.bfloat16, device=Z.device) if i < L - 1 else None
-            N.check(lib.espec_mlp_bias_gelu(Z.data_ptr(), b.data_ptr(), Z.shape[0], Z.shape[1],
-                                            int(i < L - 1), h.data_ptr() if h is not None else None,
-                                            _st(Z)), "espec_mlp_bias_gelu")
+            N.check(lib.espec_mlp_layer(rows, Wb.shape[0], b.numel(), hs[-1].data_ptr(),
+                                        Wb.data_ptr(), b.data_ptr(), int(i < L - 1), Z.data_ptr(),
+                                        h.data_ptr() if h is not None else None, st),
+                    "espec_mlp_layer")
             zs.append(Z)
             if h is not None:
                 hs.append(h)
@@ -183,18 +184,23 @@ class MLP:
         torch = _torch()
         lib = N.load()
         grads = [None] * len(self.params)
+        st = _st(dY)
         d, db16 = dY, to_bf16(dY)
+        rows = d.shape[0]
         for i in reversed(range(len(self.W))):
             dW = gemm_bf16(hs[i], db16, ta=True)
             db = torch.empty(d.shape[1], dtype=torch.float32, device=d.device)
-            N.check(lib.espec_mlp_colsum(d.data_ptr(), d.shape[0], d.shape[1], db.data_ptr(),
-                                         _st(d)), "espec_mlp_colsum")
+            N.check(lib.espec_mlp_colsum(d.data_ptr(), rows, d.shape[1], db.data_ptr(), st),
+                    "espec_mlp_colsum")
             grads[2 * i], grads[2 * i + 1] = dW, db
             if i > 0:
-                d = gemm_bf16(db16, self.Wb[i], tb=True)
-                db16 = torch.empty(d.shape, dtype=torch.bfloat16, device=d.device)
-                N.check(lib.espec_mlp_gelu_back(d.data_ptr(), zs[i - 1].data_ptr(), d.numel(),
-                                                db16.data_ptr(), _st(d)), "espec_mlp_gelu_back")
+                Wb, z = self.Wb[i], zs[i - 1]
+                dz = torch.empty_like(z)
+                dz16 = torch.empty(z.shape, dtype=torch.bfloat16, device=z.device)
+                N.check(lib.espec_mlp_layer_back(rows, Wb.shape[0], Wb.shape[1], db16.data_ptr(),
+                                                 Wb.data_ptr(), z.data_ptr(), dz.data_ptr(),
+                                                 dz16.data_ptr(), st), "espec_mlp_layer_back")
+                d, db16 = dz, dz16
         return grads
 
     def loss_grad(self, Y, T):

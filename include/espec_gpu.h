@@ -561,6 +561,17 @@ int espec_mlp_bias_gelu(float* z, const float* b, int rows, int cols, int act, v
                         void* stream);
 /* dh *= GELU'(z) (z = the layer's pre-activation); dz_bf16 = bf16(dh) */
 int espec_mlp_gelu_back(float* dh, const float* z, long count, void* dz_bf16, void* stream);
+/* One layer in one kernel, on row-major BF16 operands with FP32 accumulation:
+ * z[rows,fout] = x[rows,fin] w[fin,fout] + b, h = bf16(GELU(z)) (act != 0) or
+ * bf16(z); h may be NULL.  The same values as espec_gemm_bf16 followed by
+ * espec_mlp_bias_gelu. */
+int espec_mlp_layer(int rows, int fin, int fout, const void* x, const void* w, const float* b,
+                    int act, float* z, void* h, void* stream);
+/* The gradient through a layer to its input's pre-activation z_in[rows,fin]:
+ * dz_in = (dz[rows,fout] w^T) * GELU'(z_in) and its BF16 copy.  The same values
+ * as espec_gemm_bf16 followed by espec_mlp_gelu_back. */
+int espec_mlp_layer_back(int rows, int fin, int fout, const void* dz, const void* w,
+                         const float* z_in, float* dz_in, void* dz_in_bf16, void* stream);
 /* y = bf16(x) */
 int espec_to_bf16(const float* x, void* y, long count, void* stream);
 /* one Adam step (Kingma & Ba) on FP32 master weights with hyper = device
