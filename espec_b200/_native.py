@@ -44,7 +44,7 @@ EXPORTS = [
     "espec_spectrum_work_bytes", "hwhm_", "spectrumtd_", "espec_eig_solve_dev",
     "espec_eig_lcg_start", "espec_eig_morse2d", "espec_gemm_f64", "espec_gemm_f32",
     "espec_gemm_bf16", "espec_gemm_bf16_status", "espec_mlp_bias_gelu", "espec_mlp_gelu_back", "espec_mlp_layer",
-    "espec_mlp_layer_back",
+    "espec_mlp_layer_back", "espec_mlp_forward", "espec_mlp_backward",
     "espec_to_bf16", "espec_mlp_adam_bf16", "espec_mlp_colsum", "espec_mlp_mse", "espec_sep_basis",
     "espec_convert", "espec_spond_create", "espec_spond_load", "espec_spond_run",
     "espec_spond_results", "espec_spond_destroy", "espec_spond_continue", "espec_spond_energies",
@@ -167,6 +167,8 @@ def load():
     lib.espec_mlp_gelu_back.argtypes = [vp, vp, cl, vp, vp]
     lib.espec_mlp_layer.argtypes = [ci, ci, ci, vp, vp, vp, ci, vp, vp, vp]
     lib.espec_mlp_layer_back.argtypes = [ci, ci, ci, vp, vp, vp, vp, vp, vp]
+    lib.espec_mlp_forward.argtypes = [ci, vp, ci, vp, vp, vp, vp, vp, vp]
+    lib.espec_mlp_backward.argtypes = [ci, vp, ci, vp, vp, vp, vp, vp, vp, vp, vp]
     lib.espec_to_bf16.argtypes = [vp, vp, cl, vp]
     lib.espec_mlp_adam_bf16.argtypes = [vp, vp, vp, vp, cl, vp, cf, cf, cf, vp, vp]
     lib.espec_spond_create.argtypes = [C.POINTER(vp), ci, i, d, d, cd, ci, ci, ci]

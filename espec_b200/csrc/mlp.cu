@@ -78,12 +78,15 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, T alpha,
 // db[c] = sum_r dy[r, c]: 32 columns x 8 row phases per CTA, each phase sums
 // rows r = phase mod 8 in order, then the 8 partials are added in order
 // (deterministic)
-__global__ void colsum_kernel(const float* dy, int rows, int cols, float* db) {
+__global__ void colsum_kernel(const float* __restrict__ dy, int rows, int cols,
+                              float* __restrict__ db) {
   __shared__ float part[8][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.0f;
-  if (c < cols)
+  if (c < cols) {
+#pragma unroll 16
     for (int r = threadIdx.y; r < rows; r += 8) s += dy[(long)r * cols + c];
+  }
   part[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
   if (threadIdx.y == 0 && c < cols) {
@@ -95,12 +98,13 @@ __global__ void colsum_kernel(const float* dy, int rows, int cols, float* db) {
 }
 
 // loss = mean over rows of sum (y - t)^2 / cols; dy = 2 (y - t) / (rows cols)
-__global__ void mse_kernel(const float* y, const float* t, int rows, int cols, float* dy,
-                           float* row_loss) {
+__global__ void mse_kernel(const float* __restrict__ y, const float* __restrict__ t, int rows,
+                           int cols, float* __restrict__ dy, float* row_loss) {
   const int r = blockIdx.x;
   float s = 0.0f;
   const float sc = 2.0f / ((float)rows * (float)cols);
-  for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+#pragma unroll 8
+  for (int c = threadIdx.x; c < cols; c += 256) {
     const float d = y[(long)r * cols + c] - t[(long)r * cols + c];
     dy[(long)r * cols + c] = sc * d;
     s += d * d;

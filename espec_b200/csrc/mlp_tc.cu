@@ -7,17 +7,17 @@
 // operands; every product accumulates in FP32.
 //
 // GEMM: C[M,N] (f32) = alpha op(A) op(B) + beta C, A and B bfloat16.  One CTA
-// of 128 threads owns a 128 x BN output tile whose FP32 accumulator lives in
+// of 256 threads owns a 128 x BN output tile whose FP32 accumulator lives in
 // tensor memory (TMEM lane = tile row, column = tile column).  K advances in
-// stages of 64 through a ring of four shared-memory buffers: all threads copy the
-// A and B tiles two stages ahead with cp.async (16-byte pieces, zero-filled at the
+// stages of 64 through a ring of four or eight shared-memory buffers: all threads
+// copy the A and B tiles ahead with cp.async (16-byte pieces, zero-filled at the
 // edges) as "core matrices" (8 x 16 bytes, no swizzle; K-major or MN-major,
 // whichever keeps the source's 16-byte runs whole), one thread issues four
 // tcgen05.mma (M = 128, N = BN, K = 16, kind::f16 with BF16 inputs) per stage and
 // commits them to the buffer's mbarrier.  BN is the largest of 256, 128, 64 that
 // gives every SM a tile, else 32: the network's products have few tiles, and what
 // bounds them is the chain of stages.  The epilogue reads the accumulator with
-// tcgen05.ld (one warp per 32 TMEM lanes) and turns it in shared memory so that
+// tcgen05.ld (a warp: 32 TMEM lanes, 32 columns) and turns it in shared memory so that
 // rows are written 128 bytes at a time, adding the bias and the activation (or
 // its derivative) on the way.  Every mbarrier wait is bounded: on timeout the
 // kernel records it in a device status word, skips the epilogue and still releases
@@ -36,7 +36,8 @@ namespace {
 
 constexpr int kBM = 128;         // tile rows = TMEM lanes
 constexpr int kBK = 64;          // k per stage: four MMAs of k = 16
-constexpr int kTcThreads = 128;  // four warps, one per 32 TMEM lanes
+constexpr int kTcThreads = 256;  // staging and epilogue: warp w reads TMEM lanes 32 (w % 4) ...
+constexpr int kTcBlock = kTcThreads + 32;  // and one warp that issues the MMAs
 constexpr long kWaitLimit = 1L << 22;
 
 __device__ int g_tc_status;  // non-zero: a bounded wait gave up (sticky until read)
@@ -84,52 +85,91 @@ __device__ __forceinline__ uint32_t pack2(uint16_t lo, uint16_t hi) {
   return (uint32_t)lo | ((uint32_t)hi << 16);
 }
 
-// Operand tile of R rows (M or N) x 64 k as 8 x 8 core matrices of 16-byte
-// rows: core matrix (row group g, k group q) at q * 16 R + g * 128 bytes, so
-// that one descriptor serves both forms (stride byte offset 128 between row
-// groups, leading byte offset 16 R between k groups).
-//  * kcontig source (element (row, k) at X[row ld + k]): K-major core
-//    matrices, 16-byte row = 8 consecutive k of one row;
-//  * otherwise (element at X[k ld + row]): MN-major core matrices, 16-byte
-//    row = 8 consecutive rows at one k.
+// Operand tile of R rows (M or N) x 64 k as 8 x 8 core matrices of 16-byte rows:
+//  * kcontig source (element (row, k) at X[row ld + k]): K-major core matrices,
+//    16-byte row = 8 consecutive k of one row; 128 bytes between row groups (the
+//    stride byte offset), 16 R + 16 between k groups (the leading byte offset);
+//  * otherwise (element at X[k ld + row]): MN-major core matrices, 16-byte row = 8
+//    consecutive rows at one k; 144 bytes between row groups, 18 R between k
+//    groups.
 // Either way a 16-byte row is 16 contiguous source bytes, copied asynchronously
 // when vec (aligned; the part beyond nrows or K is zero-filled), else element by
-// element.  Eight consecutive threads fill one core matrix (128 contiguous bytes
-// of shared memory), a warp four neighbouring ones (64 contiguous source bytes).
+// element.  Consecutive threads take consecutive 16-byte pieces of the source,
+// whole 128-byte lines per eight threads (in half lines a CTA drew 29 GB/s); the
+// odd group strides put those pieces on distinct banks.
+// A thread's pieces keep their places from stage to stage: their addresses and
+// sizes are formed once and then advance by a constant.
 template <int R>
-__device__ __forceinline__ void stage_tile(uint8_t* dst, const uint16_t* X, int ld, bool kcontig,
-                                           bool vec, int row0, int nrows, int k0, int K) {
-  constexpr int kIter = R * (kBK / 8) / kTcThreads;  // 16-byte pieces per thread
+__host__ __device__ constexpr uint32_t lead_bytes(bool kcontig) {
+  return kcontig ? R * 16 + 16 : R * 18;
+}
+__host__ __device__ constexpr uint32_t stride_bytes(bool kcontig) { return kcontig ? 128 : 144; }
+template <int R>
+constexpr int kTileBytes = R * 18 * (kBK / 8);
+template <int R>
+struct Stager {
+  static constexpr int kIter = (R * (kBK / 8) + kTcThreads - 1) / kTcThreads;  // pieces per thread
+  const uint16_t* src[kIter];
+  int cnt[kIter];  // elements that exist: along k (kcontig: at stage 0), else along the rows
+  int k[kIter];    // first k of the piece, stage 0
+  long step;       // elements from stage to stage
+  bool kcontig, vec;
+  int K;
+  static __device__ __forceinline__ bool live(int i) {
+    return R * (kBK / 8) % kTcThreads == 0 || (int)threadIdx.x + i * kTcThreads < R * (kBK / 8);
+  }
+  static __device__ __forceinline__ int place(int i, bool kcontig) {
+    const int it = threadIdx.x + i * kTcThreads;
+    const int row = it >> 3, g = it % (R / 8), kk = it / (R / 8);
+    return kcontig ? (it & 7) * (int)lead_bytes<R>(true) + (row >> 3) * 128 + (row & 7) * 16
+                   : (kk >> 3) * (int)lead_bytes<R>(false) + g * 144 + (kk & 7) * 16;
+  }
+  __device__ __forceinline__ void init(const uint16_t* X, int ld, bool kc, bool v, int row0,
+                                       int nrows, int K_) {
+    kcontig = kc;
+    vec = v;
+    K = K_;
+    step = kc ? kBK : (long)kBK * ld;
 #pragma unroll
-  for (int i = 0; i < kIter; ++i) {
-    const int it = threadIdx.x + i * kTcThreads, lo = it & 7, hi = it >> 3;
-    int off, cnt;      // place; elements that exist
-    const uint16_t* src;
-    if (kcontig) {
-      const int q = hi & 7, g = hi >> 3, row = row0 + g * 8 + lo, kb = k0 + 8 * q;
-      off = q * (R * 16) + g * 128 + lo * 16;
-      cnt = row < nrows ? min(max(K - kb, 0), 8) : 0;
-      src = X + (long)row * ld + kb;
-    } else {
-      const int g = hi % (R / 8), kq = hi / (R / 8), kk = k0 + 8 * kq + lo, m = row0 + 8 * g;
-      off = kq * (R * 16) + g * 128 + lo * 16;
-      cnt = kk < K ? min(max(nrows - m, 0), 8) : 0;
-      src = X + (long)kk * ld + m;
-    }
-    if (cnt == 0) src = X;
-    if (vec) {
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst + off)),
-                   "l"(src), "r"(2 * cnt)
-                   : "memory");
-    } else {
-      uint16_t e[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) e[j] = j < cnt ? src[j] : (uint16_t)0;
-      *reinterpret_cast<uint4*>(dst + off) =
-          make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]), pack2(e[4], e[5]), pack2(e[6], e[7]));
+    for (int i = 0; i < kIter; ++i) {
+      const int it = threadIdx.x + i * kTcThreads;
+      if (kc) {
+        const int row = row0 + (it >> 3);
+        k[i] = 8 * (it & 7);
+        cnt[i] = row < nrows ? 8 : 0;
+        src[i] = X + (cnt[i] ? (long)row * ld + k[i] : 0);
+      } else {
+        const int m = row0 + 8 * (it % (R / 8));
+        k[i] = it / (R / 8);
+        cnt[i] = min(max(nrows - m, 0), 8);
+        src[i] = X + (cnt[i] ? (long)k[i] * ld + m : 0);
+      }
     }
   }
-}
+  // stage kt into dst
+  __device__ __forceinline__ void stage(uint8_t* dst, int kt) const {
+#pragma unroll
+    for (int i = 0; i < kIter; ++i) {
+      if (!live(i)) continue;
+      const int left = K - kt * kBK - k[i];  // values of k from the piece's first on
+      const int n = kcontig ? (cnt[i] ? min(max(left, 0), 8) : 0) : (left > 0 ? cnt[i] : 0);
+      // an empty piece reads nothing: any valid address (src's first element)
+      const uint16_t* p = n > 0 ? src[i] + kt * step : src[i];
+      uint8_t* d = dst + place(i, kcontig);
+      if (vec) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(d)), "l"(p),
+                     "r"(2 * n)
+                     : "memory");
+      } else {
+        uint16_t e[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) e[j] = j < n ? p[j] : (uint16_t)0;
+        *reinterpret_cast<uint4*>(d) = make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]),
+                                                  pack2(e[4], e[5]), pack2(e[6], e[7]));
+      }
+    }
+  }
+};
 
 // bounded wait for the completion of the mbarrier phase with this parity
 __device__ __forceinline__ bool wait_phase(uint64_t* bar, uint32_t parity,
@@ -178,46 +218,41 @@ __device__ __forceinline__ float gelu_grad(float z) {
          z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-constexpr int kRing = 4;   // stage buffers
-constexpr int kAhead = 2;  // stages copied ahead of the one multiplied
-
-template <int BN>
+// stage buffers, filled ahead of the stage multiplied: 8 where a narrow
+// tile has a long K (an L2 round trip is several stages long), else 4, which lets
+// two CTAs share an SM
+template <int BN, int RING>
 constexpr size_t tc_smem_bytes() {
-  return 1024 + kRing * (size_t)(kBM + BN) * kBK * 2 + 64;
+  return 1024 + RING * (size_t)(kTileBytes<kBM> + kTileBytes<BN>) + 192;
 }
 
-template <int BN, int EPI>
-__global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
+template <int BN, int EPI, int RING>
+__global__ void __launch_bounds__(kTcBlock) gemm_bf16_tc(TcGemm g) {
   static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256,
                 "TMEM columns: a power of two from 32, N tile of one MMA");
-  constexpr int kA = kBM * kBK * 2, kB = BN * kBK * 2;
+  constexpr int kA = kTileBytes<kBM>, kB = kTileBytes<BN>, kRing = RING;
   static_assert(kRing * kA >= kTcThreads * 33 * 4, "the epilogue turns tiles in the stage buffers");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = base;
   uint8_t* sB = base + kRing * kA;
-  uint64_t* bar = (uint64_t*)(base + kRing * (kA + kB));
-  uint32_t* tmem_slot = (uint32_t*)(bar + kRing);
+  uint64_t* full = (uint64_t*)(base + kRing * (kA + kB));  // a buffer's copies have landed
+  uint64_t* done = full + kRing;                           // its MMAs have read it
+  uint32_t* tmem_slot = (uint32_t*)(done + kRing);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
-  const bool a_kc = !g.ta, b_kc = g.tb != 0;
+  const bool a_kc = !g.ta, b_kc = g.tb != 0, mma_warp = warp == kTcThreads / 32;
   const int nk = (g.K + kBK - 1) / kBK;
-  auto stage = [&](int kt) {
-    if (kt < nk) {
-      const int b = kt % kRing;
-      stage_tile<kBM>(sA + b * kA, g.A, g.lda, a_kc, g.a_vec, m0, g.M, kt * kBK, g.K);
-      stage_tile<BN>(sB + b * kB, g.B, g.ldb, b_kc, g.b_vec, n0, g.N, kt * kBK, g.K);
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
 
-  for (int kt = 0; kt < kAhead; ++kt) stage(kt);
   if (threadIdx.x == 0) {
-    for (int b = 0; b < kRing; ++b)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(bar + b)));
+    for (int b = 0; b < kRing; ++b) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(full + b)),
+                   "r"(kTcThreads));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(done + b)));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 0) {
+  if (mma_warp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                      smem_u32(tmem_slot)),
                  "r"(BN));
@@ -227,23 +262,44 @@ __global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t idesc = idesc_bf16<BN>(a_kc ? 0u : 1u, b_kc ? 0u : 1u);
   bool ok = true;
-  for (int kt = 0; kt < nk; ++kt) {
-    // buffer (kt + kAhead) % kRing was read by the MMAs of stage kt + kAhead - kRing
-    const int old = kt + kAhead - kRing;
-    if (old >= 0) ok = wait_phase(bar + old % kRing, (old / kRing) & 1) && ok;
-    stage(kt + kAhead);
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(kAhead) : "memory");
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x == 0) {
+  if (!mma_warp) {
+    Stager<kBM> ta;
+    Stager<BN> tb;
+    ta.init(g.A, g.lda, a_kc, g.a_vec, m0, g.M, g.K);
+    tb.init(g.B, g.ldb, b_kc, g.b_vec, n0, g.N, g.K);
+    const bool async = g.a_vec && g.b_vec;
+    for (int kt = 0; kt < nk; ++kt) {
       const int b = kt % kRing;
+      if (kt >= kRing && !(ok = wait_phase(done + b, (kt / kRing - 1) & 1))) break;
+      ta.stage(sA + b * kA, kt);
+      tb.stage(sB + b * kB, kt);
+      if (async) {  // arrives by itself when this thread's copies have landed
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];\n" ::"r"(smem_u32(full + b))
+                     : "memory");
+      } else {
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}\n" ::"r"(
+                         smem_u32(full + b))
+                     : "memory");
+      }
+    }
+  } else if (lane == 0) {
+    // a thread without copies of its own: the proxy fence waits for all of a
+    // thread's outstanding copies, also those of later stages (issued by a staging
+    // thread it held every stage for a full memory round trip, 1.1 us)
+    const uint32_t idesc = idesc_bf16<BN>(a_kc ? 0u : 1u, b_kc ? 0u : 1u);
+    const uint32_t a_lead = lead_bytes<kBM>(a_kc), b_lead = lead_bytes<BN>(b_kc);
+    for (int kt = 0; kt < nk; ++kt) {
+      const int b = kt % kRing;
+      if (!(ok = wait_phase(full + b, (kt / kRing) & 1))) break;
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       const uint32_t a0 = smem_u32(sA + b * kA), b0 = smem_u32(sB + b * kB);
 #pragma unroll
       for (int j = 0; j < kBK / 16; ++j) {
-        const uint64_t da = smem_desc(a0 + j * 2 * (kBM * 16), kBM * 16, 128);
-        const uint64_t db = smem_desc(b0 + j * 2 * (BN * 16), BN * 16, 128);
+        const uint64_t da = smem_desc(a0 + j * 2 * a_lead, a_lead, stride_bytes(a_kc));
+        const uint64_t db = smem_desc(b0 + j * 2 * b_lead, b_lead, stride_bytes(b_kc));
         const uint32_t acc = (kt > 0 || j > 0) ? 1u : 0u;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -253,25 +309,35 @@ __global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
       }
       asm volatile(
           "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-              smem_u32(bar + b))
+              smem_u32(done + b))
           : "memory");
     }
   }
-  // the commits not waited for above: the last kRing - kAhead stages
-  for (int kt = max(0, nk - (kRing - kAhead)); kt < nk; ++kt)
-    ok = wait_phase(bar + kt % kRing, (kt / kRing) & 1) && ok;
+  __syncwarp();
+  // warp w: rows 32 (w % 4) of the tile, columns from 32 (w / 4) on, 64 apart
+  const int row0 = m0 + (warp & 3) * 32, col0 = (warp >> 2) * 32;
+  // the first columns' pre-activations, on their way while the last MMAs run
+  float zf[EPI == kGeluBack ? 32 : 1];
+  if (EPI == kGeluBack) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      zf[i] = !mma_warp && col0 < BN && row0 + i < g.M && n0 + col0 + lane < g.N
+                  ? g.z[(long)(row0 + i) * g.ldc + n0 + col0 + lane]
+                  : 0.0f;
+  }
+  // the last commit covers every MMA before it
+  if (nk > 0) ok = wait_phase(done + (nk - 1) % kRing, ((nk - 1) / kRing) & 1) && ok;
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   ok = __syncthreads_and(ok) != 0;
-  if (ok) {
+  if (ok && !mma_warp) {
     // 32 columns at a time: each warp's 32 x 32 piece through shared memory
     float* turn = reinterpret_cast<float*>(base) + warp * (32 * 33);
-    const int row0 = m0 + warp * 32;
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
+    for (int c0 = col0; c0 < BN; c0 += 64) {
       uint32_t r[32];
       if (nk > 0) {
-        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
+        tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, r);
       } else {  // empty sum
 #pragma unroll
         for (int j = 0; j < 32; ++j) r[j] = 0u;
@@ -281,7 +347,7 @@ __global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
       __syncwarp();
       const int n = n0 + c0 + lane;
       const float bias = EPI == kBias && n < g.N ? g.bias[n] : 0.0f;
-#pragma unroll 8
+#pragma unroll
       for (int i = 0; i < 32; ++i) {
         const int row = row0 + i;
         if (row < g.M && n < g.N) {
@@ -295,7 +361,7 @@ __global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
             v = v + bias;
             if (g.h) g.h[o] = bf16_bits(g.act ? gelu(v) : v);
           } else {
-            v = v * gelu_grad(g.z[o]);
+            v = v * gelu_grad(c0 == col0 ? zf[i] : g.z[o]);
             g.h[o] = bf16_bits(v);
           }
           g.C[o] = v;
@@ -306,7 +372,7 @@ __global__ void __launch_bounds__(kTcThreads) gemm_bf16_tc(TcGemm g) {
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (warp == 0)
+  if (mma_warp)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN));
 }
 
@@ -353,15 +419,16 @@ __global__ void adam_bf16_kernel(float* w, const float* g, float* m1, float* m2,
 
 inline unsigned nblk(long count) { return (unsigned)((count + 255) / 256); }
 
-template <int BN, int EPI>
+template <int BN, int EPI, int RING>
 int launch_tc(const TcGemm& g, cudaStream_t st) {
   static DeviceFlags attr;
+  constexpr size_t smem = tc_smem_bytes<BN, RING>();
   {
-    const cudaError_t e = set_max_smem_once(attr, gemm_bf16_tc<BN, EPI>, tc_smem_bytes<BN>());
+    const cudaError_t e = set_max_smem_once(attr, gemm_bf16_tc<BN, EPI, RING>, smem);
     if (e != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute", e);
   }
   dim3 grid((g.N + BN - 1) / BN, (g.M + kBM - 1) / kBM);
-  gemm_bf16_tc<BN, EPI><<<grid, kTcThreads, tc_smem_bytes<BN>(), st>>>(g);
+  gemm_bf16_tc<BN, EPI, RING><<<grid, kTcBlock, smem, st>>>(g);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_cuda_error("tensor-core GEMM launch", e);
   return ESPEC_OK;
@@ -373,10 +440,10 @@ int launch_any(const TcGemm& g, cudaStream_t st) {
   auto tiles = [&](int bn) {
     return (long)((g.N + bn - 1) / bn) * ((g.M + kBM - 1) / kBM);
   };
-  if (tiles(256) >= 148) return launch_tc<256, EPI>(g, st);
-  if (tiles(128) >= 148) return launch_tc<128, EPI>(g, st);
-  if (tiles(64) >= 148) return launch_tc<64, EPI>(g, st);
-  return launch_tc<32, EPI>(g, st);
+  if (tiles(256) >= 148) return launch_tc<256, EPI, 4>(g, st);
+  if (tiles(128) >= 148) return launch_tc<128, EPI, 4>(g, st);
+  if (tiles(64) >= 148) return launch_tc<64, EPI, 4>(g, st);
+  return g.K > 8 * kBK ? launch_tc<32, EPI, 8>(g, st) : launch_tc<32, EPI, 4>(g, st);
 }
 
 inline int vec_ok(const void* p, int ld) { return ld % 8 == 0 && ((uintptr_t)p & 15) == 0; }
@@ -499,4 +566,48 @@ extern "C" int espec_mlp_adam_bf16(float* w, const float* g, float* m1, float* m
                                                                   b2, eps, (uint16_t*)w_bf16);
   TC_CK();
   return ESPEC_OK;
+}
+
+extern "C" int espec_mlp_forward(int nlayers, const int* width, int rows, const void* x,
+                                 const void* const* w, const float* const* b, float* const* z,
+                                 void* const* h, void* stream) {
+  if (nlayers < 1 || !width || !w || !b || !z || (nlayers > 1 && !h))
+    return set_error(ESPEC_EINVAL, "bad network");
+  const void* in = x;
+  for (int i = 0; i < nlayers; ++i) {
+    void* out = i + 1 < nlayers ? h[i] : nullptr;
+    const int rc = espec_mlp_layer(rows, width[i], width[i + 1], in, w[i], b[i], i + 1 < nlayers,
+                                   z[i], out, stream);
+    if (rc) return rc;
+    in = out;
+  }
+  return ESPEC_OK;
+}
+
+extern "C" int espec_mlp_backward(int nlayers, const int* width, int rows, const void* const* hs,
+                                  const float* const* z, const void* const* w, const float* dy,
+                                  float* const* dw, float* const* db, void* work, void* stream) {
+  if (nlayers < 1 || rows < 1 || !width || !hs || !z || !w || !dy || !dw || !db || !work)
+    return set_error(ESPEC_EINVAL, "bad network");
+  size_t wmax = 0;
+  for (int i = 1; i <= nlayers; ++i) wmax = width[i] > (int)wmax ? (size_t)width[i] : wmax;
+  // the current layer's dz (FP32, two in turn) and its BF16 copies
+  const size_t n = (size_t)rows * wmax;
+  float* dz[2] = {(float*)work, (float*)work + n};
+  uint16_t* d16[2] = {(uint16_t*)(dz[1] + n), (uint16_t*)(dz[1] + n) + n};
+  const float* d = dy;
+  int cur = 0;
+  int rc = espec_to_bf16(dy, d16[0], (long)rows * width[nlayers], stream);
+  for (int i = nlayers - 1; i >= 0 && rc == ESPEC_OK; --i) {
+    const int fi = width[i], fo = width[i + 1];
+    rc = espec_gemm_bf16(fi, fo, rows, 1.0f, hs[i], fi, 1, d16[cur], fo, 0, 0.0f, dw[i], fo, stream);
+    if (rc == ESPEC_OK) rc = espec_mlp_colsum(d, rows, fo, db[i], stream);
+    if (rc == ESPEC_OK && i > 0) {
+      rc = espec_mlp_layer_back(rows, fi, fo, d16[cur], w[i], z[i - 1], dz[cur ^ 1], d16[cur ^ 1],
+                                stream);
+      cur ^= 1;
+      d = dz[cur];
+    }
+  }
+  return rc;
 }

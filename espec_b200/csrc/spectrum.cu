@@ -79,15 +79,24 @@ __device__ __forceinline__ double2 prep_value(const PrepArgs& a, long p, long i)
   return z;
 }
 
-// twiddles w_k = exp(+i twopi k / N), k < N/2 (the backward sign of FFTNT),
-// and, when asked for, the factor of every time
-__global__ void spec_table_kernel(PrepArgs a, double2* tw, double2* factor, double twopi_over_n) {
+// twiddles w_k = exp(+i twopi k / N), k < N/2 (the backward sign of FFTNT), those
+// of each earlier pass s gathered where its threads read them (2^s values from
+// 2^s - 1 on), and, when asked for, the factor of every time
+struct Twiddles {
+  const double2* w;     // w_k, k < N/2: the last pass's values
+  const double2* pass;  // the earlier passes' values, or null (no room): w by stride
+};
+__global__ void spec_table_kernel(PrepArgs a, double2* tw, double2* pass, double2* factor,
+                                  double twopi_over_n) {
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const long N = 1L << a.mf;
   if (k < N / 2) {
     double s, c;
     sincos(twopi_over_n * (double)k, &s, &c);
     tw[k] = make_double2(c, s);
+    if (pass)  // k = q 2^(mf-1-s) is value q of pass s
+      for (int s2 = a.mf - 2; s2 >= 0 && (k & ((1L << (a.mf - 1 - s2)) - 1)) == 0; --s2)
+        pass[(1L << s2) - 1 + (k >> (a.mf - 1 - s2))] = make_double2(c, s);
   }
   if (factor && k < N) factor[k] = time_factor(a, k);
 }
@@ -115,15 +124,16 @@ __host__ __device__ constexpr int brev_c(int v, int bits) {
   return r;
 }
 template <int LOGR>
-__device__ __forceinline__ void passes(double2* v, const double2* __restrict__ tw, long k, int s,
-                                       int mf) {
+__device__ __forceinline__ void passes(double2* v, const Twiddles& tw, long k, int s, int mf) {
   constexpr int R = 1 << LOGR;
 #pragma unroll
   for (int p = 0; p < LOGR; ++p) {
     const int half = R >> (p + 1);
 #pragma unroll
     for (int blk = 0; blk < (1 << p); ++blk) {
-      const double2 w = __ldg(tw + ((k + ((long)brev_c(blk, p) << s)) << (mf - 1 - s - p)));
+      const long q0 = k + ((long)brev_c(blk, p) << s);
+      const double2 w = __ldg(tw.pass && s + p < mf - 1 ? tw.pass + ((1L << (s + p)) - 1 + q0)
+                                                        : tw.w + (q0 << (mf - 1 - s - p)));
 #pragma unroll
       for (int q = 0; q < half; ++q) {
         double2& x = v[blk * 2 * half + q];
@@ -150,8 +160,8 @@ constexpr int kOneThreads = 256;
 __device__ __forceinline__ int padded(int i) { return i + (i >> 4); }
 
 template <int REM, int T>
-__global__ void __launch_bounds__(T, 512 / T) spec_one_kernel(PrepArgs a, const double2* __restrict__ tw,
-                                                     double scale) {
+__global__ void __launch_bounds__(T, 512 / T) spec_one_kernel(PrepArgs a, Twiddles tw,
+                                                                      double scale) {
   extern __shared__ double2 spec_sm[];
   const int mf = a.mf, n = 1 << mf, tp = n >> 4;  // threads of a packet
   const int g = threadIdx.x / tp, t = threadIdx.x % tp;
@@ -206,8 +216,7 @@ __global__ void __launch_bounds__(T, 512 / T) spec_one_kernel(PrepArgs a, const 
 // kOneMax; one thread per group of 2^LOGR points
 template <int LOGR>
 __global__ void __launch_bounds__(256) spec_pass_kernel(PrepArgs a, const double2* x, double2* y,
-                                                        const double2* __restrict__ tw, int s,
-                                                        double scale) {
+                                                        Twiddles tw, int s, double scale) {
   constexpr int R = 1 << LOGR;
   const int mf = a.mf;
   const long N = 1L << mf, M = N >> LOGR;
@@ -226,7 +235,7 @@ __global__ void __launch_bounds__(256) spec_pass_kernel(PrepArgs a, const double
 }
 
 template <int REM, int T>
-cudaError_t launch_one(const PrepArgs& a, const double2* tw, double scale, cudaStream_t st) {
+cudaError_t launch_one(const PrepArgs& a, const Twiddles& tw, double scale, cudaStream_t st) {
   static DeviceFlags attr;
   const size_t smem = sizeof(double2) * 17 * T;
   cudaError_t e = set_max_smem_once(attr, spec_one_kernel<REM, T>, smem);
@@ -237,7 +246,7 @@ cudaError_t launch_one(const PrepArgs& a, const double2* tw, double scale, cudaS
 }
 
 cudaError_t launch_pass(int logr, const PrepArgs& a, const double2* x, double2* y,
-                        const double2* tw, int s, double scale, cudaStream_t st) {
+                        const Twiddles& tw, int s, double scale, cudaStream_t st) {
   const long th = ((1L << a.mf) >> logr) * a.npk;
   const unsigned nb = (unsigned)((th + 255) / 256);
   switch (logr) {
@@ -325,19 +334,24 @@ extern "C" int espec_spectrum_dev(int npk, int mf, const void* in, long ld, int 
   double2* dst = one || ngroups % 2 == 1 ? a.out : wk;
   double2* factor = scaled ? (dst == a.out ? wk : a.out) : nullptr;
   a.factor = factor;
-  spec_table_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(a, tw, factor, twopi / N);
+  // a whole-transform call leaves work's signal part free: the factors, then the
+  // earlier passes' twiddles
+  double2* pass = nullptr;
+  if (one && (factor == nullptr || npk >= 2)) pass = factor == wk ? wk + N : wk;
+  spec_table_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(a, tw, pass, factor, twopi / N);
   SPEC_CK(cudaGetLastError());
+  const Twiddles tws{tw, pass};
   const double rn = 1.0 / N;  // cfft.f:102-105
   if (one) {
     cudaError_t e;
     if (mf == kOneMax) {
-      e = launch_one<1, 2 * kOneThreads>(a, tw, rn, st);
+      e = launch_one<1, 2 * kOneThreads>(a, tws, rn, st);
     } else {
       switch (mf % 4) {
-        case 0: e = launch_one<4, kOneThreads>(a, tw, rn, st); break;
-        case 1: e = launch_one<1, kOneThreads>(a, tw, rn, st); break;
-        case 2: e = launch_one<2, kOneThreads>(a, tw, rn, st); break;
-        default: e = launch_one<3, kOneThreads>(a, tw, rn, st); break;
+        case 0: e = launch_one<4, kOneThreads>(a, tws, rn, st); break;
+        case 1: e = launch_one<1, kOneThreads>(a, tws, rn, st); break;
+        case 2: e = launch_one<2, kOneThreads>(a, tws, rn, st); break;
+        default: e = launch_one<3, kOneThreads>(a, tws, rn, st); break;
       }
     }
     SPEC_CK(e);
@@ -346,7 +360,7 @@ extern "C" int espec_spectrum_dev(int npk, int mf, const void* in, long ld, int 
   const double2* src = nullptr;
   for (int s = 0; s < mf;) {
     const int lr = s == 0 && mf % 4 ? mf % 4 : 4;
-    SPEC_CK(launch_pass(lr, a, src, dst, tw, s, s + lr == mf ? rn : 1.0, st));
+    SPEC_CK(launch_pass(lr, a, src, dst, tws, s, s + lr == mf ? rn : 1.0, st));
     src = dst;
     dst = dst == a.out ? wk : a.out;
     s += lr;

@@ -16,6 +16,7 @@ Everything here runs on the GPU through the C-ABI; torch only holds device
 memory.  The host does the bookkeeping of a data set: sampling parameters,
 the sign convention of the training eigenvectors, the learning-rate schedule.
 """
+import ctypes as C
 import math
 from types import SimpleNamespace
 
@@ -36,6 +37,10 @@ def _torch():
     import torch
 
     return torch
+
+
+def _ptrs(ts):
+    return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
 
 def _st(t):
@@ -154,6 +159,7 @@ class MLP:
             self.W.append(w)
             self.Wb.append(to_bf16(w))
             self.b.append(torch.zeros(fo, dtype=torch.float32, device=dev))
+        self._widths = (C.c_int * len(self.sizes))(*self.sizes)
         self.params = [p for pair in zip(self.W, self.b) for p in pair]
         self.copies = [c for w in self.Wb for c in (w, None)]  # BF16 copy of each parameter
         self.m1 = [torch.zeros_like(p) for p in self.params]
@@ -164,43 +170,27 @@ class MLP:
         the network's output is the last pre-activation."""
         torch = _torch()
         lib = N.load()
-        hs, zs = [Xb.contiguous()], []
-        rows, L, st = hs[0].shape[0], len(self.W), _st(Xb)
-        for i, (Wb, b) in enumerate(zip(self.Wb, self.b)):
-            Z = torch.empty((rows, b.numel()), dtype=torch.float32, device=b.device)
-            h = torch.empty(Z.shape, dtype=torch.bfloat16, device=Z.device) if i < L - 1 else None
-            N.check(lib.espec_mlp_layer(rows, Wb.shape[0], b.numel(), hs[-1].data_ptr(),
-                                        Wb.data_ptr(), b.data_ptr(), int(i < L - 1), Z.data_ptr(),
-                                        h.data_ptr() if h is not None else None, st),
-                    "espec_mlp_layer")
-            zs.append(Z)
-            if h is not None:
-                hs.append(h)
-        return hs, zs
+        X = Xb.contiguous()
+        rows, L, dev = X.shape[0], len(self.W), X.device
+        zs = [torch.empty((rows, n), dtype=torch.float32, device=dev) for n in self.sizes[1:]]
+        hs = [torch.empty((rows, n), dtype=torch.bfloat16, device=dev) for n in self.sizes[1:-1]]
+        N.check(lib.espec_mlp_forward(L, self._widths, rows, X.data_ptr(), _ptrs(self.Wb),
+                                      _ptrs(self.b), _ptrs(zs), _ptrs(hs), _st(X)),
+                "espec_mlp_forward")
+        return [X, *hs], zs
 
     def backward(self, hs, zs, dY):
         """Gradients [dW0, db0, dW1, db1, ...] (FP32) for the loss whose output
         gradient is dY (FP32)."""
         torch = _torch()
         lib = N.load()
-        grads = [None] * len(self.params)
-        st = _st(dY)
-        d, db16 = dY, to_bf16(dY)
-        rows = d.shape[0]
-        for i in reversed(range(len(self.W))):
-            dW = gemm_bf16(hs[i], db16, ta=True)
-            db = torch.empty(d.shape[1], dtype=torch.float32, device=d.device)
-            N.check(lib.espec_mlp_colsum(d.data_ptr(), rows, d.shape[1], db.data_ptr(), st),
-                    "espec_mlp_colsum")
-            grads[2 * i], grads[2 * i + 1] = dW, db
-            if i > 0:
-                Wb, z = self.Wb[i], zs[i - 1]
-                dz = torch.empty_like(z)
-                dz16 = torch.empty(z.shape, dtype=torch.bfloat16, device=z.device)
-                N.check(lib.espec_mlp_layer_back(rows, Wb.shape[0], Wb.shape[1], db16.data_ptr(),
-                                                 Wb.data_ptr(), z.data_ptr(), dz.data_ptr(),
-                                                 dz16.data_ptr(), st), "espec_mlp_layer_back")
-                d, db16 = dz, dz16
+        rows, L, dev = dY.shape[0], len(self.W), dY.device
+        grads = [torch.empty(p.shape, dtype=torch.float32, device=dev) for p in self.params]
+        work = torch.empty(12 * rows * max(self.sizes[1:]), dtype=torch.uint8, device=dev)
+        N.check(lib.espec_mlp_backward(L, self._widths, rows, _ptrs(hs), _ptrs(zs),
+                                       _ptrs(self.Wb), dY.data_ptr(), _ptrs(grads[0::2]),
+                                       _ptrs(grads[1::2]), work.data_ptr(), _st(dY)),
+                "espec_mlp_backward")
         return grads
 
     def loss_grad(self, Y, T):

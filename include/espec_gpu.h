@@ -572,6 +572,19 @@ int espec_mlp_layer(int rows, int fin, int fout, const void* x, const void* w, c
  * as espec_gemm_bf16 followed by espec_mlp_gelu_back. */
 int espec_mlp_layer_back(int rows, int fin, int fout, const void* dz, const void* w,
                          const float* z_in, float* dz_in, void* dz_in_bf16, void* stream);
+/* A whole network from one call each way.  width: nlayers + 1 widths; w, b: the
+ * layers' BF16 weights [width[i], width[i+1]] and FP32 biases; z: the layers'
+ * pre-activations (the last is the output); h: the BF16 inputs of layers 1 to
+ * nlayers - 1 (GELU of the layer before), x that of layer 0. */
+int espec_mlp_forward(int nlayers, const int* width, int rows, const void* x,
+                      const void* const* w, const float* const* b, float* const* z,
+                      void* const* h, void* stream);
+/* Gradients of the weights dw[i] and biases db[i] (FP32) for the output's
+ * gradient dy[rows, width[nlayers]]; hs: the BF16 inputs of every layer (x, then
+ * the forward call's h).  work: 12 rows max(width) bytes. */
+int espec_mlp_backward(int nlayers, const int* width, int rows, const void* const* hs,
+                       const float* const* z, const void* const* w, const float* dy,
+                       float* const* dw, float* const* db, void* work, void* stream);
 /* y = bf16(x) */
 int espec_to_bf16(const float* x, void* y, long count, void* stream);
 /* one Adam step (Kingma & Ba) on FP32 master weights with hyper = device
