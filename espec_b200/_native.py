@@ -23,6 +23,7 @@ Q_PSOD_COPY = 32
 PULSE_NONE, PULSE_GAUS, PULSE_GGAUS, PULSE_SIN2 = 0, 1, 2, 3
 SPO, SOD, SIL, PSOD = 0, 1, 2, 3
 MEM_HOST, MEM_DEVICE, MEM_HOST_ASYNC = 0, 1, 2
+MEM_INTERLEAVED = 16  # added to one of them: complex arrays as (re, im) pairs
 LAUNCH_CLASSES, LAUNCH_PERSISTENT = 0, 1
 VARIANT_TC = 5
 SHFS = 2.4188843243e-2
@@ -206,6 +207,18 @@ def ptr(a):
     if hasattr(a, "data_ptr"):
         return a.data_ptr()
     return a.ctypes.data
+
+
+def complex_host(psi):
+    """(arrays kept alive, re pointer, im pointer, MEM_HOST flags) of a host wave
+    function: complex data as it lies, real data without an imaginary part."""
+    psi = np.asarray(psi)
+    if np.iscomplexobj(psi):
+        z = np.ascontiguousarray(psi.ravel(order="F") if psi.ndim > 1 else psi,
+                                 dtype=np.complex128)
+        return z, z.ctypes.data, None, MEM_HOST | MEM_INTERLEAVED
+    re = f64(psi.ravel(order="F") if psi.ndim > 1 else psi)
+    return re, re.ctypes.data, None, MEM_HOST
 
 
 def f64(a):

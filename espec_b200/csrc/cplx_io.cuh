@@ -95,6 +95,20 @@ inline int get_complex(HostStage& s, const double2* src, double* re, double* im,
   return ESPEC_OK;
 }
 
+// interleaved user arrays (ESPEC_MEM_INTERLEAVED): one copy as they lie
+inline int put_pairs(double2* dst, const double* src, size_t n, int where, cudaStream_t st) {
+  if (n == 0) return ESPEC_OK;
+  IO_CK(cudaMemcpyAsync(dst, src, 16 * n,
+                        on_host(where) ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
+  return ESPEC_OK;
+}
+inline int get_pairs(const double2* src, double* dst, size_t n, int where, cudaStream_t st) {
+  if (!dst || n == 0) return ESPEC_OK;
+  IO_CK(cudaMemcpyAsync(dst, src, 16 * n,
+                        on_host(where) ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, st));
+  return ESPEC_OK;
+}
+
 #undef IO_CK
 
 }  // namespace

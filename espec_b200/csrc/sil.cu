@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "espec_gpu.h"
+#include "cplx_io.cuh"
 #include "espec_internal.h"
 #include "sil.cuh"
 
@@ -1223,6 +1224,7 @@ struct espec_grid_plan {
   int* d_err = nullptr;
   double2* d_c = nullptr;
   int c_cap = -1;  // nsteps of the C(t) buffer
+  HostStage stage; // interleaved user arrays
 };
 
 static void grid_free(espec_grid_plan* p) {
@@ -1231,6 +1233,7 @@ static void grid_free(espec_grid_plan* p) {
                p->d_up, p->d_vp, p->d_dm, p->d_ef, p->d_ppart};
   for (void* x : b)
     if (x) cudaFree(x);
+  p->stage.release();
 }
 
 #define GRID_CK(call)                                        \
@@ -1429,13 +1432,29 @@ extern "C" int espec_grid_load(espec_grid_plan* p, const double* vpot, const dou
   if (!p || !vpot || !psi_re) return set_error(ESPEC_EINVAL, "null argument");
   if (p->absorb != ESPEC_ABS_NONE && !vabc) return set_error(ESPEC_EINVAL, "absorber table missing");
   cudaStream_t st = (cudaStream_t)stream;
+  const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
+  where &= ~ESPEC_MEM_INTERLEAVED;
   const cudaMemcpyKind kind =
       where == ESPEC_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   const size_t nb = (size_t)p->n * 8;
   GRID_CK(cudaMemcpyAsync(p->d_vpot, vpot, nb, kind, st));
   if (p->absorb != ESPEC_ABS_NONE) GRID_CK(cudaMemcpyAsync(p->d_mask, vabc, nb, kind, st));
-  GRID_CK(cudaMemcpyAsync(p->d_u0, psi_re, nb, kind, st));
-  if (psi_im) {
+  if (pairs) {
+    const double2* src = (const double2*)psi_re;
+    if (where == ESPEC_MEM_HOST) {
+      const int rc = stage_reserve(p->stage, 2 * nb);
+      if (rc) return rc;
+      GRID_CK(cudaMemcpyAsync(p->stage.d, psi_re, 2 * nb, kind, st));
+      src = (const double2*)p->stage.d;
+    }
+    deinterleave_kernel<<<io_blocks(p->n), 256, 0, st>>>(src, p->d_u0, p->d_v0, (size_t)p->n);
+    GRID_CK(cudaGetLastError());
+  } else {
+    GRID_CK(cudaMemcpyAsync(p->d_u0, psi_re, nb, kind, st));
+  }
+  if (pairs) {
+    // both parts are in place
+  } else if (psi_im) {
     GRID_CK(cudaMemcpyAsync(p->d_v0, psi_im, nb, kind, st));
   } else {
     GRID_CK(cudaMemsetAsync(p->d_v0, 0, nb, st));
@@ -1545,9 +1564,27 @@ extern "C" int espec_grid_results(espec_grid_plan* p, double* c_re, double* c_im
                                   double* psi_im, int where, void* stream) {
   if (!p || p->c_cap < 0) return set_error(ESPEC_EINVAL, "no results: run the plan first");
   cudaStream_t st = (cudaStream_t)stream;
+  const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
+  where &= ~ESPEC_MEM_INTERLEAVED;
   const cudaMemcpyKind kind =
       where == ESPEC_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
   const size_t nc = (size_t)p->c_cap + 1;
+  if (pairs) {
+    if (c_re) GRID_CK(cudaMemcpyAsync(c_re, p->d_c, 16 * nc, kind, st));
+    if (psi_re) {
+      double2* dst = (double2*)psi_re;
+      if (where == ESPEC_MEM_HOST) {
+        const int rc = stage_reserve(p->stage, 16 * (size_t)p->n);
+        if (rc) return rc;
+        dst = (double2*)p->stage.d;
+      }
+      interleave_kernel<<<io_blocks(p->n), 256, 0, st>>>(p->d_u, p->d_v, dst, (size_t)p->n);
+      GRID_CK(cudaGetLastError());
+      if (where == ESPEC_MEM_HOST)
+        GRID_CK(cudaMemcpyAsync(psi_re, dst, 16 * (size_t)p->n, kind, st));
+    }
+    c_re = c_im = psi_re = psi_im = nullptr;
+  }
   if (c_re) GRID_CK(cudaMemcpy2DAsync(c_re, 8, p->d_c, 16, 8, nc, kind, st));
   if (c_im) GRID_CK(cudaMemcpy2DAsync(c_im, 8, (char*)p->d_c + 8, 16, 8, nc, kind, st));
   const size_t nb = (size_t)p->n * 8;

@@ -691,11 +691,14 @@ extern "C" int espec_spond_load(espec_spond_plan* p, const double* vpot, const d
   if (p->absorb != ESPEC_ABS_NONE && !vabc) return set_error(ESPEC_EINVAL, "absorber table missing");
   cudaStream_t st = (cudaStream_t)stream;
   const size_t n = (size_t)p->n;
+  const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
+  where &= ~ESPEC_MEM_INTERLEAVED;
   const cudaMemcpyKind kind =
       where == ESPEC_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   ND_CK(cudaMemcpyAsync(p->d_vpot, vpot, 8 * n, kind, st));
   if (p->absorb != ESPEC_ABS_NONE) ND_CK(cudaMemcpyAsync(p->d_vabc, vabc, 8 * n, kind, st));
-  const int rp = put_complex(p->stage, p->d_psi0, psi_re, psi_im, n, where, st);
+  const int rp = pairs ? put_pairs(p->d_psi0, psi_re, n, where, st)
+                       : put_complex(p->stage, p->d_psi0, psi_re, psi_im, n, where, st);
   if (rp) return rp;
   const int rc = p->precision == ESPEC_FP64 ? build_tables<double>(p, st)
                                             : build_tables<float>(p, st);
@@ -807,8 +810,13 @@ extern "C" int espec_spond_results(espec_spond_plan* p, double* c_re, double* c_
   if (!p || p->c_cap < 0) return set_error(ESPEC_EINVAL, "no results: run the plan first");
   cudaStream_t st = (cudaStream_t)stream;
   const size_t nc = (size_t)p->c_cap + 1, n = (size_t)p->n;
-  int rc = get_complex(p->stage, p->d_c, c_re, c_im, nc, where, st);
-  if (rc == ESPEC_OK) rc = get_complex(p->stage, p->d_out, psi_re, psi_im, n, where, st);
+  const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
+  where &= ~ESPEC_MEM_INTERLEAVED;
+  int rc = pairs ? get_pairs(p->d_c, c_re, nc, where, st)
+                 : get_complex(p->stage, p->d_c, c_re, c_im, nc, where, st);
+  if (rc == ESPEC_OK)
+    rc = pairs ? get_pairs(p->d_out, psi_re, n, where, st)
+               : get_complex(p->stage, p->d_out, psi_re, psi_im, n, where, st);
   if (rc) return rc;
   if (where == ESPEC_MEM_HOST) {
     int err = 0;

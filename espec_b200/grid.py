@@ -39,14 +39,11 @@ class SilGrid:
         self.nsteps = None
 
     def load(self, vpot, psi, vabc=None, stream=None):
-        psi = np.asarray(psi)
-        self._keep = [N.f64(np.ravel(vpot, order="F") if np.ndim(vpot) > 1 else vpot),
-                      N.f64(np.real(psi).ravel(order="F") if psi.ndim > 1 else np.real(psi)),
-                      N.f64(np.imag(psi).ravel(order="F") if psi.ndim > 1 else np.imag(psi)),
+        z, re, im, where = N.complex_host(psi)
+        self._keep = [N.f64(np.ravel(vpot, order="F") if np.ndim(vpot) > 1 else vpot), z,
                       None if vabc is None else N.f64(np.ravel(vabc, order="F"))]
-        v, re, im, ab = self._keep
-        rc = N.load().espec_grid_load(self._h, N.ptr(v), N.ptr(ab), N.ptr(re), N.ptr(im),
-                                      N.MEM_HOST, stream)
+        rc = N.load().espec_grid_load(self._h, N.ptr(self._keep[0]), N.ptr(self._keep[2]), re, im,
+                                      where, stream)
         N.check(rc, "espec_grid_load")
 
     def run(self, nsteps, stream=None):
@@ -59,13 +56,11 @@ class SilGrid:
 
     def results(self, stream=None):
         """(C(t) complex [nsteps+1], psi complex [n] flattened x fastest)."""
-        ns = self.nsteps
-        cr, ci = np.zeros(ns + 1), np.zeros(ns + 1)
-        pr, pi = np.zeros(self.n), np.zeros(self.n)
-        rc = N.load().espec_grid_results(self._h, N.ptr(cr), N.ptr(ci), N.ptr(pr), N.ptr(pi),
-                                         N.MEM_HOST, stream)
+        c, psi = np.empty(self.nsteps + 1, complex), np.empty(self.n, complex)
+        rc = N.load().espec_grid_results(self._h, N.ptr(c), None, N.ptr(psi), None,
+                                         N.MEM_HOST | N.MEM_INTERLEAVED, stream)
         N.check(rc, "espec_grid_results")
-        return cr + 1j * ci, pr + 1j * pi
+        return c, psi
 
     def energies(self, stream=None):
         """(<u|H u> + <v|H v>, |u|^2 + |v|^2) of the current state (eigenerg.f)."""
@@ -178,12 +173,10 @@ class SpoGrid:
         self.nsteps = None
 
     def load(self, vpot, psi, vabc=None, stream=None):
-        psi = np.asarray(psi)
-        self._keep = [N.f64(vpot), N.f64(np.real(psi)), N.f64(np.imag(psi)),
-                      None if vabc is None else N.f64(vabc)]
-        v, re, im, ab = self._keep
-        N.check(N.load().espec_spond_load(self._h, N.ptr(v), N.ptr(ab), N.ptr(re), N.ptr(im),
-                                          N.MEM_HOST, stream), "espec_spond_load")
+        z, re, im, where = N.complex_host(psi)
+        self._keep = [N.f64(vpot), z, None if vabc is None else N.f64(vabc)]
+        N.check(N.load().espec_spond_load(self._h, N.ptr(self._keep[0]), N.ptr(self._keep[2]), re,
+                                          im, where, stream), "espec_spond_load")
 
     def run(self, nsteps, stream=None):
         N.check(N.load().espec_spond_run(self._h, int(nsteps), stream), "espec_spond_run")
@@ -203,12 +196,11 @@ class SpoGrid:
         return e.value, nr.value
 
     def results(self, stream=None):
-        ns = self.nsteps
-        cr, ci = np.zeros(ns + 1), np.zeros(ns + 1)
-        pr, pi = np.zeros(self.n), np.zeros(self.n)
-        N.check(N.load().espec_spond_results(self._h, N.ptr(cr), N.ptr(ci), N.ptr(pr), N.ptr(pi),
-                                             N.MEM_HOST, stream), "espec_spond_results")
-        return cr + 1j * ci, pr + 1j * pi
+        c, psi = np.empty(self.nsteps + 1, complex), np.empty(self.n, complex)
+        N.check(N.load().espec_spond_results(self._h, N.ptr(c), None, N.ptr(psi), None,
+                                             N.MEM_HOST | N.MEM_INTERLEAVED, stream),
+                "espec_spond_results")
+        return c, psi
 
     def close(self):
         if self._h:

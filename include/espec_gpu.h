@@ -88,6 +88,11 @@ extern "C" {
  * synchronises the stream before it reads or reuses the buffers */
 #define ESPEC_MEM_HOST_ASYNC 2
 
+/* added to `where` in espec_grid_load, espec_grid_results, espec_spond_load and
+ * espec_spond_results: complex arrays are interleaved (re, im) pairs at the _re
+ * pointer, the _im pointer is not used */
+#define ESPEC_MEM_INTERLEAVED 16
+
 /* launch shape of a batched split-operator run (espec_spo_set_launch) */
 #define ESPEC_LAUNCH_CLASSES 0     /* one kernel per packet size, concurrent streams */
 #define ESPEC_LAUNCH_PERSISTENT 1  /* one persistent kernel over every packet size   */
