@@ -2,22 +2,63 @@
 // real and imaginary float64 arrays: the reference's U/V and LNZVC columns)
 // and the device form (interleaved double2).  Host transfers go through a
 // contiguous (re | im) staging block owned by the plan, so each is one linear
-// copy; device arguments are (de)interleaved in place by a kernel.
+// copy; results of up to kStageSmall bytes are written by the kernel straight into
+// page-locked memory of the plan and copied on by the host after the caller's
+// synchronisation (a row of a printed table: no device-to-host copies, 8 us each);
+// device arguments are (de)interleaved in place by a kernel.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <cstring>
 
 #include "espec_gpu.h"
 #include "espec_internal.h"
 
 namespace espec {
 
+constexpr size_t kStageSmall = 64 * 1024;
+
 struct HostStage {
   double* d = nullptr;
   size_t bytes = 0;
+  double* h = nullptr;  // page-locked, kStageSmall bytes
+  struct Pending {
+    double* dst;
+    const double* src;
+    size_t bytes;
+  } pending[4];
+  int npending = 0;
+  size_t used = 0;  // bytes of h taken by the pending results
   void release() {
     if (d) cudaFree(d);
-    d = nullptr;
+    if (h) cudaFreeHost(h);
+    d = h = nullptr;
     bytes = 0;
+  }
+  // page-locked space for `size` bytes, or null (too large, or none to be had)
+  double* small(size_t size) {
+    if (used + size > kStageSmall || npending + 2 > 4) return nullptr;
+    if (!h && cudaHostAlloc((void**)&h, kStageSmall, cudaHostAllocPortable | cudaHostAllocMapped) !=
+                  cudaSuccess) {
+      (void)cudaGetLastError();
+      h = nullptr;
+      return nullptr;
+    }
+    double* p = h + used / sizeof(double);
+    used += size;
+    return p;
+  }
+  void later(double* dst, const double* src, size_t size) {
+    if (dst) pending[npending++] = Pending{dst, src, size};
+  }
+  // before a call's first result, and after its synchronisation
+  void drop() {
+    npending = 0;
+    used = 0;
+  }
+  void flush() {
+    for (int i = 0; i < npending; ++i) std::memcpy(pending[i].dst, pending[i].src, pending[i].bytes);
+    drop();
   }
 };
 
@@ -77,7 +118,9 @@ inline int put_complex(HostStage& s, double2* dst, const double* re, const doubl
   return ESPEC_OK;
 }
 
-// (re, im) at `where` <- src (device, n complex); either output may be null
+// (re, im) at `where` <- src (device, n complex); either output may be null.
+// ESPEC_MEM_HOST: complete once the caller has synchronised the stream and
+// called s.flush()
 inline int get_complex(HostStage& s, const double2* src, double* re, double* im, size_t n,
                        int where, cudaStream_t st) {
   if ((!re && !im) || n == 0) return ESPEC_OK;
@@ -85,6 +128,15 @@ inline int get_complex(HostStage& s, const double2* src, double* re, double* im,
     deinterleave_kernel<<<io_blocks(n), 256, 0, st>>>(src, re, im, n);
     IO_CK(cudaGetLastError());
     return ESPEC_OK;
+  }
+  if (where == ESPEC_MEM_HOST) {
+    if (double* p = s.small(16 * n)) {
+      deinterleave_kernel<<<io_blocks(n), 256, 0, st>>>(src, p, p + n, n);
+      IO_CK(cudaGetLastError());
+      s.later(re, p, 8 * n);
+      s.later(im, p + n, 8 * n);
+      return ESPEC_OK;
+    }
   }
   const int rc = stage_reserve(s, 16 * n);
   if (rc) return rc;

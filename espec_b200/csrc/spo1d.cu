@@ -722,10 +722,13 @@ extern "C" int espec_spo_load(espec_spo_plan* p, const double* vpot, const doubl
   if (p->absorb != ESPEC_ABS_NONE && !vabc) return set_error(ESPEC_EINVAL, "absorber table missing");
   cudaStream_t st = (cudaStream_t)stream;
   const size_t np = p->npts;
+  const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
+  where &= ~ESPEC_MEM_INTERLEAVED;
   const cudaMemcpyKind kind = on_host(where) ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   ESPEC_CK(cudaMemcpyAsync(p->d_vpot, vpot, np * 8, kind, st));
   if (vabc) ESPEC_CK(cudaMemcpyAsync(p->d_vabc, vabc, np * 8, kind, st));
-  int rc = put_complex(p->stage, p->d_psi0, psi_re, psi_im, np, where, st);
+  int rc = pairs ? put_pairs(p->d_psi0, psi_re, np, where, st)
+                 : put_complex(p->stage, p->d_psi0, psi_re, psi_im, np, where, st);
   if (rc) return rc;
   // the current state of a freshly loaded plan is psi0
   ESPEC_CK(cudaMemcpyAsync(p->d_psi, p->d_psi0, np * 16, cudaMemcpyDeviceToDevice, st));
@@ -847,11 +850,13 @@ static int prop_launch(espec_spo_plan* p, int nsteps, bool resume, cudaStream_t 
     }
     return persist_launch(p, nsteps, resume, st);
   }
-  ESPEC_CK(cudaEventRecord(p->ev_fork, st));
+  // packets of one size run on the caller's stream; several sizes side by side
+  const bool fork = p->classes.size() > 1;
+  if (fork) ESPEC_CK(cudaEventRecord(p->ev_fork, st));
   for (size_t ci = 0; ci < p->classes.size(); ++ci) {
     auto& c = p->classes[ci];
-    cudaStream_t cs = p->streams[ci];
-    ESPEC_CK(cudaStreamWaitEvent(cs, p->ev_fork, 0));
+    cudaStream_t cs = fork ? p->streams[ci] : st;
+    if (fork) ESPEC_CK(cudaStreamWaitEvent(cs, p->ev_fork, 0));
     cudaError_t e;
     if (p->method == ESPEC_SOD) {
       SodArgs a{};
@@ -900,8 +905,10 @@ static int prop_launch(espec_spo_plan* p, int nsteps, bool resume, cudaStream_t 
                                          : launch_n<float>(c.n, c.variant, a, c.count, false, cs);
     }
     if (e != cudaSuccess) return set_cuda_error("spo1d_kernel launch", e);
-    ESPEC_CK(cudaEventRecord(p->events[ci], cs));
-    ESPEC_CK(cudaStreamWaitEvent(st, p->events[ci], 0));
+    if (fork) {
+      ESPEC_CK(cudaEventRecord(p->events[ci], cs));
+      ESPEC_CK(cudaStreamWaitEvent(st, p->events[ci], 0));
+    }
   }
   if (p->method == ESPEC_SOD) p->has_prev = true;
   return ESPEC_OK;
@@ -925,18 +932,25 @@ extern "C" int espec_prop_energies(espec_spo_plan* p, double* e, double* norm, v
   if (!p || !e || !norm) return set_error(ESPEC_EINVAL, "null argument");
   if (!p->loaded) return set_error(ESPEC_EINVAL, "espec_spo_load has not been called");
   cudaStream_t st = (cudaStream_t)stream;
+  // few packets: the kernels write into page-locked memory
+  p->stage.drop();
+  double2* hd = (double2*)p->stage.small(16 * (size_t)p->npk);
+  p->stage.drop();
   for (auto& c : p->classes) {
-    DiagArgs a{p->d_psi, p->d_vpot, p->d_tc, c.d_kfreq, c.d_pkd, p->d_diag};
+    DiagArgs a{p->d_psi, p->d_vpot, p->d_tc, c.d_kfreq, c.d_pkd, hd ? hd : p->d_diag};
     cudaError_t err = c.any ? diag_any_launch(a, c.ap, c.d_tw, c.count, st)
                             : diag_launch(c.n, a, c.count, st);
     if (err != cudaSuccess) return set_cuda_error("diag1d_kernel launch", err);
   }
-  std::vector<double2> h(p->npk);
-  ESPEC_CK(cudaMemcpyAsync(h.data(), p->d_diag, 16 * (size_t)p->npk, cudaMemcpyDeviceToHost, st));
+  std::vector<double2> h(hd ? 0 : p->npk);
+  if (!hd) {
+    ESPEC_CK(cudaMemcpyAsync(h.data(), p->d_diag, 16 * (size_t)p->npk, cudaMemcpyDeviceToHost, st));
+    hd = h.data();
+  }
   ESPEC_CK(cudaStreamSynchronize(st));
   for (int i = 0; i < p->npk; ++i) {
-    e[i] = h[i].x;
-    norm[i] = h[i].y;
+    e[i] = hd[i].x;
+    norm[i] = hd[i].y;
   }
   return ESPEC_OK;
 }
@@ -946,10 +960,19 @@ extern "C" int espec_spo_results(espec_spo_plan* p, double* c_re, double* c_im, 
   if (!p || p->c_cap_steps < 0) return set_error(ESPEC_EINVAL, "no results: run the plan first");
   cudaStream_t st = (cudaStream_t)stream;
   const size_t nc = (size_t)p->npk * (p->c_cap_steps + 1);
-  int rc = get_complex(p->stage, p->d_c, c_re, c_im, nc, where, st);
-  if (rc == ESPEC_OK) rc = get_complex(p->stage, p->d_psi, psi_re, psi_im, p->npts, where, st);
+  const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
+  where &= ~ESPEC_MEM_INTERLEAVED;
+  p->stage.drop();
+  int rc = pairs ? get_pairs(p->d_c, c_re, nc, where, st)
+                 : get_complex(p->stage, p->d_c, c_re, c_im, nc, where, st);
+  if (rc == ESPEC_OK)
+    rc = pairs ? get_pairs(p->d_psi, psi_re, p->npts, where, st)
+               : get_complex(p->stage, p->d_psi, psi_re, psi_im, p->npts, where, st);
   if (rc) return rc;
-  if (where == ESPEC_MEM_HOST) ESPEC_CK(cudaStreamSynchronize(st));
+  if (where == ESPEC_MEM_HOST) {
+    ESPEC_CK(cudaStreamSynchronize(st));
+    p->stage.flush();
+  }
   return ESPEC_OK;
 }
 
@@ -973,8 +996,12 @@ extern "C" int espec_prop_previous(espec_spo_plan* p, double* psi_re, double* ps
   if (!p || p->method != ESPEC_SOD || p->c_cap_steps < 0)
     return set_error(ESPEC_EINVAL, "previous state exists for run SOD plans only");
   cudaStream_t st = (cudaStream_t)stream;
+  p->stage.drop();
   const int rc = get_complex(p->stage, p->d_psi_prev, psi_re, psi_im, p->npts, where, st);
   if (rc) return rc;
-  if (where == ESPEC_MEM_HOST) ESPEC_CK(cudaStreamSynchronize(st));
+  if (where == ESPEC_MEM_HOST) {
+    ESPEC_CK(cudaStreamSynchronize(st));
+    p->stage.flush();
+  }
   return ESPEC_OK;
 }

@@ -678,9 +678,13 @@ extern "C" int espec_spond_previous(espec_spond_plan* p, double* psi_re, double*
   if (!p || p->method != ESPEC_SOD || !p->has_state)
     return set_error(ESPEC_EINVAL, "previous state exists for run SOD plans only");
   cudaStream_t st = (cudaStream_t)stream;
+  p->stage.drop();
   const int rc = get_complex(p->stage, p->d_prev, psi_re, psi_im, (size_t)p->n, where, st);
   if (rc) return rc;
-  if (where == ESPEC_MEM_HOST) ND_CK(cudaStreamSynchronize(st));
+  if (where == ESPEC_MEM_HOST) {
+    ND_CK(cudaStreamSynchronize(st));
+    p->stage.flush();
+  }
   return ESPEC_OK;
 }
 
@@ -812,6 +816,7 @@ extern "C" int espec_spond_results(espec_spond_plan* p, double* c_re, double* c_
   const size_t nc = (size_t)p->c_cap + 1, n = (size_t)p->n;
   const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
   where &= ~ESPEC_MEM_INTERLEAVED;
+  p->stage.drop();
   int rc = pairs ? get_pairs(p->d_c, c_re, nc, where, st)
                  : get_complex(p->stage, p->d_c, c_re, c_im, nc, where, st);
   if (rc == ESPEC_OK)
@@ -822,6 +827,7 @@ extern "C" int espec_spond_results(espec_spond_plan* p, double* c_re, double* c_
     int err = 0;
     ND_CK(cudaMemcpyAsync(&err, p->d_bar + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     ND_CK(cudaStreamSynchronize(st));
+    p->stage.flush();
     if (err) return set_error(ESPEC_ECUDA, "a grid barrier of the split-operator kernel timed out");
   }
   return ESPEC_OK;

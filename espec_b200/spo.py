@@ -70,12 +70,10 @@ class SpoBatch:
             rc = lib.espec_spo_load(self._h, N.ptr(vpot), N.ptr(vabc), N.ptr(re), N.ptr(im),
                                     N.MEM_DEVICE, stream)
         else:
-            psi = np.asarray(psi)
-            self._keep = [N.f64(vpot), N.f64(psi.real), N.f64(np.imag(psi)),
-                          None if vabc is None else N.f64(vabc)]
-            v, re, im, ab = self._keep
-            rc = lib.espec_spo_load(self._h, N.ptr(v), N.ptr(ab), N.ptr(re), N.ptr(im),
-                                    N.MEM_HOST, stream)
+            z, re, im, where = N.complex_host(psi)
+            self._keep = [N.f64(vpot), z, None if vabc is None else N.f64(vabc)]
+            rc = lib.espec_spo_load(self._h, N.ptr(self._keep[0]), N.ptr(self._keep[2]), re, im,
+                                    where, stream)
         N.check(rc, "espec_spo_load")
 
     def run(self, nsteps, stream=None):
@@ -100,15 +98,12 @@ class SpoBatch:
 
     def results(self, stream=None):
         """(C(t) [npk, nsteps+1] complex, psi(TF) concatenated complex), host."""
-        ns = self.nsteps
-        cr = np.zeros(self.npk * (ns + 1))
-        ci = np.zeros_like(cr)
-        pr = np.zeros(self.total)
-        pi = np.zeros(self.total)
-        rc = N.load().espec_spo_results(self._h, N.ptr(cr), N.ptr(ci), N.ptr(pr), N.ptr(pi),
-                                        N.MEM_HOST, stream)
+        c = np.empty((self.npk, self.nsteps + 1), complex)
+        psi = np.empty(self.total, complex)
+        rc = N.load().espec_spo_results(self._h, N.ptr(c), None, N.ptr(psi), None,
+                                        N.MEM_HOST | N.MEM_INTERLEAVED, stream)
         N.check(rc, "espec_spo_results")
-        return (cr + 1j * ci).reshape(self.npk, ns + 1), pr + 1j * pi
+        return c, psi
 
     def results_into(self, c_re, c_im, psi_re, psi_im, stream=None, asynchronous=False):
         """Copy C(t) ([npk * (nsteps+1)], packet-major) and psi(TF) as separate

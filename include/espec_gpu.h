@@ -88,8 +88,8 @@ extern "C" {
  * synchronises the stream before it reads or reuses the buffers */
 #define ESPEC_MEM_HOST_ASYNC 2
 
-/* added to `where` in espec_grid_load, espec_grid_results, espec_spond_load and
- * espec_spond_results: complex arrays are interleaved (re, im) pairs at the _re
+/* added to `where` in the load and results calls of the plans (espec_spo_*,
+ * espec_grid_*, espec_spond_*): complex arrays are interleaved (re, im) pairs at the _re
  * pointer, the _im pointer is not used */
 #define ESPEC_MEM_INTERLEAVED 16
 
