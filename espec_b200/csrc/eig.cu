@@ -1,8 +1,9 @@
 // eig.cu -- batched initial-state eigensolver on 2D grids (eSPec's LANCZSG,
 // lanczsc.f:56-120, with LNZ lnz.f:76-119 and REORT reort.f:65-80), FP64.
 //
-// One CTA per problem (one potential): for each of nstates target states,
-// explicitly restarted Lanczos -- m Lanczos steps with full classical
+// One CTA per problem (one potential), or a cluster of two where that leaves no SM
+// without a problem: for each of nstates target states, explicitly restarted
+// Lanczos -- m Lanczos steps with full classical
 // Gram-Schmidt reorthogonalisation from the current vector, the lowest Ritz
 // pair of the m x m tridiagonal matrix, restart from that Ritz vector --
 // until the true residual |H v - theta v| (one more H*v) is at most tol.  The
@@ -16,6 +17,7 @@
 // Cold start: the reference's LCG vectors (rans.f:38-39, NSEED = 1, first N
 // draws discarded, lanczsc.f:56-62); warm start: any given vectors.
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include <cmath>
 #include <vector>
@@ -33,6 +35,7 @@ constexpr int kEigThreads = 512;
 constexpr int kEigChains = 1024;
 // points of a current vector kept in shared memory (beside 31 KB of static arrays)
 constexpr int kEigMaxSmemN = 24 * 1024;
+constexpr int kEigMinSplitN = 2048;  // points from which two CTAs share a problem
 constexpr int kEigMaxM = 40;      // NREORT = 40 in lanczsc.f:55
 constexpr int kEigMaxStates = 16;  // locked states held in the reorthogonalisation
 
@@ -69,19 +72,51 @@ __device__ __forceinline__ double hx(const EigArgs& a, const double* V, const do
   return s;
 }
 
-// CTA sum of the two chains of every thread (chains t and t + kEigThreads)
-__device__ __forceinline__ double cta_sum(double x0, double x1, double* ws) {
+// A problem's share of this CTA: with CS = 2 the chains are split between the two
+// CTAs of a cluster (rank 0: chains 0..511), so a thread has one, and values that
+// the other CTA needs are stored in its shared memory as well.  Every sum keeps
+// the order it has in one CTA: the results do not depend on CS.
+template <int CS>
+struct Share {
+  static constexpr int kStep = CS * kEigThreads;  // from point to point of a thread
+  int rank, first;
+  __device__ __forceinline__ Share()
+      : rank(CS == 1 ? 0 : (int)(blockIdx.x & 1)), first((int)threadIdx.x + rank * kEigThreads) {}
+  // chain (of the thread's two, CS = 1) of its i-th point
+  static __device__ __forceinline__ int chain(int i) { return CS == 1 ? i & 1 : 0; }
+  __device__ __forceinline__ void sync() const {
+    if (CS == 1) {
+      __syncthreads();
+    } else {
+      asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    }
+  }
+  // *p = v here and in the other CTA (p in shared memory)
+  __device__ __forceinline__ void put(double* p, double v) const {
+    *p = v;
+    if (CS == 2) {
+      uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank ^ 1));
+      asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
+    }
+  }
+};
+
+// sum of all chains: the thread's chain sums x0 (and x1, CS = 1)
+template <int CS>
+__device__ __forceinline__ double chain_sum(const Share<CS>& sh, double x0, double x1, double* ws) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     x0 += __shfl_xor_sync(0xffffffffu, x0, o);
-    x1 += __shfl_xor_sync(0xffffffffu, x1, o);
+    if (CS == 1) x1 += __shfl_xor_sync(0xffffffffu, x1, o);
   }
   if (lane == 0) {
-    ws[warp] = x0;
-    ws[warp + kEigThreads / 32] = x1;
+    sh.put(ws + warp + sh.rank * (kEigThreads / 32), x0);
+    if (CS == 1) ws[warp + kEigThreads / 32] = x1;
   }
-  __syncthreads();
+  sh.sync();
   double s = 0.0;
   for (int w = 0; w < kEigChains / 32; ++w) s += ws[w];
   __syncthreads();
@@ -95,12 +130,14 @@ __device__ __forceinline__ double cta_sum(double x0, double x1, double* ws) {
 // kDotLoads loads of the vector in flight per lane (with two, one CTA drew
 // about 20 GB/s).  part: [2 (kEigMaxM + kEigMaxStates)][32] in shared memory.
 constexpr int kDotLoads = 32;
-__device__ __forceinline__ void warp_dots(const double* x, const double* L, int nl,
-                                          const double* lock, int nlock, int n, double* part,
-                                          double* red) {
+template <int CS>
+__device__ __forceinline__ void warp_dots(const Share<CS>& sh, const double* x, const double* L,
+                                          int nl, const double* lock, int nlock, int n,
+                                          double* part, double* red) {
+  constexpr int NW = kEigThreads / 32;  // even: a vector's two chain sets stay in one CTA
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nv = nl + nlock;
-  for (int task = warp; task < 2 * nv; task += kEigThreads / 32) {
+  for (int task = warp + sh.rank * NW; task < 2 * nv; task += CS * NW) {
     const int q = task >> 1;
     const double* y = q < nl ? L + (long)q * n : lock + (long)(q - nl) * n;
     double s = 0.0;
@@ -116,29 +153,30 @@ __device__ __forceinline__ void warp_dots(const double* x, const double* L, int 
     part[task * 32 + lane] = s;
   }
   __syncthreads();
-  for (int q = warp; q < nv; q += kEigThreads / 32) {
+  for (int q = warp; q < nv; q += NW) {
+    if (CS == 2 && (2 * q / NW & 1) != sh.rank) continue;
     double s = part[2 * q * 32 + lane] + part[(2 * q + 1) * 32 + lane];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red[q] = s;
+    if (lane == 0) sh.put(red + q, s);
   }
-  __syncthreads();
+  sh.sync();
 }
 
-// w[i] = init(k_i) - sum_j lock_j(k_i) a_j - sum_q L_q(k_i) b_q (sgn = -1), or
-// + (sgn = 1), for the thread's points k_i = t + i kEigThreads, four at a time so
-// that their loads overlap; put(k, w) takes each, in order
-template <class Init, class Put>
-__device__ __forceinline__ void combine(const double* lock, const double* ca, int nlock,
+// w[i] = init(k_i) - sum_j lock_j(k_i) a_j - sum_q L_q(k_i) b_q (or plus),
+// for the thread's points, four at a time so that their loads overlap; put(k,
+// chain, w) takes each, in order
+template <int CS, class Init, class Put>
+__device__ __forceinline__ void combine(const Share<CS>& sh, const double* lock, const double* ca, int nlock,
                                         const double* L, const double* cb, int nl, int n,
                                         bool plus, Init init, Put put) {
   constexpr int P = 4;
-  for (int k0 = threadIdx.x; k0 < n; k0 += P * kEigThreads) {
+  for (int k0 = sh.first; k0 < n; k0 += P * sh.kStep) {
     double w[P];
     int kk[P];
 #pragma unroll
     for (int i = 0; i < P; ++i) {
-      kk[i] = min(k0 + i * kEigThreads, n - 1);
+      kk[i] = min(k0 + i * sh.kStep, n - 1);
       w[i] = init(kk[i]);
     }
     for (int j = 0; j < nlock; ++j) {
@@ -163,7 +201,7 @@ __device__ __forceinline__ void combine(const double* lock, const double* ca, in
     }
 #pragma unroll
     for (int i = 0; i < P; ++i)
-      if (k0 + i * kEigThreads < n) put(k0 + i * kEigThreads, i & 1, w[i]);
+      if (k0 + i * sh.kStep < n) put(k0 + i * sh.kStep, sh.chain(i), w[i]);
   }
 }
 
@@ -223,10 +261,11 @@ __host__ __device__ inline void tri_solve_pivoted(int m, const double* al, const
 
 }  // namespace
 
-// SM: the current vector in shared memory (grids up to kEigMaxSmemN points);
-// otherwise it is the work array in global memory
-template <bool SM>
-__global__ void __launch_bounds__(kEigThreads) eig_kernel(EigArgs a) {
+// SM: the current vector in shared memory (grids up to kEigMaxSmemN points), all
+// of it in each CTA of a cluster; otherwise it is the work array in global memory
+template <bool SM, int CS>
+__global__ void __launch_bounds__(kEigThreads, 1) eig_kernel(EigArgs a) {
+  static_assert(SM || CS == 1, "a cluster exchanges the current vector through shared memory");
   constexpr int NV = kEigMaxM + kEigMaxStates;
   extern __shared__ double eig_dyn[];
   __shared__ double part[2 * NV * 32];
@@ -235,7 +274,9 @@ __global__ void __launch_bounds__(kEigThreads) eig_kernel(EigArgs a) {
   __shared__ double s_al[kEigMaxM], s_bt[kEigMaxM], s_e2[kEigMaxM], s_y[kEigMaxM];
   __shared__ double s_theta;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int p = blockIdx.x, n = a.n, m = a.m;
+  const int p = blockIdx.x / CS, n = a.n, m = a.m;
+  const Share<CS> sh;
+  const int k1 = sh.first, step = sh.kStep;
   const double* V = a.vpot + (long)p * n;
   double* L = a.L + (long)p * m * n;
   double* work = a.work + (long)p * n;
@@ -245,42 +286,42 @@ __global__ void __launch_bounds__(kEigThreads) eig_kernel(EigArgs a) {
     const double* st = a.start + ((long)p * a.nstates + K) * n;
     double* v = a.vec + ((long)p * a.nstates + K) * n;
     for (int k = t; k < n; k += kEigThreads) F[k] = st[k];
-    __syncthreads();
+    sh.sync();  // and the state before is in a.vec
     int count = 0;
     double res = 0.0;
     const double* lock = a.vec + (long)p * a.nstates * n;  // states 0..K-1
     for (int rs = 0; rs < a.maxrest; ++rs) {
       // ---- project the locked states out of the current vector
       if (K > 0) {
-        warp_dots(F, nullptr, 0, lock, K, n, part, red);
-        combine(lock, red, K, nullptr, nullptr, 0, n, false, [&](int k) { return F[k]; },
+        warp_dots(sh, F, nullptr, 0, lock, K, n, part, red);
+        combine(sh, lock, red, K, nullptr, nullptr, 0, n, false, [&](int k) { return F[k]; },
                 [&](int k, int, double w) { F[k] = w; });
         __syncthreads();
       }
       // ---- m Lanczos steps (lnz.f:76-119)
       double nn[2] = {0.0, 0.0};
-      for (int k = t, c = 0; k < n; k += kEigThreads, c ^= 1) {
-        if (c) nn[1] += F[k] * F[k];
+      for (int k = k1, i = 0; k < n; k += step, ++i) {
+        if (sh.chain(i)) nn[1] += F[k] * F[k];
         else nn[0] += F[k] * F[k];
       }
-      double bt0 = sqrt(cta_sum(nn[0], nn[1], ws));
+      double bt0 = sqrt(chain_sum(sh, nn[0], nn[1], ws));
       for (int it = 0; it < m; ++it) {
         double* Li = L + (long)it * n;
         const double* Lp = it ? L + (long)(it - 1) * n : nullptr;
 #pragma unroll 4
-        for (int k = t; k < n; k += kEigThreads) {
+        for (int k = k1; k < n; k += step) {
           const double vi = F[k] / bt0;
           Li[k] = vi;
-          if (SM) F[k] = vi;
+          if (SM) sh.put(F + k, vi);
         }
-        __syncthreads();
+        sh.sync();
         // w = H vi - bt0 v_prev into work, al = <vi, w> (lnz.f:96-107)
         const double* x = SM ? F : Li;
         nn[0] = nn[1] = 0.0;
 #pragma unroll 2
-        for (int k0 = t; k0 < n; k0 += kEigChains) {
+        for (int k0 = k1; k0 < n; k0 += kEigChains) {
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
+          for (int c = 0; c < 2 / CS; ++c) {
             const int k = k0 + c * kEigThreads;
             if (k < n) {
               const double vp = it ? Lp[k] : 0.0;
@@ -290,23 +331,27 @@ __global__ void __launch_bounds__(kEigThreads) eig_kernel(EigArgs a) {
             }
           }
         }
-        const double al = cta_sum(nn[0], nn[1], ws);
+        const double al = chain_sum(sh, nn[0], nn[1], ws);
         if (t == 0) s_al[it] = al;
         ++count;
         // work = w - al vi, then classical Gram-Schmidt against the locked
         // states and L_0..L_it (reort.f:65-80: all dot products, then all
         // updates): one pass for the dots, one for the updates and the norm
 #pragma unroll 4
-        for (int k = t; k < n; k += kEigThreads) F[k] = work[k] - al * x[k];
-        __syncthreads();
-        warp_dots(F, L, it + 1, lock, K, n, part, red);
+        for (int k = k1; k < n; k += step) {
+          const double w = work[k] - al * x[k];
+          if (SM) sh.put(F + k, w);
+          else F[k] = w;
+        }
+        sh.sync();
+        warp_dots(sh, F, L, it + 1, lock, K, n, part, red);
         nn[0] = nn[1] = 0.0;
-        combine(lock, red + it + 1, K, L, red, it + 1, n, false, [&](int k) { return F[k]; },
+        combine(sh, lock, red + it + 1, K, L, red, it + 1, n, false, [&](int k) { return F[k]; },
                 [&](int k, int c, double w) {
                   F[k] = w;
                   nn[c] += w * w;
                 });
-        bt0 = sqrt(cta_sum(nn[0], nn[1], ws));
+        bt0 = sqrt(chain_sum(sh, nn[0], nn[1], ws));
         if (t == 0) s_bt[it] = bt0;
       }
       __syncthreads();
@@ -357,28 +402,31 @@ __global__ void __launch_bounds__(kEigThreads) eig_kernel(EigArgs a) {
       __syncthreads();
       // ---- the new vector L y, normalised (lanczsc.f:99-113, FATN = ECNORM)
       nn[0] = nn[1] = 0.0;
-      combine(nullptr, nullptr, 0, L, s_y, m, n, true, [](int) { return 0.0; },
+      combine(sh, nullptr, nullptr, 0, L, s_y, m, n, true, [](int) { return 0.0; },
               [&](int k, int c, double w) {
                 F[k] = w;
                 nn[c] += w * w;
               });
-      const double inv = 1.0 / sqrt(cta_sum(nn[0], nn[1], ws));
-      for (int k = t; k < n; k += kEigThreads) F[k] *= inv;
-      __syncthreads();
+      const double inv = 1.0 / sqrt(chain_sum(sh, nn[0], nn[1], ws));
+      for (int k = k1; k < n; k += step) {
+        if (SM) sh.put(F + k, F[k] * inv);
+        else F[k] *= inv;
+      }
+      sh.sync();
       // ---- true residual |H v - theta v|
       const double th = s_theta;
       nn[0] = nn[1] = 0.0;
-      for (int k = t, c = 0; k < n; k += kEigThreads, c ^= 1) {
+      for (int k = k1, i = 0; k < n; k += step, ++i) {
         const double r = hx(a, V, F, k, 1.0) - th * F[k];
-        if (c) nn[1] += r * r;
+        if (sh.chain(i)) nn[1] += r * r;
         else nn[0] += r * r;
       }
       ++count;
-      res = sqrt(cta_sum(nn[0], nn[1], ws));
+      res = sqrt(chain_sum(sh, nn[0], nn[1], ws));
       if (res <= a.tol) break;
     }
-    for (int k = t; k < n; k += kEigThreads) v[k] = F[k];
-    if (t == 0) {
+    for (int k = k1; k < n; k += step) v[k] = F[k];
+    if (t == 0 && sh.rank == 0) {
       const long o = (long)p * a.nstates + K;
       a.eval[o] = s_theta;
       a.resid[o] = res;
@@ -490,12 +538,32 @@ extern "C" int espec_eig_solve_dev(int nprob, const int* np, const double* shm,
   a.m = m;
   a.maxrest = maxrest;
   a.tol = tol;
+  cudaStream_t st = (cudaStream_t)stream;
+  const size_t smem = sizeof(double) * (size_t)a.n, most = sizeof(double) * kEigMaxSmemN;
+  int dev = 0, nsm = 0;
+  EIG_CK(cudaGetDevice(&dev));
+  EIG_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   if (a.n > kEigMaxSmemN) {
-    eig_kernel<false><<<nprob, kEigThreads, 0, (cudaStream_t)stream>>>(a);
+    eig_kernel<false, 1><<<nprob, kEigThreads, 0, st>>>(a);
+  } else if (2 * nprob <= nsm && a.n >= kEigMinSplitN) {
+    static DeviceFlags attr;
+    EIG_CK(set_max_smem_once(attr, eig_kernel<true, 2>, most));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2 * (unsigned)nprob);
+    cfg.blockDim = dim3(kEigThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute la{};
+    la.id = cudaLaunchAttributeClusterDimension;
+    la.val.clusterDim.x = 2;
+    la.val.clusterDim.y = la.val.clusterDim.z = 1;
+    cfg.attrs = &la;
+    cfg.numAttrs = 1;
+    EIG_CK(cudaLaunchKernelEx(&cfg, eig_kernel<true, 2>, a));
   } else {
     static DeviceFlags attr;
-    EIG_CK(set_max_smem_once(attr, eig_kernel<true>, sizeof(double) * kEigMaxSmemN));
-    eig_kernel<true><<<nprob, kEigThreads, sizeof(double) * a.n, (cudaStream_t)stream>>>(a);
+    EIG_CK(set_max_smem_once(attr, eig_kernel<true, 1>, most));
+    eig_kernel<true, 1><<<nprob, kEigThreads, smem, st>>>(a);
   }
   EIG_CK(cudaGetLastError());
   return ESPEC_OK;
