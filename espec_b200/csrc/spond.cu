@@ -2,23 +2,19 @@
 // spofft.f:64-200) on one 2D or 3D grid, FP64 or mixed (FP32 data, FP64
 // tables), and the plan behind espec_spond_* (include/espec_gpu.h).
 //
-// Line transforms: one warp per line of N = 32 P points (P = 1..16); lane l
-// holds points 32 j + l in register j.  Forward = four-step: a P-point DFT
-// in registers (radix-2 decimation in frequency), twiddles W_N^(l k1), then a
-// 32-point DFT across the lanes by __shfl_xor butterflies (decimation in
-// frequency): lane l, register r ends with frequency brev_P(r) + P brev_32(l).
-// The inverse is the exact mirror with conjugate twiddles (unnormalised).
-// Between the passes of a step each row stays in that permuted frequency
-// order; only the kinetic pass needs the frequencies, via its table.
-//
-// Passes per step (the V half-steps of consecutive steps merged, g = h^2):
+// A run is one cooperative kernel (spond.cuh, nd_kernel) of at most one CTA per
+// SM; its passes are separated by grid barriers with a bounded wait.  Passes
+// per step, the V half-steps of consecutive steps merged (g = h^2):
 //   2D: x pass [inverse x, C(t), x-space phase, forward x]; y pass [forward y,
 //       kinetic phase, inverse y]
 //   3D: x pass; y pass [forward y]; z pass [forward z, kinetic, inverse z];
-//       y pass [inverse y]
-// Strided passes stage a tile of 8 adjacent x columns in shared memory.  The
-// fftshift swaps of spofft.f:120-133/178-191 cancel and are not done; the
-// 1/N of the reference's B factor is folded into the kinetic table.
+//       y pass [inverse y]; or, where an xy plane fits in shared memory, one
+//       pass [inverse y, x pass, forward y] over whole planes and the z pass
+// Lines are transformed in the registers of 4 to 32 lanes (LineFft); between
+// the passes a line stays in the transform's storage order, and only the
+// kinetic pass needs the frequencies, via its table (freq_at).  The fftshift
+// swaps of spofft.f:120-133/178-191 cancel and are not done; the 1/N of the
+// reference's B factor is folded into the kinetic table.
 #include <cuda/atomic>
 #include <cuda_runtime.h>
 
@@ -324,7 +320,7 @@ void digt_nd(const espec_spond_plan* p, std::vector<double>& tc) {
 
 // how a grid's passes are cut
 struct NdConfig {
-  int threads = 256, grid = 1, lc = 3, fused = 0;
+  int threads = 256, grid = 1, lc = 3, fused = 0, kstage = 0;
   size_t smem = 0;
   NdLayout layout{};
 };
@@ -343,9 +339,9 @@ size_t packed_bytes(int ln) {
 
 // Threads: 512 where a thread's points, twiddles and preloaded factors fit 128
 // registers, else 256 (FP64 lines of 256 and 512 points, FP32 of 512).
-// Fused xy planes: where a plane fits in shared memory and there are planes
-// for most SMs -- the y passes then cost no memory traffic and no grid
-// barrier, but a plane runs on one SM.
+// Fused xy planes: where a plane and the copies of its rows' inputs fit in
+// shared memory and there are planes for most SMs -- the y passes then cost no
+// memory traffic and no grid barrier, but a plane runs on one SM.
 // Tiles of the column passes: 8 adjacent columns (128 bytes in FP64), fewer
 // where that would leave SMs without a tile.  CTAs: the fewest that keep the
 // largest share, at most one per SM.
@@ -364,7 +360,7 @@ NdConfig nd_config(const espec_spond_plan* p) {
   const size_t plane = sizeof(cpx<R>) * (size_t)p->np[0] * p->np[1];
   size_t tw = 0;
   for (int ax = 0; ax < p->ndim; ++ax) tw += packed_bytes<R>(ln[ax]);
-  c.fused = p->ndim == 3 && tw + plane <= kNdMaxSmem && p->np[2] >= kFusedMinPlanes;
+  c.fused = p->ndim == 3 && tw + plane + 65536 <= kNdMaxSmem && p->np[2] >= kFusedMinPlanes;
   for (int ax = 0; ax < 2; ++ax) c.layout.by_pos[ax] = c.fused;
   auto threads_of = [&](int ax) { return ln[ax] == 9 ? 5 : ln[ax] - 3; };  // log2, per line
   auto tiles = [&](int lc) {
@@ -387,7 +383,18 @@ NdConfig nd_config(const espec_spond_plan* p) {
   if (!c.fused && (p->n >> ln[0]) / (32 >> threads_of(0)) <= 8L * c.grid) c.threads = 256;
   const int e = mx == 9 ? 16 : 8;
   size_t ex = sizeof(cpx<R>) * (size_t)c.threads * e * 9 / 8;
-  if (c.fused) ex = std::max(ex, plane);
+  if (c.fused) ex = std::max(ex, plane + (size_t)c.threads / 32 * 4096);
+  // the kinetic pass copies tiles ahead where a group has more than one (with
+  // one there is nothing to overlap), their rows are whole 16-byte pieces, the
+  // buffers fit and a line has 8 points per thread
+  const int ka = p->ndim - 1, gt = 1 << (threads_of(ka) + c.lc), groups = c.threads / gt;
+  const size_t tile = (sizeof(cpx<R>) + sizeof(typename Ph<R>::type)) * (size_t)p->np[ka] << c.lc;
+  const size_t kst = sizeof(cpx<R>) * (size_t)c.threads * 9 + 2 * groups * tile;
+  if (ln[ka] <= 8 && c.lc >= 2 && !(p->quirks & ESPEC_Q_SPO_INPLACE) &&
+      tiles(c.lc) > (long)c.grid * groups && tw + kst <= kNdMaxSmem) {
+    c.kstage = 1;
+    ex = std::max(ex, kst);
+  }
   c.smem = tw + ex;
   return c;
 }
@@ -477,6 +484,7 @@ NdArgs<R> nd_args(const espec_spond_plan* p, const NdConfig& c) {
   a.n = p->n;
   a.fused = c.fused;
   a.lc = c.lc;
+  a.kstage = c.kstage;
   a.psi0 = p->d_psi0;
   a.bar = p->d_bar;
   a.err = (int*)(p->d_bar + 1);

@@ -274,6 +274,7 @@ struct NdArgs {
   int nsteps, from_start;
   int fused;          // 3D: xy planes whole in shared memory
   int lc;             // log2 of the adjacent columns of a tile
+  int kstage;         // the kinetic pass copies its tiles ahead (kin_staged)
   unsigned long long* bar;  // grid barrier arrivals of the launch (zeroed before it)
   int* err;                 // set when a barrier wait gave up
   long spin_limit;
@@ -301,15 +302,37 @@ enum { kFirst = 0, kMid = 1, kLast = 2, kFwd0 = 3, kUpd = 4, kUpdFwd = 5 };
 __host__ __device__ constexpr bool row_inverse(int mode) { return mode != kFirst && mode != kFwd0; }
 __host__ __device__ constexpr bool row_forward(int mode) { return mode != kLast && mode != kUpd; }
 
-// what row_points reads of a row's points; loaded before the inverse transform
-// where the registers allow (8 points per thread, 256 threads), so that the
-// two overlap
-template <typename R, int E, int MODE, int T>
+// asynchronous copies into shared memory
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int PENDING>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// what row_points reads of a row's points; loaded before the inverse transform so
+// that the two overlap: into registers where they allow it (8 points per thread,
+// 256 threads), or (ST) the 16-byte values into the lane's places of shared memory
+template <typename R, int E, int MODE, int T, bool ST = false>
 struct RowIn {
-  static constexpr bool kEarlyP = E == 8 && row_inverse(MODE) && T == 256;
-  static constexpr bool kEarlyQ = kEarlyP;
+  static constexpr bool kStaged = ST && E == 8 && row_inverse(MODE);
+  static constexpr bool kEarlyP = E == 8 && row_inverse(MODE) && T == 256 && !kStaged;
+  static constexpr bool kEarlyQ = kEarlyP || (kStaged && (T == 256 || sizeof(R) == 4));
   double2 p[E], q[E];
   typename Ph<R>::type ph[E];
+  double2* st;  // kStaged: [E][32]
+  __device__ __forceinline__ const double2* source(const NdArgs<R>& a, const SodRow& o) const {
+    return MODE == kMid || MODE == kLast ? a.w : o.src;
+  }
   __device__ __forceinline__ void load_p(const NdArgs<R>& a, const SodRow& o, int e, int x) {
     if (MODE == kFirst || MODE == kFwd0) p[e] = a.psi_start[x];
     else if (MODE == kMid || MODE == kLast) p[e] = __ldg(a.w + x);
@@ -322,6 +345,13 @@ struct RowIn {
     else if (MODE == kUpd || MODE == kUpdFwd) q[e] = o.old[x];
   }
   __device__ __forceinline__ void early(const NdArgs<R>& a, const SodRow& o, int x0, int step) {
+    if (kStaged) {
+      const double2* src = source(a, o);
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        copy_async<16>(st + 32 * e + (threadIdx.x & 31), src + x0 + e * step);
+      copy_commit();
+    }
     if (kEarlyP) {
 #pragma unroll
       for (int e = 0; e < E; ++e) load_p(a, o, e, x0 + e * step);
@@ -333,18 +363,20 @@ struct RowIn {
   }
 };
 
-template <typename R, int LN, int MODE, int T>
+template <typename R, int LN, int MODE, int T, bool ST>
 __device__ __forceinline__ void row_points(const NdArgs<R>& a, const SodRow& o, cpx<R>* v,
-                                           RowIn<R, LineFft<R, LN>::E, MODE, T>& in,
+                                           RowIn<R, LineFft<R, LN>::E, MODE, T, ST>& in,
                                            const LineFft<R, LN>& fft, int base, double& cr,
                                            double& ci) {
   constexpr int E = LineFft<R, LN>::E, L = LineFft<R, LN>::L;
+  if (in.kStaged) copy_wait<0>();  // a lane reads its own copies only
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int x = base + e * L + fft.t;
     // 128 registers: the loads of half a row's points at a time
     if (T == 512 && e == E / 2) asm volatile("" ::: "memory");
-    if (!in.kEarlyP) in.load_p(a, o, e, x);
+    if (in.kStaged) in.p[e] = in.st[32 * e + (threadIdx.x & 31)];
+    else if (!in.kEarlyP) in.load_p(a, o, e, x);
     if (!in.kEarlyQ) in.load_q(a, o, e, x);
     const double2 p = in.p[e];
     if (MODE == kFirst) {
@@ -424,7 +456,7 @@ __device__ __noinline__ double2 rows_phase(const NdArgs<R>& a, const SodRow& o,
       in.early(a, o, base + fft.t, L);
       fft.inverse(v, at, sync);
     }
-    row_points<R, LN, MODE, T>(a, o, v, in, fft, base, cr, ci);
+    row_points<R, LN, MODE, T, false>(a, o, v, in, fft, base, cr, ci);
     if (row_forward(MODE)) {
       fft.forward(v, at, sync);
 #pragma unroll
@@ -493,6 +525,73 @@ __device__ __noinline__ void cols_phase(const NdArgs<R>& a, int axis,
   }
 }
 
+// the kinetic pass with each group's next tile (state and factors) copied into
+// shared memory while the current one is transformed: two buffers per group
+// behind the exchange space.  Without the copies all warps load, transform and
+// store in step and neither the memory nor the FP units stay busy: with them
+// (and those of plane_rows) a 128^3 mixed step takes 57 us instead of 80, a
+// 256 x 32 x 64 FP64 step 31 instead of 39, 64^3 18.7 instead of 19.6
+template <typename R, int LN, int T>
+__device__ __noinline__ void kin_staged(const NdArgs<R>& a, int axis,
+                                        const typename Rot<R>::type* tab, cpx<R>* sm) {
+  using F = LineFft<R, LN>;
+  using PhT = typename Ph<R>::type;
+  constexpr int N = F::N, E = F::E, L = F::L;
+  const int lc = a.lc, gt = L << lc, tid = threadIdx.x & (gt - 1);
+  const int group = threadIdx.x / gt, ng = T / gt;
+  const int c = threadIdx.x & ((1 << lc) - 1);
+  cpx<R>* ex = sm + ((group * (N + N / 8)) << lc) + c;
+  const int tile = (N << lc) * (int)(sizeof(cpx<R>) + sizeof(PhT));
+  unsigned char* buf = reinterpret_cast<unsigned char*>(sm + T / L * (N + N / 8)) + 2 * group * tile;
+  F fft;
+  fft.init(tab, (threadIdx.x >> lc) & (L - 1));
+  auto at = [&](int p) { return ex + (skew(p) << lc); };
+  auto sync = [&]() { bar_group(1 + group, gt); };
+  const int ltx = a.ln[0] - lc;
+  const int stride = axis == 1 ? 1 << a.ln[0] : 1 << (a.ln[0] + a.ln[1]);
+  const int lset = axis == 1 ? a.ln[0] + a.ln[1] : a.ln[0];
+  const int items = (int)(a.n >> (LN + lc)), step = gridDim.x * ng;
+  auto first = [&](int it) { return ((it >> ltx) << lset) + ((it & ((1 << ltx) - 1)) << lc); };
+  auto fetch = [&](int it, int s) {
+    unsigned char* d = buf + s * tile;
+    const int b0 = first(it);
+    const int pc = (int)(sizeof(cpx<R>) << lc) / 16, kc = (int)(sizeof(PhT) << lc) / 16;
+    for (int i = tid; i < N * pc; i += gt) {
+      const int r = i / pc;
+      copy_async<16>(d + 16 * i, reinterpret_cast<const char*>(a.psi + b0 + r * stride) +
+                                     16 * (i - r * pc));
+    }
+    d += (N << lc) * sizeof(cpx<R>);
+    for (int i = tid; i < N * kc; i += gt) {
+      const int r = i / kc;
+      copy_async<16>(d + 16 * i, reinterpret_cast<const char*>(a.K + b0 + r * stride) +
+                                     16 * (i - r * kc));
+    }
+  };
+  int it = blockIdx.x + gridDim.x * group, s = 0;
+  if (it < items) fetch(it, 0);
+  copy_commit();
+  for (; it < items; it += step, s ^= 1) {
+    if (it + step < items) fetch(it + step, s ^ 1);
+    copy_commit();
+    copy_wait<1>();
+    sync();
+    const cpx<R>* x = reinterpret_cast<const cpx<R>*>(buf + s * tile) + c;
+    const PhT* kf = reinterpret_cast<const PhT*>(buf + s * tile + (N << lc) * sizeof(cpx<R>)) + c;
+    cpx<R> v[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = x[(e * L + fft.t) << lc];
+    fft.forward(v, at, sync);
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = apply_ph(kf[(e * L + fft.t) << lc], v[e]);
+    fft.inverse(v, at, sync);
+    const int base = first(it) + c;
+#pragma unroll
+    for (int e = 0; e < E; ++e) a.psi[base + (e * L + fft.t) * stride] = v[e];
+    sync();
+  }
+}
+
 // the columns of a plane in shared memory, in place (positions along y), the
 // exchange through the lines' own places
 template <typename R, int LN, bool INV, int THREADS>
@@ -521,7 +620,8 @@ __device__ __noinline__ void plane_cols(const NdArgs<R>& a, const typename Rot<R
   }
 }
 
-// the rows of a plane in shared memory, in place
+// the rows of a plane in shared memory, in place; behind the plane, 4 KB per warp
+// for the rows' 16-byte inputs
 template <typename R, int LN, int MODE, int T>
 __device__ __noinline__ double2 plane_rows(const NdArgs<R>& a, const SodRow& o,
                                            const typename Rot<R>::type* tab, cpx<R>* sm,
@@ -539,14 +639,15 @@ __device__ __noinline__ double2 plane_rows(const NdArgs<R>& a, const SodRow& o,
     auto at = [&](int p) { return row + slot_of<R>(p); };
     const int base = ((plane << a.ln[1]) + y) << LN;
     cpx<R> v[E];
-    RowIn<R, E, MODE, T> in;
+    RowIn<R, E, MODE, T, true> in;
+    in.st = reinterpret_cast<double2*>(sm + (N << a.ln[1])) + warp * (32 * 8);
     if (row_inverse(MODE)) {
       in.early(a, o, base + fft.t, F::L);
 #pragma unroll
       for (int e = 0; e < E; ++e) v[e] = *at(F::pos(F::NG - 1, fft.t, e));
       fft.inverse(v, at, sync);
     }
-    row_points<R, LN, MODE, T>(a, o, v, in, fft, base, cr, ci);
+    row_points<R, LN, MODE, T, true>(a, o, v, in, fft, base, cr, ci);
     if (row_forward(MODE)) {
       fft.forward(v, at, sync);
 #pragma unroll
@@ -588,7 +689,10 @@ __device__ __forceinline__ double2 x_phase(const NdArgs<R>& a, const SodRow& o,
   };
     if (row_inverse(MODE)) {
 #pragma unroll 8
-      for (int i = threadIdx.x; i < (1 << lp); i += blockDim.x) *slot(i) = g[i];
+      for (int i = threadIdx.x; i < (1 << lp); i += blockDim.x)
+        copy_async<sizeof(cpx<R>)>(slot(i), g + i);
+      copy_commit();
+      copy_wait<0>();
       __syncthreads();
       for_len<MAXLN>(a.ln[1], [&](auto ln) {
         plane_cols<R, decltype(ln)::value, true, T>(a, tab[1], sm);
@@ -618,6 +722,12 @@ template <typename R, int T, int MAXLN, int MODE>
 __device__ __forceinline__ void axis_phase(const NdArgs<R>& a, int axis,
                                            const typename Rot<R>::type* const* tab, cpx<R>* sm) {
   for_len<MAXLN>(a.ln[axis], [&](auto ln) {
+    if constexpr (MODE == kKin && decltype(ln)::value <= 8) {
+      if (a.kstage) {
+        kin_staged<R, decltype(ln)::value, T>(a, axis, tab[axis], sm);
+        return;
+      }
+    }
     cols_phase<R, decltype(ln)::value, MODE, T>(a, axis, tab[axis], sm);
   });
 }
