@@ -6,27 +6,26 @@
 // copies of weights, activations and back-propagated gradients as GEMM
 // operands; every product accumulates in FP32.
 //
-// GEMM: C[M,N] (f32) = alpha op(A) op(B) + beta C, A and B bfloat16.  One CTA
-// of 256 threads owns a 128 x BN output tile whose FP32 accumulator lives in
-// tensor memory (TMEM lane = tile row, column = tile column).  K advances in
-// stages of 64 through a ring of four or eight shared-memory buffers: all threads
-// copy the A and B tiles ahead with cp.async (16-byte pieces, zero-filled at the
-// edges) as "core matrices" (8 x 16 bytes, no swizzle; K-major or MN-major,
-// whichever keeps the source's 16-byte runs whole), one thread issues four
-// tcgen05.mma (M = 128, N = BN, K = 16, kind::f16 with BF16 inputs) per stage and
-// commits them to the buffer's mbarrier.  BN is the largest of 256, 128, 64 that
-// gives every SM a tile, else 32: the network's products have few tiles, and what
-// bounds them is the chain of stages.  The epilogue reads the accumulator with
-// tcgen05.ld (a warp: 32 TMEM lanes, 32 columns) and turns it in shared memory so that
-// rows are written 128 bytes at a time, adding the bias and the activation (or
-// its derivative) on the way.  Every mbarrier wait is bounded: on timeout the
-// kernel records it in a device status word, skips the epilogue and still releases
-// its TMEM.
-// 256 x 256 x 4096 (4 tiles of 128 x 128, staged through registers one stage
-// ahead with 8-way bank conflicts, rows written 4 bytes per lane): 248 us before.
+// GEMM: C[M,N] (f32) = alpha op(A) op(B) + beta C, A and B bfloat16.  One CTA owns a
+// 128 x BN output tile whose FP32 accumulator lives in tensor memory (TMEM lane =
+// tile row, column = tile column).  K advances in stages of 64 through a ring of
+// shared-memory buffers: one thread fetches the A and B tiles by TMA
+// (gemm_bf16_tma), or 256 threads copy them where TMA's alignment rules do not hold
+// (gemm_bf16_tc); one thread issues four tcgen05.mma (M = 128, N = BN, K = 16,
+// kind::f16 with BF16 inputs) per stage and commits them to the buffer's mbarrier.
+// BN is the largest of 256, 128, 64 that gives every SM a tile, else 32: the
+// network's products have few tiles, and what bounds them is the chain of stages.
+// The epilogue reads the accumulator with tcgen05.ld (a warp: 32 TMEM lanes, 32
+// columns) and turns it in shared memory so that rows are written 128 bytes at a
+// time, adding the bias and the activation (or its derivative) on the way.  Every
+// mbarrier wait is bounded: on timeout the kernel records it in a device status
+// word, skips the epilogue and still releases its TMEM.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "espec_gpu.h"
 #include "espec_internal.h"
@@ -92,11 +91,10 @@ __device__ __forceinline__ uint32_t pack2(uint16_t lo, uint16_t hi) {
 //  * otherwise (element at X[k ld + row]): MN-major core matrices, 16-byte row = 8
 //    consecutive rows at one k; 144 bytes between row groups, 18 R between k
 //    groups.
-// Either way a 16-byte row is 16 contiguous source bytes, copied asynchronously
-// when vec (aligned; the part beyond nrows or K is zero-filled), else element by
-// element.  Consecutive threads take consecutive 16-byte pieces of the source,
-// whole 128-byte lines per eight threads (in half lines a CTA drew 29 GB/s); the
-// odd group strides put those pieces on distinct banks.
+// Either way a 16-byte row is 16 contiguous source bytes, one copy when vec
+// (aligned; the part beyond nrows or K is zero-filled), else element by element.
+// Consecutive threads take consecutive 16-byte pieces of the source, whole 128-byte
+// lines per eight threads; the odd group strides put those pieces on distinct banks.
 // A thread's pieces keep their places from stage to stage: their addresses and
 // sizes are formed once and then advance by a constant.
 template <int R>
@@ -218,19 +216,88 @@ __device__ __forceinline__ float gelu_grad(float z) {
          z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-// stage buffers, filled ahead of the stage multiplied: 8 where a narrow
-// tile has a long K (an L2 round trip is several stages long), else 4, which lets
-// two CTAs share an SM
-template <int BN, int RING>
+constexpr int kCopyRing = 4;  // stage buffers
+template <int BN>
 constexpr size_t tc_smem_bytes() {
-  return 1024 + RING * (size_t)(kTileBytes<kBM> + kTileBytes<BN>) + 192;
+  return 1024 + kCopyRing * (size_t)(kTileBytes<kBM> + kTileBytes<BN>) + 192;
 }
 
-template <int BN, int EPI, int RING>
+// What follows the MMAs of a tile: wait for the last commit, write the tile, give
+// the tensor memory back.  Warp 8 issued the MMAs; `turn` space: the stage buffers.
+template <int BN, int EPI>
+__device__ __forceinline__ void finish_tile(const TcGemm& g, uint32_t tmem, uint8_t* base,
+                                            uint64_t* last, uint32_t parity, bool some, bool ok,
+                                            int m0, int n0) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool mma_warp = warp == kTcThreads / 32;
+  __syncwarp();
+  // warp w: rows 32 (w % 4) of the tile, columns from 32 (w / 4) on, 64 apart
+  const int row0 = m0 + (warp & 3) * 32, col0 = (warp >> 2) * 32;
+  // the first columns' pre-activations, on their way while the last MMAs run
+  float zf[EPI == kGeluBack ? 32 : 1];
+  if (EPI == kGeluBack) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      zf[i] = !mma_warp && col0 < BN && row0 + i < g.M && n0 + col0 + lane < g.N
+                  ? g.z[(long)(row0 + i) * g.ldc + n0 + col0 + lane]
+                  : 0.0f;
+  }
+  // the last commit covers every MMA before it
+  if (some) ok = wait_phase(last, parity) && ok;
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  ok = __syncthreads_and(ok) != 0;
+  if (ok && !mma_warp) {
+    // 32 columns at a time: each warp's 32 x 32 piece through shared memory
+    float* turn = reinterpret_cast<float*>(base) + warp * (32 * 33);
+#pragma unroll 1
+    for (int c0 = col0; c0 < BN; c0 += 64) {
+      uint32_t r[32];
+      if (some) {
+        tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, r);
+      } else {  // empty sum
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = __uint_as_float(r[j]);
+      __syncwarp();
+      const int n = n0 + c0 + lane;
+      const float bias = EPI == kBias && n < g.N ? g.bias[n] : 0.0f;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int row = row0 + i;
+        if (row < g.M && n < g.N) {
+          const long o = (long)row * g.ldc + n;
+          float v = turn[i * 33 + lane];
+          if (EPI == kPlain) {
+            v = g.alpha * v;
+            if (g.beta != 0.0f) v = some ? fmaf(g.beta, g.C[o], v) : g.beta * g.C[o];
+            else if (!some) v = 0.0f;
+          } else if (EPI == kBias) {
+            v = v + bias;
+            if (g.h) g.h[o] = bf16_bits(g.act ? gelu(v) : v);
+          } else {
+            v = v * gelu_grad(c0 == col0 ? zf[i] : g.z[o]);
+            g.h[o] = bf16_bits(v);
+          }
+          g.C[o] = v;
+        }
+      }
+      __syncwarp();
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (mma_warp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN));
+}
+
+template <int BN, int EPI>
 __global__ void __launch_bounds__(kTcBlock) gemm_bf16_tc(TcGemm g) {
   static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256,
                 "TMEM columns: a power of two from 32, N tile of one MMA");
-  constexpr int kA = kTileBytes<kBM>, kB = kTileBytes<BN>, kRing = RING;
+  constexpr int kA = kTileBytes<kBM>, kB = kTileBytes<BN>, kRing = kCopyRing;
   static_assert(kRing * kA >= kTcThreads * 33 * 4, "the epilogue turns tiles in the stage buffers");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -268,33 +335,23 @@ __global__ void __launch_bounds__(kTcBlock) gemm_bf16_tc(TcGemm g) {
     Stager<BN> tb;
     ta.init(g.A, g.lda, a_kc, g.a_vec, m0, g.M, g.K);
     tb.init(g.B, g.ldb, b_kc, g.b_vec, n0, g.N, g.K);
-    const bool async = g.a_vec && g.b_vec;
     for (int kt = 0; kt < nk; ++kt) {
       const int b = kt % kRing;
       if (kt >= kRing && !(ok = wait_phase(done + b, (kt / kRing - 1) & 1))) break;
       ta.stage(sA + b * kA, kt);
       tb.stage(sB + b * kB, kt);
-      if (async) {  // arrives by itself when this thread's copies have landed
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];\n" ::"r"(smem_u32(full + b))
-                     : "memory");
-      } else {
-        asm volatile("cp.async.wait_all;\n" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}\n" ::"r"(
-                         smem_u32(full + b))
-                     : "memory");
-      }
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}\n" ::"r"(
+                       smem_u32(full + b))
+                   : "memory");
     }
   } else if (lane == 0) {
-    // a thread without copies of its own: the proxy fence waits for all of a
-    // thread's outstanding copies, also those of later stages (issued by a staging
-    // thread it held every stage for a full memory round trip, 1.1 us)
     const uint32_t idesc = idesc_bf16<BN>(a_kc ? 0u : 1u, b_kc ? 0u : 1u);
     const uint32_t a_lead = lead_bytes<kBM>(a_kc), b_lead = lead_bytes<BN>(b_kc);
     for (int kt = 0; kt < nk; ++kt) {
       const int b = kt % kRing;
       if (!(ok = wait_phase(full + b, (kt / kRing) & 1))) break;
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       const uint32_t a0 = smem_u32(sA + b * kA), b0 = smem_u32(sB + b * kB);
 #pragma unroll
       for (int j = 0; j < kBK / 16; ++j) {
@@ -313,67 +370,142 @@ __global__ void __launch_bounds__(kTcBlock) gemm_bf16_tc(TcGemm g) {
           : "memory");
     }
   }
-  __syncwarp();
-  // warp w: rows 32 (w % 4) of the tile, columns from 32 (w / 4) on, 64 apart
-  const int row0 = m0 + (warp & 3) * 32, col0 = (warp >> 2) * 32;
-  // the first columns' pre-activations, on their way while the last MMAs run
-  float zf[EPI == kGeluBack ? 32 : 1];
-  if (EPI == kGeluBack) {
+  finish_tile<BN, EPI>(g, tmem, base, done + (nk - 1) % kRing, ((nk - 1) / kRing) & 1, nk > 0, ok,
+                       m0, n0);
+}
+
+// The same product with tiles brought by TMA, for operands whose base and rows are
+// 16-byte aligned.  What bounds the network's products is the chain of stages of
+// one CTA (16 tiles of 128 x 32 at 256 x 256), and copies by 256 threads, which
+// wait, form addresses, issue 16-byte pieces and arrive at every stage, drew 25 GB/s
+// per SM.  Here one thread asks for boxes of 64 k and the ring of stages stays in
+// flight.  The MMAs, their order and the sums are those of gemm_bf16_tc.
+// Against an asynchronous ring filled by the threads (us, before -> now):
+// 256 x 256 x 256 7.7 -> 5.6, 256 x 256 x 1024 16.6 -> 9.7, 256 x 256 x 4096
+// 51 -> 25, 2048 x 4096 x 256 35 -> 23, 1024 x 1024 x 1024 32 -> 18.
+//
+// Tiles in shared memory, op(X) of R rows x 64 k:
+//  * K-major source: one box, R rows of 64 k (128 bytes, 128-byte swizzle); 1024
+//    bytes between groups of 8 rows;
+//  * MN-major source: R / 64 boxes of 64 k rows of 64 row values each (128-byte
+//    swizzle); 8 KB between boxes, 1024 bytes between groups of 8 k; for R = 32 one
+//    box of 64-byte rows (64-byte swizzle), 512 bytes between groups of 8 k.
+template <int R>
+constexpr int kBoxBytes = R * kBK * 2;
+template <int BN, int RING>
+constexpr size_t tma_smem_bytes() {
+  return 1024 + RING * (size_t)(kBoxBytes<kBM> + kBoxBytes<BN>) + 192;
+}
+
+// descriptor of the 16 k from 16 j on of the tile at addr
+template <int R>
+__device__ __forceinline__ uint64_t box_desc(uint32_t addr, bool kcontig, int j) {
+  const uint32_t at = addr + (kcontig ? 32 : (R == 32 ? 1024 : 2048)) * j;
+  const uint32_t lead = 64 * kBK * 2, stride = !kcontig && R == 32 ? 512 : 1024;
+  const uint64_t swizzle = !kcontig && R == 32 ? 4 : 2;
+  return (uint64_t)((at & 0x3FFFFu) >> 4) | ((uint64_t)(lead >> 4) << 16) |
+         ((uint64_t)(stride >> 4) << 32) | (1ull << 46) | (swizzle << 61);
+}
+
+// the map's box from (x, y) on; x is a multiple of 32 values, so the copy starts on
+// a 16-byte boundary
+__device__ __forceinline__ void tma_box(void* dst, const CUtensorMap* map, int x, int y,
+                                        uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+      : "memory");
+}
+
+template <int R>
+__device__ __forceinline__ void tma_tile(uint8_t* dst, const CUtensorMap* map, bool kcontig, int k0,
+                                         int row0, uint64_t* bar) {
+  if (kcontig) {
+    tma_box(dst, map, k0, row0, bar);
+  } else {
 #pragma unroll
-    for (int i = 0; i < 32; ++i)
-      zf[i] = !mma_warp && col0 < BN && row0 + i < g.M && n0 + col0 + lane < g.N
-                  ? g.z[(long)(row0 + i) * g.ldc + n0 + col0 + lane]
-                  : 0.0f;
+    for (int r = 0; r < R; r += 64) tma_box(dst + r * kBK * 2, map, row0 + r, k0, bar);
   }
-  // the last commit covers every MMA before it
-  if (nk > 0) ok = wait_phase(done + (nk - 1) % kRing, ((nk - 1) / kRing) & 1) && ok;
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  ok = __syncthreads_and(ok) != 0;
-  if (ok && !mma_warp) {
-    // 32 columns at a time: each warp's 32 x 32 piece through shared memory
-    float* turn = reinterpret_cast<float*>(base) + warp * (32 * 33);
-#pragma unroll 1
-    for (int c0 = col0; c0 < BN; c0 += 64) {
-      uint32_t r[32];
-      if (nk > 0) {
-        tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, r);
-      } else {  // empty sum
-#pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = 0u;
-      }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = __uint_as_float(r[j]);
-      __syncwarp();
-      const int n = n0 + c0 + lane;
-      const float bias = EPI == kBias && n < g.N ? g.bias[n] : 0.0f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int row = row0 + i;
-        if (row < g.M && n < g.N) {
-          const long o = (long)row * g.ldc + n;
-          float v = turn[i * 33 + lane];
-          if (EPI == kPlain) {
-            v = g.alpha * v;
-            if (g.beta != 0.0f) v = nk > 0 ? fmaf(g.beta, g.C[o], v) : g.beta * g.C[o];
-            else if (nk == 0) v = 0.0f;
-          } else if (EPI == kBias) {
-            v = v + bias;
-            if (g.h) g.h[o] = bf16_bits(g.act ? gelu(v) : v);
-          } else {
-            v = v * gelu_grad(c0 == col0 ? zf[i] : g.z[o]);
-            g.h[o] = bf16_bits(v);
-          }
-          g.C[o] = v;
-        }
-      }
-      __syncwarp();
+}
+
+template <int BN, int EPI, int RING>
+__global__ void __launch_bounds__(kTcBlock)
+    gemm_bf16_tma(const TcGemm g, const __grid_constant__ CUtensorMap map_a,
+                  const __grid_constant__ CUtensorMap map_b) {
+  constexpr int kA = kBoxBytes<kBM>, kB = kBoxBytes<BN>, kRing = RING;
+  static_assert(kRing * kA >= kTcThreads * 33 * 4, "the epilogue turns tiles in the stage buffers");
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* sA = base;
+  uint8_t* sB = base + kRing * kA;
+  uint64_t* full = (uint64_t*)(base + kRing * (kA + kB));  // a buffer's boxes have landed
+  uint64_t* done = full + kRing;                                 // its MMAs have read it
+  uint32_t* tmem_slot = (uint32_t*)(done + kRing);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
+  const bool a_kc = !g.ta, b_kc = g.tb != 0, mma_warp = warp == kTcThreads / 32;
+  const int nk = (g.K + kBK - 1) / kBK;
+
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < kRing; ++b) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(full + b)));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(done + b)));
     }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (mma_warp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(BN));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (mma_warp)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN));
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  bool ok = true;
+  if (threadIdx.x == 0) {
+    int kt = 0;
+    for (; kt < nk; ++kt) {
+      const int b = kt % kRing;
+      if (kt >= kRing && !(ok = wait_phase(done + b, (kt / kRing - 1) & 1))) break;
+      asm volatile(
+          "{\n\t.reg .b64 t;\n\t"
+          "mbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}\n" ::"r"(smem_u32(full + b)),
+          "r"(kA + kB)
+          : "memory");
+      tma_tile<kBM>(sA + b * kA, &map_a, a_kc, kt * kBK, m0, full + b);
+      tma_tile<BN>(sB + b * kB, &map_b, b_kc, kt * kBK, n0, full + b);
+    }
+    // after a wait that gave up: the boxes still on their way
+    if (!ok)
+      for (int j = kt > kRing ? kt - kRing : 0; j < kt; ++j)
+        wait_phase(full + j % kRing, (j / kRing) & 1);
+  } else if (mma_warp && lane == 0) {
+    const uint32_t idesc = idesc_bf16<BN>(a_kc ? 0u : 1u, b_kc ? 0u : 1u);
+    for (int kt = 0; kt < nk; ++kt) {
+      const int b = kt % kRing;
+      if (!(ok = wait_phase(full + b, (kt / kRing) & 1))) break;
+      const uint32_t a0 = smem_u32(sA + b * kA), b0 = smem_u32(sB + b * kB);
+#pragma unroll
+      for (int j = 0; j < kBK / 16; ++j) {
+        const uint64_t da = box_desc<kBM>(a0, a_kc, j), db = box_desc<BN>(b0, b_kc, j);
+        const uint32_t acc = (kt > 0 || j > 0) ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
+            "l"(da), "l"(db), "r"(idesc), "r"(acc));
+      }
+      asm volatile(
+          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+              smem_u32(done + b))
+          : "memory");
+    }
+  }
+  finish_tile<BN, EPI>(g, tmem, base, done + (nk - 1) % kRing, ((nk - 1) / kRing) & 1, nk > 0,
+                           ok, m0, n0);
 }
 
 // z += b (row broadcast); h = bf16(gelu(z)) when act, else bf16(z) (h optional)
@@ -419,16 +551,63 @@ __global__ void adam_bf16_kernel(float* w, const float* g, float* m1, float* m2,
 
 inline unsigned nblk(long count) { return (unsigned)((count + 255) / 256); }
 
+// tensor map of op(X), `rows` x K, as it lies (tma_tile's boxes)
+bool operand_map(CUtensorMap* map, const uint16_t* X, int ld, bool kcontig, int rows, int K,
+                 int tile_rows) {
+  using Encode = decltype(&cuTensorMapEncodeTiled);
+  static const Encode encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000,
+                                                           cudaEnableDefault, &q);
+    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? (Encode)fn : (Encode) nullptr;
+  }();
+  if (!encode) return false;
+  const cuuint64_t dim[2] = {(cuuint64_t)(kcontig ? K : rows), (cuuint64_t)(kcontig ? rows : K)};
+  const cuuint64_t stride[1] = {2 * (cuuint64_t)ld};
+  const cuuint32_t box[2] = {(cuuint32_t)(kcontig ? kBK : std::min(tile_rows, 64)),
+                             (cuuint32_t)(kcontig ? tile_rows : kBK)};
+  const cuuint32_t one[2] = {1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(X), dim, stride,
+                box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                box[0] == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int BN, int EPI, int RING>
-int launch_tc(const TcGemm& g, cudaStream_t st) {
+int launch_tma(const TcGemm& g, const CUtensorMap& ma, const CUtensorMap& mb, cudaStream_t st) {
   static DeviceFlags attr;
-  constexpr size_t smem = tc_smem_bytes<BN, RING>();
-  {
-    const cudaError_t e = set_max_smem_once(attr, gemm_bf16_tc<BN, EPI, RING>, smem);
-    if (e != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute", e);
+  constexpr size_t smem = tma_smem_bytes<BN, RING>();
+  const cudaError_t a = set_max_smem_once(attr, gemm_bf16_tma<BN, EPI, RING>, smem);
+  if (a != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute", a);
+  const dim3 grid((g.N + BN - 1) / BN, (g.M + kBM - 1) / kBM);
+  gemm_bf16_tma<BN, EPI, RING><<<grid, kTcBlock, smem, st>>>(g, ma, mb);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return set_cuda_error("tensor-core GEMM launch", e);
+  return ESPEC_OK;
+}
+
+// TMA wherever a tensor map can describe the operands (base and rows at multiples of
+// 16 bytes): it was the faster form at every size measured (gemm_bf16_tma).  The
+// ring: 8 stages of a narrow tile where K has more than 4 (an L2 round trip is several
+// stages long), else 4, which lets two CTAs share an SM.
+template <int BN, int EPI>
+int launch_tc(const TcGemm& g, cudaStream_t st) {
+  if (g.K > 0 && g.a_vec && g.b_vec) {
+    CUtensorMap ma, mb;
+    if (operand_map(&ma, g.A, g.lda, !g.ta, g.M, g.K, kBM) &&
+        operand_map(&mb, g.B, g.ldb, g.tb != 0, g.N, g.K, BN)) {
+      if (BN <= 64 && g.K > 4 * kBK) return launch_tma<BN, EPI, BN <= 64 ? 8 : 4>(g, ma, mb, st);
+      return launch_tma<BN, EPI, 4>(g, ma, mb, st);
+    }
   }
-  dim3 grid((g.N + BN - 1) / BN, (g.M + kBM - 1) / kBM);
-  gemm_bf16_tc<BN, EPI, RING><<<grid, kTcBlock, smem, st>>>(g);
+  static DeviceFlags attr;
+  constexpr size_t smem = tc_smem_bytes<BN>();
+  const cudaError_t a = set_max_smem_once(attr, gemm_bf16_tc<BN, EPI>, smem);
+  if (a != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute", a);
+  const dim3 grid((g.N + BN - 1) / BN, (g.M + kBM - 1) / kBM);
+  gemm_bf16_tc<BN, EPI><<<grid, kTcBlock, smem, st>>>(g);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_cuda_error("tensor-core GEMM launch", e);
   return ESPEC_OK;
@@ -440,10 +619,10 @@ int launch_any(const TcGemm& g, cudaStream_t st) {
   auto tiles = [&](int bn) {
     return (long)((g.N + bn - 1) / bn) * ((g.M + kBM - 1) / kBM);
   };
-  if (tiles(256) >= 148) return launch_tc<256, EPI, 4>(g, st);
-  if (tiles(128) >= 148) return launch_tc<128, EPI, 4>(g, st);
-  if (tiles(64) >= 148) return launch_tc<64, EPI, 4>(g, st);
-  return g.K > 8 * kBK ? launch_tc<32, EPI, 8>(g, st) : launch_tc<32, EPI, 4>(g, st);
+  if (tiles(256) >= 148) return launch_tc<256, EPI>(g, st);
+  if (tiles(128) >= 148) return launch_tc<128, EPI>(g, st);
+  if (tiles(64) >= 148) return launch_tc<64, EPI>(g, st);
+  return launch_tc<32, EPI>(g, st);
 }
 
 inline int vec_ok(const void* p, int ld) { return ld % 8 == 0 && ((uintptr_t)p & 15) == 0; }
