@@ -8,6 +8,7 @@
 // outputs per thread.
 #include <cuda_runtime.h>
 
+#include "chain.cuh"
 #include "espec_gpu.h"
 #include "espec_internal.h"
 
@@ -81,6 +82,8 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, T alpha,
 __global__ void colsum_kernel(const float* __restrict__ dy, int rows, int cols,
                               float* __restrict__ db) {
   __shared__ float part[8][33];
+  chain_start();
+  chain_wait();
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.0f;
   if (c < cols) {
@@ -103,6 +106,8 @@ __global__ void mse_kernel(const float* __restrict__ y, const float* __restrict_
   const int r = blockIdx.x;
   float s = 0.0f;
   const float sc = 2.0f / ((float)rows * (float)cols);
+  chain_start();
+  chain_wait();
 #pragma unroll 8
   for (int c = threadIdx.x; c < cols; c += 256) {
     const float d = y[(long)r * cols + c] - t[(long)r * cols + c];
@@ -231,16 +236,17 @@ extern "C" int espec_gemm_f32(int M, int N, int K, float alpha, const float* A, 
 }
 
 extern "C" int espec_mlp_colsum(const float* dy, int rows, int cols, float* db, void* stream) {
-  colsum_kernel<<<(unsigned)((cols + 31) / 32), dim3(32, 8), 0, (cudaStream_t)stream>>>(dy, rows,
-                                                                                       cols, db);
-  MLP_CK();
+  const cudaError_t e = launch_chained(colsum_kernel, (unsigned)((cols + 31) / 32), dim3(32, 8), 0,
+                                       (cudaStream_t)stream, dy, rows, cols, db);
+  if (e != cudaSuccess) return set_cuda_error("mlp kernel launch", e);
   return ESPEC_OK;
 }
 
 extern "C" int espec_mlp_mse(const float* y, const float* t, int rows, int cols, float* dy,
                              float* row_loss, void* stream) {
-  mse_kernel<<<rows, 256, 0, (cudaStream_t)stream>>>(y, t, rows, cols, dy, row_loss);
-  MLP_CK();
+  const cudaError_t e =
+      launch_chained(mse_kernel, rows, 256, 0, (cudaStream_t)stream, y, t, rows, cols, dy, row_loss);
+  if (e != cudaSuccess) return set_cuda_error("mlp kernel launch", e);
   return ESPEC_OK;
 }
 

@@ -27,6 +27,7 @@
 
 #include <algorithm>
 
+#include "chain.cuh"
 #include "espec_gpu.h"
 #include "espec_internal.h"
 
@@ -299,6 +300,7 @@ __global__ void __launch_bounds__(kTcBlock) gemm_bf16_tc(TcGemm g) {
                 "TMEM columns: a power of two from 32, N tile of one MMA");
   constexpr int kA = kTileBytes<kBM>, kB = kTileBytes<BN>, kRing = kCopyRing;
   static_assert(kRing * kA >= kTcThreads * 33 * 4, "the epilogue turns tiles in the stage buffers");
+  chain_start();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = base;
@@ -329,6 +331,7 @@ __global__ void __launch_bounds__(kTcBlock) gemm_bf16_tc(TcGemm g) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  chain_wait();
   bool ok = true;
   if (!mma_warp) {
     Stager<kBM> ta;
@@ -381,7 +384,7 @@ __global__ void __launch_bounds__(kTcBlock) gemm_bf16_tc(TcGemm g) {
 // per SM.  Here one thread asks for boxes of 64 k and the ring of stages stays in
 // flight.  The MMAs, their order and the sums are those of gemm_bf16_tc.
 // Against an asynchronous ring filled by the threads (us, before -> now):
-// 256 x 256 x 256 7.7 -> 5.6, 256 x 256 x 1024 16.6 -> 9.7, 256 x 256 x 4096
+// 256 x 256 x 256 7.7 -> 5.6 (4.9 as part of a chain, chain.cuh), 256 x 256 x 1024 16.6 -> 9.7, 256 x 256 x 4096
 // 51 -> 25, 2048 x 4096 x 256 35 -> 23, 1024 x 1024 x 1024 32 -> 18.
 //
 // Tiles in shared memory, op(X) of R rows x 64 k:
@@ -435,6 +438,7 @@ __global__ void __launch_bounds__(kTcBlock)
                   const __grid_constant__ CUtensorMap map_b) {
   constexpr int kA = kBoxBytes<kBM>, kB = kBoxBytes<BN>, kRing = RING;
   static_assert(kRing * kA >= kTcThreads * 33 * 4, "the epilogue turns tiles in the stage buffers");
+  chain_start();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = base;
@@ -464,6 +468,7 @@ __global__ void __launch_bounds__(kTcBlock)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  chain_wait();
   bool ok = true;
   if (threadIdx.x == 0) {
     int kt = 0;
@@ -528,6 +533,8 @@ __global__ void gelu_back_kernel(float* dh, const float* z, long count, uint16_t
 }
 
 __global__ void to_bf16_kernel(const float* x, uint16_t* y, long count) {
+  chain_start();
+  chain_wait();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) y[i] = bf16_bits(x[i]);
 }
@@ -582,8 +589,8 @@ int launch_tma(const TcGemm& g, const CUtensorMap& ma, const CUtensorMap& mb, cu
   const cudaError_t a = set_max_smem_once(attr, gemm_bf16_tma<BN, EPI, RING>, smem);
   if (a != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute", a);
   const dim3 grid((g.N + BN - 1) / BN, (g.M + kBM - 1) / kBM);
-  gemm_bf16_tma<BN, EPI, RING><<<grid, kTcBlock, smem, st>>>(g, ma, mb);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e =
+      launch_chained(gemm_bf16_tma<BN, EPI, RING>, grid, kTcBlock, smem, st, g, ma, mb);
   if (e != cudaSuccess) return set_cuda_error("tensor-core GEMM launch", e);
   return ESPEC_OK;
 }
@@ -607,8 +614,7 @@ int launch_tc(const TcGemm& g, cudaStream_t st) {
   const cudaError_t a = set_max_smem_once(attr, gemm_bf16_tc<BN, EPI>, smem);
   if (a != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute", a);
   const dim3 grid((g.N + BN - 1) / BN, (g.M + kBM - 1) / kBM);
-  gemm_bf16_tc<BN, EPI><<<grid, kTcBlock, smem, st>>>(g);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_chained(gemm_bf16_tc<BN, EPI>, grid, kTcBlock, smem, st, g);
   if (e != cudaSuccess) return set_cuda_error("tensor-core GEMM launch", e);
   return ESPEC_OK;
 }
@@ -733,8 +739,9 @@ extern "C" int espec_mlp_gelu_back(float* dh, const float* z, long count, void* 
 }
 
 extern "C" int espec_to_bf16(const float* x, void* y, long count, void* stream) {
-  to_bf16_kernel<<<nblk(count), 256, 0, (cudaStream_t)stream>>>(x, (uint16_t*)y, count);
-  TC_CK();
+  const cudaError_t e =
+      launch_chained(to_bf16_kernel, nblk(count), 256, 0, (cudaStream_t)stream, x, (uint16_t*)y, count);
+  if (e != cudaSuccess) return set_cuda_error("mlp bf16 kernel launch", e);
   return ESPEC_OK;
 }
 
