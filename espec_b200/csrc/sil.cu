@@ -6,6 +6,7 @@
 #include <cuda/atomic>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <utility>
@@ -50,7 +51,7 @@ __device__ __forceinline__ double ld_state(const double* p) { return *p; }
 // every thread of every CTA): a CTA runs at most one barrier ahead of the
 // slowest, which can still be reading the other buffer.  false = a wait
 // gave up.
-template <int kInFlight = 16>
+template <int kInFlight>
 __device__ bool grid_reduce(const SilArgs& a, const double* sp, double* st, int nq,
                             int* s_flag, double* s_red /* kSilThreads doubles */,
                             unsigned& phase) {
@@ -123,6 +124,40 @@ __device__ bool grid_reduce(const SilArgs& a, const double* sp, double* st, int 
   return true;
 }
 
+// Grid barrier (grid_reduce's, without the sums); between this CTA's arrival and
+// the others', threads 32 on run meanwhile().  false = a wait gave up.
+template <class F>
+__device__ __forceinline__ bool grid_barrier(const SilArgs& a, int* s_flag, unsigned& phase,
+                                             F meanwhile) {
+  const unsigned G = gridDim.x;
+  const unsigned long long target = (unsigned long long)(phase + 1u) * G;
+  ++phase;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_flag[1] = 1;
+    if (G > 1) {
+      cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> cnt(
+          *reinterpret_cast<unsigned long long*>(a.bar));
+      cuda::atomic_ref<int, cuda::thread_scope_device> err(*a.err);
+      if (cnt.fetch_add(1ull, cuda::memory_order_acq_rel) + 1ull < target) {
+        long spins = 0;
+        while (cnt.load(cuda::memory_order_acquire) < target) {
+          if (++spins > a.spin_limit || err.load(cuda::memory_order_relaxed) != 0) {
+            err.store(1, cuda::memory_order_relaxed);
+            s_flag[1] = 0;
+            break;
+          }
+          if (spins > 4096) __nanosleep(32);
+        }
+      }
+    }
+  } else if (threadIdx.x >= 32) {
+    meanwhile();
+  }
+  __syncthreads();
+  return s_flag[1] != 0;
+}
+
 // sum of nv per-thread values over the CTA into sp[0..nv)
 template <int NV>
 __device__ __forceinline__ void block_sum(const double (&x)[NV], double* sp, double* scratch) {
@@ -172,7 +207,7 @@ __device__ __forceinline__ void grid_index(const SilArgs& a, int k, int (&idx)[3
 // from the next point's; the sums skip the off-grid terms.
 template <int NDIM, typename T = double>
 __device__ __forceinline__ T apply_h_nd(const SilArgs& a, const T* x, int k, T d,
-                                        const int (&idx)[3]) {
+                                        const int (&idx)[3], T vk) {
   const int len[3] = {a.nx, a.ny, a.nz}, str[3] = {1, a.nx, a.nx * a.ny};
   T xm2[NDIM], xm1[NDIM], xp1[NDIM], xp2[NDIM];
 #pragma unroll
@@ -183,7 +218,7 @@ __device__ __forceinline__ T apply_h_nd(const SilArgs& a, const T* x, int k, T d
     xp1[ax] = x[i + 1 < L ? k + st : k];
     xp2[ax] = x[i + 2 < L ? k + 2 * st : k];
   }
-  T s = ((T)a.sht30 + (T)__ldg(a.vpot + k)) * (x[k] * d);
+  T s = ((T)a.sht30 + vk) * (x[k] * d);
 #pragma unroll
   for (int ax = 0; ax < NDIM; ++ax) {
     const T h = (T)a.shm[ax];
@@ -194,6 +229,12 @@ __device__ __forceinline__ T apply_h_nd(const SilArgs& a, const T* x, int k, T d
     if (i + 2 < L) s += h * (xp2[ax] * d);
   }
   return s;
+}
+
+template <int NDIM, typename T = double>
+__device__ __forceinline__ T apply_h_nd(const SilArgs& a, const T* x, int k, T d,
+                                        const int (&idx)[3]) {
+  return apply_h_nd<NDIM, T>(a, x, k, d, idx, (T)__ldg(a.vpot + k));
 }
 
 // Krylov coefficients of both chains (every CTA computes the same values):
@@ -847,10 +888,23 @@ __global__ void __launch_bounds__(kSilThreads, 1) sil_kernel(SilArgs a) {
 template <int NDIM>
 constexpr int kPsodIlp = NDIM == 3 ? 2 : 4;
 
-template <int KABS, bool DM, int NDIM>
-__device__ __forceinline__ void psod_points(const SilArgs& a, Range r, const double* un,
-                                            const double* vn, double* um, double* vm, double c,
-                                            double e, double (&q)[4]);
+// What a PSOD step reads of a point and never writes: V, psi0 and the absorber.
+// With KS the CTA's values stay in shared memory for the whole run ([4][cnt],
+// every thread reads back what it stored), and a step moves 48 instead of 80 bytes
+// per point to and from L2 (1023 x 769: 10.3 -> 9.6 us a step).
+template <bool KS>
+struct PsodConst {
+  const double *v, *u0, *v0, *w;  // global arrays, or the CTA's copies
+  // i: the point k, or with KS its place i in the CTA
+  static __device__ __forceinline__ double get(const double* p, long k, int i) {
+    return KS ? p[i] : __ldg(p + k);
+  }
+};
+
+template <int KABS, bool DM, int NDIM, bool KS>
+__device__ __forceinline__ void psod_points(const SilArgs& a, const PsodConst<KS>& cs, Range r,
+                                            const double* un, const double* vn, double* um,
+                                            double* vm, double c, double e, double (&q)[4]);
 
 // PSOD on a 2D grid by column strips: CTA b owns columns [256 s, 256 s + 256)
 // (s = b mod nstrips) of a band of rows; each thread walks its column down the
@@ -858,7 +912,6 @@ __device__ __forceinline__ void psod_points(const SilArgs& a, Range r, const dou
 // from memory once per band (plus two halo rows at each end), the x
 // neighbours come from the row the warp has just loaded (L1), and every other
 // array is one streaming read or write per point.
-constexpr int kBandMinRows = 16;
 
 struct Band {
   int col, r0, r1;
@@ -877,8 +930,8 @@ __device__ __forceinline__ Band my_band(const SilArgs& a) {
 
 // (psi_n and psi_{n-1} are distinct buffers within a step: the loads of later
 // rows may move ahead of this row's stores)
-template <int KABS, bool DM>
-__device__ __forceinline__ void psod2d_band(const SilArgs& a, const Band& B,
+template <int KABS, bool DM, bool KS>
+__device__ __forceinline__ void psod2d_band(const SilArgs& a, const PsodConst<KS>& cs, const Band& B,
                                             const double* __restrict__ un,
                                             const double* __restrict__ vn,
                                             double* __restrict__ um, double* __restrict__ vm,
@@ -898,6 +951,7 @@ __device__ __forceinline__ void psod2d_band(const SilArgs& a, const Band& B,
 #pragma unroll 4
   for (int r = B.r0; r < B.r1; ++r) {
     const long k = (long)r * nx + col;
+    const int i = (r - B.r0) * kSilThreads + threadIdx.x;
     // x neighbours of row r, issued unconditionally (from k when off the grid)
     const long xm2 = col >= 2 ? k - 2 : k, xm1 = col >= 1 ? k - 1 : k;
     const long xp1 = col + 1 < nx ? k + 1 : k, xp2 = col + 2 < nx ? k + 2 : k;
@@ -905,9 +959,9 @@ __device__ __forceinline__ void psod2d_band(const SilArgs& a, const Band& B,
     const double up1 = ld_state(un + xp1), up2 = ld_state(un + xp2);
     const double vm2 = ld_state(vn + xm2), vm1 = ld_state(vn + xm1);
     const double vp1 = ld_state(vn + xp1), vp2 = ld_state(vn + xp2);
-    const double vk = __ldg(a.vpot + k);
+    const double vk = cs.get(cs.v, k, i);
     const double umk = um[k], vmk = vm[k];
-    const double u0k = __ldg(a.u0 + k), v0k = __ldg(a.v0 + k);
+    const double u0k = cs.get(cs.u0, k, i), v0k = cs.get(cs.v0, k, i);
     // the next window row
     const int rn = r + 3;
     const bool inn = rn < ny;
@@ -931,11 +985,11 @@ __device__ __forceinline__ void psod2d_band(const SilArgs& a, const Band& B,
     }
     double nu, nv;
     if (KABS == 1) {
-      const double w = a.vabc[k];
+      const double w = cs.get(cs.w, k, i);
       nu = umk + c * hv - c * w * uk;
       nv = vmk - c * hu - c * w * vkk;
     } else if (KABS == 2) {
-      const double w = a.vabc[k];
+      const double w = cs.get(cs.w, k, i);
       nu = w * (umk + c * hv);
       nv = w * (vmk - c * hu);
     } else {
@@ -958,53 +1012,56 @@ __device__ __forceinline__ void psod2d_band(const SilArgs& a, const Band& B,
   }
 }
 
-template <int NDIM>
-__device__ __forceinline__ void psod_dispatch(const SilArgs& a, Range r, const double* un,
-                                              const double* vn, double* um, double* vm, double c,
-                                              double e, double (&q)[4]) {
+template <int NDIM, bool KS>
+__device__ __forceinline__ void psod_dispatch(const SilArgs& a, const PsodConst<KS>& cs, Range r,
+                                              const double* un, const double* vn, double* um,
+                                              double* vm, double c, double e, double (&q)[4]) {
   if (NDIM == 2 && a.nstrips > 0) {
     const Band B = my_band(a);
     switch (a.kabs + (a.dm ? 3 : 0)) {
-      case 0: psod2d_band<0, false>(a, B, un, vn, um, vm, c, e, q); break;
-      case 1: psod2d_band<1, false>(a, B, un, vn, um, vm, c, e, q); break;
-      case 2: psod2d_band<2, false>(a, B, un, vn, um, vm, c, e, q); break;
-      case 3: psod2d_band<0, true>(a, B, un, vn, um, vm, c, e, q); break;
-      case 4: psod2d_band<1, true>(a, B, un, vn, um, vm, c, e, q); break;
-      default: psod2d_band<2, true>(a, B, un, vn, um, vm, c, e, q); break;
+      case 0: psod2d_band<0, false>(a, cs, B, un, vn, um, vm, c, e, q); break;
+      case 1: psod2d_band<1, false>(a, cs, B, un, vn, um, vm, c, e, q); break;
+      case 2: psod2d_band<2, false>(a, cs, B, un, vn, um, vm, c, e, q); break;
+      case 3: psod2d_band<0, true>(a, cs, B, un, vn, um, vm, c, e, q); break;
+      case 4: psod2d_band<1, true>(a, cs, B, un, vn, um, vm, c, e, q); break;
+      default: psod2d_band<2, true>(a, cs, B, un, vn, um, vm, c, e, q); break;
     }
     return;
   }
   switch (a.kabs + (a.dm ? 3 : 0)) {
-    case 0: psod_points<0, false, NDIM>(a, r, un, vn, um, vm, c, e, q); break;
-    case 1: psod_points<1, false, NDIM>(a, r, un, vn, um, vm, c, e, q); break;
-    case 2: psod_points<2, false, NDIM>(a, r, un, vn, um, vm, c, e, q); break;
-    case 3: psod_points<0, true, NDIM>(a, r, un, vn, um, vm, c, e, q); break;
-    case 4: psod_points<1, true, NDIM>(a, r, un, vn, um, vm, c, e, q); break;
-    default: psod_points<2, true, NDIM>(a, r, un, vn, um, vm, c, e, q); break;
+    case 0: psod_points<0, false, NDIM>(a, cs, r, un, vn, um, vm, c, e, q); break;
+    case 1: psod_points<1, false, NDIM>(a, cs, r, un, vn, um, vm, c, e, q); break;
+    case 2: psod_points<2, false, NDIM>(a, cs, r, un, vn, um, vm, c, e, q); break;
+    case 3: psod_points<0, true, NDIM>(a, cs, r, un, vn, um, vm, c, e, q); break;
+    case 4: psod_points<1, true, NDIM>(a, cs, r, un, vn, um, vm, c, e, q); break;
+    default: psod_points<2, true, NDIM>(a, cs, r, un, vn, um, vm, c, e, q); break;
   }
 }
 
 // psi_{n-1}(k) <- psi_{n-1}(k) - i c H psi_n(k) with absorber KABS (0 none,
 // 1 .VOPTIC, 2 .SMOOTHW) and, with DM, the field term; returns the new value
-template <int KABS, bool DM, int NDIM>
-__device__ __forceinline__ void psod_point(const SilArgs& a, const double* un, const double* vn,
-                                           const double* um, const double* vm, int k, double c,
-                                           double e, double& nu, double& nv) {
+template <int KABS, bool DM, int NDIM, bool KS>
+__device__ __forceinline__ void psod_point(const SilArgs& a, const PsodConst<KS>& cs,
+                                           const double* un, const double* vn, const double* um,
+                                           const double* vm, int k, int i, double c, double e,
+                                           double& nu, double& nv) {
   const double uk = ld_state(un + k), vk = ld_state(vn + k);
   int idx[3];
   grid_index<NDIM>(a, k, idx);
-  double hv = apply_h_nd<NDIM>(a, vn, k, 1.0, idx), hu = apply_h_nd<NDIM>(a, un, k, 1.0, idx);
+  const double pot = cs.get(cs.v, k, i);
+  double hv = apply_h_nd<NDIM>(a, vn, k, 1.0, idx, pot);
+  double hu = apply_h_nd<NDIM>(a, un, k, 1.0, idx, pot);
   if (DM) {
     const double de = __ldg(a.dm + k) * e;
     hv -= de * vk;
     hu -= de * uk;
   }
   if (KABS == 1) {
-    const double w = a.vabc[k];
+    const double w = cs.get(cs.w, k, i);
     nu = um[k] + c * hv - c * w * uk;
     nv = vm[k] - c * hu - c * w * vk;
   } else if (KABS == 2) {
-    const double w = a.vabc[k];
+    const double w = cs.get(cs.w, k, i);
     nu = w * (um[k] + c * hv);
     nv = w * (vm[k] - c * hu);
   } else {
@@ -1017,10 +1074,10 @@ __device__ __forceinline__ void psod_point(const SilArgs& a, const double* un, c
 // with all their loads issued before the first store (no branch between
 // them), then the rest one by one; q gets <psi0|psi_{n+1}>'s four sums in
 // point order
-template <int KABS, bool DM, int NDIM>
-__device__ __forceinline__ void psod_points(const SilArgs& a, Range r, const double* un,
-                                            const double* vn, double* um, double* vm, double c,
-                                            double e, double (&q)[4]) {
+template <int KABS, bool DM, int NDIM, bool KS>
+__device__ __forceinline__ void psod_points(const SilArgs& a, const PsodConst<KS>& cs, Range r,
+                                            const double* un, const double* vn, double* um,
+                                            double* vm, double c, double e, double (&q)[4]) {
   const int t = threadIdx.x;
   int k0 = r.lo + t;
   for (; k0 + (kPsodIlp<NDIM> - 1) * kSilThreads < r.hi; k0 += kPsodIlp<NDIM> * kSilThreads) {
@@ -1028,9 +1085,9 @@ __device__ __forceinline__ void psod_points(const SilArgs& a, Range r, const dou
 #pragma unroll
     for (int j = 0; j < kPsodIlp<NDIM>; ++j) {
       const int k = k0 + j * kSilThreads;
-      psod_point<KABS, DM, NDIM>(a, un, vn, um, vm, k, c, e, nu[j], nv[j]);
-      u0k[j] = __ldg(a.u0 + k);
-      v0k[j] = __ldg(a.v0 + k);
+      psod_point<KABS, DM, NDIM>(a, cs, un, vn, um, vm, k, k - r.lo, c, e, nu[j], nv[j]);
+      u0k[j] = cs.get(cs.u0, k, k - r.lo);
+      v0k[j] = cs.get(cs.v0, k, k - r.lo);
     }
 #pragma unroll
     for (int j = 0; j < kPsodIlp<NDIM>; ++j) {
@@ -1045,8 +1102,8 @@ __device__ __forceinline__ void psod_points(const SilArgs& a, Range r, const dou
   }
   for (; k0 < r.hi; k0 += kSilThreads) {
     double nu, nv;
-    psod_point<KABS, DM, NDIM>(a, un, vn, um, vm, k0, c, e, nu, nv);
-    const double u0k = __ldg(a.u0 + k0), v0k = __ldg(a.v0 + k0);
+    psod_point<KABS, DM, NDIM>(a, cs, un, vn, um, vm, k0, k0 - r.lo, c, e, nu, nv);
+    const double u0k = cs.get(cs.u0, k0, k0 - r.lo), v0k = cs.get(cs.v0, k0, k0 - r.lo);
     um[k0] = nu;
     vm[k0] = nv;
     q[0] += u0k * nu;
@@ -1065,29 +1122,95 @@ __device__ __forceinline__ void psod_points(const SilArgs& a, Range r, const dou
 // c = CST/4 and a midpoint step of CST/2 to TI + DT, psi_{n-1} reset to psi0
 // (with the reference's copy defect on request), then steps of CST.
 //
-// Two CTAs per SM (128 registers, no spills): the passes over a large grid are
-// load-latency bound, and more warps hide it.
-template <int NDIM>
+// Two CTAs per SM (128 registers): the passes over a large grid are load-latency
+// bound, and more warps hide it.  1023 x 769: 32 us a step with points in two fields'
+// arrays and the sums read by every CTA, 14.7 with loads in flight together, 9.3 with
+// bands, V, psi0 and the absorber in shared memory (10.3 without) and the sums beside
+// the barrier (9.6 without; 200 x 150: 3.8 -> 3.2).
+template <int NDIM, bool KS>
 __global__ void __launch_bounds__(kSilThreads, 2) psod_kernel(SilArgs a) {
-  __shared__ double sp[4], st[4], scratch[(kSilThreads / 32) * 8];
-  __shared__ double s_red[kSilThreads];
+  extern __shared__ __align__(16) unsigned char psod_dyn[];
+  __shared__ double scratch[(kSilThreads / 32) * 8];
+  __shared__ double s_red[128];
   __shared__ int s_flag[2];
   const Range r = my_range(a.n);
   const int t = threadIdx.x;
   unsigned phase = 0;  // grid barriers passed in this launch
   double *un = a.u, *vn = a.v, *um = a.up, *vm = a.vp;
+  // the CTA's points as its threads walk them: f(point, place in the CTA)
+  auto each_point = [&](auto f) {
+    if (NDIM == 2 && a.nstrips > 0) {
+      const Band B = my_band(a);
+      if (B.col < a.nx)
+        for (int row = B.r0; row < B.r1; ++row)
+          f((long)row * a.nx + B.col, (row - B.r0) * kSilThreads + t);
+    } else {
+      for (int k = r.lo + t; k < r.hi; k += kSilThreads) f((long)k, k - r.lo);
+    }
+  };
+  PsodConst<KS> cs{a.vpot, a.u0, a.v0, a.vabc};
+  if (KS) {
+    const int cnt = a.cta_points;
+    double* sm = reinterpret_cast<double*>(psod_dyn);
+    each_point([&](long k, int i) {
+      sm[i] = a.vpot[k];
+      sm[cnt + i] = a.u0[k];
+      sm[2 * cnt + i] = a.v0[k];
+      if (a.kabs) sm[3 * cnt + i] = a.vabc[k];
+    });
+    cs = PsodConst<KS>{sm, sm + cnt, sm + 2 * cnt, sm + 3 * cnt};
+  }
+  // The four sums of a C(t) sample: every CTA publishes its own ([4][G][4] by
+  // barrier count) before the step's barrier, and one CTA, another one each step,
+  // adds them up in CTA order while it waits at the NEXT barrier: nobody needs the
+  // total meanwhile, and read by all CTAs after the barrier it cost 1 to 2 us of
+  // every step.  A buffer is written again four barriers on, by when the summing
+  // CTA has arrived at two more.
+  int pending = -1;        // sample published before the last barrier
+  unsigned pending_at = 0;  // that barrier
+  auto sum_pending = [&] {  // threads 32..159
+    const int G = gridDim.x, i = t - 32;
+    if (i < 0 || i >= 128) return;
+    const double* part = a.part + (size_t)(pending_at & 3u) * G * 4;
+    const int q = i & 3, row = i >> 2;
+    double s = 0.0;
+    for (int i0 = row; i0 < G; i0 += 10 * 32) {
+      double x[10];
+#pragma unroll
+      for (int j = 0; j < 10; ++j) {
+        const int b = i0 + 32 * j;
+        x[j] = b < G ? __ldcg(part + 4 * b + q) : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < 10; ++j) s += x[j];
+    }
+    s_red[i] = s;
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (i < 32) {
+      double st = 0.0;
+      for (int j = 0; j < 32; ++j) st += s_red[4 * j + (i & 3)];
+      const double other = __shfl_down_sync(0xffffffffu, st, 1);
+      if (i == 0) a.c_out[pending].x = st + other;
+      if (i == 2) a.c_out[pending].y = st - other;
+    }
+  };
   auto reduce_c = [&](double (&q)[4], int slot) -> bool {
-    block_sum<4>(q, sp, scratch);
-    if (!grid_reduce(a, sp, st, 4, s_flag, s_red, phase)) return false;
-    if (t == 0 && blockIdx.x == 0 && slot >= 0)
-      a.c_out[slot] = make_double2(st[0] + st[1], st[2] - st[3]);
+    const unsigned at = phase;
+    block_sum<4>(q, a.part + ((size_t)(at & 3u) * gridDim.x + blockIdx.x) * 4, scratch);
+    const bool mine = pending >= 0 && blockIdx.x == pending_at % gridDim.x;
+    if (!grid_barrier(a, s_flag, phase, [&] {
+          if (mine) sum_pending();
+        }))
+      return false;
+    pending = slot;
+    pending_at = at;
     return true;
   };
   auto step = [&](double c, int slot, long call) __attribute__((always_inline)) -> bool {
     double q[4] = {0.0, 0.0, 0.0, 0.0};
     const double e = a.ef ? a.ef[call] : 0.0;  // chpot.f:46-50: V - DM EF
     // the absorber, the field and the dimension as template arguments
-    psod_dispatch<NDIM>(a, r, un, vn, um, vm, c, e, q);
+    psod_dispatch<NDIM, KS>(a, cs, r, un, vn, um, vm, c, e, q);
     if (!reduce_c(q, slot)) return false;
     double* x = un;
     un = um;
@@ -1113,22 +1236,16 @@ __global__ void __launch_bounds__(kSilThreads, 2) psod_kernel(SilArgs a) {
     if (!step(0.25 * a.cst, -1, 0)) return;  // psod.f:120-121
     if (!step(0.5 * a.cst, 1, 1)) return;    // psod.f:123-124
     // psod.f:136-141, over the points this CTA's steps write
-    auto copy_back = [&](long k) {
+    each_point([&](long k, int) {
       um[k] = __ldg(a.u0 + k);
       vm[k] = (a.copy_quirk && (k & 1)) ? __ldg(a.v0 + k - 1) : __ldg(a.v0 + k);
-    };
-    if (NDIM == 2 && a.nstrips > 0) {
-      const Band B = my_band(a);
-      if (B.col < a.nx)
-        for (int row = B.r0; row < B.r1; ++row) copy_back((long)row * a.nx + B.col);
-    } else {
-      for (int k = r.lo + t; k < r.hi; k += kSilThreads) copy_back(k);
-    }
+    });
     __syncthreads();
     s0 = 2;
   }
   for (int s = s0; s <= a.nsteps; ++s)
     if (!step(a.cst, s, a.slot0 + s)) return;
+  if (pending >= 0 && blockIdx.x == 0) sum_pending();
 }
 
 // <u|H u> + <v|H v> and |u|^2 + |v|^2 (EIGENERG, eigenerg.f:56-66): per-CTA
@@ -1212,6 +1329,7 @@ struct espec_grid_plan {
   int m = 0, absorb = 0, quirks = 0;
   int precision = ESPEC_FP64;  // ESPEC_MIXED (SIL): FP32 Lanczos vectors and H psi
   int nblocks = 0, nblocks_max = 0;  // CTAs of the cooperative launches (<= co-resident)
+  bool bands = false;                // PSOD by column strips (psod2d_band)
   bool loaded = false, has_state = false;
   double *d_vpot = nullptr, *d_mask = nullptr, *d_u = nullptr, *d_v = nullptr;
   double *d_u0 = nullptr, *d_v0 = nullptr, *d_L = nullptr, *d_work = nullptr, *d_wbuf = nullptr;
@@ -1255,14 +1373,12 @@ long grid_wait_limit() { return g_wait_limit.load(); }
 }  // namespace espec
 
 // column strips of the PSOD pass on a 2D grid (0: contiguous point ranges):
-// used when the CTA count is a multiple of the strip count and every band
-// holds at least kBandMinRows rows
+// planned by espec_grid_create, and the CTA count is a multiple of the strip count
 static int band_strips(const espec_grid_plan* p) {
-  if (p->method != ESPEC_PSOD || p->ndim != 2) return 0;
+  if (!p->bands) return 0;
   const int ns = (p->np[0] + kSilThreads - 1) / kSilThreads;
   if (p->nblocks % ns != 0) return 0;
-  const int nb = p->nblocks / ns;
-  return p->np[1] / nb >= kBandMinRows ? ns : 0;
+  return ns;
 }
 
 static SilArgs sil_args(const espec_grid_plan* p) {
@@ -1312,6 +1428,25 @@ static SilArgs sil_args(const espec_grid_plan* p) {
   return a;
 }
 
+// the PSOD kernel, with the points' constants in shared memory or not
+static const void* psod_form(int ndim, bool in_smem) {
+  if (in_smem)
+    return ndim == 1   ? (const void*)psod_kernel<1, true>
+           : ndim == 2 ? (const void*)psod_kernel<2, true>
+                       : (const void*)psod_kernel<3, true>;
+  return ndim == 1   ? (const void*)psod_kernel<1, false>
+         : ndim == 2 ? (const void*)psod_kernel<2, false>
+                     : (const void*)psod_kernel<3, false>;
+}
+
+// places of a CTA's points (my_range, my_band)
+static int psod_cta_points(const espec_grid_plan* p) {
+  const int ns = band_strips(p);
+  if (ns == 0) return (int)((p->n + p->nblocks - 1) / p->nblocks);
+  const int nb = p->nblocks / ns;
+  return (p->np[1] + nb - 1) / nb * kSilThreads;
+}
+
 extern "C" int espec_grid_create(espec_grid_plan** out, int method, int ndim, const int* np,
                                  const double* shm, double dt_fs, int mp, int precision,
                                  int absorb, int quirks) {
@@ -1358,9 +1493,7 @@ extern "C" int espec_grid_create(espec_grid_plan** out, int method, int ndim, co
   // co-resident CTAs for the cooperative launch
   int dev = 0, nsm = 0, occ = 0;
   const void* kern =
-      psod ? (ndim == 1   ? (const void*)psod_kernel<1>
-              : ndim == 2 ? (const void*)psod_kernel<2>
-                          : (const void*)psod_kernel<3>)
+      psod ? psod_form(ndim, false)
            : (ndim == 1   ? (const void*)sil_kernel<1, false, double>
               : ndim == 2 ? (const void*)sil_kernel<2, false, double>
                           : (const void*)sil_kernel<3, false, double>);
@@ -1372,10 +1505,11 @@ extern "C" int espec_grid_create(espec_grid_plan** out, int method, int ndim, co
     return set_cuda_error("device query", e);
   }
   long want = (n + kSilThreads - 1) / kSilThreads;
-  // one CTA per SM keeps the barriers short; a PSOD pass over a large grid
-  // (16 points or more per thread) takes every co-resident CTA instead
-  long cap = nsm;
-  if (psod && n >= 16L * nsm * kSilThreads) cap = (long)nsm * occ;
+  // one CTA per SM keeps the barriers short; a PSOD pass of more than a point per
+  // thread is bound by the latency of its loads and takes every co-resident CTA
+  // (per step, one -> two CTAs per SM: 80^3 18.6 -> 11.5 us, 50^3 8.0 -> 5.7)
+  const bool wide = psod && n > (long)nsm * kSilThreads;
+  long cap = wide ? (long)nsm * occ : nsm;
   if (cap > (long)nsm * occ) cap = (long)nsm * occ;
   // the fewest CTAs that keep the largest per-CTA share: a grid barrier costs
   // about one arrival per CTA, so 65536 points take 128 CTAs of two 256-point
@@ -1385,11 +1519,17 @@ extern "C" int espec_grid_create(espec_grid_plan** out, int method, int ndim, co
     const long per = (want + cap - 1) / cap;
     want = (want + per - 1) / per;
   }
-  // a PSOD pass over a large 2D grid runs by column strips: every co-resident
-  // CTA, a multiple of the strip count, each band at least kBandMinRows rows
-  if (psod && ndim == 2) {
-    const long ns = (np[0] + kSilThreads - 1) / kSilThreads, nb = cap / ns;
-    if (nb >= 1 && np[1] / nb >= kBandMinRows) want = ns * nb;
+  // On a 2D grid such a pass runs by column strips, where these fill a quarter of
+  // their lanes or more: a multiple of the strip count, bands of two rows or more.
+  // Per step, points -> bands: 1023 x 769 14.7 -> 9.6 us, 600 x 500 11.9 -> 6.9,
+  // 400 x 300 8.3 -> 5.0; 100 x 100, below the line, 3.8 -> 4.2.
+  if (wide && ndim == 2) {
+    const long ns = (np[0] + kSilThreads - 1) / kSilThreads;
+    const long nb = std::min((long)nsm * occ / ns, (long)np[1] / 2);
+    if (nb >= 1 && 4L * np[0] >= ns * kSilThreads) {
+      want = ns * nb;
+      p->bands = true;
+    }
   }
   p->nblocks = (int)(want > 0 ? want : 1);
   p->nblocks_max = p->nblocks;
@@ -1499,11 +1639,26 @@ static int grid_launch(espec_grid_plan* p, int nsteps, bool from_start, cudaStre
     if (p->d_dm && a.slot0 + nsteps >= p->n_ef)
       return set_error(ESPEC_EINVAL, "the pulse field table ends before the run does");
     void* args[] = {&a};
-    const void* kern = p->ndim == 1   ? (const void*)psod_kernel<1>
-                       : p->ndim == 2 ? (const void*)psod_kernel<2>
-                                      : (const void*)psod_kernel<3>;
-    GRID_CK(cudaLaunchCooperativeKernel(kern, dim3(p->nblocks),
-                                        dim3(kSilThreads), args, 0, st));
+    // V, psi0 and the absorber of a CTA's points in its shared memory where all
+    // CTAs then still run together
+    a.cta_points = psod_cta_points(p);
+    const size_t dyn = sizeof(double) * (size_t)a.cta_points * (a.kabs ? 4 : 3);
+    const void* kern = psod_form(p->ndim, true);
+    int dev = 0, nsm = 0, optin = 0, occ = 0;
+    cudaFuncAttributes fa{};
+    GRID_CK(cudaGetDevice(&dev));
+    GRID_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    GRID_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    GRID_CK(cudaFuncGetAttributes(&fa, kern));
+    if (fa.sharedSizeBytes + dyn <= (size_t)optin) {
+      GRID_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   optin - (int)fa.sharedSizeBytes));
+      GRID_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kSilThreads, dyn));
+    }
+    const bool in_smem = (long)occ * nsm >= p->nblocks;
+    if (!in_smem) kern = psod_form(p->ndim, false);
+    GRID_CK(cudaLaunchCooperativeKernel(kern, dim3(p->nblocks), dim3(kSilThreads), args,
+                                        in_smem ? dyn : 0, st));
     // the kernel swaps the roles of the two state buffers once per step
     const long swaps = from_start ? (nsteps >= 1 ? nsteps + 1 : 0) : nsteps;
     if (swaps & 1) {

@@ -43,6 +43,7 @@ struct SilArgs {
   double sht30;   // 30 * (shm[0] + shm[1] + shm[2])
   double inv_nx, inv_ny;  // 1/nx, 1/ny: grid indices by multiplication
   int nstrips;  // PSOD on a 2D grid: column strips of kSilThreads (0: point ranges)
+  int cta_points;  // PSOD: places for a CTA's points in shared memory
   const double* vpot;
   const double* mask;  // .SMOOTHW mask or null
   double* u;           // state (in / out)
