@@ -146,30 +146,33 @@ __device__ __forceinline__ void passes(double2* v, const Twiddles& tw, long k, i
   }
 }
 
-// Transforms of 2^mf points, 4 <= mf <= kOneMax, whole in shared memory: 16
-// points per thread, the passes taken four at a time in registers (REM of them,
+// Transforms of 2^mf points, 4 <= mf <= kOneMax, whole in shared memory: 8
+// points per thread, the passes taken three at a time in registers (REM of them,
 // the remainder, first), one exchange through shared memory between the groups; the
 // input is prepared as it is read and the last group writes the result.
-// Small transforms share a CTA.  The exchange adds one element in 16, which
-// keeps the stride-16 writes of the first groups on distinct banks.
+// Small transforms share a CTA.  The exchange adds one element in 8, which
+// keeps the stride-8 writes of the first groups on distinct banks.
 // HBM then carries the samples once and the spectrum once; with one kernel per
 // radix-2 pass every pass moved the whole batch (1024 x 4096 points: 12 passes
-// of 134 MB and a prep pass, 295 us).
+// of 134 MB and a prep pass, 295 us).  What is left is latency: 32 warps per SM
+// take 64 us; with 16 points per thread and four passes at a time, one exchange
+// less but 16 warps, it was 70 us.
 constexpr int kOneMax = 13;
-constexpr int kOneThreads = 256;
-__device__ __forceinline__ int padded(int i) { return i + (i >> 4); }
+constexpr int kOneLog = 3, kOneP = 1 << kOneLog;  // points per thread
+constexpr int kOneThreads = 512;
+__host__ __device__ __forceinline__ constexpr int padded(int i) { return i + (i >> kOneLog); }
 
 template <int REM, int T>
-__global__ void __launch_bounds__(T, 512 / T) spec_one_kernel(PrepArgs a, Twiddles tw,
+__global__ void __launch_bounds__(T, 1024 / T) spec_one_kernel(PrepArgs a, Twiddles tw,
                                                                       double scale) {
   extern __shared__ double2 spec_sm[];
-  const int mf = a.mf, n = 1 << mf, tp = n >> 4;  // threads of a packet
+  const int mf = a.mf, n = 1 << mf, tp = n >> kOneLog;  // threads of a packet
   const int g = threadIdx.x / tp, t = threadIdx.x % tp;
   const long p = (long)blockIdx.x * (T / tp) + g;
   const bool on = p < a.npk;
-  double2* sm = spec_sm + (size_t)g * (n + (n >> 4));
-  double2 v[16];
-  constexpr int R = 1 << REM, B = 16 / R;  // B groups of 2^REM points, k = 0
+  double2* sm = spec_sm + (size_t)g * padded(n);
+  double2 v[kOneP];
+  constexpr int R = 1 << REM, B = kOneP / R;  // B groups of 2^REM points, k = 0
 #pragma unroll
   for (int i = 0; i < B; ++i) {
     const int j0 = t + i * tp;
@@ -181,32 +184,26 @@ __global__ void __launch_bounds__(T, 512 / T) spec_one_kernel(PrepArgs a, Twiddl
   for (int i = 0; i < B; ++i) {
     passes<REM>(v + i * R, tw, 0, 0, mf);
     const int j0 = t + i * tp;
-    if (mf > REM) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) sm[padded(j0 * R + brev_c(r, REM))] = v[i * R + r];
-    } else if (on) {  // 16 points: one group is the whole transform
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-        a.out[p * n + brev_c(r, REM)] = make_double2(v[r].x * scale, v[r].y * scale);
-    }
+    for (int r = 0; r < R; ++r) sm[padded(j0 * R + brev_c(r, REM))] = v[i * R + r];
   }
   __syncthreads();
-  for (int s = REM; s < mf; s += 4) {
+  for (int s = REM; s < mf; s += kOneLog) {
     const int k = t & ((1 << s) - 1);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = sm[padded(t + q * tp)];
-    passes<4>(v, tw, k, s, mf);
-    const int o = (t - k) * 16 + k;
-    if (s + 4 < mf) {
+    for (int q = 0; q < kOneP; ++q) v[q] = sm[padded(t + q * tp)];
+    passes<kOneLog>(v, tw, k, s, mf);
+    const int o = (t - k) * kOneP + k;
+    if (s + kOneLog < mf) {
       __syncthreads();
 #pragma unroll
-      for (int r = 0; r < 16; ++r) sm[padded(o + (brev_c(r, 4) << s))] = v[r];
+      for (int r = 0; r < kOneP; ++r) sm[padded(o + (brev_c(r, kOneLog) << s))] = v[r];
       __syncthreads();
     } else if (on) {
       double2* out = a.out + p * n;
 #pragma unroll
-      for (int r = 0; r < 16; ++r)
-        out[o + (brev_c(r, 4) << s)] = make_double2(v[r].x * scale, v[r].y * scale);
+      for (int r = 0; r < kOneP; ++r)
+        out[o + (brev_c(r, kOneLog) << s)] = make_double2(v[r].x * scale, v[r].y * scale);
     }
   }
 }
@@ -237,10 +234,10 @@ __global__ void __launch_bounds__(256) spec_pass_kernel(PrepArgs a, const double
 template <int REM, int T>
 cudaError_t launch_one(const PrepArgs& a, const Twiddles& tw, double scale, cudaStream_t st) {
   static DeviceFlags attr;
-  const size_t smem = sizeof(double2) * 17 * T;
+  const size_t smem = sizeof(double2) * padded(kOneP * T);
   cudaError_t e = set_max_smem_once(attr, spec_one_kernel<REM, T>, smem);
   if (e != cudaSuccess) return e;
-  const int per = T >> (a.mf - 4);  // packets per CTA
+  const int per = T >> (a.mf - kOneLog);  // packets per CTA
   spec_one_kernel<REM, T><<<(a.npk + per - 1) / per, T, smem, st>>>(a, tw, scale);
   return cudaGetLastError();
 }
@@ -347,11 +344,10 @@ extern "C" int espec_spectrum_dev(int npk, int mf, const void* in, long ld, int 
     if (mf == kOneMax) {
       e = launch_one<1, 2 * kOneThreads>(a, tws, rn, st);
     } else {
-      switch (mf % 4) {
-        case 0: e = launch_one<4, kOneThreads>(a, tws, rn, st); break;
+      switch (mf % kOneLog) {
+        case 0: e = launch_one<kOneLog, kOneThreads>(a, tws, rn, st); break;
         case 1: e = launch_one<1, kOneThreads>(a, tws, rn, st); break;
-        case 2: e = launch_one<2, kOneThreads>(a, tws, rn, st); break;
-        default: e = launch_one<3, kOneThreads>(a, tws, rn, st); break;
+        default: e = launch_one<2, kOneThreads>(a, tws, rn, st); break;
       }
     }
     SPEC_CK(e);
