@@ -9,10 +9,10 @@
 // and 2, then every odd prime factor), natural order in and out: each thread
 // takes one butterfly of a stage into registers, twiddles it from a per-size
 // table w[e] = e^{+2 pi i e / N} and writes its r outputs (radix 2, 3, 4 and 5
-// written out, other radices up to 16 as a direct sum in registers, larger
-// primes output by output: N r complex multiply-adds for such a stage).  The step, the tables (x order, and the kinetic
-// table in natural FFT order) and the C(t) samples are those of the register
-// kernels: spo_packet (spo1d.cuh) and sod1d_kernel (sod1d.cuh).
+// written out, other primes as direct sums, prime_stage).  The step, the tables
+// (x order, and the kinetic table in natural FFT order) and the C(t) samples are
+// those of the register kernels: spo_packet (spo1d.cuh) and sod1d_kernel
+// (sod1d.cuh).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -65,9 +65,7 @@ __device__ __forceinline__ cpx<double> rot90(cpx<double> x, bool inv) {
 }
 
 // y_k = sum_q x_q w_R^{qk}, w_R = e^{+2 pi i/R} (conjugated for the
-// inverse), in registers: the radix-2, 3, 4 and 5 butterflies written out,
-// other radices up to kAnyRegRadix as the direct sum with the table's w_R
-constexpr int kAnyRegRadix = 16;
+// inverse), in registers: the radix-2, 3, 4 and 5 butterflies written out
 template <int R>
 __device__ __forceinline__ void dft_small(cpx<double>* x, const double2* __restrict__ tw, int n,
                                           bool inv) {
@@ -111,81 +109,97 @@ __device__ __forceinline__ void dft_small(cpx<double>* x, const double2* __restr
   }
 }
 
-// one Stockham stage of radix R (compile time) or r (run time): butterfly j
-// takes x_q = src[j + q m], q < r, twiddles them by w_N^{(j % ns) q N/span},
-// and writes its r-point DFT to dst[(j / ns) span + k ns + j % ns]
+// one Stockham stage of radix R: butterfly j takes x_q = src[j + q m], q < R,
+// twiddles them by w_N^{(j % ns) q N/span}, and writes its R-point DFT to
+// dst[(j / ns) span + k ns + j % ns]
 template <int R>
 __device__ __forceinline__ void any_stage(const double2* __restrict__ tw, const cpx<double>* src,
-                                          cpx<double>* dst, int n, int r, int ns, bool inv) {
+                                          cpx<double>* dst, int n, int ns, bool inv) {
   const int T = blockDim.x, t = threadIdx.x;
-  const int m = n / r, span = ns * r, tws = n / span;
+  const int m = n / R, span = ns * R, tws = n / span;
   for (int j = t; j < m; j += T) {
     const int jm = j % ns, base = (j / ns) * span + jm;
-    if (R > 0 || r <= kAnyRegRadix) {
-      constexpr int RR = R > 0 ? R : kAnyRegRadix;
-      cpx<double> x[RR];
-      const int e1 = jm * tws;  // < n / r
-      int e = 0;
+    cpx<double> x[R];
+    const int e1 = jm * tws;  // < n / R
+    int e = 0;
 #pragma unroll
-      for (int q = 0; q < RR; ++q) {
-        if (R == 0 && q >= r) break;
-        x[q] = src[j + q * m];
-        if (q > 0) x[q] = twid(x[q], __ldg(tw + e), inv);
-        e += e1;  // q e1 < n: no wrap
-      }
-      if constexpr (R > 0) {
-        dft_small<R>(x, tw, n, inv);
-#pragma unroll
-        for (int k = 0; k < R; ++k) dst[base + k * ns] = x[k];
-      } else {
-        for (int k = 0; k < r; ++k) {  // direct sum with w_r^{qk} = w_N^{qk m}
-          double sr = 0.0, si = 0.0;
-          int f = 0;
-          for (int q = 0; q < r; ++q) {
-            const cpx<double> y = twid(x[q], __ldg(tw + f), inv);
-            sr += y.x;
-            si += y.y;
-            f += k * m;
-            if (f >= n) f -= n;
-          }
-          dst[base + k * ns] = mk(sr, si);
-        }
-      }
-    } else {
-      // a prime radix above kAnyRegRadix: each output from the r inputs
-      for (int k = 0; k < r; ++k) {
-        int e1 = jm * tws + k * m;
-        if (e1 >= n) e1 -= n;
-        double sr = 0.0, si = 0.0;
-        int e = 0;
-        for (int q = 0; q < r; ++q) {
-          const cpx<double> y = twid(src[j + q * m], __ldg(tw + e), inv);
-          sr += y.x;
-          si += y.y;
-          e += e1;
-          if (e >= n) e -= n;
-        }
-        dst[base + k * ns] = mk(sr, si);
-      }
+    for (int q = 0; q < R; ++q) {
+      x[q] = src[j + q * m];
+      if (q > 0) x[q] = twid(x[q], __ldg(tw + e), inv);
+      e += e1;  // q e1 < n: no wrap
     }
+    dft_small<R>(x, tw, n, inv);
+#pragma unroll
+    for (int k = 0; k < R; ++k) dst[base + k * ns] = x[k];
+  }
+}
+
+// The stage of an odd prime radix r as direct sums.  The inputs are twiddled in
+// place first; then a thread takes outputs k and r - k of one butterfly together:
+//   x_q w^{qk} + x_{r-q} w^{-qk} = (x_q + x_{r-q}) cos + i (x_q - x_{r-q}) sin,
+// which serves both outputs, so a pair of them costs 2 (r - 1) real multiply-adds
+// and 2 (r - 1) additions, and every pair has a thread.  What bounds it: shared
+// memory, three 16-byte reads per term, the roots gathered.  With a thread per
+// butterfly, which formed its r outputs one by one, a size 2 p ran on two threads;
+// us per step of one packet, before -> now: 34 points 32 -> 4.6, 578 (17 17 2) 69 ->
+// 14, 1022 (73 7 2) 541 -> 28, 1322 (661 2) 35 000 -> 129, 1326 (17 13 3 2) 128 -> 19.
+// wr: shared memory for the r values w_r^f, or null (no room): read from tw.
+__device__ __noinline__ void prime_stage(const double2* __restrict__ tw, cpx<double>* src,
+                                         cpx<double>* dst, double2* wr, int n, int r, int ns,
+                                         bool inv) {
+  const int T = blockDim.x, t = threadIdx.x;
+  const int m = n / r, span = ns * r, tws = n / span, h = (r - 1) / 2;
+  if (ns > 1)
+    for (int i = m + t; i < n; i += T) {
+      const int q = i / m, j = i - q * m;
+      src[i] = twid(src[i], __ldg(tw + (j % ns) * tws * q), inv);  // < n: q jm tws < n
+    }
+  if (wr)
+    for (int i = t; i < r; i += T) wr[i] = __ldg(tw + i * m);
+  __syncthreads();
+  for (int it = t; it < m * (h + 1); it += T) {
+    const int k = it / m, j = it - k * m, jm = j % ns;
+    const cpx<double>* x = src + j;
+    cpx<double>* y = dst + (j / ns) * span + jm;
+    const cpx<double> x0 = x[0];
+    double cr = 0.0, ci = 0.0, sr = 0.0, si = 0.0;  // sums of (x_q +- x_{r-q}) cos / sin
+    int f = 0;
+#pragma unroll 4
+    for (int q = 1; q <= h; ++q) {
+      f += k;
+      if (f >= r) f -= r;
+      const double2 w = wr ? wr[f] : __ldg(tw + f * m);
+      const cpx<double> a = x[q * m], b = x[(r - q) * m];
+      cr = fma(a.x + b.x, w.x, cr);
+      ci = fma(a.y + b.y, w.x, ci);
+      sr = fma(a.x - b.x, w.y, sr);
+      si = fma(a.y - b.y, w.y, si);
+    }
+    if (inv) {
+      sr = -sr;
+      si = -si;
+    }
+    y[k * ns] = mk(x0.x + cr - si, x0.y + ci + sr);
+    if (k > 0) y[(r - k) * ns] = mk(x0.x + cr + si, x0.y + ci - sr);
   }
 }
 
 // out = src transformed (forward: e^{+2 pi i jk/N}, inverse: conjugate, no
 // scaling); src and dst are the two N-point buffers, the result lands in one
-// of them (returned).  Ends with a CTA barrier.
+// of them (returned).  wr: shared memory for prime_stage, or null.  Ends with a CTA
+// barrier.
 __device__ cpx<double>* any_fft(const AnyPlan& pl, const double2* __restrict__ tw,
-                                cpx<double>* src, cpx<double>* dst, bool inv) {
+                                cpx<double>* src, cpx<double>* dst, double2* wr, bool inv) {
   const int n = pl.n;
   int ns = 1;  // size of the sub-transforms done so far
   for (int s = 0; s < pl.ns; ++s) {
     const int r = pl.r[s];
     switch (r) {
-      case 2: any_stage<2>(tw, src, dst, n, r, ns, inv); break;
-      case 3: any_stage<3>(tw, src, dst, n, r, ns, inv); break;
-      case 4: any_stage<4>(tw, src, dst, n, r, ns, inv); break;
-      case 5: any_stage<5>(tw, src, dst, n, r, ns, inv); break;
-      default: any_stage<0>(tw, src, dst, n, r, ns, inv); break;
+      case 2: any_stage<2>(tw, src, dst, n, ns, inv); break;
+      case 3: any_stage<3>(tw, src, dst, n, ns, inv); break;
+      case 4: any_stage<4>(tw, src, dst, n, ns, inv); break;
+      case 5: any_stage<5>(tw, src, dst, n, ns, inv); break;
+      default: prime_stage(tw, src, dst, wr, n, r, ns, inv); break;
     }
     __syncthreads();
     cpx<double>* tmp = src;
@@ -224,6 +238,7 @@ __global__ void __launch_bounds__(kAnyThreads) spo_any_kernel(SpoArgs<double> a,
   cpx<double>* b0 = reinterpret_cast<cpx<double>*>(smem_raw);
   cpx<double>* b1 = b0 + n;
   double2* red = reinterpret_cast<double2*>(b1 + n);
+  double2* wr = pl.wr ? red + 3 * (kAnyThreads / 32) : nullptr;
   const SpoPacket pk = a.pk[blockIdx.x];
   const int base = pk.off;
   double2* cout = a.c_out + pk.c_off;
@@ -243,7 +258,7 @@ __global__ void __launch_bounds__(kAnyThreads) spo_any_kernel(SpoArgs<double> a,
     const TB::phase_t* ph = step == 1 ? a.tab.h : a.tab.g;
     for (int x = t; x < n; x += T) v[x] = TB::apply(ph[base + x], v[x]);
     __syncthreads();
-    cpx<double>* f = any_fft(pl, tw, v, v == b0 ? b1 : b0, false);
+    cpx<double>* f = any_fft(pl, tw, v, v == b0 ? b1 : b0, wr, false);
     for (int x = t; x < n; x += T) {
       if (quirk) {  // spofft.f:148-154 as written: V(I) uses the updated U(I)
         const double c = a.kq_c[base + x], s = a.kq_s[base + x];
@@ -255,7 +270,7 @@ __global__ void __launch_bounds__(kAnyThreads) spo_any_kernel(SpoArgs<double> a,
       }
     }
     __syncthreads();
-    v = any_fft(pl, tw, f, f == b0 ? b1 : b0, true);
+    v = any_fft(pl, tw, f, f == b0 ? b1 : b0, wr, true);
     double cr = 0.0, ci = 0.0;
     for (int x = t; x < n; x += T) {
       const cpx<double> w = a.tab.w[base + x];
@@ -286,6 +301,7 @@ __global__ void __launch_bounds__(kAnyThreads) sod_any_kernel(SodArgs a, AnyPlan
   cpx<double>* f0 = prev + n;
   cpx<double>* f1 = f0 + n;
   double2* red = reinterpret_cast<double2*>(f1 + n);
+  double2* wr = pl.wr ? red + 3 * (kAnyThreads / 32) : nullptr;
   const SpoPacket pk = a.pk[blockIdx.x];
   const int base = pk.off;
   double2* cout = a.c_out + pk.c_off;
@@ -305,13 +321,13 @@ __global__ void __launch_bounds__(kAnyThreads) sod_any_kernel(SodArgs a, AnyPlan
   auto sod_update = [&](const cpx<double>* src, cpx<double>* dst, double f) {
     for (int x = t; x < n; x += T) f0[x] = src[x];
     __syncthreads();
-    cpx<double>* k = any_fft(pl, tw, f0, f1, false);
+    cpx<double>* k = any_fft(pl, tw, f0, f1, wr, false);
     for (int x = t; x < n; x += T) {
       const double kc = a.tab.kc[base + x];
       k[x] = mk(k[x].x * kc, k[x].y * kc);
     }
     __syncthreads();
-    const cpx<double>* h = any_fft(pl, tw, k, k == f0 ? f1 : f0, true);
+    const cpx<double>* h = any_fft(pl, tw, k, k == f0 ? f1 : f0, wr, true);
     for (int x = t; x < n; x += T) {
       const double vc = a.tab.vc[base + x];
       const double hx = fma(vc, src[x].x, h[x].x), hy = fma(vc, src[x].y, h[x].y);
@@ -381,6 +397,7 @@ __global__ void __launch_bounds__(kAnyThreads) diag_any_kernel(DiagArgs a, AnyPl
   cpx<double>* b0 = reinterpret_cast<cpx<double>*>(smem_raw);
   cpx<double>* b1 = b0 + n;
   double2* red = reinterpret_cast<double2*>(b1 + n);
+  double2* wr = pl.wr ? red + 3 * (kAnyThreads / 32) : nullptr;
   const SpoPacket pk = a.pk[blockIdx.x];
   const int base = pk.off;
   double epot = 0.0, nrm = 0.0, ekin = 0.0;
@@ -392,7 +409,7 @@ __global__ void __launch_bounds__(kAnyThreads) diag_any_kernel(DiagArgs a, AnyPl
     nrm += p.x * p.x + p.y * p.y;
   }
   __syncthreads();
-  const cpx<double>* f = any_fft(pl, tw, b0, b1, false);
+  const cpx<double>* f = any_fft(pl, tw, b0, b1, wr, false);
   for (int x = t; x < n; x += T) ekin += a.tc[base + x] * (f[x].x * f[x].x + f[x].y * f[x].y);
   ekin /= (double)n;
   const double2 s = cta_sum2(epot, nrm, red);
@@ -400,14 +417,21 @@ __global__ void __launch_bounds__(kAnyThreads) diag_any_kernel(DiagArgs a, AnyPl
   if (t == 0) a.out[pk.c_off] = make_double2(s.x + k.x, s.y);
 }
 
-template <class K, class... A>
-cudaError_t any_launch(K kern, DeviceFlags& flags, int n, int method, int nblocks,
-                       cudaStream_t st, const A&... args) {
-  const size_t smem = any_smem_bytes(n, method);
+// kern(a, plan, tw, rest...); the largest prime's table joins the buffers in shared
+// memory where it fits
+template <class K, class Args, class... Rest>
+cudaError_t any_launch(K kern, DeviceFlags& flags, AnyPlan pl, int method, int nblocks,
+                       cudaStream_t st, const Args& a, const double2* tw, Rest... rest) {
+  size_t smem = any_smem_bytes(pl.n, method);
   if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
+  int r = 0;
+  for (int s = 0; s < pl.ns; ++s)
+    if (pl.r[s] > 5 && pl.r[s] > r) r = pl.r[s];
+  pl.wr = r > 0 && smem + sizeof(double2) * r <= kMaxSmem;
+  if (pl.wr) smem += sizeof(double2) * r;
   cudaError_t e = set_max_smem_once(flags, kern, kMaxSmem);
   if (e != cudaSuccess) return e;
-  kern<<<nblocks, kAnyThreads, smem, st>>>(args...);
+  kern<<<nblocks, kAnyThreads, smem, st>>>(a, pl, tw, rest...);
   return cudaGetLastError();
 }
 
@@ -416,19 +440,19 @@ cudaError_t any_launch(K kern, DeviceFlags& flags, int n, int method, int nblock
 cudaError_t spo_any_launch(const SpoArgs<double>& a, const AnyPlan& pl, const double2* tw,
                            bool quirk, int nblocks, cudaStream_t st) {
   static DeviceFlags f;
-  return any_launch(spo_any_kernel, f, pl.n, ESPEC_SPO, nblocks, st, a, pl, tw, quirk ? 1 : 0);
+  return any_launch(spo_any_kernel, f, pl, ESPEC_SPO, nblocks, st, a, tw, quirk ? 1 : 0);
 }
 
 cudaError_t sod_any_launch(const SodArgs& a, const AnyPlan& pl, const double2* tw, int kabs,
                            int nblocks, cudaStream_t st) {
   static DeviceFlags f;
-  return any_launch(sod_any_kernel, f, pl.n, ESPEC_SOD, nblocks, st, a, pl, tw, kabs);
+  return any_launch(sod_any_kernel, f, pl, ESPEC_SOD, nblocks, st, a, tw, kabs);
 }
 
 cudaError_t diag_any_launch(const DiagArgs& a, const AnyPlan& pl, const double2* tw, int nblocks,
                             cudaStream_t st) {
   static DeviceFlags f;
-  return any_launch(diag_any_kernel, f, pl.n, ESPEC_SPO, nblocks, st, a, pl, tw);
+  return any_launch(diag_any_kernel, f, pl, ESPEC_SPO, nblocks, st, a, tw);
 }
 
 // w[e] = (cos 2 pi e / N, sin 2 pi e / N), from long-double cosines and sines

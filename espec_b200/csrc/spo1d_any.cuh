@@ -17,6 +17,7 @@ constexpr int kAnyMaxN = 1 << 16;  // the shared-memory bound below is the tight
 struct AnyPlan {
   int n, ns;               // size, number of stages
   int r[kAnyMaxStages];    // radix of each stage (product n)
+  int wr = 0;              // shared memory holds a prime radix's table (set by the launch)
 };
 
 // radices for size n (even, 4 <= n <= kAnyMaxN); false if n has none
