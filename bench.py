@@ -830,7 +830,7 @@ def profile_case(name, dev):
         st = EG.lcg_start(g.n, 4, dev).expand(32, 4, g.n).contiguous()
         r = EG.solve(g, v, st, nstates=4, m=40, tol=1e-9, maxrest=300)
         return float(r["resid"].max())
-    if name in ("spond2d", "spond3d"):  # x_pass / axis_pass passes
+    if name in ("spond2d", "spond3d"):  # the cooperative split-operator kernel
         np_, prec, nsteps = ([256, 256], "fp64", 20) if name == "spond2d" else \
             ([128, 128, 128], "mixed", 10)
         axes = [np.linspace(0.6, 3.6, k) for k in np_]
