@@ -340,8 +340,11 @@ size_t packed_bytes(int ln) {
 // Threads: 512 where a thread's points, twiddles and preloaded factors fit 128
 // registers, else 256 (FP64 lines of 256 and 512 points, FP32 of 512).
 // Fused xy planes: where a plane and the copies of its rows' inputs fit in
-// shared memory and there are planes for most SMs -- the y passes then cost no
-// memory traffic and no grid barrier, but a plane runs on one SM.
+// shared memory and there are planes for most SMs, or for half of them and a plane
+// is one line per group of lanes -- the y passes then cost no memory traffic and no
+// grid barrier, but a plane runs on one SM.  Us per step, fused and separate: 128^3
+// mixed 57 and 64, 64 x 32 x 128 15.1 and 17.8, 32 x 64 x 64 14.1 and 14.7; 64^3 18.7
+// and 16.9, 128 x 64 x 64 mixed 23.0 and 19.7, 64 x 64 x 32 18.2 and 14.2.
 // Tiles of the column passes: 8 adjacent columns (128 bytes in FP64), fewer
 // where that would leave SMs without a tile.  CTAs: the fewest that keep the
 // largest share, at most one per SM.
@@ -360,7 +363,8 @@ NdConfig nd_config(const espec_spond_plan* p) {
   const size_t plane = sizeof(cpx<R>) * (size_t)p->np[0] * p->np[1];
   size_t tw = 0;
   for (int ax = 0; ax < p->ndim; ++ax) tw += packed_bytes<R>(ln[ax]);
-  c.fused = p->ndim == 3 && tw + plane + 65536 <= kNdMaxSmem && p->np[2] >= kFusedMinPlanes;
+  const bool planes = p->np[2] >= 128 || (p->np[2] >= 64 && p->np[0] * p->np[1] <= 2048);
+  c.fused = p->ndim == 3 && planes && tw + plane + 65536 <= kNdMaxSmem;
   for (int ax = 0; ax < 2; ++ax) c.layout.by_pos[ax] = c.fused;
   auto threads_of = [&](int ax) { return ln[ax] == 9 ? 5 : ln[ax] - 3; };  // log2, per line
   auto tiles = [&](int lc) {
@@ -379,8 +383,16 @@ NdConfig nd_config(const espec_spond_plan* p) {
     want = (want + per - 1) / per;
   }
   c.grid = (int)want;
-  // a grid that gives 8 warps of a CTA no second line keeps 256 threads
-  if (!c.fused && (p->n >> ln[0]) / (32 >> threads_of(0)) <= 8L * c.grid) c.threads = 256;
+  // a grid that gives 8 warps of a CTA no second line (of the plane, or of the z
+  // tiles) keeps 256 threads
+  if (c.fused) {
+    const long gt = 1L << (threads_of(2) + c.lc);
+    if ((long)p->np[0] << threads_of(1) <= 256 && (long)p->np[1] << threads_of(0) <= 256 &&
+        tiles(c.lc) * gt <= 256L * c.grid)
+      c.threads = 256;  // 64 x 32 x 128: SOD 23.2 -> 18.4 us a step, SPO 18.9 -> 15.2
+  } else if ((p->n >> ln[0]) / (32 >> threads_of(0)) <= 8L * c.grid) {
+    c.threads = 256;
+  }
   const int e = mx == 9 ? 16 : 8;
   size_t ex = sizeof(cpx<R>) * (size_t)c.threads * e * 9 / 8;
   if (c.fused) ex = std::max(ex, plane + (size_t)c.threads / 32 * 4096);

@@ -16,9 +16,7 @@
 namespace espec {
 namespace nd {
 
-
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kFusedMinPlanes = 64;
 // dynamic shared memory of a CTA: 227 KB less the kernels' static part
 constexpr size_t kNdMaxSmem = 227 * 1024 - 2048;
 
@@ -529,8 +527,7 @@ __device__ __noinline__ void cols_phase(const NdArgs<R>& a, int axis,
 // shared memory while the current one is transformed: two buffers per group
 // behind the exchange space.  Without the copies all warps load, transform and
 // store in step and neither the memory nor the FP units stay busy: with them
-// (and those of plane_rows) a 128^3 mixed step takes 57 us instead of 80, a
-// 256 x 32 x 64 FP64 step 31 instead of 39, 64^3 18.7 instead of 19.6
+// (and those of plane_rows) a 128^3 mixed step takes 57 us instead of 80
 template <typename R, int LN, int T>
 __device__ __noinline__ void kin_staged(const NdArgs<R>& a, int axis,
                                         const typename Rot<R>::type* tab, cpx<R>* sm) {

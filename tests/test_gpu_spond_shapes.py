@@ -13,9 +13,9 @@ import espec_b200 as E
 pytestmark = pytest.mark.gpu
 
 SHAPES = [[32, 32], [512, 32], [32, 512], [256, 128], [128, 256], [64, 512],  # 2D
-          [32, 32, 32], [32, 32, 512], [512, 32, 32], [32, 256, 32],         # separate passes
-          [32, 32, 64], [64, 32, 128], [32, 64, 256], [256, 32, 64],         # fused planes
-          [128, 64, 64], [64, 64, 128]]                                      # ..., staged tiles
+          [32, 32, 32], [32, 32, 512], [512, 32, 32], [32, 256, 32],         # 3D
+          [32, 32, 64], [64, 32, 128], [32, 64, 256], [256, 32, 64],
+          [128, 64, 64], [64, 64, 128]]
 DT = 0.002 * NAT.SHFS
 
 
