@@ -92,7 +92,10 @@ inline unsigned io_blocks(size_t n) {
 
 inline int stage_reserve(HostStage& s, size_t bytes) {
   if (s.bytes >= bytes) return ESPEC_OK;
-  s.release();
+  // the device block alone: results of this call may be pending in s.h
+  if (s.d) cudaFree(s.d);
+  s.d = nullptr;
+  s.bytes = 0;
   IO_CK(cudaMalloc(&s.d, bytes));
   s.bytes = bytes;
   return ESPEC_OK;
