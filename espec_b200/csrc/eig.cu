@@ -103,10 +103,16 @@ struct Share {
   }
 };
 
-// sum of all chains: the thread's chain sums x0 (and x1, CS = 1)
+// sum of all chains: the thread's chain sums x0 (and x1, CS = 1).  Two buffers
+// [2][kEigChains / 32] in turn: a CTA may store its part of the next sum in its
+// partner while that one still reads this sum, but not of the sum after it, since the
+// partner has arrived at the next sum's barrier by then.
 template <int CS>
-__device__ __forceinline__ double chain_sum(const Share<CS>& sh, double x0, double x1, double* ws) {
+__device__ __forceinline__ double chain_sum(const Share<CS>& sh, double x0, double x1,
+                                            double* bufs, int& turn) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* ws = bufs + turn * (kEigChains / 32);
+  turn ^= 1;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     x0 += __shfl_xor_sync(0xffffffffu, x0, o);
@@ -269,13 +275,14 @@ __global__ void __launch_bounds__(kEigThreads, 1) eig_kernel(EigArgs a) {
   constexpr int NV = kEigMaxM + kEigMaxStates;
   extern __shared__ double eig_dyn[];
   __shared__ double part[2 * NV * 32];
-  __shared__ double ws[kEigChains / 32];
+  __shared__ double ws[2 * (kEigChains / 32)];
   __shared__ double red[NV];
   __shared__ double s_al[kEigMaxM], s_bt[kEigMaxM], s_e2[kEigMaxM], s_y[kEigMaxM];
   __shared__ double s_theta;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int p = blockIdx.x / CS, n = a.n, m = a.m;
   const Share<CS> sh;
+  int turn = 0;  // chain_sum's buffer
   const int k1 = sh.first, step = sh.kStep;
   const double* V = a.vpot + (long)p * n;
   double* L = a.L + (long)p * m * n;
@@ -304,7 +311,7 @@ __global__ void __launch_bounds__(kEigThreads, 1) eig_kernel(EigArgs a) {
         if (sh.chain(i)) nn[1] += F[k] * F[k];
         else nn[0] += F[k] * F[k];
       }
-      double bt0 = sqrt(chain_sum(sh, nn[0], nn[1], ws));
+      double bt0 = sqrt(chain_sum(sh, nn[0], nn[1], ws, turn));
       for (int it = 0; it < m; ++it) {
         double* Li = L + (long)it * n;
         const double* Lp = it ? L + (long)(it - 1) * n : nullptr;
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(kEigThreads, 1) eig_kernel(EigArgs a) {
             }
           }
         }
-        const double al = chain_sum(sh, nn[0], nn[1], ws);
+        const double al = chain_sum(sh, nn[0], nn[1], ws, turn);
         if (t == 0) s_al[it] = al;
         ++count;
         // work = w - al vi, then classical Gram-Schmidt against the locked
@@ -351,7 +358,7 @@ __global__ void __launch_bounds__(kEigThreads, 1) eig_kernel(EigArgs a) {
                   F[k] = w;
                   nn[c] += w * w;
                 });
-        bt0 = sqrt(chain_sum(sh, nn[0], nn[1], ws));
+        bt0 = sqrt(chain_sum(sh, nn[0], nn[1], ws, turn));
         if (t == 0) s_bt[it] = bt0;
       }
       __syncthreads();
@@ -407,7 +414,7 @@ __global__ void __launch_bounds__(kEigThreads, 1) eig_kernel(EigArgs a) {
                 F[k] = w;
                 nn[c] += w * w;
               });
-      const double inv = 1.0 / sqrt(chain_sum(sh, nn[0], nn[1], ws));
+      const double inv = 1.0 / sqrt(chain_sum(sh, nn[0], nn[1], ws, turn));
       for (int k = k1; k < n; k += step) {
         if (SM) sh.put(F + k, F[k] * inv);
         else F[k] *= inv;
@@ -422,7 +429,7 @@ __global__ void __launch_bounds__(kEigThreads, 1) eig_kernel(EigArgs a) {
         else nn[0] += r * r;
       }
       ++count;
-      res = sqrt(chain_sum(sh, nn[0], nn[1], ws));
+      res = sqrt(chain_sum(sh, nn[0], nn[1], ws, turn));
       if (res <= a.tol) break;
     }
     for (int k = k1; k < n; k += step) v[k] = F[k];
