@@ -209,15 +209,15 @@ def ptr(a):
     return a.ctypes.data
 
 
-def complex_host(psi):
+def complex_host(psi, order="C"):
     """(arrays kept alive, re pointer, im pointer, MEM_HOST flags) of a host wave
-    function: complex data as it lies, real data without an imaginary part."""
-    psi = np.asarray(psi)
+    function: complex data as it lies, real data without an imaginary part.  order:
+    in which several dimensions are taken, the one of the plan's potential."""
+    psi = np.asarray(psi).ravel(order=order)
     if np.iscomplexobj(psi):
-        z = np.ascontiguousarray(psi.ravel(order="F") if psi.ndim > 1 else psi,
-                                 dtype=np.complex128)
+        z = np.ascontiguousarray(psi, dtype=np.complex128)
         return z, z.ctypes.data, None, MEM_HOST | MEM_INTERLEAVED
-    re = f64(psi.ravel(order="F") if psi.ndim > 1 else psi)
+    re = f64(psi)
     return re, re.ctypes.data, None, MEM_HOST
 
 

@@ -39,7 +39,7 @@ class SilGrid:
         self.nsteps = None
 
     def load(self, vpot, psi, vabc=None, stream=None):
-        z, re, im, where = N.complex_host(psi)
+        z, re, im, where = N.complex_host(psi, order="F")
         self._keep = [N.f64(np.ravel(vpot, order="F") if np.ndim(vpot) > 1 else vpot), z,
                       None if vabc is None else N.f64(np.ravel(vabc, order="F"))]
         rc = N.load().espec_grid_load(self._h, N.ptr(self._keep[0]), N.ptr(self._keep[2]), re, im,
