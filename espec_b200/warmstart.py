@@ -43,6 +43,12 @@ def _ptrs(ts):
     return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
 
+def _packed(t, count, size):
+    """t, `count` values of `size` bytes in GPU memory, without gaps"""
+    assert t.is_cuda and t.numel() == count and t.element_size() == size
+    return t.contiguous()
+
+
 def _st(t):
     return _torch().cuda.current_stream(t.device).cuda_stream
 
@@ -170,6 +176,7 @@ class MLP:
         the network's output is the last pre-activation."""
         torch = _torch()
         lib = N.load()
+        assert Xb.dim() == 2 and Xb.shape[1] == self.sizes[0] and Xb.element_size() == 2
         X = Xb.contiguous()
         rows, L, dev = X.shape[0], len(self.W), X.device
         zs = [torch.empty((rows, n), dtype=torch.float32, device=dev) for n in self.sizes[1:]]
@@ -185,6 +192,11 @@ class MLP:
         torch = _torch()
         lib = N.load()
         rows, L, dev = dY.shape[0], len(self.W), dY.device
+        assert dY.shape == (rows, self.sizes[-1]) and len(hs) >= L and len(zs) >= L - 1
+        assert all(h.shape == (rows, n) for h, n in zip(hs, self.sizes[:-1]))
+        dY = _packed(dY, dY.numel(), 4)
+        hs = [_packed(h, rows * n, 2) for h, n in zip(hs, self.sizes[:-1])]
+        zs = [_packed(z, rows * n, 4) for z, n in zip(zs, self.sizes[1:-1])]
         grads = [torch.empty(p.shape, dtype=torch.float32, device=dev) for p in self.params]
         work = torch.empty(12 * rows * max(self.sizes[1:]), dtype=torch.uint8, device=dev)
         N.check(lib.espec_mlp_backward(L, self._widths, rows, _ptrs(hs), _ptrs(zs),
