@@ -43,6 +43,10 @@ def _ptrs(ts):
     return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
 
+def _ints(v):
+    return (C.c_int * len(v))(*v)
+
+
 def _packed(t, count, size):
     """t, `count` values of `size` bytes in GPU memory, without gaps"""
     assert t.is_cuda and t.numel() == count and t.element_size() == size
@@ -165,7 +169,6 @@ class MLP:
             self.W.append(w)
             self.Wb.append(to_bf16(w))
             self.b.append(torch.zeros(fo, dtype=torch.float32, device=dev))
-        self._widths = (C.c_int * len(self.sizes))(*self.sizes)
         self.params = [p for pair in zip(self.W, self.b) for p in pair]
         self.copies = [c for w in self.Wb for c in (w, None)]  # BF16 copy of each parameter
         self.m1 = [torch.zeros_like(p) for p in self.params]
@@ -181,7 +184,7 @@ class MLP:
         rows, L, dev = X.shape[0], len(self.W), X.device
         zs = [torch.empty((rows, n), dtype=torch.float32, device=dev) for n in self.sizes[1:]]
         hs = [torch.empty((rows, n), dtype=torch.bfloat16, device=dev) for n in self.sizes[1:-1]]
-        N.check(lib.espec_mlp_forward(L, self._widths, rows, X.data_ptr(), _ptrs(self.Wb),
+        N.check(lib.espec_mlp_forward(L, _ints(self.sizes), rows, X.data_ptr(), _ptrs(self.Wb),
                                       _ptrs(self.b), _ptrs(zs), _ptrs(hs), _st(X)),
                 "espec_mlp_forward")
         return [X, *hs], zs
@@ -199,7 +202,7 @@ class MLP:
         zs = [_packed(z, rows * n, 4) for z, n in zip(zs, self.sizes[1:-1])]
         grads = [torch.empty(p.shape, dtype=torch.float32, device=dev) for p in self.params]
         work = torch.empty(12 * rows * max(self.sizes[1:]), dtype=torch.uint8, device=dev)
-        N.check(lib.espec_mlp_backward(L, self._widths, rows, _ptrs(hs), _ptrs(zs),
+        N.check(lib.espec_mlp_backward(L, _ints(self.sizes), rows, _ptrs(hs), _ptrs(zs),
                                        _ptrs(self.Wb), dY.data_ptr(), _ptrs(grads[0::2]),
                                        _ptrs(grads[1::2]), work.data_ptr(), _st(dY)),
                 "espec_mlp_backward")
