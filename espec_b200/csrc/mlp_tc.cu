@@ -13,8 +13,9 @@
 // (gemm_bf16_tma), or 256 threads copy them where TMA's alignment rules do not hold
 // (gemm_bf16_tc); one thread issues four tcgen05.mma (M = 128, N = BN, K = 16,
 // kind::f16 with BF16 inputs) per stage and commits them to the buffer's mbarrier.
-// BN is the largest of 256, 128, 64 that gives every SM a tile, else 32: the
-// network's products have few tiles, and what bounds them is the chain of stages.
+// BN is the largest of 256, 128, 64 that gives every SM a tile more than half full,
+// else 32 (launch_any): the network's products have few tiles, and what bounds them is
+// the chain of stages.
 // The epilogue reads the accumulator with tcgen05.ld (a warp: 32 TMEM lanes, 32
 // columns) and turns it in shared memory so that rows are written 128 bytes at a
 // time, adding the bias and the activation (or its derivative) on the way.  Every
@@ -619,15 +620,19 @@ int launch_tc(const TcGemm& g, cudaStream_t st) {
   return ESPEC_OK;
 }
 
-// the widest tiles that still give every SM one
+// the widest tiles that still give every SM one, of whose columns more than half exist:
+// else the next narrower tile does the same work with half the MMA, copies and shared
+// memory.  us per product with the tile of 256 columns and now: 20000 x 16 x 256 20.6 ->
+// 8.9, 65536 x 64 x 256 40.8 -> 13.1, 65536 x 128 x 256 41.5 -> 28.4, 262144 x 100 x 64
+// 163 -> 112; 20000 x 160 x 256 keeps it, 20.8.
 template <int EPI>
 int launch_any(const TcGemm& g, cudaStream_t st) {
   auto tiles = [&](int bn) {
     return (long)((g.N + bn - 1) / bn) * ((g.M + kBM - 1) / kBM);
   };
-  if (tiles(256) >= 148) return launch_tc<256, EPI>(g, st);
-  if (tiles(128) >= 148) return launch_tc<128, EPI>(g, st);
-  if (tiles(64) >= 148) return launch_tc<64, EPI>(g, st);
+  if (g.N > 128 && tiles(256) >= 148) return launch_tc<256, EPI>(g, st);
+  if (g.N > 64 && tiles(128) >= 148) return launch_tc<128, EPI>(g, st);
+  if (g.N > 32 && tiles(64) >= 148) return launch_tc<64, EPI>(g, st);
   return launch_tc<32, EPI>(g, st);
 }
 
