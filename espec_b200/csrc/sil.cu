@@ -1439,14 +1439,6 @@ static const void* psod_form(int ndim, bool in_smem) {
                      : (const void*)psod_kernel<3, false>;
 }
 
-// places of a CTA's points (my_range, my_band)
-static int psod_cta_points(const espec_grid_plan* p) {
-  const int ns = band_strips(p);
-  if (ns == 0) return (int)((p->n + p->nblocks - 1) / p->nblocks);
-  const int nb = p->nblocks / ns;
-  return (p->np[1] + nb - 1) / nb * kSilThreads;
-}
-
 extern "C" int espec_grid_create(espec_grid_plan** out, int method, int ndim, const int* np,
                                  const double* shm, double dt_fs, int mp, int precision,
                                  int absorb, int quirks) {
@@ -1641,8 +1633,9 @@ static int grid_launch(espec_grid_plan* p, int nsteps, bool from_start, cudaStre
     void* args[] = {&a};
     // V, psi0 and the absorber of a CTA's points in its shared memory where all
     // CTAs then still run together
-    a.cta_points = psod_cta_points(p);
-    const size_t dyn = sizeof(double) * (size_t)a.cta_points * (a.kabs ? 4 : 3);
+    const long places = psod_places(a.nstrips, p->n, p->np[1], p->nblocks);
+    const size_t dyn = sizeof(double) * (size_t)places * (a.kabs ? 4 : 3);
+    a.cta_points = (int)places;  // read where `dyn` fits in shared memory
     const void* kern = psod_form(p->ndim, true);
     int dev = 0, nsm = 0, optin = 0, occ = 0;
     cudaFuncAttributes fa{};

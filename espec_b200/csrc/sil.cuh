@@ -79,4 +79,12 @@ struct SilArgs {
   long slot0;
 };
 
+// places for the points of a PSOD pass's largest CTA: a range of points (strips = 0),
+// or the rows of a band, kSilThreads columns each (my_range and my_band in sil.cu)
+inline long psod_places(int strips, long n, int ny, int nblocks) {
+  if (strips == 0) return (n + nblocks - 1) / nblocks;
+  const int bands = nblocks / strips;
+  return ((long)ny + bands - 1) / bands * kSilThreads;
+}
+
 }  // namespace espec
