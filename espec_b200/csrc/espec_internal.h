@@ -19,6 +19,9 @@ void digt_nd_table(int ndim, const int* np, const double* sh, const double* sm, 
 std::string spectrum_table(int mf, double dt, double de, const double* u, const double* v);
 // polls before a grid-barrier wait gives up (espec_set_wait_limit)
 long grid_wait_limit();
+// whether the next grid launch starts its arrival count one short
+// (espec_selftest_short_arrivals; counts the launch)
+bool grid_short_start();
 inline int ck(cudaError_t e, const char* what) {
   return e == cudaSuccess ? 0 : set_cuda_error(what, e);
 }

@@ -1370,6 +1370,9 @@ static std::atomic<int> g_short_arrivals{0};
 
 namespace espec {
 long grid_wait_limit() { return g_wait_limit.load(); }
+bool grid_short_start() {
+  return g_short_arrivals.load() > 0 && g_short_arrivals.fetch_sub(1) > 0;
+}
 }  // namespace espec
 
 // column strips of the PSOD pass on a 2D grid (0: contiguous point ranges):
@@ -1612,8 +1615,7 @@ static int grid_launch(espec_grid_plan* p, int nsteps, bool from_start, cudaStre
   }
   // the 64-bit arrival count starts at 0, or at 2^64 - 1 (one short of the
   // first barrier's G arrivals, modulo 2^64) for a self-test launch
-  const bool short_start = g_short_arrivals.load() > 0 && g_short_arrivals.fetch_sub(1) > 0;
-  GRID_CK(cudaMemsetAsync(p->d_bar, short_start ? 0xFF : 0, sizeof(unsigned) * 2, st));
+  GRID_CK(cudaMemsetAsync(p->d_bar, grid_short_start() ? 0xFF : 0, sizeof(unsigned) * 2, st));
   GRID_CK(cudaMemsetAsync(p->d_bar + 2, 0, sizeof(unsigned) * p->nblocks, st));
   GRID_CK(cudaMemsetAsync(p->d_err, 0, sizeof(int), st));
   SilArgs a = sil_args(p);

@@ -225,7 +225,8 @@ struct espec_spond_plan {
   int nsm = 0;
   double* d_tax = nullptr;         // DIGT axis tables (or the defect's TC(1..NP1))
   bool k_ready = false;            // the kinetic table is built (it depends on the plan alone)
-  unsigned long long* d_bar = nullptr;  // grid barrier arrivals, then the error flag
+  // grid barrier arrivals and error flag of the propagation, then of the energies' transform
+  unsigned long long* d_bar = nullptr;
   bool has_state = false;          // d_out holds the state of the last run
   // energy diagnostics (FP64 in both forms)
   cpx<double>* d_khat = nullptr;
@@ -499,17 +500,19 @@ NdArgs<R> nd_args(const espec_spond_plan* p, const NdConfig& c) {
   a.kstage = c.kstage;
   a.psi0 = p->d_psi0;
   a.bar = p->d_bar;
-  a.err = (int*)(p->d_bar + 1);
   a.spin_limit = grid_wait_limit();
   return a;
 }
 
 template <typename R>
 int nd_launch(espec_spond_plan* p, const NdConfig& c, NdArgs<R>& a, cudaStream_t st) {
-  // the arrival count; a diagnostic transform keeps the last run's error flag,
-  // so that it fails too
-  ND_CK(cudaMemsetAsync(p->d_bar, 0, (a.op == kOpForward ? 1 : 2) * sizeof(unsigned long long),
-                        st));
+  a.err = (int*)(a.bar + 1);
+  // the arrival count, and the error flag unless the run continues from a state that
+  // an earlier one may have spoiled
+  const size_t word = sizeof(unsigned long long);
+  const bool fresh = a.op == kOpForward || a.from_start;
+  ND_CK(cudaMemsetAsync(a.bar, 0, fresh ? 2 * word : word, st));
+  if (grid_short_start()) ND_CK(cudaMemsetAsync(a.bar, 0xFF, word, st));
   cudaError_t e;
   if constexpr (sizeof(R) == 8)
     e = c.threads == 256 ? nd_launch_f64_256(a, c.grid, c.smem, st)
@@ -677,8 +680,8 @@ extern "C" int espec_spond_create_method(espec_spond_plan** out, int method, int
   size_t tax = 0;
   for (int ax = 0; ax < ndim; ++ax) tax += np[ax];
   if ((rc = ck(cudaMalloc(&p->d_tax, 8 * tax), "cudaMalloc"))) return fail(rc);
-  if ((rc = ck(cudaMalloc(&p->d_bar, 2 * sizeof(unsigned long long)), "cudaMalloc"))) return fail(rc);
-  if ((rc = ck(cudaMemset(p->d_bar, 0, 2 * sizeof(unsigned long long)), "cudaMemset")))
+  if ((rc = ck(cudaMalloc(&p->d_bar, 4 * sizeof(unsigned long long)), "cudaMalloc"))) return fail(rc);
+  if ((rc = ck(cudaMemset(p->d_bar, 0, 4 * sizeof(unsigned long long)), "cudaMemset")))
     return fail(rc);
   for (int ax = 0; ax < ndim; ++ax)
     if ((rc = ck(cudaMalloc(&p->d_tw[ax], sizeof(RotD) * np[ax]), "cudaMalloc"))) return fail(rc);
@@ -693,6 +696,17 @@ extern "C" int espec_spond_create(espec_spond_plan** out, int ndim, const int* n
                                    quirks);
 }
 
+static const char* const kTimedOut = "a grid barrier of the split-operator kernel timed out";
+
+// results in host memory: complete, or the last run's wait gave up
+static int nd_finish(espec_spond_plan* p, cudaStream_t st) {
+  int err = 0;
+  ND_CK(cudaMemcpyAsync(&err, p->d_bar + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ND_CK(cudaStreamSynchronize(st));
+  p->stage.flush();
+  return err ? set_error(ESPEC_ECUDA, kTimedOut) : ESPEC_OK;
+}
+
 extern "C" int espec_spond_previous(espec_spond_plan* p, double* psi_re, double* psi_im,
                                     int where, void* stream) {
   if (!p || p->method != ESPEC_SOD || !p->has_state)
@@ -701,10 +715,7 @@ extern "C" int espec_spond_previous(espec_spond_plan* p, double* psi_re, double*
   p->stage.drop();
   const int rc = get_complex(p->stage, p->d_prev, psi_re, psi_im, (size_t)p->n, where, st);
   if (rc) return rc;
-  if (where == ESPEC_MEM_HOST) {
-    ND_CK(cudaStreamSynchronize(st));
-    p->stage.flush();
-  }
+  if (where == ESPEC_MEM_HOST) return nd_finish(p, st);
   return ESPEC_OK;
 }
 
@@ -812,6 +823,7 @@ extern "C" int espec_spond_energies(espec_spond_plan* p, double* e, double* norm
   const NdConfig c = nd_config<double>(p);
   NdArgs<double> a = nd_args<double>(p, c);
   a.op = kOpForward;
+  a.bar = p->d_bar + 2;
   a.psi = p->d_khat;
   a.psi_start = p->has_state ? p->d_out : p->d_psi0;
   for (int ax = 0; ax < p->ndim; ++ax) a.tw[ax] = p->d_tw64[ax];
@@ -822,8 +834,11 @@ extern "C" int espec_spond_energies(espec_spond_plan* p, double* e, double* norm
   csum_kernel<<<1, 32, 0, st>>>(p->d_epart, nb, 0, 0, p->d_epart + nb, a.err);
   ND_CK(cudaGetLastError());
   double2 h;
+  unsigned long long flags[3];  // the run's flag, the arrivals, the transform's flag
   ND_CK(cudaMemcpyAsync(&h, p->d_epart + nb, sizeof h, cudaMemcpyDeviceToHost, st));
+  ND_CK(cudaMemcpyAsync(flags, p->d_bar + 1, sizeof flags, cudaMemcpyDeviceToHost, st));
   ND_CK(cudaStreamSynchronize(st));
+  if (flags[2] || (p->has_state && flags[0])) return set_error(ESPEC_ECUDA, kTimedOut);
   *e = h.x;
   *norm = h.y;
   return ESPEC_OK;
@@ -843,13 +858,7 @@ extern "C" int espec_spond_results(espec_spond_plan* p, double* c_re, double* c_
     rc = pairs ? get_pairs(p->d_out, psi_re, n, where, st)
                : get_complex(p->stage, p->d_out, psi_re, psi_im, n, where, st);
   if (rc) return rc;
-  if (where == ESPEC_MEM_HOST) {
-    int err = 0;
-    ND_CK(cudaMemcpyAsync(&err, p->d_bar + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ND_CK(cudaStreamSynchronize(st));
-    p->stage.flush();
-    if (err) return set_error(ESPEC_ECUDA, "a grid barrier of the split-operator kernel timed out");
-  }
+  if (where == ESPEC_MEM_HOST) return nd_finish(p, st);
   return ESPEC_OK;
 }
 

@@ -417,10 +417,11 @@ int espec_grid_previous(espec_grid_plan* plan, double* psi_re, double* psi_im, i
 long espec_grid_npoints(const espec_grid_plan* plan);
 void espec_grid_destroy(espec_grid_plan* plan);
 /* Bounded waits of the grid kernels (no counterpart in the reference, which
- * has no device waits).  Every grid-barrier wait of the SIL and PSOD kernels
- * gives up after `polls` polls of the arrival count (0: the default, 2^24,
- * seconds); the kernel then sets its error flag and returns, and
- * espec_grid_results reports ESPEC_ECUDA ("timed out"), the drop-ins INFO = 2.
+ * has no device waits).  Every grid-barrier wait of the SIL and PSOD kernels and
+ * of the 2D/3D FFT kernels (espec_spond_*) gives up after `polls` polls of the
+ * arrival count (0: the default, 2^24, seconds); the kernel then sets its error
+ * flag and returns, and espec_grid_results, espec_spond_results, _previous (host
+ * memory) and _energies report ESPEC_ECUDA ("timed out"), the drop-ins INFO = 2.
  * espec_selftest_short_arrivals(k): the next k grid launches start their
  * arrival count one short, so their first barrier never completes and every
  * wait runs out -- the time-out path exercised without any fault; the device
