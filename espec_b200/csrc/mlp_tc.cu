@@ -244,7 +244,9 @@ __device__ __forceinline__ void finish_tile(const TcGemm& g, uint32_t tmem, uint
                   ? g.z[(long)(row0 + i) * g.ldc + n0 + col0 + lane]
                   : 0.0f;
   }
-  // the last commit covers every MMA before it
+  // The last commit covers every MMA before it.  Where the MMA thread gave up at an
+  // earlier stage nobody makes that commit, and all threads stay here for the whole
+  // limit: the wait for the boxes and MMAs still in flight.
   if (some) ok = wait_phase(last, parity) && ok;
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
