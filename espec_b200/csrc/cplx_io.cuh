@@ -101,10 +101,19 @@ inline int stage_reserve(HostStage& s, size_t bytes) {
   return ESPEC_OK;
 }
 
-// dst (device, n complex) <- (re, im) at `where`; im may be null (zero)
 // a user pointer in host memory (synchronous or in-flight copies)
 inline bool on_host(int where) { return where == ESPEC_MEM_HOST || where == ESPEC_MEM_HOST_ASYNC; }
 
+inline bool memory_is(const void* p, cudaMemoryType type) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return at.type == type;
+}
+
+// dst (device, n complex) <- (re, im) at `where`; im may be null (zero)
 inline int put_complex(HostStage& s, double2* dst, const double* re, const double* im, size_t n,
                        int where, cudaStream_t st) {
   if (n == 0) return ESPEC_OK;
@@ -132,7 +141,9 @@ inline int get_complex(HostStage& s, const double2* src, double* re, double* im,
     IO_CK(cudaGetLastError());
     return ESPEC_OK;
   }
-  if (where == ESPEC_MEM_HOST) {
+  // (device pointers given as host memory are left to the copies below, which take them)
+  if (where == ESPEC_MEM_HOST && !memory_is(re, cudaMemoryTypeDevice) &&
+      !memory_is(im, cudaMemoryTypeDevice)) {
     if (double* p = s.small(16 * n)) {
       deinterleave_kernel<<<io_blocks(n), 256, 0, st>>>(src, p, p + n, n);
       IO_CK(cudaGetLastError());
