@@ -3,13 +3,14 @@
 // and the device form (interleaved double2).  Host transfers go through a
 // contiguous (re | im) staging block owned by the plan, so each is one linear
 // copy; results of up to kStageSmall bytes are written by the kernel straight into
-// page-locked memory of the plan and copied on by the host after the caller's
-// synchronisation (a row of a printed table: no device-to-host copies, 8 us each);
-// device arguments are (de)interleaved in place by a kernel.
+// a page-locked block that the plan holds (HostBlocks) and copied on by the host
+// after the caller's synchronisation (a row of a printed table: no device-to-host
+// copies, 8 us each); device arguments are (de)interleaved in place by a kernel.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <mutex>
 
 #include "espec_gpu.h"
 #include "espec_internal.h"
@@ -18,10 +19,63 @@ namespace espec {
 
 constexpr size_t kStageSmall = 64 * 1024;
 
+// Page-locked blocks of kStageSmall bytes, one for each plan that reads small results;
+// a plan holds its block from its first such result until it is destroyed.  Page-locking
+// and releasing a block cost 1 to 3 ms, more than a short-lived plan gains (with a block
+// of its own, the first result of a new plan took 2.5 ms; 40 us by copies, 20 us through
+// a block): all plans share kCount blocks of one allocation, made once and only when
+// results have asked kPatience times, by when their copies have cost about as much.  A
+// plan that finds no block free has its results copied.
+class HostBlocks {
+ public:
+  static HostBlocks& get() {
+    static HostBlocks b;
+    return b;
+  }
+  double* take() {
+    std::lock_guard<std::mutex> lock(m_);
+    if (!base_ && !allocate()) return nullptr;
+    if (!free_) return nullptr;
+    int i = 0;
+    while (!(free_ >> i & 1)) ++i;
+    free_ &= free_ - 1;
+    return reinterpret_cast<double*>(base_ + i * kStageSmall);
+  }
+  void give(double* block) {
+    std::lock_guard<std::mutex> lock(m_);
+    if (base_) free_ |= 1u << (reinterpret_cast<char*>(block) - base_) / kStageSmall;
+  }
+  // at the end of the process; plans may still give blocks back afterwards
+  ~HostBlocks() {
+    if (base_) cudaFreeHost(base_);
+    base_ = nullptr;
+    asked_ = 0;
+  }
+
+ private:
+  static constexpr int kCount = 16, kPatience = 64;
+  bool allocate() {
+    if (++asked_ < kPatience) return false;
+    asked_ = 0;
+    if (cudaHostAlloc((void**)&base_, kCount * kStageSmall,
+                      cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      (void)cudaGetLastError();
+      base_ = nullptr;
+      return false;
+    }
+    free_ = (1u << kCount) - 1;
+    return true;
+  }
+  std::mutex m_;
+  char* base_ = nullptr;
+  unsigned free_ = 0;  // one bit per block
+  int asked_ = 0;
+};
+
 struct HostStage {
   double* d = nullptr;
   size_t bytes = 0;
-  double* h = nullptr;  // page-locked, kStageSmall bytes
+  double* h = nullptr;  // a page-locked block of kStageSmall bytes
   struct Pending {
     double* dst;
     const double* src;
@@ -31,19 +85,14 @@ struct HostStage {
   size_t used = 0;  // bytes of h taken by the pending results
   void release() {
     if (d) cudaFree(d);
-    if (h) cudaFreeHost(h);
+    if (h) HostBlocks::get().give(h);  // no kernel writes to it: cudaFree has waited
     d = h = nullptr;
     bytes = 0;
   }
   // page-locked space for `size` bytes, or null (too large, or none to be had)
   double* small(size_t size) {
     if (used + size > kStageSmall || npending + 2 > 4) return nullptr;
-    if (!h && cudaHostAlloc((void**)&h, kStageSmall, cudaHostAllocPortable | cudaHostAllocMapped) !=
-                  cudaSuccess) {
-      (void)cudaGetLastError();
-      h = nullptr;
-      return nullptr;
-    }
+    if (!h && !(h = HostBlocks::get().take())) return nullptr;
     double* p = h + used / sizeof(double);
     used += size;
     return p;
