@@ -153,13 +153,20 @@ inline int stage_reserve(HostStage& s, size_t bytes) {
 // a user pointer in host memory (synchronous or in-flight copies)
 inline bool on_host(int where) { return where == ESPEC_MEM_HOST || where == ESPEC_MEM_HOST_ASYNC; }
 
-inline bool memory_is(const void* p, cudaMemoryType type) {
+inline cudaMemoryType memory_type(const void* p) {
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     (void)cudaGetLastError();
-    return false;
+    return cudaMemoryTypeUnregistered;
   }
-  return at.type == type;
+  return at.type;
+}
+// ESPEC_MEM_HOST: the caller may reuse its array once the call returns; a copy from
+// memory that CUDA knows of (page-locked) is then still in flight
+inline int wait_source(const void* p, int where, cudaStream_t st) {
+  if (where == ESPEC_MEM_HOST && memory_type(p) != cudaMemoryTypeUnregistered)
+    IO_CK(cudaStreamSynchronize(st));
+  return ESPEC_OK;
 }
 
 // dst (device, n complex) <- (re, im) at `where`; im may be null (zero)
@@ -191,8 +198,8 @@ inline int get_complex(HostStage& s, const double2* src, double* re, double* im,
     return ESPEC_OK;
   }
   // (device pointers given as host memory are left to the copies below, which take them)
-  if (where == ESPEC_MEM_HOST && !memory_is(re, cudaMemoryTypeDevice) &&
-      !memory_is(im, cudaMemoryTypeDevice)) {
+  if (where == ESPEC_MEM_HOST && memory_type(re) != cudaMemoryTypeDevice &&
+      memory_type(im) != cudaMemoryTypeDevice) {
     if (double* p = s.small(16 * n)) {
       deinterleave_kernel<<<io_blocks(n), 256, 0, st>>>(src, p, p + n, n);
       IO_CK(cudaGetLastError());
@@ -215,7 +222,7 @@ inline int put_pairs(double2* dst, const double* src, size_t n, int where, cudaS
   if (n == 0) return ESPEC_OK;
   IO_CK(cudaMemcpyAsync(dst, src, 16 * n,
                         on_host(where) ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st));
-  return ESPEC_OK;
+  return wait_source(src, where, st);
 }
 inline int get_pairs(const double2* src, double* dst, size_t n, int where, cudaStream_t st) {
   if (!dst || n == 0) return ESPEC_OK;

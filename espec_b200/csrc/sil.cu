@@ -1581,6 +1581,8 @@ extern "C" int espec_grid_load(espec_grid_plan* p, const double* vpot, const dou
       if (rc) return rc;
       GRID_CK(cudaMemcpyAsync(p->stage.d, psi_re, 2 * nb, kind, st));
       src = (const double2*)p->stage.d;
+      const int rw = wait_source(psi_re, where, st);
+      if (rw) return rw;
     }
     deinterleave_kernel<<<io_blocks(p->n), 256, 0, st>>>(src, p->d_u0, p->d_v0, (size_t)p->n);
     GRID_CK(cudaGetLastError());
