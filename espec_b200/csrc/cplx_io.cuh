@@ -18,6 +18,8 @@
 namespace espec {
 
 constexpr size_t kStageSmall = 64 * 1024;
+inline constexpr const char* kPreviousParts =
+    "the previous state comes as separate real and imaginary arrays";
 
 // Page-locked blocks of kStageSmall bytes, one for each plan that reads small results;
 // a plan holds its block from its first such result until it is destroyed.  Page-locking

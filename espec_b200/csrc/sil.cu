@@ -1569,14 +1569,13 @@ extern "C" int espec_grid_load(espec_grid_plan* p, const double* vpot, const dou
   cudaStream_t st = (cudaStream_t)stream;
   const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
   where &= ~ESPEC_MEM_INTERLEAVED;
-  const cudaMemcpyKind kind =
-      where == ESPEC_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
+  const cudaMemcpyKind kind = on_host(where) ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   const size_t nb = (size_t)p->n * 8;
   GRID_CK(cudaMemcpyAsync(p->d_vpot, vpot, nb, kind, st));
   if (p->absorb != ESPEC_ABS_NONE) GRID_CK(cudaMemcpyAsync(p->d_mask, vabc, nb, kind, st));
   if (pairs) {
     const double2* src = (const double2*)psi_re;
-    if (where == ESPEC_MEM_HOST) {
+    if (on_host(where)) {  // the kernel does not read host memory
       const int rc = stage_reserve(p->stage, 2 * nb);
       if (rc) return rc;
       GRID_CK(cudaMemcpyAsync(p->stage.d, psi_re, 2 * nb, kind, st));
@@ -1718,21 +1717,20 @@ extern "C" int espec_grid_results(espec_grid_plan* p, double* c_re, double* c_im
   cudaStream_t st = (cudaStream_t)stream;
   const bool pairs = (where & ESPEC_MEM_INTERLEAVED) != 0;
   where &= ~ESPEC_MEM_INTERLEAVED;
-  const cudaMemcpyKind kind =
-      where == ESPEC_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
+  const cudaMemcpyKind kind = on_host(where) ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
   const size_t nc = (size_t)p->c_cap + 1;
   if (pairs) {
     if (c_re) GRID_CK(cudaMemcpyAsync(c_re, p->d_c, 16 * nc, kind, st));
     if (psi_re) {
       double2* dst = (double2*)psi_re;
-      if (where == ESPEC_MEM_HOST) {
+      if (on_host(where)) {
         const int rc = stage_reserve(p->stage, 16 * (size_t)p->n);
         if (rc) return rc;
         dst = (double2*)p->stage.d;
       }
       interleave_kernel<<<io_blocks(p->n), 256, 0, st>>>(p->d_u, p->d_v, dst, (size_t)p->n);
       GRID_CK(cudaGetLastError());
-      if (where == ESPEC_MEM_HOST)
+      if (on_host(where))
         GRID_CK(cudaMemcpyAsync(psi_re, dst, 16 * (size_t)p->n, kind, st));
     }
     c_re = c_im = psi_re = psi_im = nullptr;
@@ -1775,6 +1773,7 @@ extern "C" int espec_grid_previous(espec_grid_plan* p, double* psi_re, double* p
                                    void* stream) {
   if (!p || p->method != ESPEC_PSOD || !p->has_state)
     return set_error(ESPEC_EINVAL, "previous state exists for run PSOD plans only");
+  if (where & ESPEC_MEM_INTERLEAVED) return set_error(ESPEC_EINVAL, kPreviousParts);
   cudaStream_t st = (cudaStream_t)stream;
   const cudaMemcpyKind kind =
       where == ESPEC_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;

@@ -995,6 +995,7 @@ extern "C" int espec_prop_previous(espec_spo_plan* p, double* psi_re, double* ps
                                    void* stream) {
   if (!p || p->method != ESPEC_SOD || p->c_cap_steps < 0)
     return set_error(ESPEC_EINVAL, "previous state exists for run SOD plans only");
+  if (where & ESPEC_MEM_INTERLEAVED) return set_error(ESPEC_EINVAL, kPreviousParts);
   cudaStream_t st = (cudaStream_t)stream;
   p->stage.drop();
   const int rc = get_complex(p->stage, p->d_psi_prev, psi_re, psi_im, p->npts, where, st);

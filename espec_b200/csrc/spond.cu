@@ -711,6 +711,7 @@ extern "C" int espec_spond_previous(espec_spond_plan* p, double* psi_re, double*
                                     int where, void* stream) {
   if (!p || p->method != ESPEC_SOD || !p->has_state)
     return set_error(ESPEC_EINVAL, "previous state exists for run SOD plans only");
+  if (where & ESPEC_MEM_INTERLEAVED) return set_error(ESPEC_EINVAL, kPreviousParts);
   cudaStream_t st = (cudaStream_t)stream;
   p->stage.drop();
   const int rc = get_complex(p->stage, p->d_prev, psi_re, psi_im, (size_t)p->n, where, st);

@@ -90,7 +90,7 @@ extern "C" {
 
 /* added to `where` in the load and results calls of the plans (espec_spo_*,
  * espec_grid_*, espec_spond_*): complex arrays are interleaved (re, im) pairs at the _re
- * pointer, the _im pointer is not used */
+ * pointer, the _im pointer is not used (the _previous calls refuse it) */
 #define ESPEC_MEM_INTERLEAVED 16
 
 /* launch shape of a batched split-operator run (espec_spo_set_launch) */
