@@ -125,15 +125,15 @@ __device__ bool grid_reduce(const SilArgs& a, const double* sp, double* st, int 
 }
 
 // Grid barrier (grid_reduce's, without the sums); between this CTA's arrival and
-// the others', threads 32 on run meanwhile().  false = a wait gave up.
+// the others', threads 32 on run meanwhile().  s_flag[0] (shared): barriers passed in
+// this launch, thread 0's.  false = a wait gave up.
 template <class F>
-__device__ __forceinline__ bool grid_barrier(const SilArgs& a, int* s_flag, unsigned& phase,
-                                             F meanwhile) {
-  const unsigned G = gridDim.x;
-  const unsigned long long target = (unsigned long long)(phase + 1u) * G;
-  ++phase;
+__device__ __forceinline__ bool grid_barrier(const SilArgs& a, int* s_flag, F meanwhile) {
   __syncthreads();
   if (threadIdx.x == 0) {
+    const unsigned G = gridDim.x;
+    const unsigned long long target = (unsigned long long)((unsigned)s_flag[0] + 1u) * G;
+    s_flag[0] = (int)((unsigned)s_flag[0] + 1u);
     s_flag[1] = 1;
     if (G > 1) {
       cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> cnt(
@@ -1135,7 +1135,6 @@ __global__ void __launch_bounds__(kSilThreads, 2) psod_kernel(SilArgs a) {
   __shared__ int s_flag[2];
   const Range r = my_range(a.n);
   const int t = threadIdx.x;
-  unsigned phase = 0;  // grid barriers passed in this launch
   double *un = a.u, *vn = a.v, *um = a.up, *vm = a.vp;
   // the CTA's points as its threads walk them: f(point, place in the CTA)
   auto each_point = [&](auto f) {
@@ -1166,12 +1165,20 @@ __global__ void __launch_bounds__(kSilThreads, 2) psod_kernel(SilArgs a) {
   // total meanwhile, and read by all CTAs after the barrier it cost 1 to 2 us of
   // every step.  A buffer is written again four barriers on, by when the summing
   // CTA has arrived at two more.
-  int pending = -1;        // sample published before the last barrier
-  unsigned pending_at = 0;  // that barrier
-  auto sum_pending = [&] {  // threads 32..159
-    const int G = gridDim.x, i = t - 32;
-    if (i < 0 || i >= 128) return;
-    const double* part = a.part + (size_t)(pending_at & 3u) * G * 4;
+  // The sample (or -1) published before the last barrier, and that barrier's count: in
+  // shared memory, as the count of barriers passed is.  In registers they made the bands
+  // without constants in shared memory spill in the row loop (us a step with them there
+  // -> now: 2048 x 2048 67.4 -> 65.0, 1536 x 1536 41.6 -> 39.2, 1023 x 769 9.3 -> 9.1).
+  __shared__ int s_pending[2];
+  if (t == 0) {
+    s_pending[0] = -1;
+    s_flag[0] = 0;
+  }
+  __syncthreads();
+  auto sum_pending = [&](unsigned cta) {  // threads 32..159 of CTA `cta`
+    const int G = gridDim.x, i = t - 32, slot = s_pending[0];
+    if (i < 0 || i >= 128 || slot < 0 || blockIdx.x != cta) return;
+    const double* part = a.part + (size_t)(s_pending[1] & 3) * G * 4;
     const int q = i & 3, row = i >> 2;
     double s = 0.0;
     for (int i0 = row; i0 < G; i0 += 10 * 32) {
@@ -1190,20 +1197,19 @@ __global__ void __launch_bounds__(kSilThreads, 2) psod_kernel(SilArgs a) {
       double st = 0.0;
       for (int j = 0; j < 32; ++j) st += s_red[4 * j + (i & 3)];
       const double other = __shfl_down_sync(0xffffffffu, st, 1);
-      if (i == 0) a.c_out[pending].x = st + other;
-      if (i == 2) a.c_out[pending].y = st - other;
+      if (i == 0) a.c_out[slot].x = st + other;
+      if (i == 2) a.c_out[slot].y = st - other;
     }
   };
   auto reduce_c = [&](double (&q)[4], int slot) -> bool {
-    const unsigned at = phase;
-    block_sum<4>(q, a.part + ((size_t)(at & 3u) * gridDim.x + blockIdx.x) * 4, scratch);
-    const bool mine = pending >= 0 && blockIdx.x == pending_at % gridDim.x;
-    if (!grid_barrier(a, s_flag, phase, [&] {
-          if (mine) sum_pending();
-        }))
+    block_sum<4>(q, a.part + ((size_t)(s_flag[0] & 3) * gridDim.x + blockIdx.x) * 4, scratch);
+    if (!grid_barrier(a, s_flag,
+                      [&] { sum_pending((unsigned)s_pending[1] % gridDim.x); }))
       return false;
-    pending = slot;
-    pending_at = at;
+    if (t == 0) {  // read again after the barriers of block_sum
+      s_pending[0] = slot;
+      s_pending[1] = s_flag[0] - 1;
+    }
     return true;
   };
   auto step = [&](double c, int slot, long call) __attribute__((always_inline)) -> bool {
@@ -1245,7 +1251,8 @@ __global__ void __launch_bounds__(kSilThreads, 2) psod_kernel(SilArgs a) {
   }
   for (int s = s0; s <= a.nsteps; ++s)
     if (!step(a.cst, s, a.slot0 + s)) return;
-  if (pending >= 0 && blockIdx.x == 0) sum_pending();
+  __syncthreads();
+  sum_pending(0);
 }
 
 // <u|H u> + <v|H v> and |u|^2 + |v|^2 (EIGENERG, eigenerg.f:56-66): per-CTA
