@@ -894,7 +894,10 @@ constexpr int kPsodIlp = NDIM == 3 ? 2 : 4;
 // per point to and from L2 (1023 x 769: 10.3 -> 9.6 us a step).
 template <bool KS>
 struct PsodConst {
-  const double *v, *u0, *v0, *w;  // global arrays, or the CTA's copies
+  // global arrays, or the CTA's copies (w: read with KS only; without, the absorber by its
+  // address in the parameters and not through the read-only path took 2048 x 2048 from
+  // 78.2 to 76.9 us a step)
+  const double *v, *u0, *v0, *w;
   // i: the point k, or with KS its place i in the CTA
   static __device__ __forceinline__ double get(const double* p, long k, int i) {
     return KS ? p[i] : __ldg(p + k);
@@ -985,11 +988,11 @@ __device__ __forceinline__ void psod2d_band(const SilArgs& a, const PsodConst<KS
     }
     double nu, nv;
     if (KABS == 1) {
-      const double w = cs.get(cs.w, k, i);
+      const double w = KS ? cs.w[i] : a.vabc[k];
       nu = umk + c * hv - c * w * uk;
       nv = vmk - c * hu - c * w * vkk;
     } else if (KABS == 2) {
-      const double w = cs.get(cs.w, k, i);
+      const double w = KS ? cs.w[i] : a.vabc[k];
       nu = w * (umk + c * hv);
       nv = w * (vmk - c * hu);
     } else {
@@ -1057,11 +1060,11 @@ __device__ __forceinline__ void psod_point(const SilArgs& a, const PsodConst<KS>
     hu -= de * uk;
   }
   if (KABS == 1) {
-    const double w = cs.get(cs.w, k, i);
+    const double w = KS ? cs.w[i] : a.vabc[k];
     nu = um[k] + c * hv - c * w * uk;
     nv = vm[k] - c * hu - c * w * vk;
   } else if (KABS == 2) {
-    const double w = cs.get(cs.w, k, i);
+    const double w = KS ? cs.w[i] : a.vabc[k];
     nu = w * (um[k] + c * hv);
     nv = w * (vm[k] - c * hu);
   } else {
@@ -1168,7 +1171,7 @@ __global__ void __launch_bounds__(kSilThreads, 2) psod_kernel(SilArgs a) {
   // The sample (or -1) published before the last barrier, and that barrier's count: in
   // shared memory, as the count of barriers passed is.  In registers they made the bands
   // without constants in shared memory spill in the row loop (us a step with them there
-  // -> now: 2048 x 2048 67.4 -> 65.0, 1536 x 1536 41.6 -> 39.2, 1023 x 769 9.3 -> 9.1).
+  // -> now: 2048 x 2048 67.3 -> 64.6, 1536 x 1536 41.5 -> 39.0, 1023 x 769 9.3 -> 9.0).
   __shared__ int s_pending[2];
   if (t == 0) {
     s_pending[0] = -1;
