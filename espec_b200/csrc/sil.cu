@@ -1512,7 +1512,8 @@ extern "C" int espec_grid_create(espec_grid_plan** out, int method, int ndim, co
   long want = (n + kSilThreads - 1) / kSilThreads;
   // one CTA per SM keeps the barriers short; a PSOD pass of more than a point per
   // thread is bound by the latency of its loads and takes every co-resident CTA
-  // (per step, one -> two CTAs per SM: 80^3 18.6 -> 11.5 us, 50^3 8.0 -> 5.7)
+  // (per step, one -> two CTAs per SM: 80^3 18.6 -> 11.5 us, 50^3 8.0 -> 5.7, just above
+  // the line 34^3 5.1 -> 3.2, 38000 points 2.8 -> 2.1, but 45000 2.4 -> 2.6)
   const bool wide = psod && n > (long)nsm * kSilThreads;
   long cap = wide ? (long)nsm * occ : nsm;
   if (cap > (long)nsm * occ) cap = (long)nsm * occ;
@@ -1524,14 +1525,18 @@ extern "C" int espec_grid_create(espec_grid_plan** out, int method, int ndim, co
     const long per = (want + cap - 1) / cap;
     want = (want + per - 1) / per;
   }
-  // On a 2D grid such a pass runs by column strips, where these fill a quarter of
-  // their lanes or more: a multiple of the strip count, bands of two rows or more.
-  // Per step, points -> bands: 1023 x 769 14.7 -> 9.6 us, 600 x 500 11.9 -> 6.9,
-  // 400 x 300 8.3 -> 5.0; 100 x 100, below the line, 3.8 -> 4.2.
+  // On a 2D grid such a pass runs by column strips, where these fill 72 of their 256
+  // lanes or more: a multiple of the strip count, bands of two rows or more.  Us per
+  // step, points and bands: 2048 x 2048 110 and 65, 1536 x 1536 52 and 39, 513 x 500 7.6
+  // and 6.0, 320 x 300 4.3 and 4.1, 128 x 4000 9.5 and 7.2, 80 x 2000 5.4 and 4.7, 76 x
+  // 1000 4.1 and 3.8; below the line 68 x 1000 3.2 and 3.8, 64 x 1000 3.1 and 3.8, 64 x
+  // 4000 5.3 and 6.6 (with a mask 5.3 and 8.3), 64 x 40000 65 and 106.  Above it some would
+  // be better off with points: little more than a point per thread (200 x 192 3.0 and 3.3),
+  // tall grids of half-filled strips (300 x 1000 5.3 and 6.1, 96 x 20000 47 and 56).
   if (wide && ndim == 2) {
     const long ns = (np[0] + kSilThreads - 1) / kSilThreads;
     const long nb = std::min((long)nsm * occ / ns, (long)np[1] / 2);
-    if (nb >= 1 && 4L * np[0] >= ns * kSilThreads) {
+    if (nb >= 1 && np[0] >= 72 * ns) {
       want = ns * nb;
       p->bands = true;
     }

@@ -1,8 +1,8 @@
 """The PSOD kernel's column strips and its points with the constants in shared memory
 against the oracle, with what changes the arithmetic of a point: both absorbers, the
 restart-copy defect, a pulse.  Strips with the constants in shared memory (400 x 300,
-257 x 300, 64 x 700) and without (1300 x 1250), points in 1D and 3D.  Some roundings of
-1.1e-16 per point and step on values of at most 1: |dC|, |dpsi| <= 1e-10."""
+257 x 300, 72 x 700) and without (1300 x 1250), points in 1D, 2D (71 x 700) and 3D.  Some
+roundings of 1.1e-16 per point and step on values of at most 1: |dC|, |dpsi| <= 1e-10."""
 import numpy as np
 import pytest
 
@@ -14,8 +14,8 @@ import golden_cases as G
 from test_gpu_psod import packet
 
 pytestmark = pytest.mark.gpu
-SIZES = {"400x300": 1e-4, "257x300": 1e-4, "64x700": 1e-4, "1300x1250": 1e-5, "90001": 2e-8,
-         "50x51x52": 1e-3}
+SIZES = {"400x300": 1e-4, "257x300": 1e-4, "72x700": 1e-4, "71x700": 1e-4,
+         "1300x1250": 1e-5, "90001": 2e-8, "50x51x52": 1e-3}
 
 
 @pytest.mark.parametrize("extra", ["plain", "copy", "pulse"])
