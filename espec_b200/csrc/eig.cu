@@ -35,7 +35,10 @@ constexpr int kEigThreads = 512;
 constexpr int kEigChains = 1024;
 // points of a current vector kept in shared memory (beside 31 KB of static arrays)
 constexpr int kEigMaxSmemN = 24 * 1024;
-constexpr int kEigMinSplitN = 2048;  // points from which two CTAs share a problem
+// points from which two CTAs share a problem: six restarts of two states, 16 problems, ms
+// with one CTA and with two: 1024 points 4.9 and 5.3, 1440 5.7 and 5.9, 2025 7.7 and 7.2,
+// 2048 6.0 and 6.0, 2304 7.4 and 6.6, 4096 9.5 and 7.7, 16384 33 and 21
+constexpr int kEigMinSplitN = 2048;
 constexpr int kEigMaxM = 40;      // NREORT = 40 in lanczsc.f:55
 constexpr int kEigMaxStates = 16;  // locked states held in the reorthogonalisation
 
