@@ -95,6 +95,11 @@ struct Share {
       asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     }
   }
+  // vectors in global memory: with one CTA by way of L1, which holds those of a small
+  // grid; with two past it, since the other CTA writes to them
+  __device__ __forceinline__ double load(const double* p) const {
+    return CS == 1 ? *p : __ldcg(p);
+  }
   // *p = v here and in the other CTA (p in shared memory)
   __device__ __forceinline__ void put(double* p, double v) const {
     *p = v;
@@ -138,7 +143,7 @@ __device__ __forceinline__ double chain_sum(const Share<CS>& sh, double x0, doub
 // that even the first iterations of a restart keep every warp loading, with
 // kDotLoads loads of the vector in flight per lane (with two, one CTA drew
 // about 20 GB/s).  part: [2 (kEigMaxM + kEigMaxStates)][32] in shared memory.
-constexpr int kDotLoads = 32;
+constexpr int kDotLoads = 32, kTailLoads = 8;
 template <int CS>
 __device__ __forceinline__ void warp_dots(const Share<CS>& sh, const double* x, const double* L,
                                           int nl, const double* lock, int nlock, int n,
@@ -146,6 +151,33 @@ __device__ __forceinline__ void warp_dots(const Share<CS>& sh, const double* x, 
   constexpr int NW = kEigThreads / 32;  // even: a vector's two chain sets stay in one CTA
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nv = nl + nlock;
+  if (CS == 1 && n < kEigMinSplitN) {
+    // a small grid: both chains of a vector in one warp, no exchange (three restarts of
+    // two states, with it and the loads by way of L1: 35 points 1.58 -> 1.01 ms, 256 1.32
+    // -> 1.07, 1024 1.70 -> 1.53, 2025 2.53 -> 2.29)
+    for (int q = warp; q < nv; q += NW) {
+      const double* y = q < nl ? L + (long)q * n : lock + (long)(q - nl) * n;
+      double s[2] = {0.0, 0.0};
+      for (int k = lane; k < n; k += 32 * kTailLoads) {
+        double v[kTailLoads], u[kTailLoads];
+#pragma unroll
+        for (int j = 0; j < kTailLoads; ++j) {
+          const bool in = k + 32 * j < n;
+          v[j] = in ? sh.load(y + k + 32 * j) : 0.0;
+          u[j] = in ? x[k + 32 * j] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < kTailLoads; ++j)
+          if (k + 32 * j < n) s[j & 1] += u[j] * v[j];
+      }
+      double d = s[0] + s[1];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+      if (lane == 0) red[q] = d;
+    }
+    __syncthreads();
+    return;
+  }
   for (int task = warp + sh.rank * NW; task < 2 * nv; task += CS * NW) {
     const int q = task >> 1;
     const double* y = q < nl ? L + (long)q * n : lock + (long)(q - nl) * n;
@@ -154,11 +186,22 @@ __device__ __forceinline__ void warp_dots(const Share<CS>& sh, const double* x, 
     for (; k + 64 * (kDotLoads - 1) < n; k += 64 * kDotLoads) {
       double v[kDotLoads];
 #pragma unroll
-      for (int j = 0; j < kDotLoads; ++j) v[j] = __ldcg(y + k + 64 * j);
+      for (int j = 0; j < kDotLoads; ++j) v[j] = sh.load(y + k + 64 * j);
 #pragma unroll
       for (int j = 0; j < kDotLoads; ++j) s += x[k + 64 * j] * v[j];
     }
-    for (; k < n; k += 64) s += x[k] * __ldcg(y + k);
+    for (; k < n; k += 64 * kTailLoads) {
+      double v[kTailLoads], u[kTailLoads];
+#pragma unroll
+      for (int j = 0; j < kTailLoads; ++j) {
+        const bool in = k + 64 * j < n;
+        v[j] = in ? sh.load(y + k + 64 * j) : 0.0;
+        u[j] = in ? x[k + 64 * j] : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < kTailLoads; ++j)
+        if (k + 64 * j < n) s += u[j] * v[j];
+    }
     part[task * 32 + lane] = s;
   }
   __syncthreads();
@@ -191,21 +234,21 @@ __device__ __forceinline__ void combine(const Share<CS>& sh, const double* lock,
     for (int j = 0; j < nlock; ++j) {
       const double c = ca[j];
 #pragma unroll
-      for (int i = 0; i < P; ++i) w[i] -= c * __ldcg(lock + (long)j * n + kk[i]);
+      for (int i = 0; i < P; ++i) w[i] -= c * sh.load(lock + (long)j * n + kk[i]);
     }
     if (plus) {
 #pragma unroll 4
       for (int q = 0; q < nl; ++q) {
         const double c = cb[q];
 #pragma unroll
-        for (int i = 0; i < P; ++i) w[i] += c * __ldcg(L + (long)q * n + kk[i]);
+        for (int i = 0; i < P; ++i) w[i] += c * sh.load(L + (long)q * n + kk[i]);
       }
     } else {
 #pragma unroll 4
       for (int q = 0; q < nl; ++q) {
         const double c = cb[q];
 #pragma unroll
-        for (int i = 0; i < P; ++i) w[i] -= c * __ldcg(L + (long)q * n + kk[i]);
+        for (int i = 0; i < P; ++i) w[i] -= c * sh.load(L + (long)q * n + kk[i]);
       }
     }
 #pragma unroll
