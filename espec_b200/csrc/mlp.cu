@@ -79,11 +79,14 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, T alpha,
 // db[c] = sum_r dy[r, c]: 32 columns x 8 row phases per CTA, each phase sums
 // rows r = phase mod 8 in order, then the 8 partials are added in order
 // (deterministic)
+template <bool CHAIN>
 __global__ void colsum_kernel(const float* __restrict__ dy, int rows, int cols,
                               float* __restrict__ db) {
   __shared__ float part[8][33];
-  chain_start();
-  chain_wait();
+  if (CHAIN) {
+    chain_start();
+    chain_wait();
+  }
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.0f;
   if (c < cols) {
@@ -101,13 +104,16 @@ __global__ void colsum_kernel(const float* __restrict__ dy, int rows, int cols,
 }
 
 // loss = mean over rows of sum (y - t)^2 / cols; dy = 2 (y - t) / (rows cols)
+template <bool CHAIN>
 __global__ void mse_kernel(const float* __restrict__ y, const float* __restrict__ t, int rows,
                            int cols, float* __restrict__ dy, float* row_loss) {
   const int r = blockIdx.x;
   float s = 0.0f;
   const float sc = 2.0f / ((float)rows * (float)cols);
-  chain_start();
-  chain_wait();
+  if (CHAIN) {
+    chain_start();
+    chain_wait();
+  }
 #pragma unroll 8
   for (int c = threadIdx.x; c < cols; c += 256) {
     const float d = y[(long)r * cols + c] - t[(long)r * cols + c];
@@ -236,16 +242,17 @@ extern "C" int espec_gemm_f32(int M, int N, int K, float alpha, const float* A, 
 }
 
 extern "C" int espec_mlp_colsum(const float* dy, int rows, int cols, float* db, void* stream) {
-  const cudaError_t e = launch_chained(colsum_kernel, (unsigned)((cols + 31) / 32), dim3(32, 8), 0,
-                                       (cudaStream_t)stream, dy, rows, cols, db);
+  const cudaError_t e =
+      launch_either(colsum_kernel<true>, colsum_kernel<false>, (unsigned)((cols + 31) / 32),
+                    dim3(32, 8), (cudaStream_t)stream, dy, rows, cols, db);
   if (e != cudaSuccess) return set_cuda_error("mlp kernel launch", e);
   return ESPEC_OK;
 }
 
 extern "C" int espec_mlp_mse(const float* y, const float* t, int rows, int cols, float* dy,
                              float* row_loss, void* stream) {
-  const cudaError_t e =
-      launch_chained(mse_kernel, rows, 256, 0, (cudaStream_t)stream, y, t, rows, cols, dy, row_loss);
+  const cudaError_t e = launch_either(mse_kernel<true>, mse_kernel<false>, rows, 256,
+                                      (cudaStream_t)stream, y, t, rows, cols, dy, row_loss);
   if (e != cudaSuccess) return set_cuda_error("mlp kernel launch", e);
   return ESPEC_OK;
 }

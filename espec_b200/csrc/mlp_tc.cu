@@ -535,9 +535,12 @@ __global__ void gelu_back_kernel(float* dh, const float* z, long count, uint16_t
   dzb[i] = bf16_bits(d);
 }
 
+template <bool CHAIN>
 __global__ void to_bf16_kernel(const float* x, uint16_t* y, long count) {
-  chain_start();
-  chain_wait();
+  if (CHAIN) {
+    chain_start();
+    chain_wait();
+  }
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) y[i] = bf16_bits(x[i]);
 }
@@ -746,8 +749,8 @@ extern "C" int espec_mlp_gelu_back(float* dh, const float* z, long count, void* 
 }
 
 extern "C" int espec_to_bf16(const float* x, void* y, long count, void* stream) {
-  const cudaError_t e =
-      launch_chained(to_bf16_kernel, nblk(count), 256, 0, (cudaStream_t)stream, x, (uint16_t*)y, count);
+  const cudaError_t e = launch_either(to_bf16_kernel<true>, to_bf16_kernel<false>, nblk(count), 256,
+                                      (cudaStream_t)stream, x, (uint16_t*)y, count);
   if (e != cudaSuccess) return set_cuda_error("mlp bf16 kernel launch", e);
   return ESPEC_OK;
 }
