@@ -8,6 +8,8 @@
 // outputs per thread.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "chain.cuh"
 #include "espec_gpu.h"
 #include "espec_internal.h"
@@ -76,11 +78,25 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, T alpha,
   }
 }
 
+// s + x[r cols] + x[(r + 8) cols] + ..., U rows in flight, as long as U are left
+template <int U>
+__device__ __forceinline__ float add_rows(const float* x, int& r, int rows, int cols, float s) {
+  for (; r + 8 * (U - 1) < rows; r += 8 * U) {
+    float v[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) v[j] = x[(long)(r + 8 * j) * cols];
+#pragma unroll
+    for (int j = 0; j < U; ++j) s += v[j];
+  }
+  return s;
+}
+
 // db[c] = sum_r dy[r, c]: 32 columns x 8 row phases per CTA, each phase sums
 // rows r = phase mod 8 in order, then the 8 partials are added in order
 // (deterministic)
-template <bool CHAIN>
-__global__ void colsum_kernel(const float* __restrict__ dy, int rows, int cols,
+// (U rows of a phase in flight)
+template <bool CHAIN, int U>
+__global__ void __launch_bounds__(256, 8) colsum_kernel(const float* __restrict__ dy, int rows, int cols,
                               float* __restrict__ db) {
   __shared__ float part[8][33];
   if (CHAIN) {
@@ -90,8 +106,12 @@ __global__ void colsum_kernel(const float* __restrict__ dy, int rows, int cols,
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.0f;
   if (c < cols) {
-#pragma unroll 16
-    for (int r = threadIdx.y; r < rows; r += 8) s += dy[(long)r * cols + c];
+    const float* x = dy + c;
+    int r = threadIdx.y;
+    s = add_rows<U>(x, r, rows, cols, s);
+    s = add_rows<4>(x, r, rows, cols, s);
+    s = add_rows<2>(x, r, rows, cols, s);
+    s = add_rows<1>(x, r, rows, cols, s);
   }
   part[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
@@ -104,7 +124,8 @@ __global__ void colsum_kernel(const float* __restrict__ dy, int rows, int cols,
 }
 
 // loss = mean over rows of sum (y - t)^2 / cols; dy = 2 (y - t) / (rows cols)
-template <bool CHAIN>
+// (W points of a thread in flight)
+template <bool CHAIN, int W>
 __global__ void mse_kernel(const float* __restrict__ y, const float* __restrict__ t, int rows,
                            int cols, float* __restrict__ dy, float* row_loss) {
   const int r = blockIdx.x;
@@ -114,12 +135,20 @@ __global__ void mse_kernel(const float* __restrict__ y, const float* __restrict_
     chain_start();
     chain_wait();
   }
-#pragma unroll 8
-  for (int c = threadIdx.x; c < cols; c += 256) {
+  auto point = [&](int c) {
     const float d = y[(long)r * cols + c] - t[(long)r * cols + c];
     dy[(long)r * cols + c] = sc * d;
     s += d * d;
+  };
+  int c = threadIdx.x;
+  if (W > 1) {
+    for (; c + (W - 1) * 256 < cols; c += W * 256) {
+#pragma unroll
+      for (int j = 0; j < W; ++j) point(c + 256 * j);
+    }
   }
+#pragma unroll 1
+  for (; c < cols; c += 256) point(c);
   __shared__ float red[256];
   red[threadIdx.x] = s;
   __syncthreads();
@@ -241,18 +270,33 @@ extern "C" int espec_gemm_f32(int M, int N, int K, float alpha, const float* A, 
   return gemm_launch<float>(M, N, K, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc, stream);
 }
 
+// 16 rows in flight where a phase has as many; with fewer the registers only cost warps
+// (us, 16 and 8 in flight: 8192 x 4096 49 and 75, 30000 x 1024 159 and 266; 64 x 400000 31
+// and 21)
 extern "C" int espec_mlp_colsum(const float* dy, int rows, int cols, float* db, void* stream) {
+  const dim3 grid((unsigned)((cols + 31) / 32)), block(32, 8);
+  const cudaStream_t st = (cudaStream_t)stream;
   const cudaError_t e =
-      launch_either(colsum_kernel<true>, colsum_kernel<false>, (unsigned)((cols + 31) / 32),
-                    dim3(32, 8), (cudaStream_t)stream, dy, rows, cols, db);
+      rows >= 128 ? launch_either(colsum_kernel<true, 16>, colsum_kernel<false, 16>, grid, block, st,
+                                  dy, rows, cols, db)
+                  : launch_either(colsum_kernel<true, 8>, colsum_kernel<false, 8>, grid, block, st,
+                                  dy, rows, cols, db);
   if (e != cudaSuccess) return set_cuda_error("mlp kernel launch", e);
   return ESPEC_OK;
 }
 
 extern "C" int espec_mlp_mse(const float* y, const float* t, int rows, int cols, float* dy,
                              float* row_loss, void* stream) {
-  const cudaError_t e = launch_either(mse_kernel<true>, mse_kernel<false>, rows, 256,
-                                      (cudaStream_t)stream, y, t, rows, cols, dy, row_loss);
+  const cudaStream_t st = (cudaStream_t)stream;
+  auto run = [&](auto w) {
+    return launch_either(mse_kernel<true, decltype(w)::value>, mse_kernel<false, decltype(w)::value>,
+                         rows, 256, st, y, t, rows, cols, dy, row_loss);
+  };
+  // as many points in flight as a row gives every thread (us: 64 x 400000 211 with 4, 157
+  // with 8; 30000 x 1024 92 with 8, 62 with 4; 200000 x 64 261 with 8, 248 with one)
+  const cudaError_t e = cols >= 2048   ? run(std::integral_constant<int, 8>{})
+                        : cols >= 1024 ? run(std::integral_constant<int, 4>{})
+                                       : run(std::integral_constant<int, 1>{});
   if (e != cudaSuccess) return set_cuda_error("mlp kernel launch", e);
   return ESPEC_OK;
 }
