@@ -344,8 +344,11 @@ size_t packed_bytes(int ln) {
 // shared memory and there are planes for most SMs, or for half of them and a plane
 // is one line per group of lanes -- the y passes then cost no memory traffic and no
 // grid barrier, but a plane runs on one SM.  Us per step, fused and separate: 128^3
-// mixed 57 and 64, 64 x 32 x 128 15.1 and 17.8, 32 x 64 x 64 14.1 and 14.7; 64^3 18.7
-// and 16.9, 128 x 64 x 64 mixed 23.0 and 19.7, 64 x 64 x 32 18.2 and 14.2.
+// mixed 57 and 64, 64 x 64 x 256 44 and 49, 64 x 32 x 128 15.1 and 17.8, 32 x 64 x 64
+// 14.1 and 14.7; 64^3 18.7 and 16.9, 128 x 64 x 64 mixed 23.0 and 19.7, 64 x 64 x 32 18.2
+// and 14.2.  Not with z lines of 512 points, whose CTAs have 256 threads: 32 x 32 x 512
+// 45.1 and 38.5 (SOD 69.7 and 51.7), 128 x 32 x 512 120 and 114, 64 x 64 x 512 113 and 114
+// (SOD 174 and 169).
 // Tiles of the column passes: 8 adjacent columns (128 bytes in FP64), fewer
 // where that would leave SMs without a tile.  CTAs: the fewest that keep the
 // largest share, at most one per SM.
@@ -364,7 +367,8 @@ NdConfig nd_config(const espec_spond_plan* p) {
   const size_t plane = sizeof(cpx<R>) * (size_t)p->np[0] * p->np[1];
   size_t tw = 0;
   for (int ax = 0; ax < p->ndim; ++ax) tw += packed_bytes<R>(ln[ax]);
-  const bool planes = p->np[2] >= 128 || (p->np[2] >= 64 && p->np[0] * p->np[1] <= 2048);
+  const bool planes = (p->np[2] >= 128 && p->np[2] < 512) ||
+                      (p->np[2] >= 64 && p->np[2] < 128 && p->np[0] * p->np[1] <= 2048);
   c.fused = p->ndim == 3 && planes && tw + plane + 65536 <= kNdMaxSmem;
   for (int ax = 0; ax < 2; ++ax) c.layout.by_pos[ax] = c.fused;
   auto threads_of = [&](int ax) { return ln[ax] == 9 ? 5 : ln[ax] - 3; };  // log2, per line
