@@ -90,8 +90,31 @@ __global__ void csum_kernel(const double2* cpart, int nparts, int nsteps, int fi
     sr += __shfl_xor_sync(kFull, sr, o);
     si += __shfl_xor_sync(kFull, si, o);
   }
-  if (err && *err) sr = si = nan("");
+  if (*err) sr = si = nan("");
   if (lane == 0) c_out[s] = make_double2(sr, si);
+}
+
+// after the energies' transform: (energy, norm) from the CTAs' sums, one warp, and whether
+// a wait of the transform or of the last run gave up (bar: arrivals and flags, the run's
+// first).  The transform's arrivals and flag go back to zero for the next one.
+__global__ void nd_energy_sum_kernel(const double2* part, int nparts, unsigned long long* bar,
+                                     double2* out) {
+  const int lane = threadIdx.x & 31;
+  double e = 0.0, nr = 0.0;
+  for (int i = lane; i < nparts; i += 32) {
+    e += part[i].x;
+    nr += part[i].y;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    e += __shfl_xor_sync(kFull, e, o);
+    nr += __shfl_xor_sync(kFull, nr, o);
+  }
+  if (lane == 0) {
+    out[0] = make_double2(e, nr);
+    out[1] = make_double2(*(const int*)(bar + 3), *(const int*)(bar + 1));
+    bar[2] = bar[3] = 0;
+  }
 }
 
 // Frequency (FFT order) at place s of an axis's transform.  Positions p of the
@@ -512,10 +535,10 @@ template <typename R>
 int nd_launch(espec_spond_plan* p, const NdConfig& c, NdArgs<R>& a, cudaStream_t st) {
   a.err = (int*)(a.bar + 1);
   // the arrival count, and the error flag unless the run continues from a state that
-  // an earlier one may have spoiled
+  // an earlier one may have spoiled; those of the energies' transform are left at zero
+  // by nd_energy_sum_kernel
   const size_t word = sizeof(unsigned long long);
-  const bool fresh = a.op == kOpForward || a.from_start;
-  ND_CK(cudaMemsetAsync(a.bar, 0, fresh ? 2 * word : word, st));
+  if (a.op != kOpForward) ND_CK(cudaMemsetAsync(a.bar, 0, a.from_start ? 2 * word : word, st));
   if (grid_short_start()) ND_CK(cudaMemsetAsync(a.bar, 0xFF, word, st));
   cudaError_t e;
   if constexpr (sizeof(R) == 8)
@@ -811,7 +834,7 @@ extern "C" int espec_spond_energies(espec_spond_plan* p, double* e, double* norm
   if (!p->d_khat) {
     ND_CK(cudaMalloc(&p->d_khat, sizeof(cpx<double>) * n));
     ND_CK(cudaMalloc(&p->d_tcp, 8 * n));
-    ND_CK(cudaMalloc(&p->d_epart, sizeof(double2) * (nb + 1)));
+    ND_CK(cudaMalloc(&p->d_epart, sizeof(double2) * (nb + 2)));
     for (int ax = 0; ax < p->ndim; ++ax) {
       ND_CK(cudaMalloc(&p->d_tw64[ax], sizeof(RotD) * p->np[ax]));
       tw_table_kernel<double><<<(p->np[ax] + 255) / 256, 256, 0, st>>>(p->d_tw64[ax], p->np[ax]);
@@ -836,16 +859,22 @@ extern "C" int espec_spond_energies(espec_spond_plan* p, double* e, double* norm
   if (rl) return rl;
   nd_energy_kernel<<<nb, 256, 0, st>>>(a.psi_start, p->d_vpot, p->d_khat, p->d_tcp, n,
                                        1.0 / (double)n, p->d_epart);
-  csum_kernel<<<1, 32, 0, st>>>(p->d_epart, nb, 0, 0, p->d_epart + nb, a.err);
+  // the sums go straight into page-locked memory where the plan has some
+  p->stage.drop();
+  double2* hd = (double2*)p->stage.small(2 * sizeof(double2));
+  p->stage.drop();
+  nd_energy_sum_kernel<<<1, 32, 0, st>>>(p->d_epart, nb, p->d_bar, hd ? hd : p->d_epart + nb);
   ND_CK(cudaGetLastError());
-  double2 h;
-  unsigned long long flags[3];  // the run's flag, the arrivals, the transform's flag
-  ND_CK(cudaMemcpyAsync(&h, p->d_epart + nb, sizeof h, cudaMemcpyDeviceToHost, st));
-  ND_CK(cudaMemcpyAsync(flags, p->d_bar + 1, sizeof flags, cudaMemcpyDeviceToHost, st));
+  double2 h[2];
+  if (!hd) {
+    ND_CK(cudaMemcpyAsync(h, p->d_epart + nb, sizeof h, cudaMemcpyDeviceToHost, st));
+    hd = h;
+  }
   ND_CK(cudaStreamSynchronize(st));
-  if (flags[2] || (p->has_state && flags[0])) return set_error(ESPEC_ECUDA, kTimedOut);
-  *e = h.x;
-  *norm = h.y;
+  if (hd[1].x != 0.0 || (p->has_state && hd[1].y != 0.0))
+    return set_error(ESPEC_ECUDA, kTimedOut);
+  *e = hd[0].x;
+  *norm = hd[0].y;
   return ESPEC_OK;
 }
 
