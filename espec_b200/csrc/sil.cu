@@ -1346,6 +1346,8 @@ struct espec_grid_plan {
   int precision = ESPEC_FP64;  // ESPEC_MIXED (SIL): FP32 Lanczos vectors and H psi
   int nblocks = 0, nblocks_max = 0;  // CTAs of the cooperative launches (<= co-resident)
   bool bands = false;                // PSOD by column strips (psod2d_band)
+  int smem_ctas = 0;                 // the CTA count for which in_smem has been found
+  bool in_smem = false;              // PSOD: the points' constants fit in shared memory
   bool loaded = false, has_state = false;
   double *d_vpot = nullptr, *d_mask = nullptr, *d_u = nullptr, *d_v = nullptr;
   double *d_u0 = nullptr, *d_v0 = nullptr, *d_L = nullptr, *d_work = nullptr, *d_wbuf = nullptr;
@@ -1660,20 +1662,24 @@ static int grid_launch(espec_grid_plan* p, int nsteps, bool from_start, cudaStre
     const long places = psod_places(a.nstrips, p->n, p->np[1], p->nblocks);
     const size_t dyn = sizeof(double) * (size_t)places * (a.kabs ? 4 : 3);
     a.cta_points = (int)places;  // read where `dyn` fits in shared memory
-    const void* kern = psod_form(p->ndim, true);
-    int dev = 0, nsm = 0, optin = 0, occ = 0;
-    cudaFuncAttributes fa{};
-    GRID_CK(cudaGetDevice(&dev));
-    GRID_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    GRID_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    GRID_CK(cudaFuncGetAttributes(&fa, kern));
-    if (fa.sharedSizeBytes + dyn <= (size_t)optin) {
-      GRID_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   optin - (int)fa.sharedSizeBytes));
-      GRID_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kSilThreads, dyn));
+    if (p->smem_ctas != p->nblocks) {  // once per CTA count: 1 to 2 us of host calls
+      const void* kern = psod_form(p->ndim, true);
+      int dev = 0, nsm = 0, optin = 0, occ = 0;
+      cudaFuncAttributes fa{};
+      GRID_CK(cudaGetDevice(&dev));
+      GRID_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+      GRID_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+      GRID_CK(cudaFuncGetAttributes(&fa, kern));
+      if (fa.sharedSizeBytes + dyn <= (size_t)optin) {
+        GRID_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     optin - (int)fa.sharedSizeBytes));
+        GRID_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kSilThreads, dyn));
+      }
+      p->in_smem = (long)occ * nsm >= p->nblocks;
+      p->smem_ctas = p->nblocks;
     }
-    const bool in_smem = (long)occ * nsm >= p->nblocks;
-    if (!in_smem) kern = psod_form(p->ndim, false);
+    const bool in_smem = p->in_smem;
+    const void* kern = psod_form(p->ndim, in_smem);
     GRID_CK(cudaLaunchCooperativeKernel(kern, dim3(p->nblocks), dim3(kSilThreads), args,
                                         in_smem ? dyn : 0, st));
     // the kernel swaps the roles of the two state buffers once per step
