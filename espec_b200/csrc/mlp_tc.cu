@@ -247,10 +247,13 @@ __device__ __forceinline__ void finish_tile(const TcGemm& g, uint32_t tmem, uint
   // The last commit covers every MMA before it.  Where the MMA thread gave up at an
   // earlier stage nobody makes that commit, and all threads stay here for the whole
   // limit: the wait for the boxes and MMAs still in flight.
+  // (With tiles by TMA, warps 1 to 7 have followed no phase and may take an earlier one
+  // for the last: it is the barrier they wait at, which the MMA thread reaches after its
+  // own wait, and the fence has to follow it.)
   if (some) ok = wait_phase(last, parity) && ok;
   asm volatile("cp.async.wait_all;\n" ::: "memory");
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   ok = __syncthreads_and(ok) != 0;
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   if (ok && !mma_warp) {
     // 32 columns at a time: each warp's 32 x 32 piece through shared memory
     float* turn = reinterpret_cast<float*>(base) + warp * (32 * 33);
