@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "espec_gpu.h"
@@ -255,6 +256,21 @@ cudaError_t launch_pass(int logr, const PrepArgs& a, const double2* x, double2* 
   return cudaGetLastError();
 }
 
+// the transform's input into out: for samples that lie in the spectrum's memory, which
+// every other form writes to while it still reads samples
+__global__ void spec_prep_kernel(PrepArgs a) {
+  const long N = 1L << a.mf, mc = N / 2;
+  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= N * a.npk) return;
+  const long p = gid >> a.mf, i = gid & (N - 1);
+  double2 z = prep_value(a, p, i);
+  if (a.hwhm || a.window) {
+    const double2 f = time_factor(a, i < mc ? i + mc : i - mc);
+    z = make_double2(f.x * z.x - f.y * z.y, f.x * z.y + f.y * z.x);
+  }
+  a.out[gid] = z;
+}
+
 // mf = 0: the prepared sample is the spectrum (FFTNT returns at N = 1)
 __global__ void spec_copy_kernel(PrepArgs a) {
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -323,6 +339,28 @@ extern "C" int espec_spectrum_dev(int npk, int mf, const void* in, long ld, int 
   const long tot = N * npk;
   double2* wk = (double2*)work;
   double2* tw = wk + tot;
+  const double rn = 1.0 / N;  // cfft.f:102-105
+  // samples in spec's memory: prepared into work, then an odd number of groups of
+  // passes from work to spec and back
+  const double2* in_end = a.in + (npk - 1) * ld + (assemble ? N / 2 : N);
+  if (a.in < a.out + tot && a.out < in_end) {
+    PrepArgs b = a;
+    b.out = wk;
+    spec_prep_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(b);
+    SPEC_CK(cudaGetLastError());
+    spec_table_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(a, tw, nullptr, nullptr,
+                                                                   twopi / N);
+    SPEC_CK(cudaGetLastError());
+    const Twiddles tws{tw, nullptr};
+    double2 *from = wk, *to = a.out;
+    for (int s = 0, left = (mf + 3) / 4 | 1; s < mf; --left) {
+      const int lr = (mf - s + left - 1) / left;
+      SPEC_CK(launch_pass(lr, a, from, to, tws, s, s + lr == mf ? rn : 1.0, st));
+      std::swap(from, to);
+      s += lr;
+    }
+    return ESPEC_OK;
+  }
   // groups of up to four passes, the short one first; the groups ping-pong
   // between work and spec and end in spec.  The time factors sit in the
   // buffer that the first group does not write.
@@ -338,7 +376,6 @@ extern "C" int espec_spectrum_dev(int npk, int mf, const void* in, long ld, int 
   spec_table_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(a, tw, pass, factor, twopi / N);
   SPEC_CK(cudaGetLastError());
   const Twiddles tws{tw, pass};
-  const double rn = 1.0 / N;  // cfft.f:102-105
   if (one) {
     cudaError_t e;
     if (mf == kOneMax) {

@@ -632,7 +632,8 @@ long espec_pplnz_field(int shape, const double* par, double ti, double tf, doubl
  * window of SPECTRUMTD (window 1 = .SG with parameter wp, 0 = none), the half
  * swap and the backward DFT / N of FFTNT (spectrumtd.f:58-81, cfft.f).
  * spec: device double2 [npk][2^mf] in FFTNT's natural order.  work: device
- * scratch of espec_spectrum_work_bytes(npk, mf).  quirks: ESPEC_Q_FFTNT_SP.
+ * scratch of espec_spectrum_work_bytes(npk, mf).  in may lie in spec's memory (in
+ * place: the samples then go through work).  quirks: ESPEC_Q_FFTNT_SP.
  * ---------------------------------------------------------------------- */
 int espec_spectrum_dev(int npk, int mf, const void* in, long ld, int assemble,
                        double dtf, double tf, double tal, double de, int window,
