@@ -187,7 +187,8 @@ __device__ __noinline__ void prime_stage(const double2* __restrict__ tw, cpx<dou
 // out = src transformed (forward: e^{+2 pi i jk/N}, inverse: conjugate, no
 // scaling); src and dst are the two N-point buffers, the result lands in one
 // of them (returned).  wr: shared memory for prime_stage, or null.  Ends with a CTA
-// barrier.
+// barrier.  PRIMES: the size may have a prime factor above 5.
+template <bool PRIMES>
 __device__ cpx<double>* any_fft(const AnyPlan& pl, const double2* __restrict__ tw,
                                 cpx<double>* src, cpx<double>* dst, double2* wr, bool inv) {
   const int n = pl.n;
@@ -199,7 +200,9 @@ __device__ cpx<double>* any_fft(const AnyPlan& pl, const double2* __restrict__ t
       case 3: any_stage<3>(tw, src, dst, n, ns, inv); break;
       case 4: any_stage<4>(tw, src, dst, n, ns, inv); break;
       case 5: any_stage<5>(tw, src, dst, n, ns, inv); break;
-      default: prime_stage(tw, src, dst, wr, n, r, ns, inv); break;
+      default:
+        if (PRIMES) prime_stage(tw, src, dst, wr, n, r, ns, inv);
+        break;
     }
     __syncthreads();
     cpx<double>* tmp = src;
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(kAnyThreads) spo_any_kernel(SpoArgs<double> a,
     const TB::phase_t* ph = step == 1 ? a.tab.h : a.tab.g;
     for (int x = t; x < n; x += T) v[x] = TB::apply(ph[base + x], v[x]);
     __syncthreads();
-    cpx<double>* f = any_fft(pl, tw, v, v == b0 ? b1 : b0, wr, false);
+    cpx<double>* f = any_fft<true>(pl, tw, v, v == b0 ? b1 : b0, wr, false);
     for (int x = t; x < n; x += T) {
       if (quirk) {  // spofft.f:148-154 as written: V(I) uses the updated U(I)
         const double c = a.kq_c[base + x], s = a.kq_s[base + x];
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(kAnyThreads) spo_any_kernel(SpoArgs<double> a,
       }
     }
     __syncthreads();
-    v = any_fft(pl, tw, f, f == b0 ? b1 : b0, wr, true);
+    v = any_fft<true>(pl, tw, f, f == b0 ? b1 : b0, wr, true);
     double cr = 0.0, ci = 0.0;
     for (int x = t; x < n; x += T) {
       const cpx<double> w = a.tab.w[base + x];
@@ -292,8 +295,16 @@ __global__ void __launch_bounds__(kAnyThreads) spo_any_kernel(SpoArgs<double> a,
 }
 
 // kabs: 0 none, 1 complex absorbing potential, 2 multiplicative mask
-__global__ void __launch_bounds__(kAnyThreads) sod_any_kernel(SodArgs a, AnyPlan pl,
-                                                              const double2* tw, int kabs) {
+// Four CTAs per SM (64 registers), which batches of more than two packets per SM need: a
+// step's passes wait at barriers.  Sizes without a prime factor above 5 have a form of
+// their own, since the call to prime_stage costs registers across the stages.  us, with
+// three CTAs and one form -> with four -> with both forms: 2048 packets of 250 points, 40
+// steps 1130 -> 944 -> 918, 4096 of 90 1766 -> 1424 -> 1377, 1024 of 1000, 20 steps 847 -> 784
+// -> 786, one of 250, 400 steps 1713 -> 1692 -> 1630, 300 of 250, 100 steps 557 -> 568 -> 552;
+// 1024 of 578 (17 17 2), 20 steps 1177 -> 985.
+template <bool PRIMES>
+__global__ void __launch_bounds__(kAnyThreads, 4) sod_any_kernel(SodArgs a, AnyPlan pl,
+                                                                 const double2* tw, int kabs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n = pl.n, t = threadIdx.x, T = blockDim.x;
   cpx<double>* cur = reinterpret_cast<cpx<double>*>(smem_raw);
@@ -321,13 +332,13 @@ __global__ void __launch_bounds__(kAnyThreads) sod_any_kernel(SodArgs a, AnyPlan
   auto sod_update = [&](const cpx<double>* src, cpx<double>* dst, double f) {
     for (int x = t; x < n; x += T) f0[x] = src[x];
     __syncthreads();
-    cpx<double>* k = any_fft(pl, tw, f0, f1, wr, false);
+    cpx<double>* k = any_fft<PRIMES>(pl, tw, f0, f1, wr, false);
     for (int x = t; x < n; x += T) {
       const double kc = a.tab.kc[base + x];
       k[x] = mk(k[x].x * kc, k[x].y * kc);
     }
     __syncthreads();
-    const cpx<double>* h = any_fft(pl, tw, k, k == f0 ? f1 : f0, wr, true);
+    const cpx<double>* h = any_fft<PRIMES>(pl, tw, k, k == f0 ? f1 : f0, wr, true);
     for (int x = t; x < n; x += T) {
       const double vc = a.tab.vc[base + x];
       const double hx = fma(vc, src[x].x, h[x].x), hy = fma(vc, src[x].y, h[x].y);
@@ -354,37 +365,29 @@ __global__ void __launch_bounds__(kAnyThreads) sod_any_kernel(SodArgs a, AnyPlan
     const double2 c = cta_sum2(cr, ci, red);
     if (t == 0) cout[step] = c;
   };
-  bool cur_newest = true;
-  int step = 2;
-  if (a.psi_start) {
-    step = 1;
-  } else if (a.nsteps >= 1) {
+  // one loop over all updates, so that the two transforms are compiled once: five copies of
+  // them spilled and took 80 registers
+  cpx<double>*src = cur, *dst = prev;  // the newest state and the one before
+  const int updates = a.psi_start || a.nsteps == 0 ? a.nsteps : a.nsteps + 1;
+  for (int u = 0; u < updates; ++u) {
     // start-up (psodfft.f:120-152): E = psi0 - i/2 H psi0 ; psi1 = psi0 - i/2 H E
-    sod_update(cur, prev, 0.5);
-    sod_update(prev, cur, 0.5);
-    for (int x = t; x < n; x += T) {
-      const double2 p0 = a.psi0[base + x];
-      prev[x] = mk(p0.x, p0.y);
-    }
-    c_sample(cur, 1);
-  }
-  for (; step + 1 <= a.nsteps; step += 2) {
-    sod_update(cur, prev, 1.0);
-    c_sample(prev, step);
-    sod_update(prev, cur, 1.0);
-    c_sample(cur, step + 1);
-  }
-  if (step <= a.nsteps) {
-    sod_update(cur, prev, 1.0);
-    c_sample(prev, step);
-    cur_newest = false;
+    const bool half = !a.psi_start && u < 2;
+    sod_update(src, dst, half ? 0.5 : 1.0);
+    if (half && u == 1)  // and psi(t - dt) = psi0
+      for (int x = t; x < n; x += T) {
+        const double2 p0 = a.psi0[base + x];
+        src[x] = mk(p0.x, p0.y);
+      }
+    const int step = a.psi_start ? u + 1 : u;
+    if (step > 0) c_sample(dst, step);
+    cpx<double>* x = src;
+    src = dst;
+    dst = x;
   }
   if (a.psi_out) {
-    const cpx<double>* nw = cur_newest ? cur : prev;
-    const cpx<double>* od = cur_newest ? prev : cur;
     for (int x = t; x < n; x += T) {
-      a.psi_out[base + x] = make_double2(nw[x].x, nw[x].y);
-      if (a.psi_prev_out) a.psi_prev_out[base + x] = make_double2(od[x].x, od[x].y);
+      a.psi_out[base + x] = make_double2(src[x].x, src[x].y);
+      if (a.psi_prev_out) a.psi_prev_out[base + x] = make_double2(dst[x].x, dst[x].y);
     }
   }
 }
@@ -409,12 +412,20 @@ __global__ void __launch_bounds__(kAnyThreads) diag_any_kernel(DiagArgs a, AnyPl
     nrm += p.x * p.x + p.y * p.y;
   }
   __syncthreads();
-  const cpx<double>* f = any_fft(pl, tw, b0, b1, wr, false);
+  const cpx<double>* f = any_fft<true>(pl, tw, b0, b1, wr, false);
   for (int x = t; x < n; x += T) ekin += a.tc[base + x] * (f[x].x * f[x].x + f[x].y * f[x].y);
   ekin /= (double)n;
   const double2 s = cta_sum2(epot, nrm, red);
   const double2 k = cta_sum2(ekin, 0.0, red + kAnyThreads / 32);
   if (t == 0) a.out[pk.c_off] = make_double2(s.x + k.x, s.y);
+}
+
+// largest prime factor above 5 (0: none)
+int large_prime(const AnyPlan& pl) {
+  int r = 0;
+  for (int s = 0; s < pl.ns; ++s)
+    if (pl.r[s] > 5 && pl.r[s] > r) r = pl.r[s];
+  return r;
 }
 
 // kern(a, plan, tw, rest...); the largest prime's table joins the buffers in shared
@@ -424,9 +435,7 @@ cudaError_t any_launch(K kern, DeviceFlags& flags, AnyPlan pl, int method, int n
                        cudaStream_t st, const Args& a, const double2* tw, Rest... rest) {
   size_t smem = any_smem_bytes(pl.n, method);
   if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
-  int r = 0;
-  for (int s = 0; s < pl.ns; ++s)
-    if (pl.r[s] > 5 && pl.r[s] > r) r = pl.r[s];
+  const int r = large_prime(pl);
   pl.wr = r > 0 && smem + sizeof(double2) * r <= kMaxSmem;
   if (pl.wr) smem += sizeof(double2) * r;
   cudaError_t e = set_max_smem_once(flags, kern, kMaxSmem);
@@ -445,8 +454,10 @@ cudaError_t spo_any_launch(const SpoArgs<double>& a, const AnyPlan& pl, const do
 
 cudaError_t sod_any_launch(const SodArgs& a, const AnyPlan& pl, const double2* tw, int kabs,
                            int nblocks, cudaStream_t st) {
-  static DeviceFlags f;
-  return any_launch(sod_any_kernel, f, pl, ESPEC_SOD, nblocks, st, a, tw, kabs);
+  static DeviceFlags f[2];
+  return large_prime(pl)
+             ? any_launch(sod_any_kernel<true>, f[1], pl, ESPEC_SOD, nblocks, st, a, tw, kabs)
+             : any_launch(sod_any_kernel<false>, f[0], pl, ESPEC_SOD, nblocks, st, a, tw, kabs);
 }
 
 cudaError_t diag_any_launch(const DiagArgs& a, const AnyPlan& pl, const double2* tw, int nblocks,
