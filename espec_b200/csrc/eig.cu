@@ -216,13 +216,16 @@ __device__ __forceinline__ void warp_dots(const Share<CS>& sh, const double* x, 
 }
 
 // w[i] = init(k_i) - sum_j lock_j(k_i) a_j - sum_q L_q(k_i) b_q (or plus),
-// for the thread's points, four at a time so that their loads overlap; put(k,
-// chain, w) takes each, in order
-template <int CS, class Init, class Put>
-__device__ __forceinline__ void combine(const Share<CS>& sh, const double* lock, const double* ca, int nlock,
-                                        const double* L, const double* cb, int nl, int n,
-                                        bool plus, Init init, Put put) {
-  constexpr int P = 4;
+// for the thread's points, P at a time and 16 / P vectors so that their loads overlap;
+// put(k, chain, w) takes each, in order.  Four; two on one CTA's grids of up to two points
+// per thread, where loads for points that do not exist cost as much as the others (three
+// states, 40 vectors, two restarts, ms with four and two: 256 points 1.50 and 1.42, 600 2.04 and
+// 1.87, 1024 2.32 and 2.18, but 1296 2.77 and 2.79)
+template <int P, int CS, class Init, class Put>
+__device__ __forceinline__ void combine_points(const Share<CS>& sh, const double* lock,
+                                               const double* ca, int nlock, const double* L,
+                                               const double* cb, int nl, int n, bool plus,
+                                               Init init, Put put) {
   for (int k0 = sh.first; k0 < n; k0 += P * sh.kStep) {
     double w[P];
     int kk[P];
@@ -237,14 +240,14 @@ __device__ __forceinline__ void combine(const Share<CS>& sh, const double* lock,
       for (int i = 0; i < P; ++i) w[i] -= c * sh.load(lock + (long)j * n + kk[i]);
     }
     if (plus) {
-#pragma unroll 4
+#pragma unroll 16 / P
       for (int q = 0; q < nl; ++q) {
         const double c = cb[q];
 #pragma unroll
         for (int i = 0; i < P; ++i) w[i] += c * sh.load(L + (long)q * n + kk[i]);
       }
     } else {
-#pragma unroll 4
+#pragma unroll 16 / P
       for (int q = 0; q < nl; ++q) {
         const double c = cb[q];
 #pragma unroll
@@ -255,6 +258,15 @@ __device__ __forceinline__ void combine(const Share<CS>& sh, const double* lock,
     for (int i = 0; i < P; ++i)
       if (k0 + i * sh.kStep < n) put(k0 + i * sh.kStep, sh.chain(i), w[i]);
   }
+}
+template <int CS, class Init, class Put>
+__device__ __forceinline__ void combine(const Share<CS>& sh, const double* lock, const double* ca,
+                                        int nlock, const double* L, const double* cb, int nl,
+                                        int n, bool plus, Init init, Put put) {
+  if (CS == 1 && n <= 2 * sh.kStep)
+    combine_points<2>(sh, lock, ca, nlock, L, cb, nl, n, plus, init, put);
+  else
+    combine_points<4>(sh, lock, ca, nlock, L, cb, nl, n, plus, init, put);
 }
 
 // number of eigenvalues of the tridiagonal (d, e) below x (Sturm count)
